@@ -114,7 +114,7 @@ def table_shapes(B, L, T, max_left):
     return (B, Mc, T + 2), (B, L - Mc, T + 2, max_left + 2)
 
 
-_main_chain_cache = {}  # (address of the main-chain mask, prelen) -> node list, slots, left rows
+_main_chain_cache = {}  # (address and version of the main-chain mask, prelen) -> mask, node list, slots
 
 
 class _Kernel:
@@ -590,9 +590,19 @@ class _Kernel:
         _cabi.check(rc, "pcfgnat_stage_inputs")
 
     @staticmethod
+    def main_chain_slots(main_chain):
+        """(node ids [M] int32, slot of every node or -1 [prelen] int32) of a uint8 main-chain mask.  Reads the device.
+        Whoever captures kernels that take them into a graph keeps them for as long as the graph lives."""
+        nodes = main_chain.nonzero().flatten().to(torch.int32)
+        slot_of = torch.full((main_chain.shape[0],), -1, dtype=torch.int32, device=main_chain.device)
+        slot_of[nodes.long()] = torch.arange(nodes.numel(), dtype=torch.int32, device=main_chain.device)
+        return nodes, slot_of
+
+    @staticmethod
     def _links_forward(query, key_left, key_right, gate_logits, prev_output_tokens, pad_index, left_tree_mask,
-                       right_tree_mask, main_chain):
-        """Forward of ``extract_links``; returns (links, everything the backward needs)."""
+                       right_tree_mask, main_chain, chain=None):
+        """Forward of ``extract_links``; returns (links, everything the backward needs).  ``chain``: the
+        ``main_chain_slots`` of main_chain where the caller keeps them (a step object, whose graph reads them)."""
         _require_cuda()
         if query.dim() != 4 or key_left.shape != query.shape or key_right.shape != query.shape:
             raise RuntimeError("query, key_left, key_right must be [batch, prelen, heads, head_dim] and agree")
@@ -622,16 +632,15 @@ class _Kernel:
             raise RuntimeError("tree masks must cover prelen nodes")
         nonpad = prev_output_tokens.to(dev).ne(pad_index).to(torch.uint8).contiguous()
         # main-chain nodes: the only ones that have, or are, right children -> compact score matrices
-        key = (mc.data_ptr(), L)
-        cached = _main_chain_cache.get(key)
-        if cached is None:
-            nodes = mc.nonzero().flatten().to(torch.int32)                   # [M] main-chain node ids
-            slot_of = torch.full((L,), -1, dtype=torch.int32, device=dev)
-            slot_of[nodes.long()] = torch.arange(nodes.numel(), dtype=torch.int32, device=dev)
-            cached = (mc, nodes, slot_of)  # keeps mc alive: its address is the key
-            _main_chain_cache.clear()
-            _main_chain_cache[key] = cached
-        _, nodes, slot_of = cached
+        if chain is None:
+            key = (mc.data_ptr(), mc._version, L)
+            cached = _main_chain_cache.get(key)
+            if cached is None:
+                cached = (mc, _Kernel.main_chain_slots(mc))  # keeps mc alive: its address is part of the key
+                _main_chain_cache.clear()
+                _main_chain_cache[key] = cached
+            chain = cached[1]
+        nodes, slot_of = chain
         M = nodes.numel()
         lib = _cabi.lib()
         with torch.cuda.device(dev):
@@ -684,7 +693,7 @@ class _Kernel:
 
     @staticmethod
     def extract_links(query, key_left, key_right, gate_logits, prev_output_tokens, pad_index, left_tree_mask,
-                      right_tree_mask, main_chain):
+                      right_tree_mask, main_chain, chain=None):
         """links [B, L, 2, L] f32 as the model's extract_links() forms them from the projected link features
         (models/...pcfg.py:140-201, max_left == 1): ``query``, ``key_left``, ``key_right`` [B, L, heads, head_dim]
         (outputs of the three link projections, reshaped), ``gate_logits`` [B, L, heads].  Three launches: feature
@@ -694,7 +703,7 @@ class _Kernel:
             return ExtractLinksFunc.apply(query, key_left, key_right, gate_logits, prev_output_tokens, pad_index,
                                           left_tree_mask, right_tree_mask, main_chain)
         return _Kernel._links_forward(query, key_left, key_right, gate_logits, prev_output_tokens, pad_index, left_tree_mask,
-                                      right_tree_mask, main_chain)[0]
+                                      right_tree_mask, main_chain, chain)[0]
 
     @staticmethod
     def loss_stats(sentence_loss, target_length):

@@ -321,6 +321,7 @@ class LossStep(_GraphedStep):
             u8 = lambda t: t.to(dev).ne(0).to(torch.uint8).contiguous()
             self.left_u8, self.right_u8 = u8(left_tree_mask[:L, :L]), u8(right_tree_mask[:L, :L])
             self.main_u8 = u8(main_chain[:L])
+            self.chain = self.kernel.main_chain_slots(self.main_u8)  # the graph reads them: they live as long as it
         # force_emit: the training pass after a glancing pass (criterions/nat_pcfg_loss.py:116-121): two more
         # inputs, matchmask [B,T,L] and keep_word_mask [B,L] (bool, as GlanceStep returns them); a revealed node
         # may only emit its aligned target position and gets no gradient
@@ -384,7 +385,7 @@ class LossStep(_GraphedStep):
         if self.link_features is not None:
             links, saved = self.kernel._links_forward(self.query, self.key_left, self.key_right, self.gate_logits,
                                                       self.prev_output_tokens, self.pad_index, self.left_u8, self.right_u8,
-                                                      self.main_u8)
+                                                      self.main_u8, self.chain)
         loss, mg, lg = self.kernel.pcfg_loss_fwd_bwd(em["match"], links, self.output_length, self.target_length)
         if self.force_emit:
             self.kernel.force_emit_grad(mg, self.keep_word_mask, out=mg)
@@ -499,6 +500,7 @@ class DecodeStep(_GraphedStep):
             u8 = lambda t: t.to(dev).ne(0).to(torch.uint8).contiguous()
             self.left_u8, self.right_u8 = u8(left_tree_mask[:L, :L]), u8(right_tree_mask[:L, :L])
             self.main_u8 = u8(main_chain[:L])
+            self.chain = self.kernel.main_chain_slots(self.main_u8)  # the graph reads them: they live as long as it
 
     def _inputs(self):
         if self.link_features is None:
@@ -520,7 +522,7 @@ class DecodeStep(_GraphedStep):
         links = self.links
         if self.link_features is not None:
             links = k.extract_links(self.query, self.key_left, self.key_right, self.gate_logits, self.prev_output_tokens,
-                                    self.pad_index, self.left_u8, self.right_u8, self.main_u8)
+                                    self.pad_index, self.left_u8, self.right_u8, self.main_u8, self.chain)
         if self.strategy != "viterbi":
             return k.lookahead_decode_device(links, em["max_lprob"], em["argmax"], self.output_length, self.mask,
                                              self.pad_index, self.decode_beta, self.strategy)

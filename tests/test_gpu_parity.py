@@ -1412,6 +1412,40 @@ def test_loss_step_from_link_features_matches_autograd_chain(pkg, ops, syn):
     assert dq.abs().sum() > 0 and dkr.abs().sum() > 0
 
 
+def test_steps_from_link_features_live_side_by_side(pkg, ops, syn):
+    """A captured step keeps the node lists that its graph reads: building a second step, of another shape, and letting
+    the allocator hand out what was freed leaves the first step's results as they were."""
+    import importlib
+
+    runtime = importlib.import_module("pcfg_nat_b200.runtime")
+    support = importlib.import_module("pcfg_nat_b200.support_tree")
+    heads, dim = 2, 8
+
+    def decode_step(src_max, seed):
+        b = syn.make_batch(syn.Workload("side", batch=3, vocab=300, hidden=64, src_min=4, src_max=src_max), seed=seed)
+        g = torch.Generator().manual_seed(seed)
+        feats = [torch.randn(b.B, b.L, heads, dim, generator=g) for _ in range(3)]
+        gates = torch.randn(b.B, b.L, heads, generator=g)
+        prev = torch.where(torch.arange(b.L)[None, :] < b.output_length[:, None], 3, 1)
+        lm, rm, mc = support.get_mask(b.L, 1)
+        step = runtime.DecodeStep(b.weight.to(DEV), b.B, b.L, lm, DEV, link_features=(heads, dim), right_tree_mask=rm,
+                                  main_chain=mc, strategy="greedy")
+        step.load(b.hidden, *feats, gates, prev, b.output_length)
+        return step
+
+    def held(step):  # host copies: nothing of the step is kept by accident
+        return [t.cpu() for t in step.run()]
+
+    first = decode_step(12, 1)
+    want = held(first)
+    nodes, slot_of = first.chain
+    assert nodes.tolist() == list(range(1, first.L, 2)) and int(slot_of.max()) == first.L // 2 - 1
+    second = decode_step(6, 2)
+    held(second)
+    filler = [torch.zeros(n, dtype=torch.int32, device=DEV) for n in (8, 16, 24, 48) for _ in range(64)]
+    assert all(torch.equal(x, y) for x, y in zip(held(first), want)), len(filler)
+
+
 @pytest.mark.parametrize("mode", ["links", "all"])
 def test_overlapped_load_fetching_from_host_buffers(pkg, ops, syn, mode):
     """An overlapped load whose large inputs are fetched by the kernel that reads the pinned host buffers itself
