@@ -22,9 +22,8 @@
 //   links_scores_grad_kernel   one block per (sentence, node): the row's forward quantities once more, then the
 //                              gradient of every logit (k, c, head) as X0, X1 [B][H][M][M] (left option 0 / 1,
 //                              scaled), their row sums (gradient of ab) and the gradient of the gate logits;
-//   links_features_grad_kernel one block per (sentence, head): the five small products that turn X0, X1 into the
-//                              gradients of q, kl, kr at the main-chain nodes and their left options (operands in
-//                              shared memory, 4 x 4 outputs per thread; a plain version for odd shapes).
+//   links_features_grad_kernel the small products that turn X0, X1 into the gradients of q, kl, kr at the main-chain
+//                              nodes and their left options, 64 x 64 tiles per (sentence, head).
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -426,174 +425,193 @@ __global__ void __launch_bounds__(kLinkThreads)
     }
 }
 
-// Gradients of the packed features from X0, X1 and dab, one block per (sentence, head):
+// Gradients of the packed features from X0, X1 and dab:
 //   dqm[a]      = dab[a][0] klm[0] + dab[a][1] klm[1 + a] + sum_s (X0 + X1)[a][s] krm[s]
 //   dklm[1 + a] = dab[a][1] qm[a] + sum_s X1[a][s] krm[s]
 //   dklm[0]     = sum_a ( dab[a][0] qm[a] + sum_s X0[a][s] krm[s] )
 //   dkrm[s]     = sum_a ( (X0 + X1)[a][s] qm[a] + X0[a][s] klm[0] + X1[a][s] klm[1 + a] )
 // and scattered to the nodes: dq[nodes[a]], dkr[nodes[s]], dkl[nodes[a] - 1] and dkl[0] (which also takes row 1 of the
 // first main-chain node, whose left option 1 is node 0 again).  dq, dkl, dkr [B][L][H][D] f32 were zero-filled.
-__global__ void __launch_bounds__(256)
-    links_features_grad_simple_kernel(const float *__restrict__ X0, const float *__restrict__ X1, const float *__restrict__ dab,
-                               const float *__restrict__ qm, const float *__restrict__ klm, const float *__restrict__ krm,
-                               const int *__restrict__ nodes, int M, int L, int H, int D, float *__restrict__ dq,
-                               float *__restrict__ dkl, float *__restrict__ dkr) {
-    const int h = blockIdx.x, b = blockIdx.y;
-    const size_t bh = (size_t)b * H + h;
-    const float *x0 = X0 + bh * M * M, *x1 = X1 + bh * M * M, *da = dab + bh * M * 2;
-    const float *q = qm + bh * M * D, *kl = klm + bh * (M + 1) * D, *kr = krm + bh * M * D;
-    const int HD = H * D;
-    // outputs indexed (row, d): one thread each, sums over the other node index
-    for (int i = threadIdx.x; i < M * D; i += blockDim.x) {
-        const int r = i / D, d = i - r * D;
-        // row r as a parent a
-        float s0 = 0.f, s1 = 0.f;  // sum_s X0[a][s] krm[s][d], sum_s X1[a][s] krm[s][d]
-        for (int s = 0; s < M; s++) {
-            const float k = kr[(size_t)s * D + d];
-            s0 = fmaf(x0[(size_t)r * M + s], k, s0);
-            s1 = fmaf(x1[(size_t)r * M + s], k, s1);
+//
+// Four float32 matrix products, M x M x D each, per (sentence, head).  A block makes 64 rows x 64 columns of d of the
+// parents' two products (role 0) or of the children's two (role 1), 4 x 4 outputs of both per thread, the summed index
+// walked in chunks of 32 through 27 / 33 KB of shared memory: three 16-byte shared-memory loads per 32 FMAs, so the
+// FMA pipe is what bounds it, and no shape is too large for it.  The X matrices are zero wherever a child is not
+// admissible (all children at or below the parent, padding): a chunk whose X are all zero is skipped, unless the
+// features beside it are not finite (0 x inf stays NaN).  90 sentences, M = 161, 8 x 64 features: 366 us; 3 095 us
+// with one thread per output reading its operands from global memory, as it was.
+constexpr int kFgThreads = 256, kFgTile = 64, kFgChunk = 32, kFgPitch = kFgChunk + 4;
+constexpr int kFgSmemFloats = 4 * kFgChunk * kFgTile + 4 * kFgTile;  // role 1, the larger of the two
+
+__device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) < CUDART_INF_F); }
+
+// rows r0 .. r0 + 31 (< rows), columns d0 .. d0 + 63 (< D) of src [rows][D] into dst [32][64], zero outside
+__device__ __forceinline__ bool stage_features(const float *__restrict__ src, int r0, int rows, int d0, int D, bool vec,
+                                               float *dst) {
+    bool odd = false;
+    if (vec) {
+        for (int i = threadIdx.x; i < kFgChunk * kFgTile / 4; i += kFgThreads) {
+            const int r = r0 + i / (kFgTile / 4), d = d0 + i % (kFgTile / 4) * 4;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r < rows && d < D) v = __ldg(reinterpret_cast<const float4 *>(src + (size_t)r * D + d));
+            odd |= not_finite(v.x) || not_finite(v.y) || not_finite(v.z) || not_finite(v.w);
+            reinterpret_cast<float4 *>(dst)[i] = v;
         }
-        const float d0 = da[r * 2 + 0], d1 = da[r * 2 + 1];
-        const float qv = q[(size_t)r * D + d];
-        const float g_q = d0 * kl[d] + d1 * kl[(size_t)(1 + r) * D + d] + (s0 + s1);
-        const float g_kl1 = d1 * qv + s1;      // left option 1 of node r
-        const float g_kl0 = d0 * qv + s0;      // this node's part of the "no left child" row
-        // row r as a child s
-        float t = 0.f;
-        for (int a = 0; a < M; a++) {
-            const float v0 = x0[(size_t)a * M + r], v1 = x1[(size_t)a * M + r];
-            t = fmaf(v0 + v1, q[(size_t)a * D + d], t);
-            t = fmaf(v0, kl[d], t);
-            t = fmaf(v1, kl[(size_t)(1 + a) * D + d], t);
+    } else {
+        for (int i = threadIdx.x; i < kFgChunk * kFgTile; i += kFgThreads) {
+            const int r = r0 + i / kFgTile, d = d0 + i % kFgTile;
+            const float v = r < rows && d < D ? __ldg(src + (size_t)r * D + d) : 0.f;
+            odd |= not_finite(v);
+            dst[i] = v;
         }
-        const int node = nodes[r];
-        const size_t at = ((size_t)b * L + node) * HD + (size_t)h * D + d;
-        dq[at] = g_q;
-        dkr[at] = t;
-        const int left = node - 1 > 0 ? node - 1 : 0;
-        atomicAdd(dkl + ((size_t)b * L + left) * HD + (size_t)h * D + d, g_kl1);
-        atomicAdd(dkl + ((size_t)b * L + 0) * HD + (size_t)h * D + d, g_kl0);
     }
+    return odd;
 }
 
-// The same with every operand staged in shared memory once and 4 x 4 outputs per thread (D a multiple of 4): the five
-// products are small matrix products, M x M x D each, and a thread that computes one output from global memory
-// re-reads every operand M or D times.  The contributions to the "no left child" row of kl are summed in shared
-// memory and leave as one atomic per column (all M parents share that row).  xs = row pitch of X0 / X1 in shared
-// memory, M rounded up to a multiple of 4 with the padding zero.
-constexpr int kFeatThreads = 320;
-__global__ void __launch_bounds__(kFeatThreads)
+__device__ __forceinline__ float part(const float4 &v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
+
+// vec: D a multiple of 4 and the feature matrices on 16-byte boundaries
+__global__ void __launch_bounds__(kFgThreads, 2)
     links_features_grad_kernel(const float *__restrict__ X0, const float *__restrict__ X1, const float *__restrict__ dab,
                                const float *__restrict__ qm, const float *__restrict__ klm, const float *__restrict__ krm,
-                               const int *__restrict__ nodes, int M, int L, int H, int D, int xs, float *__restrict__ dq,
+                               const int *__restrict__ nodes, int M, int L, int H, int D, int vec, float *__restrict__ dq,
                                float *__restrict__ dkl, float *__restrict__ dkr) {
-    extern __shared__ __align__(16) float s_feat[];
-    const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
-    const size_t bh = (size_t)b * H + h;
-    const float *da = dab + bh * M * 2;
-    const int HD = H * D;
-    float *sx0 = s_feat, *sx1 = sx0 + (size_t)M * xs, *sq = sx1 + (size_t)M * xs, *skr = sq + (size_t)M * D;
-    float *skl = skr + (size_t)M * D, *skl0 = skl + (size_t)(M + 1) * D;  // skl0 [D]: sum for row 0 of kl
-    {
-        const float *x0 = X0 + bh * M * M, *x1 = X1 + bh * M * M;
-        for (int i = tid; i < M * xs; i += kFeatThreads) {
-            const int r = i / xs, c = i - r * xs;
-            sx0[i] = c < M ? x0[(size_t)r * M + c] : 0.f;
-            sx1[i] = c < M ? x1[(size_t)r * M + c] : 0.f;
-        }
-        const float *q = qm + bh * M * D, *kr = krm + bh * M * D, *kl = klm + bh * (M + 1) * D;
-        for (int i = tid; i < M * D; i += kFeatThreads) sq[i] = q[i], skr[i] = kr[i];
-        for (int i = tid; i < (M + 1) * D; i += kFeatThreads) skl[i] = kl[i];
-        for (int i = tid; i < D; i += kFeatThreads) skl0[i] = 0.f;
-    }
-    __syncthreads();
-    const int CG = D / 4, micro = ((M + 3) / 4) * CG;
-    for (int mt = tid; mt < micro; mt += kFeatThreads) {
-        const int r0 = (mt / CG) * 4, d0 = (mt % CG) * 4;
-        int rr[4];  // rows of this tile, clamped: a row past the end repeats the last one and is not written
-#pragma unroll
-        for (int i = 0; i < 4; i++) rr[i] = r0 + i < M ? r0 + i : M - 1;
-        // rows as parents a: s0 = sum_s X0[a][s] krm[s], s1 = sum_s X1[a][s] krm[s]
-        float a0[4][4], a1[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) a0[i][c] = a1[i][c] = 0.f;
-        for (int s = 0; s < xs; s += 4) {
-            float4 x0v[4], x1v[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                x0v[i] = *reinterpret_cast<const float4 *>(sx0 + (size_t)rr[i] * xs + s);
-                x1v[i] = *reinterpret_cast<const float4 *>(sx1 + (size_t)rr[i] * xs + s);
+    __shared__ __align__(16) float smem[kFgSmemFloats];
+    const int role = blockIdx.x & 1, r0 = (blockIdx.x >> 1) * kFgTile, d0 = blockIdx.y * kFgTile;
+    const size_t bh = blockIdx.z;
+    const int b = blockIdx.z / H, h = blockIdx.z - b * H;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const float *x0 = X0 + bh * M * M, *x1 = X1 + bh * M * M;
+    const float *q = qm + bh * M * D, *kl = klm + bh * (M + 1) * D, *kr = krm + bh * M * D;
+    const size_t pitch = (size_t)H * D, base = (size_t)b * L * pitch + (size_t)h * D;
+    float acc0[4][4] = {}, acc1[4][4] = {};
+    if (role == 0) {  // rows are parents a; summed over the children s
+        float *sx0 = smem, *sx1 = sx0 + kFgTile * kFgPitch, *sk = sx1 + kFgTile * kFgPitch;
+        for (int s0 = 0; s0 < M; s0 += kFgChunk) {
+            bool work = false;
+#pragma unroll 4
+            for (int i = tid; i < kFgTile * kFgChunk; i += kFgThreads) {
+                const int r = i / kFgChunk, s = i % kFgChunk;
+                float v0 = 0.f, v1 = 0.f;
+                if (r0 + r < M && s0 + s < M) {
+                    v0 = __ldg(x0 + (size_t)(r0 + r) * M + s0 + s);
+                    v1 = __ldg(x1 + (size_t)(r0 + r) * M + s0 + s);
+                }
+                work |= v0 != 0.f || v1 != 0.f;
+                sx0[r * kFgPitch + s] = v0;
+                sx1[r * kFgPitch + s] = v1;
             }
+            work |= stage_features(kr, s0, M, d0, D, vec, sk);
+            if (__syncthreads_or(work)) {
+#pragma unroll 2
+                for (int s = 0; s < kFgChunk; s += 4) {
+                    float4 x0v[4], x1v[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int sr = s + j < M ? s + j : M - 1;  // padding columns of X are zero
-                const float4 kv = *reinterpret_cast<const float4 *>(skr + (size_t)sr * D + d0);
-                const float kc[4] = {kv.x, kv.y, kv.z, kv.w};
+                    for (int i = 0; i < 4; i++) {
+                        x0v[i] = *reinterpret_cast<const float4 *>(sx0 + (4 * ty + i) * kFgPitch + s);
+                        x1v[i] = *reinterpret_cast<const float4 *>(sx1 + (4 * ty + i) * kFgPitch + s);
+                    }
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float v0 = j == 0 ? x0v[i].x : j == 1 ? x0v[i].y : j == 2 ? x0v[i].z : x0v[i].w;
-                    const float v1 = j == 0 ? x1v[i].x : j == 1 ? x1v[i].y : j == 2 ? x1v[i].z : x1v[i].w;
+                    for (int j = 0; j < 4; j++) {
+                        const float4 kv = *reinterpret_cast<const float4 *>(sk + (s + j) * kFgTile + 4 * tx);
 #pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        a0[i][c] = fmaf(v0, kc[c], a0[i][c]);
-                        a1[i][c] = fmaf(v1, kc[c], a1[i][c]);
+                        for (int i = 0; i < 4; i++)
+#pragma unroll
+                            for (int c = 0; c < 4; c++) {
+                                acc0[i][c] = fmaf(part(x0v[i], j), part(kv, c), acc0[i][c]);
+                                acc1[i][c] = fmaf(part(x1v[i], j), part(kv, c), acc1[i][c]);
+                            }
                     }
                 }
             }
+            __syncthreads();
         }
         float kl0_part[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const int r = r0 + i;
+            const int r = r0 + 4 * ty + i;
             if (r >= M) continue;
-            const float w0 = da[r * 2 + 0], w1 = da[r * 2 + 1];
-            const int node = nodes[r];
-            const size_t at = ((size_t)b * L + node) * HD + (size_t)h * D + d0;
-            const int left = node - 1 > 0 ? node - 1 : 0;
-            float *dkl_row = dkl + ((size_t)b * L + left) * HD + (size_t)h * D + d0;
+            const float w0 = dab[(bh * M + r) * 2], w1 = dab[(bh * M + r) * 2 + 1];
+            const int node = nodes[r], left = node - 1 > 0 ? node - 1 : 0;
 #pragma unroll
             for (int c = 0; c < 4; c++) {
-                const float qv = sq[(size_t)r * D + d0 + c];
-                dq[at + c] = w0 * skl[d0 + c] + w1 * skl[(size_t)(1 + r) * D + d0 + c] + (a0[i][c] + a1[i][c]);
-                atomicAdd(dkl_row + c, w1 * qv + a1[i][c]);  // left option 1 of node r
-                kl0_part[c] += w0 * qv + a0[i][c];         // this node's part of the "no left child" row
+                const int d = d0 + 4 * tx + c;
+                if (d >= D) continue;
+                const float qv = q[(size_t)r * D + d];
+                dq[base + node * pitch + d] = w0 * kl[d] + w1 * kl[(size_t)(1 + r) * D + d] + (acc0[i][c] + acc1[i][c]);
+                const float g = w1 * qv + acc1[i][c];  // left option 1 of node r: a row of its own, but for node 0's
+                if (left > 0) dkl[base + left * pitch + d] = g;
+                else kl0_part[c] += g;
+                kl0_part[c] += w0 * qv + acc0[i][c];  // this node's part of the "no left child" row
             }
         }
+        // the block's part of row 0 of kl: all parents share that row
+        float *red = smem;
 #pragma unroll
-        for (int c = 0; c < 4; c++) atomicAdd(skl0 + d0 + c, kl0_part[c]);
-        // rows as children s: sum_a ( (X0 + X1)[a][s] qm[a] + X0[a][s] klm[0] + X1[a][s] klm[1 + a] )
-        float t[4][4], x0sum[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int c = 0; c < 4; c++) red[ty * kFgTile + 4 * tx + c] = kl0_part[c];
+        __syncthreads();
+        if (tid < kFgTile && d0 + tid < D) {
+            float sum = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) t[i][c] = 0.f;
-        for (int a = 0; a < M; a++) {
-            const float4 xa0 = *reinterpret_cast<const float4 *>(sx0 + (size_t)a * xs + r0);
-            const float4 xa1 = *reinterpret_cast<const float4 *>(sx1 + (size_t)a * xs + r0);
-            const float4 qv = *reinterpret_cast<const float4 *>(sq + (size_t)a * D + d0);
-            const float4 k1 = *reinterpret_cast<const float4 *>(skl + (size_t)(1 + a) * D + d0);
-            const float v0[4] = {xa0.x, xa0.y, xa0.z, xa0.w}, v1[4] = {xa1.x, xa1.y, xa1.z, xa1.w};
-            const float qc[4] = {qv.x, qv.y, qv.z, qv.w}, kc[4] = {k1.x, k1.y, k1.z, k1.w};
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                x0sum[i] += v0[i];
-#pragma unroll
-                for (int c = 0; c < 4; c++) t[i][c] = fmaf(v1[i], kc[c], fmaf(v0[i] + v1[i], qc[c], t[i][c]));
-            }
+            for (int i = 0; i < 16; i++) sum += red[i * kFgTile + tid];
+            atomicAdd(dkl + base + d0 + tid, sum);
         }
+    } else {  // rows are children s; summed over the parents a
+        float *sxs = smem, *sx1 = sxs + kFgChunk * kFgTile, *sq = sx1 + kFgChunk * kFgTile, *sk = sq + kFgChunk * kFgTile;
+        float *sums = sk + kFgChunk * kFgTile;  // [4][64]
+        const int s_own = r0 + (tid & 63);      // the column whose X this thread stages
+        float x0sum = 0.f;                      // its sum of X0 over a = tid / 64 + 4 j
+        for (int a0 = 0; a0 < M; a0 += kFgChunk) {
+            bool work = false;
+#pragma unroll
+            for (int j = 0; j < kFgChunk / 4; j++) {
+                const int a = (tid >> 6) + 4 * j;
+                float v0 = 0.f, v1 = 0.f;
+                if (a0 + a < M && s_own < M) {
+                    v0 = __ldg(x0 + (size_t)(a0 + a) * M + s_own);
+                    v1 = __ldg(x1 + (size_t)(a0 + a) * M + s_own);
+                }
+                work |= v0 != 0.f || v1 != 0.f;
+                x0sum += v0;
+                sxs[a * kFgTile + (tid & 63)] = v0 + v1;
+                sx1[a * kFgTile + (tid & 63)] = v1;
+            }
+            work |= stage_features(q, a0, M, d0, D, vec, sq);
+            work |= stage_features(kl + D, a0, M, d0, D, vec, sk);
+            if (__syncthreads_or(work)) {
+#pragma unroll 4
+                for (int a = 0; a < kFgChunk; a++) {
+                    const float4 xs = *reinterpret_cast<const float4 *>(sxs + a * kFgTile + 4 * ty);
+                    const float4 xb = *reinterpret_cast<const float4 *>(sx1 + a * kFgTile + 4 * ty);
+                    const float4 qv = *reinterpret_cast<const float4 *>(sq + a * kFgTile + 4 * tx);
+                    const float4 kv = *reinterpret_cast<const float4 *>(sk + a * kFgTile + 4 * tx);
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int c = 0; c < 4; c++) {
+                            acc0[i][c] = fmaf(part(xs, i), part(qv, c), acc0[i][c]);
+                            acc1[i][c] = fmaf(part(xb, i), part(kv, c), acc1[i][c]);
+                        }
+                }
+            }
+            __syncthreads();
+        }
+        sums[(tid >> 6) * kFgTile + (tid & 63)] = x0sum;
+        __syncthreads();
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const int r = r0 + i;
+            const int r = r0 + 4 * ty + i;
             if (r >= M) continue;
-            const size_t at = ((size_t)b * L + nodes[r]) * HD + (size_t)h * D + d0;
+            const int t = 4 * ty + i;
+            const float w = (sums[t] + sums[kFgTile + t]) + (sums[2 * kFgTile + t] + sums[3 * kFgTile + t]);
+            const size_t at = base + nodes[r] * pitch;
 #pragma unroll
-            for (int c = 0; c < 4; c++) dkr[at + c] = fmaf(x0sum[i], skl[d0 + c], t[i][c]);
+            for (int c = 0; c < 4; c++) {
+                const int d = d0 + 4 * tx + c;
+                if (d < D) dkr[at + d] = fmaf(w, kl[d], acc0[i][c] + acc1[i][c]);
+            }
         }
     }
-    __syncthreads();
-    for (int d = tid; d < D; d += kFeatThreads) atomicAdd(dkl + ((size_t)b * L + 0) * HD + (size_t)h * D + d, skl0[d]);
 }
 
 }  // namespace
@@ -621,16 +639,10 @@ int launch_links_backward(const float *links_grad, const float *ac, const float 
                                                                      X0, X1, dab, dgates);
     if (cudaGetLastError() != cudaSuccess) return PCFGNAT_ERR_CUDA;
     if (M == 0) return PCFGNAT_OK;
-    // operands in shared memory and 4 x 4 outputs per thread where D allows it and they fit (M = 80, D = 64: 113 KB)
-    const int xs = (M + 3) / 4 * 4;
-    const size_t feat_smem = ((size_t)2 * M * xs + (size_t)(3 * M + 1) * D + D) * sizeof(float);
-    if (D % 4 == 0 && feat_smem <= (size_t)kSmemLimit - 1024 &&
-        ensure_dynamic_smem(links_features_grad_kernel, feat_smem) == cudaSuccess)
-        links_features_grad_kernel<<<dim3(H, B), kFeatThreads, feat_smem, st>>>(X0, X1, dab, qm, klm, krm, nodes, M, L, H, D,
-                                                                              xs, dq, dkl, dkr);
-    else
-        links_features_grad_simple_kernel<<<dim3(H, B), 256, 0, st>>>(X0, X1, dab, qm, klm, krm, nodes, M, L, H, D, dq, dkl,
-                                                                      dkr);
+    const bool vec = D % 4 == 0 && ((reinterpret_cast<uintptr_t>(qm) | reinterpret_cast<uintptr_t>(klm) |
+                                     reinterpret_cast<uintptr_t>(krm)) & 15) == 0;
+    const dim3 grid(2 * ((M + kFgTile - 1) / kFgTile), (D + kFgTile - 1) / kFgTile, B * H);
+    links_features_grad_kernel<<<grid, kFgThreads, 0, st>>>(X0, X1, dab, qm, klm, krm, nodes, M, L, H, D, vec, dq, dkl, dkr);
     return cuda_rc(cudaGetLastError());
 }
 

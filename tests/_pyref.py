@@ -132,15 +132,19 @@ def force_emit(match_eos_masked, matchmask, keep_word_mask):
     return out, (~keep).expand_as(match_eos_masked)
 
 
-def extract_links(q, kl, kr, gate_logits, prev_output_tokens, pad, left_mask, right_mask, main_chain):
+def extract_links(q, kl, kr, gate_logits, prev_output_tokens, pad, left_mask, right_mask, main_chain, dtype=None,
+                  floor=float("-inf")):
     """Torch restatement (max_left == 1) of what the model's extract_links computes
     (fs_plugins/models/glat_decomposed_with_link_two_hands_tri_pcfg.py:140-201), from the projected link features
     q, kl, kr [B, L, heads, D] and gate logits [B, L, heads]:
-    links[b, a, k, c] = logsumexp_h( log_softmax_{(k, c)}( (ab + bc) + ac ) + log_softmax_h(gates) )."""
+    links[b, a, k, c] = logsumexp_h( log_softmax_{(k, c)}( (ab + bc) + ac ) + log_softmax_h(gates) ).
+    ``dtype`` to compute in (float32); ``floor`` in the place of -inf: with a finite one autograd goes through rows
+    that have masked cells."""
     import torch
 
+    dtype = dtype or torch.float32
     B, L, H, D = q.shape
-    q, kl, kr = q.float(), kl.float(), kr.float()
+    q, kl, kr = q.to(dtype), kl.to(dtype), kr.to(dtype)
     scale = D ** 0.5
     nonpad = prev_output_tokens.ne(pad)
     left_ok = nonpad[:, None, :] & ~left_mask.bool()[None, :L, :L]                      # [B, a, j]
@@ -150,15 +154,15 @@ def extract_links(q, kl, kr, gate_logits, prev_output_tokens, pad, left_mask, ri
     kl_opt = kl[:, left_idx]                                                             # [B, a, k, H, D]
     ab = torch.einsum("bahd,bakhd->bakh", q, kl_opt) / scale
     ab_ok = torch.gather(left_ok, 2, left_idx[None].expand(B, -1, -1))                   # [B, a, k]
-    ab = ab.masked_fill(~ab_ok[..., None] & use[:, :, None, None], float("-inf"))
+    ab = ab.masked_fill(~ab_ok[..., None] & use[:, :, None, None], floor)
     bc = torch.einsum("bakhd,bchd->bakch", kl_opt, kr) / scale
     ac = torch.einsum("bahd,bchd->bach", q, kr) / scale
-    ac = ac.masked_fill(~right_ok[..., None] & use[:, :, None, None], float("-inf"))
+    ac = ac.masked_fill(~right_ok[..., None] & use[:, :, None, None], floor)
     abc = (ab[:, :, :, None, :] + bc) + ac[:, :, None, :, :]                             # [B, a, k, c, H]
     lp = torch.log_softmax(abc.reshape(B, L, 2 * L, H), 2)
-    lg = torch.log_softmax(gate_logits.float(), -1)
+    lg = torch.log_softmax(gate_logits.to(dtype), -1)
     links = torch.logsumexp(lp + lg[:, :, None, :], -1).view(B, L, 2, L)
-    return links.masked_fill(~use[:, :, None, None], float("-inf"))
+    return links.masked_fill(~use[:, :, None, None], floor)
 
 
 def lookahead_decode(links, ob_lprob, tokens, output_length, left_tree_mask, pad, beta=1.0, lookahead=True):

@@ -1030,6 +1030,37 @@ def test_extract_links_backward_against_reference_autograd(ops, case, dtype):
         assert all(torch.isfinite(x.grad).all() for x in leaves + [gates]) and leaves[0].grad.abs().sum() > 0
 
 
+@pytest.mark.parametrize("L, heads, dim, dtype", [(2, 1, 4, torch.float32), (9, 3, 5, torch.float32), (62, 1, 33, torch.float16),
+                                                  (64, 4, 64, torch.float16), (66, 2, 68, torch.float32),
+                                                  (128, 8, 16, torch.float16), (131, 5, 64, torch.float16),
+                                                  (322, 8, 64, torch.float16)])
+def test_extract_links_and_gradient_at_tile_edges(pkg, ops, L, heads, dim, dtype):
+    """Transitions and feature gradients at node and feature counts around the tiles of the product kernels, against
+    autograd in float64: float32 sums of up to 322 terms, 1e-5 of the largest entry (half precision: its rounding)."""
+    import importlib
+
+    lm, rm, mc = importlib.import_module("pcfg_nat_b200.support_tree").get_mask(L, 1)
+    g = torch.Generator().manual_seed(L)
+    leaves = [torch.randn(3, L, heads, dim, generator=g).to(dtype) for _ in range(3)] + [torch.randn(3, L, heads, generator=g)]
+    length = torch.tensor([L, max(2, L // 2), max(2, L - 3)])
+    prev = torch.where(torch.arange(L)[None, :] < length[:, None], 3, 1)
+    ref = [t.double().requires_grad_() for t in leaves]
+    want = pyref.extract_links(*ref, prev, 1, lm, rm, mc, dtype=torch.float64, floor=-1e30)
+    ours = [t.to(DEV).requires_grad_() for t in leaves]
+    links = ops.get_pcfg_kernel().extract_links(*ours, prev.to(DEV), 1, lm, rm, mc)
+    ok = want > -1e29
+    assert torch.equal(torch.isfinite(links).cpu(), ok)
+    G = torch.randn(want.shape, generator=g) * ok
+    torch.testing.assert_close(links.detach().cpu()[ok].double(), want.detach()[ok], rtol=1e-5, atol=1e-4)
+    if not ok.any():
+        return
+    torch.where(ok, want, 0.0).mul(G).sum().backward()
+    (torch.where(ok.to(DEV), links, 0.0) * G.to(DEV)).sum().backward()
+    for x, y in zip(ours, ref):
+        err = (x.grad.cpu().double() - y.grad).abs().max()
+        assert err <= (2e-5 if x.dtype == torch.float32 else 1e-3) * y.grad.abs().max(), (tuple(x.shape), float(err))
+
+
 def test_decode_step_from_link_features(pkg, ops, syn):
     """DecodeStep fed with the projected link features gives what extract_links + the transition-fed step give."""
     import importlib
