@@ -169,6 +169,14 @@ int pcfgnat_logsoftmax_gather(void *logits, int dtype, const int64_t *select_idx
                               int64_t stride_s, int64_t rows, int64_t rows_per_batch, int V, int slen,
                               int require_gradient, float *selected, int *status, void *stream);
 
+/* Its backward, in place: probs [rows][V] (the softmax probabilities the forward left) becomes the gradient of the
+ * logits, -probs * sum_s grad_selected[s] + scatter(grad_selected); replaces the torch operators of
+ * DagLogsoftmaxGatherFunc.backward (fs_plugins/custom_ops/pcfg_loss.py:168-180).  grad_selected [rows][slen] f32
+ * contiguous; select_idx as above; an index out of range is skipped and flagged. */
+int pcfgnat_logsoftmax_gather_backward(void *probs, int dtype, const float *grad_selected, const int64_t *select_idx,
+                                       int64_t stride_b, int64_t stride_l, int64_t stride_s, int64_t rows,
+                                       int64_t rows_per_batch, int V, int slen, int *status, void *stream);
+
 /* Fused output projection + log-softmax + target gather / row max on the tensor cores; the
  * [rows, V] logits are never written to memory.  New entry point: it stands in for the chain
  * output_projection (fs_plugins/models/glat_decomposed_with_link_two_hands_tri_pcfg.py:237, a

@@ -25,6 +25,7 @@ SIGNATURES = {
     "pcfgnat_viterbi_decode": (c_int, [c_void] * 8 + [c_int, c_i64] + [c_int] * 4 + [c_void] * 5),
     "pcfgnat_lookahead_decode": (c_int, [c_void] * 5 + [c_int, ctypes.c_float, c_int, c_i64] + [c_int] * 4 + [c_void] * 4),
     "pcfgnat_logsoftmax_gather": (c_int, [c_void, c_int, c_void] + [c_i64] * 5 + [c_int] * 3 + [c_void] * 3),
+    "pcfgnat_logsoftmax_gather_backward": (c_int, [c_void, c_int] + [c_void] * 2 + [c_i64] * 5 + [c_int] * 2 + [c_void] * 2),
     "pcfgnat_proj_workspace_bytes": (c_size, [c_int] * 4),
     "pcfgnat_proj_logsoftmax_gather": (c_int, [c_void] * 5 + [c_int] * 5 + [c_void] * 5 + [c_size] + [c_void] * 2),
     "pcfgnat_proj_dlogits": (c_int, [c_void] * 7 + [c_int] * 5 + [c_void] * 2 + [c_size] + [c_void] * 2),

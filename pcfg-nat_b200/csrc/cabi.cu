@@ -335,6 +335,16 @@ int pcfgnat_logsoftmax_gather(void *logits, int dtype, const int64_t *select_idx
                                     slen, require_gradient, selected, status, static_cast<cudaStream_t>(stream));
 }
 
+int pcfgnat_logsoftmax_gather_backward(void *probs, int dtype, const float *grad_selected, const int64_t *select_idx,
+                                       int64_t stride_b, int64_t stride_l, int64_t stride_s, int64_t rows,
+                                       int64_t rows_per_batch, int V, int slen, int *status, void *stream) {
+    PCFGNAT_API_RANGE();
+    if (rows < 0 || rows_per_batch < 1 || V < 1 || slen < 0) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    if (rows && (!probs || (slen && (!select_idx || !grad_selected)))) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    return launch_logsoftmax_gather_grad(probs, dtype, grad_selected, select_idx, stride_b, stride_l, stride_s, rows,
+                                         rows_per_batch, V, slen, status, static_cast<cudaStream_t>(stream));
+}
+
 size_t pcfgnat_proj_workspace_bytes(int B, int L, int T, int V) {
     if (B < 0 || L < 1 || T < 0 || V < 1) return 0;
     return proj_workspace_bytes(B, L, T, V);

@@ -137,6 +137,8 @@ int launch_lookahead_decode(const float *links, const float *ob, const int64_t *
 int launch_logsoftmax_gather(void *logits, int dtype, const int64_t *sel, int64_t sb, int64_t sl, int64_t ss,
                              int64_t rows, int64_t rpb, int V, int slen, int req_grad, float *selected, int *status,
                              cudaStream_t st);
+int launch_logsoftmax_gather_grad(void *probs, int dtype, const float *grad, const int64_t *sel, int64_t sb, int64_t sl,
+                                  int64_t ss, int64_t rows, int64_t rpb, int V, int slen, int *status, cudaStream_t st);
 
 // row-per-thread family on its own; redo != nullptr: only the sentences the linear-space kernels left marked
 int launch_loss_fwd_rows(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B, int L,

@@ -398,6 +398,103 @@ int launch_typed(T *logits, const int64_t *sel, int64_t sb, int64_t sl, int64_t 
     return cuda_rc(cudaGetLastError());
 }
 
+// Gradient of the logits from the softmax probabilities that the forward left in their place, in place again:
+//     row[v] = -row[v] * sum_s g[s] + sum_{s: sel[s] == v} g[s]
+// (what DagLogsoftmaxGatherFunc.backward of the reference does with mul_ and scatter_add_, custom_ops/pcfg_loss.py:168-180),
+// formed in float32 and rounded to the storage type once.  HBM bound: one read and one write of [rows][V], a block
+// per row, 16-byte pieces between the row's first and last 16-byte boundary, four loads in flight per thread; the
+// blocks of an SM cover each other's two barriers.  The selected columns are worked out before the row is overwritten
+// (a column that is selected several times is added up, in order, by the first thread that names it) and stored after
+// it; more columns than threads are added atomically instead.  [14 400, 40 000] half precision: 392 us, 0.91 of the
+// measured copy bandwidth; 1 331 us as torch's broadcast multiplication and scatter.
+constexpr int kGradThreads = 256;
+
+__device__ __forceinline__ void atomic_add_to(float *p, float g) { atomicAdd(p, g); }
+__device__ __forceinline__ void atomic_add_to(__half *p, float g) { atomicAdd(p, __float2half(g)); }
+
+template <typename T>
+__device__ __forceinline__ uint4 scaled(uint4 v, float scale) {
+    T *e = reinterpret_cast<T *>(&v);
+#pragma unroll
+    for (int k = 0; k < (int)(16 / sizeof(T)); k++) e[k] = from_f<T>(to_f<T>(e[k]) * scale);
+    return v;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kGradThreads)
+    logsoftmax_gather_grad_kernel(T *probs, const float *__restrict__ grad, const int64_t *__restrict__ sel, int64_t sb,
+                                  int64_t sl, int64_t ss, int64_t rpb, int V, int slen, int *status) {
+    __shared__ int s_sel[kGradThreads];
+    __shared__ float s_g[kGradThreads];
+    constexpr int kVec = 16 / sizeof(T);
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int64_t r = blockIdx.x;
+    T *row = probs + (size_t)r * V;
+    const float *g = grad + (size_t)r * slen;
+    const int64_t *srow = sel + (r / rpb) * sb + (r % rpb) * sl;
+    float sum = 0.f;
+    for (int s = lane; s < slen; s += 32) sum += __ldg(g + s);  // every warp for itself: no barrier
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float scale = -sum;
+    int col = -1;     // the column this thread answers for, and its new value
+    float val = 0.f;
+    if (slen <= kGradThreads) {
+        if (tid < slen) {
+            const int64_t v = srow[(int64_t)tid * ss];
+            if (v >= 0 && v < V) col = (int)v;
+            else flag(status, PCFGNAT_STATUS_BAD_INDEX);
+            s_sel[tid] = col;
+            s_g[tid] = __ldg(g + tid);
+        }
+        __syncthreads();
+        if (col >= 0) {
+            for (int s = 0; s < slen; s++) {
+                if (s_sel[s] != col) continue;
+                if (s < tid) {  // an earlier thread has this column
+                    col = -1;
+                    break;
+                }
+                val += s_g[s];
+            }
+        }
+        if (col >= 0) val = fmaf(to_f<T>(row[col]), scale, val);
+        __syncthreads();  // the selected probabilities are read
+    }
+    const int head = min(V, (int)((16 - (reinterpret_cast<uintptr_t>(row) & 15)) % 16 / sizeof(T)));
+    const int n_vec = (V - head) / kVec, tail = head + n_vec * kVec;
+    uint4 *body = reinterpret_cast<uint4 *>(row + head);
+    int i = tid;
+    for (; i + 3 * kGradThreads < n_vec; i += 4 * kGradThreads) {
+        uint4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = body[i + j * kGradThreads];
+#pragma unroll
+        for (int j = 0; j < 4; j++) body[i + j * kGradThreads] = scaled<T>(v[j], scale);
+    }
+    for (; i < n_vec; i += kGradThreads) body[i] = scaled<T>(body[i], scale);
+    if (tid < head) row[tid] = from_f<T>(to_f<T>(row[tid]) * scale);
+    if (tail + tid < V) row[tail + tid] = from_f<T>(to_f<T>(row[tail + tid]) * scale);
+    __syncthreads();
+    if (slen <= kGradThreads) {
+        if (col >= 0) row[col] = from_f<T>(val);
+    } else {
+        for (int s = tid; s < slen; s += kGradThreads) {
+            const int64_t v = srow[(int64_t)s * ss];
+            if (v >= 0 && v < V) atomic_add_to(row + v, __ldg(g + s));
+            else flag(status, PCFGNAT_STATUS_BAD_INDEX);
+        }
+    }
+}
+
+template <typename T>
+int launch_grad_typed(T *probs, const float *grad, const int64_t *sel, int64_t sb, int64_t sl, int64_t ss, int64_t rows,
+                      int64_t rpb, int V, int slen, int *status, cudaStream_t st) {
+    if (rows > INT32_MAX) return PCFGNAT_ERR_TOO_LARGE;
+    logsoftmax_gather_grad_kernel<T><<<(unsigned)rows, kGradThreads, 0, st>>>(probs, grad, sel, sb, sl, ss, rpb, V, slen, status);
+    return cuda_rc(cudaGetLastError());
+}
+
 }  // namespace
 
 int launch_logsoftmax_gather(void *logits, int dtype, const int64_t *sel, int64_t sb, int64_t sl, int64_t ss,
@@ -410,6 +507,16 @@ int launch_logsoftmax_gather(void *logits, int dtype, const int64_t *sel, int64_
     if (dtype == PCFGNAT_DTYPE_F16)
         return launch_typed<__half>(static_cast<__half *>(logits), sel, sb, sl, ss, rows, rpb, V, slen, req_grad,
                                     selected, status, st);
+    return PCFGNAT_ERR_UNSUPPORTED;
+}
+
+int launch_logsoftmax_gather_grad(void *probs, int dtype, const float *grad, const int64_t *sel, int64_t sb, int64_t sl,
+                                  int64_t ss, int64_t rows, int64_t rpb, int V, int slen, int *status, cudaStream_t st) {
+    if (rows == 0) return PCFGNAT_OK;
+    if (dtype == PCFGNAT_DTYPE_F32)
+        return launch_grad_typed(static_cast<float *>(probs), grad, sel, sb, sl, ss, rows, rpb, V, slen, status, st);
+    if (dtype == PCFGNAT_DTYPE_F16)
+        return launch_grad_typed(static_cast<__half *>(probs), grad, sel, sb, sl, ss, rows, rpb, V, slen, status, st);
     return PCFGNAT_ERR_UNSUPPORTED;
 }
 

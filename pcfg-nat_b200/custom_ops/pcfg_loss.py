@@ -264,6 +264,28 @@ class _Kernel:
         return selected
 
     @staticmethod
+    def logsoftmax_gather_backward(probs, select_idx, grad_selected):
+        """Turns the softmax probabilities [B, L, V] that ``logsoftmax_gather`` left into the gradient of the logits, in
+        place: -probs * sum(grad) + scatter(grad), formed in float32 (pcfg_loss.py:168-180)."""
+        _require_cuda()
+        B, L, V = probs.shape
+        if not probs.is_contiguous() or probs.dtype not in (torch.float32, torch.float16):
+            raise RuntimeError("probs must be a contiguous float32 or float16 tensor")
+        g = _f32_cuda(grad_selected, "grad_selected", 3)
+        if tuple(select_idx.shape) != tuple(g.shape) or g.shape[:2] != probs.shape[:2] or select_idx.dtype != torch.int64:
+            raise RuntimeError("select_idx (int64) and grad_selected must be [batch, prelen, columns]")
+        dev = probs.device
+        if g.device != dev or select_idx.device != dev:
+            raise RuntimeError("probs, select_idx and grad_selected must be on the same device")
+        with torch.cuda.device(dev):
+            rc = _cabi.lib().pcfgnat_logsoftmax_gather_backward(
+                probs.data_ptr(), 0 if probs.dtype == torch.float32 else 1, g.data_ptr(), select_idx.data_ptr(),
+                *select_idx.stride(), B * L, L, V, g.shape[2], _status_ptr(dev), _stream(dev))
+        _cabi.check(rc, "pcfgnat_logsoftmax_gather_backward")
+        torch.autograd.graph.increment_version(probs)  # written in place: autograd's checks see it
+        return probs
+
+    @staticmethod
     def proj_logsoftmax_gather(hidden, weight, targets=None, output_length=None, target_length=None,
                                want_max=False, want_lse=False):
         """Fused output projection + log-softmax + gather / row max on the tensor cores.
@@ -943,9 +965,11 @@ class DagLogsoftmaxGatherFunc(Function):
         ctx.has_backward = True
         probs, idx = ctx.saved_tensors
         # d logits = -p * sum_s g_s + scatter(g): done in the saved buffer
-        probs.mul_(grad_output.sum(-1, keepdim=True).neg_().to(probs.dtype))
-        probs.scatter_add_(-1, idx, grad_output.to(probs.dtype))
-        return probs, None
+        if torch.is_grad_enabled() and grad_output.requires_grad:  # create_graph: operators autograd can follow
+            probs.mul_(grad_output.sum(-1, keepdim=True).neg_().to(probs.dtype))
+            probs.scatter_add_(-1, idx, grad_output.to(probs.dtype))
+            return probs, None
+        return get_pcfg_kernel().logsoftmax_gather_backward(probs, idx, grad_output), None
 
 
 dag_logsoftmax_gather_inplace = DagLogsoftmaxGatherFunc.apply

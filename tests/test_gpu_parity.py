@@ -364,6 +364,30 @@ def test_logsoftmax_gather_reference_golden_and_autograd(ops):
     np.testing.assert_allclose(xb.grad.cpu().numpy(), xa.grad.cpu().numpy(), atol=1e-5)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("V, slen", [(1, 1), (5, 3), (1003, 9), (8192, 256), (8200, 257), (40001, 40)])
+def test_logsoftmax_gather_backward(ops, dtype, V, slen):
+    """Rows that start off a 16-byte boundary, shorter than one block's pass and longer, repeated columns, more columns
+    than threads (added atomically in the storage type), indices out of range.  One rounding of the storage type."""
+    g = torch.Generator().manual_seed(V)
+    B, L = 2, 5
+    probs = torch.softmax(3 * torch.randn(B, L, V, generator=g), -1).to(dtype)
+    idx = torch.randint(0, V, (B, L, slen), generator=g)
+    idx[:, :, slen // 2:] = idx[:, :, slen // 2:] // 3  # repeated columns
+    grad = torch.randn(B, L, slen, generator=g)
+    want = probs.double() * -grad.double().sum(-1, keepdim=True)
+    want.scatter_add_(-1, idx, grad.double())
+    got = ops.get_pcfg_kernel().logsoftmax_gather_backward(probs.to(DEV), idx.to(DEV), grad.to(DEV))
+    eps = 1e-3 if dtype == torch.float16 else 1e-6
+    torch.testing.assert_close(got.cpu().double(), want, rtol=eps * (4 if slen > 256 else 1), atol=eps * (4 if slen > 256 else 0.01))
+    ops.read_status(DEV)
+    if V > 8:
+        idx[1, 2, 0], idx[0, 0, slen - 1] = V, -1
+        got = ops.get_pcfg_kernel().logsoftmax_gather_backward(probs.to(DEV), idx.to(DEV), grad.to(DEV))
+        assert ops.read_status(DEV) & 4 and torch.isfinite(got).all()
+        torch.testing.assert_close(got[1, 0].cpu().double(), want[1, 0], rtol=4 * eps, atol=4 * eps)
+
+
 def test_fused_loss_many_sentences_mixed_cluster_widths(ops, syn, monkeypatch):
     """More sentences than half the SMs: the fused forward + backward runs its passes as cost-ordered clusters
     of two, which the costliest sentences have to themselves and the others share, one CTA each.  Loss and gradients against the oracle, with an
