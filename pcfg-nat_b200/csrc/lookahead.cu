@@ -15,40 +15,74 @@
 // prelen, 1) with an index of batch extent 1 (:425), which for bsz > 1 hands every sentence the log-probabilities of
 // sentence 0; its published lookahead decoding runs with batch size 1, where that is the sentence's own.  Here every
 // sentence uses its own log-probabilities.
+//
+// A cluster of up to eight CTAs serves a sentence.  Its warps take the nodes in use (1 .. length - 1), read a node's
+// 2 L transitions, eight loads in flight per lane, and leave in the first CTA's shared memory one word per node: the
+// chosen child and left option, whether the walk may descend there (left_tree_mask), whether the token is emitted.
+// One thread of the first CTA then walks on that table alone; what it visits it notes as node numbers in the output,
+// which the block turns into tokens at the end.  The walk is a chain of shared-memory loads (the mask and token loads
+// it used to wait for, one L2 round trip each per node, are made by the warps beforehand), and the scan of the
+// transitions is spread over the GPU also when there are few sentences.  64 sentences, graph 240: 21 us, 220 us with a
+// block per sentence whose walk read the mask and the tokens.
+#include <cooperative_groups.h>
+
 #include <climits>
 
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace pcfgnat {
 
 namespace {
 
-constexpr int kLookThreads = 256;
+constexpr int kLookThreads = 256, kLookWarps = kLookThreads / 32;
+constexpr int kLookNodesPerCta = 16, kLookCluster = 8;
+
+// word of a node: chosen child in the low bits, and
+constexpr int kLookChild = (1 << 28) - 1;
+constexpr int kLookLeft = 1 << 28;   // left option 1 (node a - 1), else 0 (node 0)
+constexpr int kLookStop = 1 << 29;   // left_tree_mask forbids the descent
+constexpr int kLookBad = 1 << 30;    // outside the mask
+constexpr int kLookEmit = 1 << 31;   // the token is not padding
 
 __global__ void __launch_bounds__(kLookThreads)
     lookahead_decode_kernel(const float *__restrict__ links, const float *__restrict__ ob, const int64_t *__restrict__ tokens,
                             const int64_t *__restrict__ ol, const int64_t *__restrict__ mask, int mask_dim, float beta,
                             int lookahead, int64_t pad, int L, int cap, int64_t *out, int64_t *cnt, int *status) {
-    extern __shared__ int s_idx[];  // [L] chosen (k * L + c) of every node, then [L] the walk's stack
-    int *stack = s_idx + L;
-    const int b = blockIdx.x;
+    extern __shared__ int s_node[];  // first CTA: [L] words of the nodes, then [L] the walk's stack
+    __shared__ int s_kept;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), nc = (int)cluster.num_blocks();
+    const int b = blockIdx.x / nc;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float *lkb = links + (size_t)b * L * 2 * L;
     const float *obb = ob + (size_t)b * L;
-    for (int a = warp; a < L; a += kLookThreads / 32) {
+    const int64_t given = ol[b];
+    const bool fits = given >= 0 && given <= L;
+    const int length = fits ? (int)given : 0;
+    int *words = cluster.map_shared_rank(s_node, 0);
+    for (int a = 1 + rank * kLookWarps + warp; a < length; a += nc * kLookWarps) {
         const float *row = lkb + (size_t)a * 2 * L;
+        const float left0 = lookahead ? obb[0] : 0.f, left1 = lookahead ? obb[a - 1] : 0.f;
         float best = neg_inf();
         int key = INT_MAX;
-        for (int i = lane; i < 2 * L; i += 32) {  // a lane sees its candidates in increasing index order
-            const int k = i >= L, c = i - k * L;
-            float v = row[i];
-            if (lookahead) {
-                const int left = k == 0 ? 0 : (a - 1 < 0 ? 0 : a - 1);
-                v = (v + obb[c] * beta) + obb[left] * beta;
+        for (int i0 = lane; i0 < 2 * L; i0 += 8 * 32) {  // a lane sees its candidates in increasing index order
+            float v[8], o[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int i = i0 + 32 * j;
+                v[j] = i < 2 * L ? __ldg(row + i) : CUDART_NAN_F;
+                o[j] = lookahead && i < 2 * L ? __ldg(obb + (i >= L ? i - L : i)) : 0.f;
             }
-            if (v > best || (key == INT_MAX && !isnan(v))) {  // strict: the first maximum stays; -inf counts as a value
-                best = v;
-                key = i;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int i = i0 + 32 * j;
+                const float x = lookahead ? fmaf(i >= L ? left1 : left0, beta, fmaf(o[j], beta, v[j])) : v[j];
+                if (x > best || (key == INT_MAX && !isnan(x))) {  // strict: the first maximum stays; -inf counts as a value
+                    best = x;
+                    key = i;
+                }
             }
         }
 #pragma unroll
@@ -60,44 +94,55 @@ __global__ void __launch_bounds__(kLookThreads)
                 key = ok;
             }
         }
-        if (lane == 0) s_idx[a] = key == INT_MAX ? 0 : key;
+        if (lane == 0) {
+            if (key == INT_MAX) key = 0;
+            const int k = key >= L, left = k ? a - 1 : 0;
+            int word = (key - k * L) | (k ? kLookLeft : 0);
+            if (a >= mask_dim) word |= kLookBad;  // left < a
+            else if (mask[(size_t)a * mask_dim + left]) word |= kLookStop;
+            if (tokens[(size_t)b * L + a] != pad) word |= kLookEmit;
+            words[a] = word;
+        }
+    }
+    cluster.sync();
+    if (rank != 0) return;
+    int64_t *o = out + (size_t)b * cap;
+    if (tid == 0) {
+        int *stack = s_node + L;
+        int sp = 0, count = 0, now = 1;
+        bool bad = !fits;
+        long guard = 0;
+        while (!bad && ((now < length && now != 0) || sp > 0)) {
+            while (now < length && now != 0) {
+                if (sp >= L || ++guard > 4L * L + 16) {
+                    bad = true;
+                    break;
+                }
+                stack[sp++] = now;
+                const int word = s_node[now];
+                if (word & kLookBad) {
+                    bad = true;
+                    break;
+                }
+                if (word & kLookStop) break;
+                now = word & kLookLeft ? now - 1 : 0;
+            }
+            if (bad || sp == 0) break;
+            now = stack[--sp];
+            const int word = s_node[now];
+            if (word & kLookEmit) {
+                if (count < cap) o[count] = now;
+                count++;
+            }
+            now = word & kLookChild;
+        }
+        if (bad) flag(status, PCFGNAT_STATUS_BAD_TRACE);
+        s_kept = count < cap ? count : cap;
+        cnt[b] = s_kept;
     }
     __syncthreads();
-    if (tid != 0) return;
-    const int length = (int)ol[b];
-    int64_t *o = out + (size_t)b * cap;
-    int sp = 0, count = 0, now = 1;
-    bool bad = length < 0 || length > L;
-    long guard = 0;
-    while (!bad && ((now < length && now != 0) || sp > 0)) {
-        while (now < length && now != 0) {
-            if (now < 0 || now >= L || sp >= L || ++guard > 4L * L + 16) {
-                bad = true;
-                break;
-            }
-            stack[sp++] = now;
-            const int k = s_idx[now] / L;
-            const int left = k == 0 ? 0 : now - k;
-            if (left < 0 || now >= mask_dim || left >= mask_dim) {
-                bad = true;
-                break;
-            }
-            if (mask[(size_t)now * mask_dim + left]) break;
-            now = left;
-        }
-        if (bad || sp == 0) break;
-        now = stack[--sp];
-        const int64_t tok = tokens[(size_t)b * L + now];
-        if (tok != pad) {
-            if (count < cap) o[count] = tok;
-            count++;
-        }
-        now = s_idx[now] % L;
-    }
-    if (bad) flag(status, PCFGNAT_STATUS_BAD_TRACE);
-    const int kept = count < cap ? count : cap;
-    for (int i = kept; i < cap; i++) o[i] = pad;
-    cnt[b] = kept;
+    const int kept = s_kept;
+    for (int i = tid; i < cap; i += kLookThreads) o[i] = i < kept ? tokens[(size_t)b * L + o[i]] : pad;
 }
 
 }  // namespace
@@ -106,11 +151,23 @@ int launch_lookahead_decode(const float *links, const float *ob, const int64_t *
                             const int64_t *mask, int mask_dim, float beta, int lookahead, int64_t pad, int B, int L,
                             int cap, int64_t *out, int64_t *cnt, int *status, cudaStream_t st) {
     if (B == 0) return PCFGNAT_OK;
+    if (L > kLookChild) return PCFGNAT_ERR_TOO_LARGE;
     const size_t smem = (size_t)2 * L * sizeof(int);
     if (smem > 48 * 1024 && ensure_dynamic_smem(lookahead_decode_kernel, smem) != cudaSuccess) return PCFGNAT_ERR_TOO_LARGE;
-    lookahead_decode_kernel<<<B, kLookThreads, smem, st>>>(links, ob, tokens, ol, mask, mask_dim, beta, lookahead, pad, L, cap,
-                                                           out, cnt, status);
-    return cuda_rc(cudaGetLastError());
+    const int want = (L + kLookNodesPerCta - 1) / kLookNodesPerCta, nc = want < kLookCluster ? want : kLookCluster;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)B * nc);
+    cfg.blockDim = dim3(kLookThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = nc;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cuda_rc(cudaLaunchKernelEx(&cfg, lookahead_decode_kernel, links, ob, tokens, ol, mask, mask_dim, beta, lookahead,
+                                      pad, L, cap, out, cnt, status));
 }
 
 }  // namespace pcfgnat

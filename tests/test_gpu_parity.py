@@ -1430,6 +1430,36 @@ def test_lookahead_decode_step_against_restatement(pkg, ops, syn, strategy):
         assert (tokens[i, len(r):] == 1).all()
 
 
+@pytest.mark.parametrize("L", [2, 3, 16, 17, 33, 128, 129, 300])
+def test_lookahead_decode_cluster_edges(pkg, ops, L):
+    """Sentence counts and graph lengths around the nodes a CTA and a cluster take, with ties, a length of zero, an
+    emitted pad token and an invalid length (flagged, nothing decoded)."""
+    import importlib
+
+    lm = importlib.import_module("pcfg_nat_b200.support_tree").get_mask(L, 1)[0]
+    g = torch.Generator().manual_seed(L)
+    B = 5
+    links = torch.randint(-6, 0, (B, L, 2, L), generator=g).float() / 2  # ties
+    at = torch.arange(L)
+    links.masked_fill_(~((at[:, None] % 2 == 1) & (at[None, :] % 2 == 1) & (at[None, :] > at[:, None]))[None, :, None, :],
+                       float("-inf"))
+    ob = torch.randint(-4, 0, (B, L), generator=g).float()
+    tok = torch.randint(1, 9, (B, L), generator=g)
+    ol = torch.tensor([L, max(2, L // 2), max(1, L - 1), 0, L])
+    links.masked_fill_((at[None, :] >= ol[:, None])[:, None, None, :], float("-inf"))
+    k = ops.get_pcfg_kernel()
+    ops.read_status(DEV)
+    for strategy in ("lookahead", "greedy"):
+        out, cnt = k.lookahead_decode_device(links.to(DEV), ob.to(DEV), tok.to(DEV), ol.to(DEV), lm.to(DEV), 1, 0.5, strategy)
+        rows = pyref.lookahead_decode(links, ob, tok, ol, lm.bool(), 1, 0.5, strategy == "lookahead")
+        for i, r in enumerate(rows):
+            assert int(cnt[i]) == len(r) and out[i].cpu().tolist() == r + [1] * (L - len(r))
+    assert ops.read_status(DEV) == 0
+    ol[4] = L + 1
+    out, cnt = k.lookahead_decode_device(links.to(DEV), ob.to(DEV), tok.to(DEV), ol.to(DEV), lm.to(DEV), 1, 0.5, "greedy")
+    assert ops.read_status(DEV) != 0 and int(cnt[4]) == 0 and (out[4] == 1).all()
+
+
 def test_loss_step_from_link_features_matches_autograd_chain(pkg, ops, syn):
     """LossStep fed with the projected link features (transitions formed and differentiated inside the step) against
     the operators chained by autograd: extract_links -> cuda_pcfg_loss -> backward."""
