@@ -320,6 +320,11 @@ int pcfgnat_links_gather_features(const void *q, const void *kl, const void *kr,
                                   int B, int L, int heads, int head_dim, float *qm, float *klm, float *krm, void *stream);
 int pcfgnat_links_scores(const float *qm, const float *klm, const float *krm, int M, int B, int heads, int head_dim,
                          float *ac, float *bc, void *stream);
+/* The same for callers that know the masks (as for pcfgnat_links_from_scores): score cells that no admissible
+ * (node, right child) pair reads need not be formed and may be left unwritten. */
+int pcfgnat_links_scores_masked(const float *qm, const float *klm, const float *krm, const uint8_t *nonpad,
+                                const uint8_t *right_tree_mask, const uint8_t *main_chain, const int *nodes, int M, int B,
+                                int L, int heads, int head_dim, float *ac, float *bc, void *stream);
 /* Gradient of those links with respect to the link features and the gate logits (training; the reference gets it
  * from autograd through the ~30 operators of extract_links).  links_grad [B][L][2][L] f32; ac, bc, qm, klm, krm and
  * the masks as in the forward.  Scratch: X0, X1 [B][heads][M][M] and dab [B][heads][M][2] f32 (fully overwritten at

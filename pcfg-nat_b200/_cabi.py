@@ -33,6 +33,7 @@ SIGNATURES = {
     "pcfgnat_proj_backward_gemms": (c_int, [c_void] * 3 + [c_int] * 3 + [c_void] * 4),
     "pcfgnat_links_gather_features": (c_int, [c_void] * 3 + [c_int] + [c_void] + [c_int] * 5 + [c_void] * 4),
     "pcfgnat_links_scores": (c_int, [c_void] * 3 + [c_int] * 4 + [c_void] * 3),
+    "pcfgnat_links_scores_masked": (c_int, [c_void] * 7 + [c_int] * 5 + [c_void] * 3),
     "pcfgnat_links_backward": (c_int, [c_void] * 13 + [c_int] * 6 + [c_void] * 8),
     "pcfgnat_links_from_scores": (c_int, [c_void] * 11 + [c_int] * 6 + [c_void] * 2),
     "pcfgnat_copy_links_main_rows": (c_int, [c_void] * 2 + [c_int] * 3 + [c_void]),

@@ -541,7 +541,19 @@ int pcfgnat_links_scores(const float *qm, const float *klm, const float *krm, in
     PCFGNAT_API_RANGE();
     if (B < 0 || M < 0 || heads < 1 || head_dim < 1) return PCFGNAT_ERR_INVALID_ARGUMENT;
     if (B && M && (!qm || !klm || !krm || !ac || !bc)) return PCFGNAT_ERR_INVALID_ARGUMENT;
-    return launch_links_scores(qm, klm, krm, M, B, heads, head_dim, ac, bc, static_cast<cudaStream_t>(stream));
+    return launch_links_scores(qm, klm, krm, nullptr, nullptr, nullptr, nullptr, 0, M, B, heads, head_dim, ac, bc,
+                               static_cast<cudaStream_t>(stream));
+}
+
+int pcfgnat_links_scores_masked(const float *qm, const float *klm, const float *krm, const uint8_t *nonpad,
+                                const uint8_t *right_tree_mask, const uint8_t *main_chain, const int *nodes, int M, int B,
+                                int L, int heads, int head_dim, float *ac, float *bc, void *stream) {
+    PCFGNAT_API_RANGE();
+    if (B < 0 || L < 1 || M < 0 || M > L || heads < 1 || head_dim < 1) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    if (B && M && (!qm || !klm || !krm || !nonpad || !right_tree_mask || !main_chain || !nodes || !ac || !bc))
+        return PCFGNAT_ERR_INVALID_ARGUMENT;
+    return launch_links_scores(qm, klm, krm, nonpad, right_tree_mask, main_chain, nodes, L, M, B, heads, head_dim, ac, bc,
+                               static_cast<cudaStream_t>(stream));
 }
 
 int pcfgnat_links_backward(const float *links_grad, const float *ac, const float *bc, const float *qm, const float *klm,

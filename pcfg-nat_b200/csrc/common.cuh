@@ -211,8 +211,9 @@ int launch_proj(const void *hidden, const void *weight, const int64_t *targets, 
 
 int launch_links_gather(const void *q, const void *kl, const void *kr, int is_half, const int *nodes, int M, int B, int L,
                         int H, int D, float *qm, float *klm, float *krm, cudaStream_t st);
-int launch_links_scores(const float *qm, const float *klm, const float *krm, int M, int B, int H, int D, float *ac,
-                        float *bc, cudaStream_t st);
+int launch_links_scores(const float *qm, const float *klm, const float *krm, const uint8_t *nonpad, const uint8_t *right_mask,
+                        const uint8_t *main_chain, const int *nodes, int L, int M, int B, int H, int D, float *ac, float *bc,
+                        cudaStream_t st);
 int launch_links_backward(const float *links_grad, const float *ac, const float *bc, const float *qm, const float *klm,
                           const float *krm, const float *gates, const uint8_t *nonpad, const uint8_t *left_mask,
                           const uint8_t *right_mask, const uint8_t *main_chain, const int *slot_of, const int *nodes, int M,

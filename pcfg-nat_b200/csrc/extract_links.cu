@@ -16,7 +16,7 @@
 //   links_gather_kernel        packs the features of the M main-chain nodes (and of their left options) as the
 //                              float32 operands of the GEMMs:  qm, krm [B][H][M][D], klm [B][H][M+1][D];
 //   links_scores_kernel        ac [B][H][M][M] = qm krm^T,  bc [B][H][M+1][M] = klm krm^T, unscaled (small batched
-//                              float32 products, one block per sentence, head and 64 x 64 tile);
+//                              float32 products, one block per sentence, head and 128 x 64 tile);
 //   links_from_scores_kernel   one block per (sentence, node) does the rest.
 // Backward (training): links_grad [B][L][2][L] ->
 //   links_scores_grad_kernel   one block per (sentence, node): the row's forward quantities once more, then the
@@ -25,6 +25,8 @@
 //   links_features_grad_kernel the small products that turn X0, X1 into the gradients of q, kl, kr at the main-chain
 //                              nodes and their left options, 64 x 64 tiles per (sentence, head).
 #include <cuda_fp16.h>
+
+#include <initializer_list>
 
 #include "common.cuh"
 
@@ -52,21 +54,39 @@ __device__ __forceinline__ float feat(const void *p, bool half, size_t i) {
 
 // q, kl, kr [B][L][H][D] (f16 or f32); nodes [M] = ids of the main-chain nodes, ascending.
 //   qm = q[nodes], krm = kr[nodes]; klm row 0 = kl[0] (no left child), row 1 + s = kl[nodes[s] - 1].
-__global__ void links_gather_kernel(const void *__restrict__ q, const void *__restrict__ kl, const void *__restrict__ kr,
-                                    int is_half, const int *__restrict__ nodes, int M, int L, int H, int D, float *qm,
-                                    float *klm, float *krm) {
-    const int b = blockIdx.y, r = blockIdx.x;  // r = 0 .. M: row of klm; rows 1 .. M are also rows r - 1 of qm, krm
-    const int HD = H * D;
-    const int left = r == 0 ? 0 : max(nodes[r - 1] - 1, 0);
-    for (int i = threadIdx.x; i < HD; i += blockDim.x) {
-        const int h = i / D, d = i - h * D;
-        klm[(((size_t)b * H + h) * (M + 1) + r) * D + d] = feat(kl, is_half, ((size_t)b * L + left) * HD + i);
-        if (r > 0) {
-            const size_t src = ((size_t)b * L + nodes[r - 1]) * HD + i;
-            const size_t dst = (((size_t)b * H + h) * M + (r - 1)) * D + d;
-            qm[dst] = feat(q, is_half, src);
-            krm[dst] = feat(kr, is_half, src);
+// VEC: four features at a time (D a multiple of 4, everything on 16-byte boundaries).  Bound by the float32 writes.
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+    links_gather_kernel(const void *__restrict__ q, const void *__restrict__ kl, const void *__restrict__ kr, int is_half,
+                        const int *__restrict__ nodes, int M, int L, int H, int D, float *qm, float *klm, float *krm) {
+    constexpr int V = VEC ? 4 : 1;
+    const int b = blockIdx.y, HD = H * D, per_row = HD / V;
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    const int r = i / per_row, e = (i - r * per_row) * V;  // r = 0 .. M: row of klm; rows 1 .. M are also rows r - 1 of qm, krm
+    if (r > M) return;
+    const int h = e / D, d = e - h * D;
+    const int node = r == 0 ? 0 : nodes[r - 1], left = node > 0 ? node - 1 : 0;
+    auto copy = [&](const void *src, size_t from, float *dst, size_t to) {
+        if constexpr (VEC) {
+            float4 v;
+            if (is_half) {
+                const uint2 u = __ldg(reinterpret_cast<const uint2 *>(static_cast<const __half *>(src) + from));
+                const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&u.x));
+                const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
+                v = make_float4(lo.x, lo.y, hi.x, hi.y);
+            } else {
+                v = __ldg(reinterpret_cast<const float4 *>(static_cast<const float *>(src) + from));
+            }
+            *reinterpret_cast<float4 *>(dst + to) = v;
+        } else {
+            dst[to] = feat(src, is_half, from);
         }
+    };
+    copy(kl, ((size_t)b * L + left) * HD + e, klm, (((size_t)b * H + h) * (M + 1) + r) * D + d);
+    if (r > 0) {
+        const size_t src = ((size_t)b * L + node) * HD + e, dst = (((size_t)b * H + h) * M + (r - 1)) * D + d;
+        copy(q, src, qm, dst);
+        copy(kr, src, krm, dst);
     }
 }
 
@@ -195,59 +215,126 @@ __global__ void __launch_bounds__(kLinkThreads)
     }
 }
 
-// C[b][h] = A[b][h] krm[b][h]^T for the rows of A = qm (M rows -> ac) and A = klm (M + 1 rows -> bc): float32, 64 x 64
-// output tiles, the D axis walked in chunks of 16 through shared memory.
-constexpr int kScoreTile = 64, kScoreK = 16;
-__global__ void __launch_bounds__(256)
+// Which score cells anybody reads: those of (node, right child) pairs that the masks admit.  All null: every cell.
+struct ScoreMasks {
+    const uint8_t *nonpad, *right_mask, *main_chain;
+    const int *nodes;
+    int L;
+};
+
+// Asynchronous copies into shared memory (16 or 4 bytes), zero-filled where there is nothing to copy.
+__device__ __forceinline__ void copy_async16(float *dst, const float *src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dsm_smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_async4(float *dst, const float *src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dsm_smem_u32(dst)), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// C[b][h] = A[b][h] krm[b][h]^T for the rows of A = qm (M rows -> ac) and A = klm (M + 1 rows -> bc): float32, 128 x 64
+// output tiles of the 2 M + 1 stacked rows, the D axis walked in chunks of 32 through shared memory, 8 x 4 outputs per
+// thread: twelve 16-byte shared-memory loads per 128 FMAs, conflict-free at a pitch of 36 floats when a thread's rows
+// and columns lie 16 apart.  A block makes the same tile of `heads` heads, one after the other, the next chunk (or
+// head) in flight while this one is multiplied.  A tile without a cell that anybody reads (children at or below the
+// parents, padding: six tiles in ten of a ragged batch) is left alone; the test looks at a quarter of the tile's pairs
+// at a time, so that a tile in use rarely pays for more than that.  90 sentences, M = 161, 8 x 64 features: 180 us; 296 us with a block per
+// head and nothing in flight, 384 us as 64 x 64 tiles of 4 x 4 outputs, every tile formed.
+constexpr int kScoreRows = 128, kScoreCols = 64, kScoreK = 32, kScorePitch = kScoreK + 4;
+constexpr int kScoreStage = (kScoreRows + kScoreCols) * kScorePitch;  // floats; two of them
+__global__ void __launch_bounds__(256, 2)
     links_scores_kernel(const float *__restrict__ qm, const float *__restrict__ klm, const float *__restrict__ krm, int M,
-                        int D, float *__restrict__ ac, float *__restrict__ bc) {
-    __shared__ float sa[kScoreK][kScoreTile + 1], sb[kScoreK][kScoreTile + 1];
-    const int bh = blockIdx.z;
-    const int tiles_m = (M + kScoreTile - 1) / kScoreTile, tiles_r = (2 * M + 1 + kScoreTile - 1) / kScoreTile;
-    const int tr = blockIdx.y, tc = blockIdx.x;  // row tile over the 2 M + 1 stacked rows (qm then klm), column tile over M
-    if (tr >= tiles_r || tc >= tiles_m) return;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 x 16 threads, 4 x 4 outputs each
-    float acc[4][4] = {};
-    const float *qb = qm + (size_t)bh * M * D, *klb = klm + (size_t)bh * (M + 1) * D, *krb = krm + (size_t)bh * M * D;
-    for (int k0 = 0; k0 < D; k0 += kScoreK) {
-        for (int i = threadIdx.x; i < kScoreTile * kScoreK; i += 256) {
-            const int r = i / kScoreK, k = i - r * kScoreK;
-            const int row = tr * kScoreTile + r, col = tc * kScoreTile + r;
-            float va = 0.f, vb = 0.f;
-            if (k0 + k < D) {
-                if (row < M) va = qb[(size_t)row * D + k0 + k];
-                else if (row < 2 * M + 1) va = klb[(size_t)(row - M) * D + k0 + k];
-                if (col < M) vb = krb[(size_t)col * D + k0 + k];
+                        int H, int D, int heads, int vec, ScoreMasks masks, float *__restrict__ ac, float *__restrict__ bc) {
+    extern __shared__ __align__(16) float s_tiles[];
+    const int groups = (H + heads - 1) / heads, b = blockIdx.z / groups, h0 = (blockIdx.z - b * groups) * heads;
+    const int r0 = blockIdx.y * kScoreRows, c0 = blockIdx.x * kScoreCols, tid = threadIdx.x;
+    if (masks.nonpad != nullptr) {
+        const uint8_t *np = masks.nonpad + (size_t)b * masks.L;
+        bool needed = false;
+        for (int part = 0; part < 4 && !needed; part++) {  // rows part, part + 4, ... of the tile
+            bool mine = false;
+#pragma unroll
+            for (int i = tid; i < kScoreRows / 4 * kScoreCols; i += 256) {
+                const int row = r0 + part + i / kScoreCols * 4, s = c0 + i % kScoreCols;
+                if (row > 2 * M || s >= M) continue;
+                const int c = masks.nodes[s];
+                if (!np[c] || !masks.main_chain[c]) continue;
+                // row M is the left option "none", which every node shares
+                mine |= row == M || !masks.right_mask[(size_t)masks.nodes[row < M ? row : row - M - 1] * masks.L + c];
             }
-            sa[k][r] = va;
-            sb[k][r] = vb;
+            needed = __syncthreads_or(mine);
         }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kScoreK; k++) {
-            float a4[4], b4[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                a4[i] = sa[k][ty * 4 + i];
-                b4[i] = sb[k][tx * 4 + i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a4[i], b4[j], acc[i][j]);
-        }
-        __syncthreads();
+        if (!needed) return;
     }
+    const int tx = tid & 15, ty = tid >> 4;
+    const int chunks = (D + kScoreK - 1) / kScoreK, steps = chunks * min(heads, H - h0);
+    auto stage = [&](int step) {
+        const size_t bh = (size_t)b * H + h0 + step / chunks;
+        const int k0 = step % chunks * kScoreK;
+        float *tile = s_tiles + (step & 1) * kScoreStage;  // rows of A, then rows of krm
+        auto source = [&](int r, bool &in) {
+            in = r < kScoreRows ? r0 + r <= 2 * M : c0 + r - kScoreRows < M;
+            if (!in) return krm;
+            const int row = r0 + r;
+            return r >= kScoreRows ? krm + (bh * M + c0 + r - kScoreRows) * D
+                                   : row < M ? qm + (bh * M + row) * D : klm + (bh * (M + 1) + row - M) * D;
+        };
+        if (vec) {
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int row = tr * kScoreTile + ty * 4 + i;
-        if (row >= 2 * M + 1) continue;
+            for (int i = tid; i < (kScoreRows + kScoreCols) * (kScoreK / 4); i += 256) {
+                const int r = i / (kScoreK / 4), k = i % (kScoreK / 4) * 4;
+                bool in;
+                const float *src = source(r, in);
+                in &= k0 + k < D;
+                copy_async16(tile + r * kScorePitch + k, in ? src + k0 + k : krm, in);
+            }
+        } else {
+            for (int i = tid; i < (kScoreRows + kScoreCols) * kScoreK; i += 256) {
+                const int r = i / kScoreK, k = i % kScoreK;
+                bool in;
+                const float *src = source(r, in);
+                in &= k0 + k < D;
+                copy_async4(tile + r * kScorePitch + k, in ? src + k0 + k : krm, in);
+            }
+        }
+        copy_commit();
+    };
+    float acc[8][4] = {};
+    stage(0);
+    for (int step = 0; step < steps; step++) {
+        copy_wait();
+        __syncthreads();  // this chunk is there, and nobody reads the other buffer any more
+        if (step + 1 < steps) stage(step + 1);
+        const float *sa = s_tiles + (step & 1) * kScoreStage, *sb = sa + kScoreRows * kScorePitch;
+#pragma unroll 2
+        for (int k = 0; k < kScoreK; k += 4) {
+            float4 b4[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int col = tc * kScoreTile + tx * 4 + j;
-            if (col >= M) continue;
-            if (row < M) ac[((size_t)bh * M + row) * M + col] = acc[i][j];
-            else bc[((size_t)bh * (M + 1) + (row - M)) * M + col] = acc[i][j];
+            for (int j = 0; j < 4; j++) b4[j] = *reinterpret_cast<const float4 *>(sb + (tx + 16 * j) * kScorePitch + k);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float4 a4 = *reinterpret_cast<const float4 *>(sa + (ty + 16 * i) * kScorePitch + k);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    acc[i][j] = fmaf(a4.x, b4[j].x, acc[i][j]);
+                    acc[i][j] = fmaf(a4.y, b4[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(a4.z, b4[j].z, acc[i][j]);
+                    acc[i][j] = fmaf(a4.w, b4[j].w, acc[i][j]);
+                }
+            }
+        }
+        if ((step + 1) % chunks == 0) {
+            const size_t bh = (size_t)b * H + h0 + step / chunks;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int row = r0 + ty + 16 * i;
+                float *out = row < M ? ac + (bh * M + row) * M : bc + (bh * (M + 1) + (row - M)) * M;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    if (row <= 2 * M && c0 + tx + 16 * j < M) out[c0 + tx + 16 * j] = acc[i][j];
+                    acc[i][j] = 0.f;
+                }
+            }
         }
     }
 }
@@ -435,36 +522,42 @@ __global__ void __launch_bounds__(kLinkThreads)
 //
 // Four float32 matrix products, M x M x D each, per (sentence, head).  A block makes 64 rows x 64 columns of d of the
 // parents' two products (role 0) or of the children's two (role 1), 4 x 4 outputs of both per thread, the summed index
-// walked in chunks of 32 through 27 / 33 KB of shared memory: three 16-byte shared-memory loads per 32 FMAs, so the
-// FMA pipe is what bounds it, and no shape is too large for it.  The X matrices are zero wherever a child is not
+// walked in chunks of 32 through shared memory (the next chunk in flight while this one is multiplied): three 16-byte
+// shared-memory loads per 32 FMAs, and no shape is too large for it.  The X matrices are zero wherever a child is not
 // admissible (all children at or below the parent, padding): a chunk whose X are all zero is skipped, unless the
-// features beside it are not finite (0 x inf stays NaN).  90 sentences, M = 161, 8 x 64 features: 366 us; 3 095 us
+// features beside it are not finite (0 x inf stays NaN).  90 sentences, M = 161, 8 x 64 features: 284 us (366 us
+// without the next chunk in flight); 3 095 us
 // with one thread per output reading its operands from global memory, as it was.
 constexpr int kFgThreads = 256, kFgTile = 64, kFgChunk = 32, kFgPitch = kFgChunk + 4;
-constexpr int kFgSmemFloats = 4 * kFgChunk * kFgTile + 4 * kFgTile;  // role 1, the larger of the two
+constexpr int kFgStage = 4 * kFgChunk * kFgTile;  // floats of one chunk: role 1, the larger of the two; two of them
+constexpr size_t kFgSmem = (2 * kFgStage + 4 * kFgTile) * sizeof(float);
 
 __device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) < CUDART_INF_F); }
 
 // rows r0 .. r0 + 31 (< rows), columns d0 .. d0 + 63 (< D) of src [rows][D] into dst [32][64], zero outside
-__device__ __forceinline__ bool stage_features(const float *__restrict__ src, int r0, int rows, int d0, int D, bool vec,
+__device__ __forceinline__ void stage_features(const float *__restrict__ src, int r0, int rows, int d0, int D, bool vec,
                                                float *dst) {
-    bool odd = false;
     if (vec) {
+#pragma unroll
         for (int i = threadIdx.x; i < kFgChunk * kFgTile / 4; i += kFgThreads) {
             const int r = r0 + i / (kFgTile / 4), d = d0 + i % (kFgTile / 4) * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r < rows && d < D) v = __ldg(reinterpret_cast<const float4 *>(src + (size_t)r * D + d));
-            odd |= not_finite(v.x) || not_finite(v.y) || not_finite(v.z) || not_finite(v.w);
-            reinterpret_cast<float4 *>(dst)[i] = v;
+            const bool in = r < rows && d < D;
+            copy_async16(dst + 4 * i, in ? src + (size_t)r * D + d : src, in);
         }
     } else {
         for (int i = threadIdx.x; i < kFgChunk * kFgTile; i += kFgThreads) {
             const int r = r0 + i / kFgTile, d = d0 + i % kFgTile;
-            const float v = r < rows && d < D ? __ldg(src + (size_t)r * D + d) : 0.f;
-            odd |= not_finite(v);
-            dst[i] = v;
+            const bool in = r < rows && d < D;
+            copy_async4(dst + i, in ? src + (size_t)r * D + d : src, in);
         }
     }
+}
+// whether what this thread staged there has an infinity or a NaN
+__device__ __forceinline__ bool staged_not_finite(const float *dst, bool vec) {
+    bool odd = false;
+#pragma unroll
+    for (int j = 0; j < kFgChunk * kFgTile / kFgThreads; j++)
+        odd |= not_finite(vec ? dst[4 * (threadIdx.x + j / 4 * kFgThreads) + j % 4] : dst[threadIdx.x + j * kFgThreads]);
     return odd;
 }
 
@@ -476,7 +569,7 @@ __global__ void __launch_bounds__(kFgThreads, 2)
                                const float *__restrict__ qm, const float *__restrict__ klm, const float *__restrict__ krm,
                                const int *__restrict__ nodes, int M, int L, int H, int D, int vec, float *__restrict__ dq,
                                float *__restrict__ dkl, float *__restrict__ dkr) {
-    __shared__ __align__(16) float smem[kFgSmemFloats];
+    extern __shared__ __align__(16) float s_tiles[];
     const int role = blockIdx.x & 1, r0 = (blockIdx.x >> 1) * kFgTile, d0 = blockIdx.y * kFgTile;
     const size_t bh = blockIdx.z;
     const int b = blockIdx.z / H, h = blockIdx.z - b * H;
@@ -485,47 +578,58 @@ __global__ void __launch_bounds__(kFgThreads, 2)
     const float *q = qm + bh * M * D, *kl = klm + bh * (M + 1) * D, *kr = krm + bh * M * D;
     const size_t pitch = (size_t)H * D, base = (size_t)b * L * pitch + (size_t)h * D;
     float acc0[4][4] = {}, acc1[4][4] = {};
+    const int chunks = (M + kFgChunk - 1) / kFgChunk;
     if (role == 0) {  // rows are parents a; summed over the children s
-        float *sx0 = smem, *sx1 = sx0 + kFgTile * kFgPitch, *sk = sx1 + kFgTile * kFgPitch;
-        for (int s0 = 0; s0 < M; s0 += kFgChunk) {
-            bool work = false;
-#pragma unroll 4
+        constexpr int kX1 = kFgTile * kFgPitch, kK = 2 * kX1;  // X0, X1 [64][36] and krm [32][64] in a stage
+        auto stage = [&](int step) {
+            const int s0 = step * kFgChunk;
+            float *tile = s_tiles + (step & 1) * kFgStage;
+#pragma unroll
             for (int i = tid; i < kFgTile * kFgChunk; i += kFgThreads) {
                 const int r = i / kFgChunk, s = i % kFgChunk;
-                float v0 = 0.f, v1 = 0.f;
-                if (r0 + r < M && s0 + s < M) {
-                    v0 = __ldg(x0 + (size_t)(r0 + r) * M + s0 + s);
-                    v1 = __ldg(x1 + (size_t)(r0 + r) * M + s0 + s);
-                }
-                work |= v0 != 0.f || v1 != 0.f;
-                sx0[r * kFgPitch + s] = v0;
-                sx1[r * kFgPitch + s] = v1;
+                const bool in = r0 + r < M && s0 + s < M;
+                const size_t at = in ? (size_t)(r0 + r) * M + s0 + s : 0;
+                copy_async4(tile + r * kFgPitch + s, x0 + at, in);
+                copy_async4(tile + kX1 + r * kFgPitch + s, x1 + at, in);
             }
-            work |= stage_features(kr, s0, M, d0, D, vec, sk);
-            if (__syncthreads_or(work)) {
+            stage_features(kr, s0, M, d0, D, vec, tile + kK);
+            copy_commit();
+        };
+        stage(0);
+        for (int step = 0; step < chunks; step++) {
+            const float *sx0 = s_tiles + (step & 1) * kFgStage, *sx1 = sx0 + kX1, *sk = sx0 + kK;
+            copy_wait();
+            bool work = staged_not_finite(sk, vec);  // a thread looks at what it copied itself: no barrier in between
+#pragma unroll
+            for (int i = tid; i < kFgTile * kFgChunk; i += kFgThreads) {
+                const int at = i / kFgChunk * kFgPitch + i % kFgChunk;
+                work |= sx0[at] != 0.f || sx1[at] != 0.f;
+            }
+            work = __syncthreads_or(work);  // the chunk is there, and nobody reads the other buffer any more
+            if (step + 1 < chunks) stage(step + 1);
+            if (!work) continue;
 #pragma unroll 2
-                for (int s = 0; s < kFgChunk; s += 4) {
-                    float4 x0v[4], x1v[4];
+            for (int s = 0; s < kFgChunk; s += 4) {
+                float4 x0v[4], x1v[4];
 #pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        x0v[i] = *reinterpret_cast<const float4 *>(sx0 + (4 * ty + i) * kFgPitch + s);
-                        x1v[i] = *reinterpret_cast<const float4 *>(sx1 + (4 * ty + i) * kFgPitch + s);
-                    }
+                for (int i = 0; i < 4; i++) {
+                    x0v[i] = *reinterpret_cast<const float4 *>(sx0 + (4 * ty + i) * kFgPitch + s);
+                    x1v[i] = *reinterpret_cast<const float4 *>(sx1 + (4 * ty + i) * kFgPitch + s);
+                }
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const float4 kv = *reinterpret_cast<const float4 *>(sk + (s + j) * kFgTile + 4 * tx);
+                for (int j = 0; j < 4; j++) {
+                    const float4 kv = *reinterpret_cast<const float4 *>(sk + (s + j) * kFgTile + 4 * tx);
 #pragma unroll
-                        for (int i = 0; i < 4; i++)
+                    for (int i = 0; i < 4; i++)
 #pragma unroll
-                            for (int c = 0; c < 4; c++) {
-                                acc0[i][c] = fmaf(part(x0v[i], j), part(kv, c), acc0[i][c]);
-                                acc1[i][c] = fmaf(part(x1v[i], j), part(kv, c), acc1[i][c]);
-                            }
-                    }
+                        for (int c = 0; c < 4; c++) {
+                            acc0[i][c] = fmaf(part(x0v[i], j), part(kv, c), acc0[i][c]);
+                            acc1[i][c] = fmaf(part(x1v[i], j), part(kv, c), acc1[i][c]);
+                        }
                 }
             }
-            __syncthreads();
         }
+        __syncthreads();
         float kl0_part[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int i = 0; i < 4; i++) {
@@ -546,7 +650,7 @@ __global__ void __launch_bounds__(kFgThreads, 2)
             }
         }
         // the block's part of row 0 of kl: all parents share that row
-        float *red = smem;
+        float *red = s_tiles;
 #pragma unroll
         for (int c = 0; c < 4; c++) red[ty * kFgTile + 4 * tx + c] = kl0_part[c];
         __syncthreads();
@@ -557,44 +661,56 @@ __global__ void __launch_bounds__(kFgThreads, 2)
             atomicAdd(dkl + base + d0 + tid, sum);
         }
     } else {  // rows are children s; summed over the parents a
-        float *sxs = smem, *sx1 = sxs + kFgChunk * kFgTile, *sq = sx1 + kFgChunk * kFgTile, *sk = sq + kFgChunk * kFgTile;
-        float *sums = sk + kFgChunk * kFgTile;  // [4][64]
-        const int s_own = r0 + (tid & 63);      // the column whose X this thread stages
-        float x0sum = 0.f;                      // its sum of X0 over a = tid / 64 + 4 j
-        for (int a0 = 0; a0 < M; a0 += kFgChunk) {
-            bool work = false;
+        constexpr int kPart = kFgChunk * kFgTile;  // X0 (then X0 + X1), X1, qm, klm, each [32][64], in a stage
+        float *sums = s_tiles + 2 * kFgStage;      // [4][64]
+        const int s_own = r0 + (tid & 63);         // the column whose X this thread stages
+        float x0sum = 0.f;                         // its sum of X0 over a = tid / 64 + 4 j
+        auto stage = [&](int step) {
+            const int a0 = step * kFgChunk;
+            float *tile = s_tiles + (step & 1) * kFgStage;
 #pragma unroll
             for (int j = 0; j < kFgChunk / 4; j++) {
                 const int a = (tid >> 6) + 4 * j;
-                float v0 = 0.f, v1 = 0.f;
-                if (a0 + a < M && s_own < M) {
-                    v0 = __ldg(x0 + (size_t)(a0 + a) * M + s_own);
-                    v1 = __ldg(x1 + (size_t)(a0 + a) * M + s_own);
-                }
+                const bool in = a0 + a < M && s_own < M;
+                const size_t at = in ? (size_t)(a0 + a) * M + s_own : 0;
+                copy_async4(tile + a * kFgTile + (tid & 63), x0 + at, in);
+                copy_async4(tile + kPart + a * kFgTile + (tid & 63), x1 + at, in);
+            }
+            stage_features(q, a0, M, d0, D, vec, tile + 2 * kPart);
+            stage_features(kl + D, a0, M, d0, D, vec, tile + 3 * kPart);
+            copy_commit();
+        };
+        stage(0);
+        for (int step = 0; step < chunks; step++) {
+            float *sxs = s_tiles + (step & 1) * kFgStage;
+            const float *sx1 = sxs + kPart, *sq = sxs + 2 * kPart, *sk = sxs + 3 * kPart;
+            copy_wait();
+            bool work = staged_not_finite(sq, vec) || staged_not_finite(sk, vec);
+#pragma unroll
+            for (int j = 0; j < kFgChunk / 4; j++) {
+                const int at = ((tid >> 6) + 4 * j) * kFgTile + (tid & 63);
+                const float v0 = sxs[at], v1 = sx1[at];
                 work |= v0 != 0.f || v1 != 0.f;
                 x0sum += v0;
-                sxs[a * kFgTile + (tid & 63)] = v0 + v1;
-                sx1[a * kFgTile + (tid & 63)] = v1;
+                sxs[at] = v0 + v1;
             }
-            work |= stage_features(q, a0, M, d0, D, vec, sq);
-            work |= stage_features(kl + D, a0, M, d0, D, vec, sk);
-            if (__syncthreads_or(work)) {
+            work = __syncthreads_or(work);
+            if (step + 1 < chunks) stage(step + 1);
+            if (!work) continue;
 #pragma unroll 4
-                for (int a = 0; a < kFgChunk; a++) {
-                    const float4 xs = *reinterpret_cast<const float4 *>(sxs + a * kFgTile + 4 * ty);
-                    const float4 xb = *reinterpret_cast<const float4 *>(sx1 + a * kFgTile + 4 * ty);
-                    const float4 qv = *reinterpret_cast<const float4 *>(sq + a * kFgTile + 4 * tx);
-                    const float4 kv = *reinterpret_cast<const float4 *>(sk + a * kFgTile + 4 * tx);
+            for (int a = 0; a < kFgChunk; a++) {
+                const float4 xs = *reinterpret_cast<const float4 *>(sxs + a * kFgTile + 4 * ty);
+                const float4 xb = *reinterpret_cast<const float4 *>(sx1 + a * kFgTile + 4 * ty);
+                const float4 qv = *reinterpret_cast<const float4 *>(sq + a * kFgTile + 4 * tx);
+                const float4 kv = *reinterpret_cast<const float4 *>(sk + a * kFgTile + 4 * tx);
 #pragma unroll
-                    for (int i = 0; i < 4; i++)
+                for (int i = 0; i < 4; i++)
 #pragma unroll
-                        for (int c = 0; c < 4; c++) {
-                            acc0[i][c] = fmaf(part(xs, i), part(qv, c), acc0[i][c]);
-                            acc1[i][c] = fmaf(part(xb, i), part(kv, c), acc1[i][c]);
-                        }
-                }
+                    for (int c = 0; c < 4; c++) {
+                        acc0[i][c] = fmaf(part(xs, i), part(qv, c), acc0[i][c]);
+                        acc1[i][c] = fmaf(part(xb, i), part(kv, c), acc1[i][c]);
+                    }
             }
-            __syncthreads();
         }
         sums[(tid >> 6) * kFgTile + (tid & 63)] = x0sum;
         __syncthreads();
@@ -616,11 +732,27 @@ __global__ void __launch_bounds__(kFgThreads, 2)
 
 }  // namespace
 
-int launch_links_scores(const float *qm, const float *klm, const float *krm, int M, int B, int H, int D, float *ac,
-                        float *bc, cudaStream_t st) {
+static bool on_16_bytes(std::initializer_list<const void *> ptrs) {
+    uintptr_t all = 0;
+    for (const void *p : ptrs) all |= reinterpret_cast<uintptr_t>(p);
+    return (all & 15) == 0;
+}
+
+// nonpad == nullptr: every cell is formed
+int launch_links_scores(const float *qm, const float *klm, const float *krm, const uint8_t *nonpad, const uint8_t *right_mask,
+                        const uint8_t *main_chain, const int *nodes, int L, int M, int B, int H, int D, float *ac, float *bc,
+                        cudaStream_t st) {
     if (B == 0 || M == 0) return PCFGNAT_OK;
-    const dim3 grid((M + kScoreTile - 1) / kScoreTile, (2 * M + 1 + kScoreTile - 1) / kScoreTile, B * H);
-    links_scores_kernel<<<grid, 256, 0, st>>>(qm, klm, krm, M, D, ac, bc);
+    const int vec = D % 4 == 0 && on_16_bytes({qm, klm, krm});
+    const dim3 tiles((M + kScoreCols - 1) / kScoreCols, (2 * M + 1 + kScoreRows - 1) / kScoreRows);
+    // up to four heads per block (the test for tiles in use and the first chunk's latency are paid once), as long as
+    // there are four blocks for every place on the GPU: tiles that are not in use leave at once
+    int heads = 4;
+    while (heads > 1 && (long long)tiles.x * tiles.y * B * ((H + heads - 1) / heads) < 4 * 2 * 148) heads /= 2;
+    const size_t smem = 2 * kScoreStage * sizeof(float);
+    if (ensure_dynamic_smem(links_scores_kernel, smem) != cudaSuccess) return PCFGNAT_ERR_CUDA;
+    links_scores_kernel<<<dim3(tiles.x, tiles.y, B * ((H + heads - 1) / heads)), 256, smem, st>>>(
+        qm, klm, krm, M, H, D, heads, vec, ScoreMasks{nonpad, right_mask, main_chain, nodes, L}, ac, bc);
     return cuda_rc(cudaGetLastError());
 }
 
@@ -639,17 +771,24 @@ int launch_links_backward(const float *links_grad, const float *ac, const float 
                                                                      X0, X1, dab, dgates);
     if (cudaGetLastError() != cudaSuccess) return PCFGNAT_ERR_CUDA;
     if (M == 0) return PCFGNAT_OK;
-    const bool vec = D % 4 == 0 && ((reinterpret_cast<uintptr_t>(qm) | reinterpret_cast<uintptr_t>(klm) |
-                                     reinterpret_cast<uintptr_t>(krm)) & 15) == 0;
+    const int vec = D % 4 == 0 && on_16_bytes({qm, klm, krm});
     const dim3 grid(2 * ((M + kFgTile - 1) / kFgTile), (D + kFgTile - 1) / kFgTile, B * H);
-    links_features_grad_kernel<<<grid, kFgThreads, 0, st>>>(X0, X1, dab, qm, klm, krm, nodes, M, L, H, D, vec, dq, dkl, dkr);
+    if (ensure_dynamic_smem(links_features_grad_kernel, kFgSmem) != cudaSuccess) return PCFGNAT_ERR_CUDA;
+    links_features_grad_kernel<<<grid, kFgThreads, kFgSmem, st>>>(X0, X1, dab, qm, klm, krm, nodes, M, L, H, D, vec, dq, dkl, dkr);
     return cuda_rc(cudaGetLastError());
 }
 
 int launch_links_gather(const void *q, const void *kl, const void *kr, int is_half, const int *nodes, int M, int B, int L,
                         int H, int D, float *qm, float *klm, float *krm, cudaStream_t st) {
     if (B == 0) return PCFGNAT_OK;
-    links_gather_kernel<<<dim3(M + 1, B), 256, 0, st>>>(q, kl, kr, is_half, nodes, M, L, H, D, qm, klm, krm);
+    const bool vec = D % 4 == 0 && on_16_bytes({q, kl, kr, qm, klm, krm});
+    const long long items = (long long)(M + 1) * H * D / (vec ? 4 : 1);
+    if (items > INT32_MAX - 256) return PCFGNAT_ERR_TOO_LARGE;
+    const dim3 grid((unsigned)((items + 255) / 256), B);
+    if (vec)
+        links_gather_kernel<true><<<grid, 256, 0, st>>>(q, kl, kr, is_half, nodes, M, L, H, D, qm, klm, krm);
+    else
+        links_gather_kernel<false><<<grid, 256, 0, st>>>(q, kl, kr, is_half, nodes, M, L, H, D, qm, klm, krm);
     return cuda_rc(cudaGetLastError());
 }
 

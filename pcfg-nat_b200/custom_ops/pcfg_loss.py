@@ -675,9 +675,10 @@ class _Kernel:
             _cabi.check(rc, "pcfgnat_links_gather_features")
             ac = torch.empty((B, H, M, M), dtype=torch.float32, device=dev)
             bc = torch.empty((B, H, M + 1, M), dtype=torch.float32, device=dev)
-            rc = lib.pcfgnat_links_scores(qm.data_ptr(), klm.data_ptr(), krm.data_ptr(), M, B, H, D, ac.data_ptr(),
-                                          bc.data_ptr(), _stream(dev))
-            _cabi.check(rc, "pcfgnat_links_scores")
+            rc = lib.pcfgnat_links_scores_masked(qm.data_ptr(), klm.data_ptr(), krm.data_ptr(), nonpad.data_ptr(),
+                                                 rm.data_ptr(), mc.data_ptr(), nodes.data_ptr(), M, B, L, H, D,
+                                                 ac.data_ptr(), bc.data_ptr(), _stream(dev))
+            _cabi.check(rc, "pcfgnat_links_scores_masked")
             links = torch.empty((B, L, 2, L), dtype=torch.float32, device=dev)
             rc = lib.pcfgnat_links_from_scores(ac.data_ptr(), bc.data_ptr(), qm.data_ptr(), klm.data_ptr(),
                                                gates.data_ptr(), nonpad.data_ptr(), lm.data_ptr(), rm.data_ptr(),
