@@ -328,7 +328,7 @@ int pcfgnat_links_scores_masked(const float *qm, const float *klm, const float *
 /* Gradient of those links with respect to the link features and the gate logits (training; the reference gets it
  * from autograd through the ~30 operators of extract_links).  links_grad [B][L][2][L] f32; ac, bc, qm, klm, krm and
  * the masks as in the forward.  Scratch: X0, X1 [B][heads][M][M] and dab [B][heads][M][2] f32 (fully overwritten at
- * the rows of main-chain nodes; the caller zero-fills them once for the others).  Outputs, all f32: dq, dkl, dkr
+ * the rows of the main-chain nodes).  Outputs, all f32: dq, dkl, dkr
  * [B][L][heads][head_dim] (zero-filled by the caller: only main-chain nodes and their left options are written)
  * and dgates [B][L][heads] (every cell written). */
 int pcfgnat_links_backward(const float *links_grad, const float *ac, const float *bc, const float *qm, const float *klm,

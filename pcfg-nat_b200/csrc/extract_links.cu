@@ -34,8 +34,9 @@ namespace pcfgnat {
 
 namespace {
 
-constexpr int kLinkThreads = 128;
 constexpr int kMaxHeads = 32;
+constexpr size_t kRowSmem = 40 * 1024;  // a row's exponentials are kept in shared memory up to here: five blocks per SM
+inline int row_threads(int H) { return H <= 4 ? 128 : 256; }
 
 __device__ __forceinline__ float warp_sum_f(float v) {
 #pragma unroll
@@ -90,49 +91,84 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// HT: number of heads known at compile time (the terms of a cell stay in registers between the two reductions
-// over the heads), or 0 for any number up to kMaxHeads.
-// gates [B][L][H] f32 (logits); nonpad [B][L] u8; left_mask, right_mask [L][L] u8 (1 = not allowed); main_chain [L]
-// u8; slot_of [L] = index of a node among the main-chain nodes or -1; nodes [M] its inverse.
-template <int HT>
-__global__ void __launch_bounds__(kLinkThreads)
-    links_from_scores_kernel(const float *__restrict__ ac, const float *__restrict__ bc, const float *__restrict__ qm,
-                             const float *__restrict__ klm, const float *__restrict__ gates,
-                             const uint8_t *__restrict__ nonpad, const uint8_t *__restrict__ left_mask,
-                             const uint8_t *__restrict__ right_mask, const uint8_t *__restrict__ main_chain,
-                             const int *__restrict__ slot_of, const int *__restrict__ nodes, int M, int L, int H, int D,
-                             float scale, float *__restrict__ links) {
-    extern __shared__ uint8_t s_right_ok[];  // [M] right child nodes[s] admissible for this node
-    __shared__ float s_ab[2][kMaxHeads], s_lse[kMaxHeads], s_lg[kMaxHeads];
-    const int a = blockIdx.x, b = blockIdx.y;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = kLinkThreads / 32;
-    const uint8_t *np = nonpad + (size_t)b * L;
-    float *out = links + ((size_t)b * L + a) * 2 * L;
-    for (int i = tid; i < 2 * L; i += kLinkThreads) out[i] = neg_inf();  // admissible cells are overwritten below
-    const int sa = slot_of[a];
-    if (sa < 0) return;  // not on the main chain: no right child at max_left == 1
-    // admissible children of a at all?  (the reference's link_left_nouse_mask / link_right_nouse_mask)
-    int any_left = 0, any_right = 0;
-    for (int j = tid; j < L; j += kLinkThreads) any_left |= np[j] && !left_mask[(size_t)a * L + j];
-    for (int s = tid; s < M; s += kLinkThreads) {
-        const int c = nodes[s];
-        const bool r_ok = np[c] && !right_mask[(size_t)a * L + c] && main_chain[c];
-        s_right_ok[s] = r_ok;
-        any_right |= r_ok;
+// One (sentence, node) row of the transitions: what its forward and its gradient both start from.  The blocks of
+// both kernels have a warp per head, up to eight.
+struct RowArgs {
+    const float *ac, *bc, *qm, *klm, *gates;
+    const uint8_t *nonpad, *left_mask, *right_mask, *main_chain;
+    const int *slot_of, *nodes;
+    int M, L, H, D;
+    float scale;
+};
+
+// Shared memory of a row: right_ok [M] (bytes), and with STAGED e [H][2][M] = exp(logit - top[head]), each head's
+// logits relative to its largest one.  !STAGED (rows too long for that) forms e again from the scores when asked.
+template <bool STAGED>
+struct Row {
+    const RowArgs &p;
+    int a, b, sa, lo, hi;  // node, sentence, its slot; slots [lo, hi) hold every admissible right child
+    const uint8_t *right_ok;
+    float *e;
+    const float (*ab)[kMaxHeads];
+    const float *top;
+
+    // logit of (left option k, right child slot s) for head h: (ab + bc) + ac
+    __device__ __forceinline__ float logit(int h, int k, int s) const {
+        const size_t bh = (size_t)b * p.H + h;
+        const float vac = __ldg(p.ac + (bh * p.M + sa) * p.M + s) * p.scale;
+        const float vbc = __ldg(p.bc + (bh * (p.M + 1) + (k ? 1 + sa : 0)) * p.M + s) * p.scale;
+        return (ab[k][h] + vbc) + vac;
     }
-    any_left = __syncthreads_or(any_left);
-    any_right = __syncthreads_or(any_right);  // also: s_right_ok is written, and so is the -inf fill of this row
-    if (!any_left || !any_right) return;
-    const int left1 = a >= 1 ? a - 1 : 0;  // the reference's _max_left_index[a][1]
-    const bool ok_left0 = np[0] && !left_mask[(size_t)a * L + 0];
-    const bool ok_left1 = np[left1] && !left_mask[(size_t)a * L + left1];
+    // -inf and NaN logits count nothing; nor does a head with a logit of +inf (its others would be -inf, itself NaN)
+    __device__ __forceinline__ float rel(float v, float t) const { return v > neg_inf() && t < CUDART_INF_F ? expf(v - t) : 0.f; }
+    __device__ __forceinline__ float exp_at(int h, int k, int s) const {
+        if constexpr (STAGED) return e[((size_t)h * 2 + k) * p.M + s];
+        else return rel(logit(h, k, s), top[h]);
+    }
+};
+
+// A cell of the mixture is log sum_h e[h] c[h], c[h] = gate probability / sum of the head's e.  Below this sum the
+// cell is formed from the log-probabilities instead: e of all heads may be about to flush to zero.
+constexpr float kMixtureFloor = 1e-30f;
+
+// Sets up a row: false when it has no admissible child on one of the sides (or the node is not on the main chain),
+// uniformly over the block.  s_lse, s_lg: per head the log-sum-exp of the logits and the log gate probability;
+// s_c, s_inv: gate probability / sum of e, and 1 / that sum, 0 where undefined.  Ends with the block in step.
+template <bool STAGED>
+__device__ __forceinline__ bool links_row(Row<STAGED> &row, uint8_t *right_ok, float (*s_ab)[kMaxHeads], float *s_top,
+                                          float *s_lse, float *s_lg, float *s_c, float *s_inv) {
+    const RowArgs &p = row.p;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
+    const int a = row.a, sa = row.sa, M = p.M;
+    const uint8_t *np = p.nonpad + (size_t)row.b * p.L;
+    __shared__ int s_lo, s_hi;
+    if (tid == 0) {
+        s_lo = M;
+        s_hi = 0;
+    }
+    // admissible children of a at all?  (the reference's link_left_nouse_mask / link_right_nouse_mask)
+    bool any_left = false;
+    for (int j = tid; j < p.L; j += blockDim.x) any_left |= np[j] && !p.left_mask[(size_t)a * p.L + j];
+    int lo = M, hi = 0;
+    for (int s = tid; s < M; s += blockDim.x) {
+        const int c = p.nodes[s];
+        const bool r_ok = np[c] && !p.right_mask[(size_t)a * p.L + c] && p.main_chain[c];
+        right_ok[s] = r_ok;
+        if (r_ok) {
+            lo = min(lo, s);
+            hi = s + 1;
+        }
+    }
     // ab[k][h]: one warp per head at a time, lanes over the chunk dimension
-    for (int h = warp; h < H; h += n_warps) {
-        const float *qa = qm + (((size_t)b * H + h) * M + sa) * D;
-        const float *k0 = klm + (((size_t)b * H + h) * (M + 1) + 0) * D;
-        const float *k1 = klm + (((size_t)b * H + h) * (M + 1) + 1 + sa) * D;
+    const int left1 = a >= 1 ? a - 1 : 0;  // the reference's _max_left_index[a][1]
+    const bool ok_left0 = np[0] && !p.left_mask[(size_t)a * p.L + 0];
+    const bool ok_left1 = np[left1] && !p.left_mask[(size_t)a * p.L + left1];
+    for (int h = warp; h < p.H; h += n_warps) {
+        const size_t bh = (size_t)row.b * p.H + h;
+        const float *qa = p.qm + (bh * M + sa) * p.D;
+        const float *k0 = p.klm + bh * (M + 1) * p.D, *k1 = k0 + (size_t)(1 + sa) * p.D;
         float d0 = 0.f, d1 = 0.f;
-        for (int d = lane; d < D; d += 32) {
+        for (int d = lane; d < p.D; d += 32) {
             const float x = qa[d];
             d0 = fmaf(x, k0[d], d0);
             d1 = fmaf(x, k1[d], d1);
@@ -140,78 +176,113 @@ __global__ void __launch_bounds__(kLinkThreads)
         d0 = warp_sum_f(d0);
         d1 = warp_sum_f(d1);
         if (lane == 0) {
-            s_ab[0][h] = ok_left0 ? d0 * scale : neg_inf();
-            s_ab[1][h] = ok_left1 ? d1 * scale : neg_inf();
+            s_ab[0][h] = ok_left0 ? d0 * p.scale : neg_inf();
+            s_ab[1][h] = ok_left1 ? d1 * p.scale : neg_inf();
         }
     }
     if (warp == n_warps - 1) {  // log-softmax of the gate logits over the heads
-        const float gt = lane < H ? gates[((size_t)b * L + a) * H + lane] : neg_inf();
+        const float gt = lane < p.H ? p.gates[((size_t)row.b * p.L + a) * p.H + lane] : neg_inf();
         const float mx = warp_max_f(gt);
-        const float sum = warp_sum_f(lane < H ? expf(gt - mx) : 0.f);
-        if (lane < H) s_lg[lane] = gt - (mx + logf(sum));
+        const float sum = warp_sum_f(lane < p.H ? expf(gt - mx) : 0.f);
+        if (lane < p.H) s_lg[lane] = gt - (mx + logf(sum));
+    }
+    if (!__syncthreads_or(any_left)) return false;
+    if (hi > 0) {
+        atomicMin(&s_lo, lo);
+        atomicMax(&s_hi, hi);
     }
     __syncthreads();
-    // logit of (left option k, right child slot s) for head h: (ab + bc) + ac
-    auto logit = [&](int h, int k, int s) {
-        const float vac = ac[(((size_t)b * H + h) * M + sa) * M + s] * scale;
-        const float vbc = bc[(((size_t)b * H + h) * (M + 1) + (k ? 1 + sa : 0)) * M + s] * scale;
-        return (s_ab[k][h] + vbc) + vac;
-    };
-    // pass 1: log-sum-exp over (k, c) per head
-    for (int h = warp; h < H; h += n_warps) {
-        float mx = neg_inf(), sum = 0.f;
-        for (int s = lane; s < M; s += 32) {
-            if (!s_right_ok[s]) continue;
+    row.lo = s_lo;
+    row.hi = s_hi;
+    if (row.lo >= row.hi) return false;
+    // per head: the largest logit, then the exponentials relative to it and their sum
+    for (int h = warp; h < p.H; h += n_warps) {
+        float mx = neg_inf();
+        for (int s = row.lo + lane; s < row.hi; s += 32) {
+            const bool ok = right_ok[s];
 #pragma unroll
             for (int k = 0; k < 2; k++) {
-                const float v = logit(h, k, s);
-                if (v > mx) {
-                    sum = sum * expf(mx - v) + 1.f;  // exp(-inf - v) = 0 on the first finite value
-                    mx = v;
-                } else if (v > neg_inf()) {
-                    sum += expf(v - mx);
+                const float v = ok ? row.logit(h, k, s) : neg_inf();
+                if constexpr (STAGED) row.e[((size_t)h * 2 + k) * M + s] = v;
+                mx = fmaxf(mx, v);  // drops NaN
+            }
+        }
+        mx = warp_max_f(mx);
+        float sum = 0.f;
+        for (int s = row.lo + lane; s < row.hi; s += 32) {
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                if constexpr (STAGED) {
+                    float &cell = row.e[((size_t)h * 2 + k) * M + s];
+                    cell = row.rel(cell, mx);
+                    sum += cell;
+                } else {
+                    sum += right_ok[s] ? row.rel(row.logit(h, k, s), mx) : 0.f;
                 }
             }
         }
-        const float top = warp_max_f(mx);
-        sum = isinf(mx) ? 0.f : sum * expf(mx - top);
         sum = warp_sum_f(sum);
-        if (lane == 0) s_lse[h] = isinf(top) ? top : top + logf(sum);
+        if (lane == 0) {
+            const float lg = s_lg[h], gate = lg > neg_inf() ? expf(lg) : 0.f;  // NaN: the head counts nothing
+            s_top[h] = mx;
+            s_lse[h] = isinf(mx) ? mx : mx + logf(sum);
+            s_inv[h] = sum > 0.f ? 1.f / sum : 0.f;
+            s_c[h] = gate * s_inv[h];
+        }
     }
     __syncthreads();
-    // pass 2: mix the heads
-    for (int i = tid; i < 2 * M; i += kLinkThreads) {
-        const int k = i / M, s = i - k * M;
-        if (!s_right_ok[s]) continue;
-        float res = neg_inf();
-        if (HT > 0) {
-            float term[HT > 0 ? HT : 1];
-            float mx = neg_inf();
-#pragma unroll
-            for (int h = 0; h < HT; h++) {
-                term[h] = (logit(h, k, s) - s_lse[h]) + s_lg[h];
-                mx = fmaxf(mx, term[h]);  // fmaxf drops NaN
-            }
-            if (!isinf(mx)) {
-                float sum = 0.f;
-#pragma unroll
-                for (int h = 0; h < HT; h++)
-                    if (term[h] > neg_inf()) sum += expf(term[h] - mx);
-                res = mx + logf(sum);
-            }
-        } else {
-            float mx = neg_inf();
-            for (int h = 0; h < H; h++) mx = fmaxf(mx, (logit(h, k, s) - s_lse[h]) + s_lg[h]);
-            if (!isinf(mx)) {
-                float sum = 0.f;
-                for (int h = 0; h < H; h++) {
-                    const float t = (logit(h, k, s) - s_lse[h]) + s_lg[h];
-                    if (t > neg_inf()) sum += expf(t - mx);
-                }
-                res = mx + logf(sum);
-            }
+    return true;
+}
+
+// The mixture of a cell from the log-probabilities of its heads: largest term, and sum of the others relative to it.
+template <class LogProb>
+__device__ __forceinline__ float mixture_terms(int H, LogProb term, float &sum) {
+    float mx = neg_inf();
+    for (int h = 0; h < H; h++) mx = fmaxf(mx, term(h));  // drops NaN
+    sum = 0.f;
+    if (!isinf(mx))
+        for (int h = 0; h < H; h++) {
+            const float t = term(h);
+            if (t > neg_inf()) sum += expf(t - mx);
         }
-        out[(size_t)k * L + nodes[s]] = res;
+    return mx;
+}
+
+// One block per (sentence, node).  A cell takes one exponential per head, one FMA per head and one logarithm.  Bound by
+// latency (a row is a few hundred cells behind five barriers): rows of nodes that are not on the main chain, and
+// slots outside the admissible range, cost nothing but their -inf.  90 sentences, M = 161, eight heads: 136 us; 190 us
+// with two exponentials per cell and head, each from scores read again.  Against float64 the transitions are off by
+// 2.3e-7 (rms; 2.8e-7 before).
+template <bool STAGED>
+__global__ void __launch_bounds__(256)
+    links_from_scores_kernel(const RowArgs p, float *__restrict__ links) {
+    extern __shared__ __align__(16) float s_e[];  // STAGED: [H][2][M] exponentials; then [M] bytes
+    __shared__ float s_ab[2][kMaxHeads], s_top[kMaxHeads], s_lse[kMaxHeads], s_lg[kMaxHeads], s_c[kMaxHeads], s_inv[kMaxHeads];
+    const int a = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+    float *out = links + ((size_t)b * p.L + a) * 2 * p.L;
+    for (int i = tid; i < 2 * p.L; i += blockDim.x) out[i] = neg_inf();  // admissible cells are overwritten below
+    const int sa = p.slot_of[a];
+    if (sa < 0) return;  // not on the main chain: no right child at max_left == 1
+    uint8_t *right_ok = reinterpret_cast<uint8_t *>(s_e + (STAGED ? (size_t)p.H * 2 * p.M : 0));
+    Row<STAGED> row{p, a, b, sa, 0, 0, right_ok, s_e, s_ab, s_top};
+    if (!links_row(row, right_ok, s_ab, s_top, s_lse, s_lg, s_c, s_inv)) return;
+    const int span = row.hi - row.lo;
+    for (int i = tid; i < 2 * span; i += blockDim.x) {
+        const int k = i >= span, s = row.lo + i - k * span;
+        if (!right_ok[s]) continue;
+        float sum = 0.f;
+#pragma unroll 8
+        for (int h = 0; h < p.H; h++) sum = fmaf(row.exp_at(h, k, s), s_c[h], sum);
+        float res;
+        if (sum > kMixtureFloor) {
+            res = logf(sum);
+        } else {
+            float rest;
+            res = mixture_terms(p.H, [&](int h) { return (row.logit(h, k, s) - s_lse[h]) + s_lg[h]; }, rest);
+            if (!isinf(res)) res += logf(rest);
+            else res = neg_inf();
+        }
+        out[(size_t)k * p.L + p.nodes[s]] = res;
     }
 }
 
@@ -339,176 +410,118 @@ __global__ void __launch_bounds__(256, 2)
     }
 }
 
-// Gradient of the logits of one (sentence, node) row.  With G = links_grad[a][k][c], res = links[a][k][c],
-//   term[h] = logit[h] - lse[h] + lg[h],  w[h] = exp(term[h] - res)             (share of head h in the mixture)
-//   d lp[k][c][h] = G w[h],   Gs[h] = sum_{k,c} d lp[k][c][h]  (= d lg[h]),
-//   d logit[k][c][h] = d lp[k][c][h] - exp(logit[k][c][h] - lse[h]) Gs[h]
+// Gradient of the logits of one (sentence, node) row.  With G = links_grad[a][k][c], e and c as above, and
+// w = G / sum_h e[h] c[h]:
+//   d lp[k][c][h] = w e[h] c[h]                               (G times the share of head h in the mixture)
+//   Gs[h] = sum_{k,c} d lp[k][c][h]                           (= d lg[h])
+//   d logit[k][c][h] = d lp[k][c][h] - e[h] / sum e[h] Gs[h]
 // written scaled by 1/sqrt(D) (the logits are scaled dot products) as X0 (k = 0) and X1 (k = 1) [B][H][M][M] at row
 // slot(a); dab [B][H][M][2] = their row sums; dgates[a][h] = Gs[h] - softmax(gates)[h] sum_h' Gs[h'].  Rows of nodes
-// that are not on the main chain, or have no admissible child, are zero (X rows) / zero (dgates).
-__global__ void __launch_bounds__(kLinkThreads)
-    links_scores_grad_kernel(const float *__restrict__ links_grad, const float *__restrict__ ac, const float *__restrict__ bc,
-                             const float *__restrict__ qm, const float *__restrict__ klm, const float *__restrict__ gates,
-                             const uint8_t *__restrict__ nonpad, const uint8_t *__restrict__ left_mask,
-                             const uint8_t *__restrict__ right_mask, const uint8_t *__restrict__ main_chain,
-                             const int *__restrict__ slot_of, const int *__restrict__ nodes, int M, int L, int H, int D,
-                             float scale, float *__restrict__ X0, float *__restrict__ X1, float *__restrict__ dab,
-                             float *__restrict__ dgates) {
-    extern __shared__ uint8_t s_right_ok[];
-    __shared__ float s_ab[2][kMaxHeads], s_lse[kMaxHeads], s_lg[kMaxHeads], s_gs[kMaxHeads], s_red[kMaxHeads][4];
+// that are not on the main chain, or have no admissible child, are zero (X rows) / zero (dgates).  A head with a
+// logit of +inf gets NaN, as its gradient is undefined.  300 us at the size above, 562 us with the shares of a cell
+// formed twice from log-probabilities; feature gradients off by 2.2e-7 of their norm (3.3e-7 before).
+// KEEP: what stays in shared memory: 2 = e and w, 1 = w, 0 = neither (formed again when needed).
+template <int KEEP>
+__global__ void __launch_bounds__(256)
+    links_scores_grad_kernel(const RowArgs p, const float *__restrict__ links_grad, float *__restrict__ X0,
+                             float *__restrict__ X1, float *__restrict__ dab, float *__restrict__ dgates) {
+    constexpr bool STAGED = KEEP == 2;
+    extern __shared__ __align__(16) float s_e[];  // [H][2][M] exponentials; w [2][M]; bytes: [M], and [2][M] beside w
+    __shared__ float s_ab[2][kMaxHeads], s_top[kMaxHeads], s_lse[kMaxHeads], s_lg[kMaxHeads], s_c[kMaxHeads], s_inv[kMaxHeads];
+    __shared__ float s_gs[kMaxHeads];
     const int a = blockIdx.x, b = blockIdx.y;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = kLinkThreads / 32;
-    const uint8_t *np = nonpad + (size_t)b * L;
-    float *dg = dgates + ((size_t)b * L + a) * H;
-    for (int h = tid; h < H; h += kLinkThreads) dg[h] = 0.f;
-    const int sa = slot_of[a];
-    if (sa < 0) return;
-    // this node's rows of X0, X1 and dab start at zero
-    for (int i = tid; i < H * M; i += kLinkThreads) {
-        const int h = i / M, s = i - h * M;
-        X0[(((size_t)b * H + h) * M + sa) * M + s] = 0.f;
-        X1[(((size_t)b * H + h) * M + sa) * M + s] = 0.f;
-    }
-    for (int i = tid; i < 2 * H; i += kLinkThreads) dab[(((size_t)b * H + i / 2) * M + sa) * 2 + (i & 1)] = 0.f;
-    int any_left = 0, any_right = 0;
-    for (int j = tid; j < L; j += kLinkThreads) any_left |= np[j] && !left_mask[(size_t)a * L + j];
-    for (int s = tid; s < M; s += kLinkThreads) {
-        const int c = nodes[s];
-        const bool r_ok = np[c] && !right_mask[(size_t)a * L + c] && main_chain[c];
-        s_right_ok[s] = r_ok;
-        any_right |= r_ok;
-    }
-    any_left = __syncthreads_or(any_left);
-    any_right = __syncthreads_or(any_right);
-    if (!any_left || !any_right) return;
-    const int left1 = a >= 1 ? a - 1 : 0;
-    const bool ok_left0 = np[0] && !left_mask[(size_t)a * L + 0];
-    const bool ok_left1 = np[left1] && !left_mask[(size_t)a * L + left1];
-    for (int h = warp; h < H; h += n_warps) {
-        const float *qa = qm + (((size_t)b * H + h) * M + sa) * D;
-        const float *k0 = klm + (((size_t)b * H + h) * (M + 1) + 0) * D;
-        const float *k1 = klm + (((size_t)b * H + h) * (M + 1) + 1 + sa) * D;
-        float d0 = 0.f, d1 = 0.f;
-        for (int d = lane; d < D; d += 32) {
-            const float x = qa[d];
-            d0 = fmaf(x, k0[d], d0);
-            d1 = fmaf(x, k1[d], d1);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
+    const int M = p.M, H = p.H;
+    float *dg = dgates + ((size_t)b * p.L + a) * H;
+    const int sa = p.slot_of[a];
+    float *s_w = s_e + (STAGED ? (size_t)H * 2 * M : 0);
+    uint8_t *right_ok = reinterpret_cast<uint8_t *>(s_w + (KEEP ? 2 * M : 0)), *s_rare = right_ok + M;
+    Row<STAGED> row{p, a, b, sa, 0, 0, right_ok, s_e, s_ab, s_top};
+    if (sa < 0 || !links_row(row, right_ok, s_ab, s_top, s_lse, s_lg, s_c, s_inv)) {
+        for (int h = tid; h < H; h += blockDim.x) dg[h] = 0.f;
+        if (sa < 0) return;
+        for (int i = tid; i < H * M; i += blockDim.x) {
+            const size_t at = (((size_t)b * H + i / M) * M + sa) * M + i % M;
+            X0[at] = 0.f;
+            X1[at] = 0.f;
         }
-        d0 = warp_sum_f(d0);
-        d1 = warp_sum_f(d1);
-        if (lane == 0) {
-            s_ab[0][h] = ok_left0 ? d0 * scale : neg_inf();
-            s_ab[1][h] = ok_left1 ? d1 * scale : neg_inf();
-        }
+        for (int i = tid; i < 2 * H; i += blockDim.x) dab[(((size_t)b * H + i / 2) * M + sa) * 2 + (i & 1)] = 0.f;
+        return;
     }
-    float gate_p = 0.f;  // softmax(gates)[lane] in the last warp
-    if (warp == n_warps - 1) {
-        const float gt = lane < H ? gates[((size_t)b * L + a) * H + lane] : neg_inf();
-        const float mx = warp_max_f(gt);
-        const float sum = warp_sum_f(lane < H ? expf(gt - mx) : 0.f);
-        if (lane < H) {
-            s_lg[lane] = gt - (mx + logf(sum));
-            gate_p = expf(s_lg[lane]);
+    auto term = [&](int h, int k, int s) { return (row.logit(h, k, s) - s_lse[h]) + s_lg[h]; };
+    const float *grow = links_grad + ((size_t)b * p.L + a) * 2 * p.L;
+    // w of an admissible cell, or G itself (rare) below the floor of the mixture
+    auto weigh = [&](int k, int s, bool &rare) {
+        rare = false;
+        const float G = grow[(size_t)k * p.L + p.nodes[s]];
+        if (G == 0.f) return 0.f;
+        float sum = 0.f;
+#pragma unroll 8
+        for (int h = 0; h < H; h++) sum = fmaf(row.exp_at(h, k, s), s_c[h], sum);
+        rare = !(sum > kMixtureFloor);
+        return rare ? G : G / sum;
+    };
+    if constexpr (KEEP > 0) {
+        const int span = row.hi - row.lo;
+        for (int i = tid; i < 2 * span; i += blockDim.x) {
+            const int k = i >= span, s = row.lo + i - k * span;
+            bool rare = false;
+            s_w[k * M + s] = right_ok[s] ? weigh(k, s, rare) : 0.f;
+            s_rare[k * M + s] = rare;
         }
+        __syncthreads();
     }
-    __syncthreads();
-    auto logit = [&](int h, int k, int s) {
-        const float vac = ac[(((size_t)b * H + h) * M + sa) * M + s] * scale;
-        const float vbc = bc[(((size_t)b * H + h) * (M + 1) + (k ? 1 + sa : 0)) * M + s] * scale;
-        return (s_ab[k][h] + vbc) + vac;
+    // d lp of a cell: w e c, or formed from the log-probabilities where the sum is too small (-inf cells: nothing)
+    auto share = [&](int h, int k, int s, float e) {
+        float w;
+        bool rare;
+        if constexpr (KEEP > 0) {
+            w = s_w[k * M + s];
+            rare = s_rare[k * M + s];
+        } else {
+            w = weigh(k, s, rare);
+        }
+        if (!rare) return w * (e * s_c[h]);
+        float sum;
+        const float mx = mixture_terms(H, [&](int i) { return term(i, k, s); }, sum), t = term(h, k, s);
+        return !isinf(mx) && t > neg_inf() ? w * expf(t - mx) / sum : 0.f;
     };
     for (int h = warp; h < H; h += n_warps) {
-        float mx = neg_inf(), sum = 0.f;
+        float gs = 0.f;
+        for (int s = row.lo + lane; s < row.hi; s += 32) {
+            if (!right_ok[s]) continue;
+#pragma unroll
+            for (int k = 0; k < 2; k++) gs += share(h, k, s, row.exp_at(h, k, s));
+        }
+        gs = warp_sum_f(gs);
+        const float back = s_top[h] < CUDART_INF_F ? gs * s_inv[h] : CUDART_NAN_F;  // Gs / sum e
+        float sums[2] = {0.f, 0.f};
+        const size_t at = (((size_t)b * H + h) * M + sa) * M;
         for (int s = lane; s < M; s += 32) {
-            if (!s_right_ok[s]) continue;
+            const bool ok = s >= row.lo && s < row.hi && right_ok[s];
 #pragma unroll
             for (int k = 0; k < 2; k++) {
-                const float v = logit(h, k, s);
-                if (v > mx) {
-                    sum = sum * expf(mx - v) + 1.f;
-                    mx = v;
-                } else if (v > neg_inf()) {
-                    sum += expf(v - mx);
+                float d = 0.f;
+                if (ok) {
+                    const float e = row.exp_at(h, k, s);
+                    d = (share(h, k, s, e) - e * back) * p.scale;
                 }
+                (k ? X1 : X0)[at + s] = d;
+                sums[k] += d;
             }
         }
-        const float top = warp_max_f(mx);
-        sum = isinf(mx) ? 0.f : sum * expf(mx - top);
-        sum = warp_sum_f(sum);
-        if (lane == 0) s_lse[h] = isinf(top) ? top : top + logf(sum);
-    }
-    for (int i = tid; i < kMaxHeads * 4; i += kLinkThreads) s_red[i / 4][i & 3] = 0.f;
-    __syncthreads();
-    // pass A: Gs[h] = sum over the row's cells of G w[h]; every thread walks its cells, heads in registers
-    const float *grow = links_grad + ((size_t)b * L + a) * 2 * L;
-    float gs_part[kMaxHeads];
-    for (int h = 0; h < H; h++) gs_part[h] = 0.f;
-    for (int i = tid; i < 2 * M; i += kLinkThreads) {
-        const int k = i / M, s = i - k * M;
-        if (!s_right_ok[s]) continue;
-        const float G = grow[(size_t)k * L + nodes[s]];
-        if (G == 0.f) continue;
-        float mx = neg_inf();
-        for (int h = 0; h < H; h++) mx = fmaxf(mx, (logit(h, k, s) - s_lse[h]) + s_lg[h]);
-        if (isinf(mx)) continue;  // the cell is -inf: no gradient
-        float sum = 0.f;
-        for (int h = 0; h < H; h++) {
-            const float t = (logit(h, k, s) - s_lse[h]) + s_lg[h];
-            if (t > neg_inf()) sum += expf(t - mx);
-        }
-        const float inv = G / sum;
-        for (int h = 0; h < H; h++) {
-            const float t = (logit(h, k, s) - s_lse[h]) + s_lg[h];
-            if (t > neg_inf()) gs_part[h] += expf(t - mx) * inv;
+        sums[0] = warp_sum_f(sums[0]);
+        sums[1] = warp_sum_f(sums[1]);
+        if (lane == 0) {
+            s_gs[h] = gs;
+            dab[(((size_t)b * H + h) * M + sa) * 2 + 0] = sums[0];
+            dab[(((size_t)b * H + h) * M + sa) * 2 + 1] = sums[1];
         }
     }
-    for (int h = 0; h < H; h++) {
-        const float v = warp_sum_f(gs_part[h]);
-        if (lane == 0) s_red[h][warp] = v;
-    }
-    __syncthreads();
-    if (tid < H) s_gs[tid] = (s_red[tid][0] + s_red[tid][1]) + (s_red[tid][2] + s_red[tid][3]);
     __syncthreads();
     if (warp == n_warps - 1) {  // gate logits: d lg - softmax(gates) sum d lg
         const float tot = warp_sum_f(lane < H ? s_gs[lane] : 0.f);
-        if (lane < H) dg[lane] = s_gs[lane] - gate_p * tot;
-    }
-    // pass B: d logit of every cell and head, and the row sums per left option
-    float ab_part[2][kMaxHeads];
-    for (int h = 0; h < H; h++) ab_part[0][h] = ab_part[1][h] = 0.f;
-    for (int i = tid; i < 2 * M; i += kLinkThreads) {
-        const int k = i / M, s = i - k * M;
-        if (!s_right_ok[s]) continue;
-        const float G = grow[(size_t)k * L + nodes[s]];
-        float mx = neg_inf(), sum = 0.f;
-        for (int h = 0; h < H; h++) mx = fmaxf(mx, (logit(h, k, s) - s_lse[h]) + s_lg[h]);
-        if (!isinf(mx))
-            for (int h = 0; h < H; h++) {
-                const float t = (logit(h, k, s) - s_lse[h]) + s_lg[h];
-                if (t > neg_inf()) sum += expf(t - mx);
-            }
-        float *X = k ? X1 : X0;
-        for (int h = 0; h < H; h++) {
-            const float lgt = logit(h, k, s);
-            float d = 0.f;
-            if (lgt > neg_inf()) {
-                const float t = (lgt - s_lse[h]) + s_lg[h];
-                const float dlp = (G != 0.f && !isinf(mx)) ? G * expf(t - mx) / sum : 0.f;
-                d = (dlp - expf(lgt - s_lse[h]) * s_gs[h]) * scale;
-            }
-            X[(((size_t)b * H + h) * M + sa) * M + s] = d;
-            ab_part[k][h] += d;
-        }
-    }
-    __syncthreads();  // s_red is reused
-    for (int k = 0; k < 2; k++) {
-        for (int h = 0; h < H; h++) {
-            const float v = warp_sum_f(ab_part[k][h]);
-            if (lane == 0) s_red[h][warp] = v;
-        }
-        __syncthreads();
-        if (tid < H) dab[(((size_t)b * H + tid) * M + sa) * 2 + k] = (s_red[tid][0] + s_red[tid][1]) + (s_red[tid][2] + s_red[tid][3]);
-        __syncthreads();
+        if (lane < H) dg[lane] = s_gs[lane] - expf(s_lg[lane]) * tot;
     }
 }
 
@@ -763,12 +776,16 @@ int launch_links_backward(const float *links_grad, const float *ac, const float 
                           float *dgates, cudaStream_t st) {
     if (B == 0) return PCFGNAT_OK;
     if (H > kMaxHeads) return PCFGNAT_ERR_TOO_LARGE;
-    const float scale = 1.f / sqrtf((float)D);
-    const size_t smem = (size_t)(M + 16) / 16 * 16;
-    if (smem > 40 * 1024) return PCFGNAT_ERR_TOO_LARGE;
-    links_scores_grad_kernel<<<dim3(L, B), kLinkThreads, smem, st>>>(links_grad, ac, bc, qm, klm, gates, nonpad, left_mask,
-                                                                     right_mask, main_chain, slot_of, nodes, M, L, H, D, scale,
-                                                                     X0, X1, dab, dgates);
+    const RowArgs row{ac, bc, qm, klm, gates, nonpad, left_mask, right_mask, main_chain, slot_of, nodes, M, L, H, D,
+                      1.f / sqrtf((float)D)};
+    if ((size_t)M > 40 * 1024) return PCFGNAT_ERR_TOO_LARGE;
+    const size_t staged = (size_t)H * 2 * M * sizeof(float), w = (size_t)2 * M * sizeof(float) + 3 * (size_t)M;
+    if (staged + w <= kRowSmem)
+        links_scores_grad_kernel<2><<<dim3(L, B), row_threads(H), staged + w, st>>>(row, links_grad, X0, X1, dab, dgates);
+    else if (w <= kRowSmem)
+        links_scores_grad_kernel<1><<<dim3(L, B), row_threads(H), w, st>>>(row, links_grad, X0, X1, dab, dgates);
+    else
+        links_scores_grad_kernel<0><<<dim3(L, B), row_threads(H), (size_t)M, st>>>(row, links_grad, X0, X1, dab, dgates);
     if (cudaGetLastError() != cudaSuccess) return PCFGNAT_ERR_CUDA;
     if (M == 0) return PCFGNAT_OK;
     const int vec = D % 4 == 0 && on_16_bytes({qm, klm, krm});
@@ -798,15 +815,14 @@ int launch_links_from_scores(const float *ac, const float *bc, const float *qm, 
                              int D, float *links, cudaStream_t st) {
     if (B == 0) return PCFGNAT_OK;
     if (H > kMaxHeads) return PCFGNAT_ERR_TOO_LARGE;
-    const float scale = 1.f / sqrtf((float)D);
-    const size_t smem = (size_t)(M + 16) / 16 * 16;
-    if (smem > 40 * 1024) return PCFGNAT_ERR_TOO_LARGE;
-    if (H == 8)
-        links_from_scores_kernel<8><<<dim3(L, B), kLinkThreads, smem, st>>>(ac, bc, qm, klm, gates, nonpad, left_mask, right_mask,
-                                                                          main_chain, slot_of, nodes, M, L, H, D, scale, links);
+    if ((size_t)M > 40 * 1024) return PCFGNAT_ERR_TOO_LARGE;
+    const RowArgs row{ac, bc, qm, klm, gates, nonpad, left_mask, right_mask, main_chain, slot_of, nodes, M, L, H, D,
+                      1.f / sqrtf((float)D)};
+    const size_t staged = (size_t)H * 2 * M * sizeof(float);
+    if (staged + M <= kRowSmem)
+        links_from_scores_kernel<true><<<dim3(L, B), row_threads(H), staged + M, st>>>(row, links);
     else
-        links_from_scores_kernel<0><<<dim3(L, B), kLinkThreads, smem, st>>>(ac, bc, qm, klm, gates, nonpad, left_mask, right_mask,
-                                                                          main_chain, slot_of, nodes, M, L, H, D, scale, links);
+        links_from_scores_kernel<false><<<dim3(L, B), row_threads(H), M, st>>>(row, links);
     return cuda_rc(cudaGetLastError());
 }
 

@@ -699,9 +699,10 @@ class _Kernel:
         dev = g.device
         p = lambda name: saved[name].data_ptr()
         with torch.cuda.device(dev):
-            X0 = torch.zeros((B, H, M, M), dtype=torch.float32, device=dev)
-            X1 = torch.zeros((B, H, M, M), dtype=torch.float32, device=dev)
-            dab = torch.zeros((B, H, M, 2), dtype=torch.float32, device=dev)
+            # every main-chain node's block writes its whole row of these
+            X0 = torch.empty((B, H, M, M), dtype=torch.float32, device=dev)
+            X1 = torch.empty((B, H, M, M), dtype=torch.float32, device=dev)
+            dab = torch.empty((B, H, M, 2), dtype=torch.float32, device=dev)
             dq = torch.zeros((B, L, H, D), dtype=torch.float32, device=dev)
             dkl = torch.zeros_like(dq)
             dkr = torch.zeros_like(dq)
