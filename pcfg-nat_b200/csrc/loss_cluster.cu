@@ -168,6 +168,23 @@ __device__ __forceinline__ float inside_node_free(const float *r0, const float *
     return fmaf(fast_lg2(sum), kLn2, mx);
 }
 
+// One sentence's C [Lt][W][3]: C[0][t][0] = 0 for t <= n; C[leaf slot][t][1] = match[leaf][t] for t < n (pcfg_loss.cu:288-297)
+__device__ __forceinline__ void fill_leaf_table(float *Cb, const float *__restrict__ mat, int m, int n, int T, int W, int Lt,
+                                                bool ok, int ctid, int cthreads) {
+    for (int i = ctid; i < Lt * W * 3; i += cthreads) {
+        const int g = i % 3, t = (i / 3) % W, a_id = i / (3 * W);
+        float v = neg_inf();
+        if (ok) {
+            if (a_id == 0) {
+                if (g == 0 && t <= n) v = 0.f;
+            } else if (g == 1 && 2 * a_id < m && t < n) {
+                v = __ldg(mat + (size_t)(2 * a_id) * T + t);
+            }
+        }
+        Cb[i] = v;
+    }
+}
+
 // TRIPS == 0: the reference's summation order (bit-exact table).  TRIPS > 0: free order, for chains of at
 // most 32 * TRIPS main nodes (a lane holds the terms of its TRIPS children in registers between the passes).
 // SHARES (free order only): `shares` is a [B][L][T] buffer; the share of the j = 0 terms in S[a][t] goes to
@@ -222,21 +239,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
     float *Sb = S + (size_t)b * Mc * W;
 
     for (int i = ctid; i < Mc * W; i += cthreads) Sb[i] = neg_inf();
-    if (C) {  // C[0][t][0] = 0 for t <= n; C[leaf slot][t][1] = match[leaf][t] for t < n (pcfg_loss.cu:288-297)
-        float *Cb = C + (size_t)b * Lt * W * 3;
-        for (int i = ctid; i < Lt * W * 3; i += cthreads) {
-            int g = i % 3, t = (i / 3) % W, a_id = i / (3 * W);
-            float v = neg_inf();
-            if (ok) {
-                if (a_id == 0) {
-                    if (g == 0 && t <= n) v = 0.f;
-                } else if (g == 1 && 2 * a_id < m && t < n) {
-                    v = __ldg(mat + (size_t)(2 * a_id) * T + t);
-                }
-            }
-            Cb[i] = v;
-        }
-    }
+    if (C) fill_leaf_table(C + (size_t)b * Lt * W * 3, mat, m, n, T, W, Lt, ok, ctid, cthreads);
     if (!ok) {  // uniform over the cluster: nobody reaches a cluster barrier
         if (ctid == 0) {
             flag(status, PCFGNAT_STATUS_BAD_LENGTH);
@@ -399,6 +402,194 @@ __global__ void __launch_bounds__(kCThreads, 1)
             sb[(size_t)a * T + t] = own0[r * W + t];
             if (a >= 3) sb[(size_t)(a - 1) * T + t] = own1[r * W + t];
         }
+    }
+    if (loss && ctid == 0) loss[b] = (n >= 2) ? col[0] : Sb[0];
+}
+
+// ---------------------------------------------------------------------------------------
+// inside pass, reference order, G lanes per node
+// ---------------------------------------------------------------------------------------
+// The table of inside_cluster_kernel<0> bit for bit, for shapes whose terms fit shared memory beside the links.  With a
+// warp per node the kernel is bound by instruction issue (70 % of the cycles), and most of what it issues is not terms:
+// a node's fixed costs (emissions, the maximum, the 16 ordered shuffles per 32 children, logarithm, sending) are paid
+// by a whole warp, and the last trip of a node is mostly empty lanes.  Here G = 16 or 8 lanes take a node's children
+// c = a + q + G i, so that those costs are paid for 32 / G nodes at once; rows are staged with -inf where there is no
+// child (and for the first node's leaf), so that no term is tested; the exponentials go to the node's scratch in the
+// order in which the reference adds them, and four lanes per node, one per virtual lane x, add them up from 16-byte
+// loads.  Scratch of a node: xs floats per virtual lane, 8 modulo 32, nodes 4 xs + 4 apart: conflict-free both ways.
+// 64 sentences, M = 128, T = 76: 192 us (267 us with a warp per node); 90 sentences, M <= 80: 82 us (112 us).
+template <int G>
+__device__ __forceinline__ bool inside_exact_steps(float *col, const float *lk0, const float *lk1, const float *em0,
+                                                   const float *eml, float *own, float *scratch, uint64_t *col_bar, int n,
+                                                   int Mb, int my_rows, int NC, int crank, int W, int cs, int lk_stride,
+                                                   int xs, int active) {
+    constexpr int R = 32 / G, H = G / 4;  // nodes per warp; lanes per virtual lane
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int q = lane % G, sub = lane / G, x = q & 3;
+    float *node_scratch = scratch + (size_t)(warp * R + sub) * (4 * xs + 4) + x * xs;
+    float2 *cells = reinterpret_cast<float2 *>(node_scratch) + (q >> 2);
+    const float4 *terms = reinterpret_cast<const float4 *>(node_scratch);
+    uint32_t rcol = 0, rbar0 = 0, rbar1 = 0;  // lane q < NC: this CTA's columns and barriers as CTA q maps them
+    if (NC > 1 && q < NC) {
+        rcol = dsm_map_to_cta(dsm_smem_u32(col), q);
+        rbar0 = dsm_map_to_cta(dsm_smem_u32(&col_bar[0]), q);
+        rbar1 = dsm_map_to_cta(dsm_smem_u32(&col_bar[1]), q);
+    }
+    bool arrived = true;
+    for (int start = n - 2; start >= 0; start--) {
+        const float *S1 = col + ((start + 1) & 3) * cs, *S2 = col + ((start + 2) & 3) * cs;
+        float *S0 = col + (start & 3) * cs;
+        const uint32_t bar = dsm_smem_u32(&col_bar[start & 1]);
+        if (NC > 1 && tid == 0)  // this CTA expects the whole column of this step: one value per node of the chain
+            asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(4 * Mb)
+                         : "memory");
+        for (int first = warp * R; warp < active && first < my_rows; first += active * R) {  // warp-uniform
+            const bool live = first + sub < my_rows;
+            const int r = live ? first + sub : first, ai = crank + NC * r;
+            const int trips = (Mb - (crank + NC * first) + G - 1) / G;  // of the warp's first node, which has most children
+            const float ma0 = em0[r * W + start], ma1 = em0[r * W + start + 1], ml = eml[r * W + start];
+            const float *r0 = lk0 + r * lk_stride + ai + q, *r1 = lk1 + r * lk_stride + ai + q;
+            const float *s1 = S1 + ai + q, *s2 = S2 + ai + q;
+            float mx = neg_inf();
+#pragma unroll 4
+            for (int i = 0; i < trips; i++) {  // fmaxf: NaN counts as -inf, like an absent child
+                const float a = fmaxf((r0[G * i] + s1[G * i]) + ma0, neg_inf());
+                const float b = fmaxf(((r1[G * i] + s2[G * i]) + ml) + ma1, neg_inf());
+                mx = fmaxf(mx, fmaxf(a, b));
+                cells[H * i] = make_float2(a, b);
+            }
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll 4
+            for (int i = 0; i < trips; i++) {  // not looked at where mx is infinite
+                const float2 v = cells[H * i];
+                cells[H * i] = make_float2(expf(v.x - mx), expf(v.y - mx));
+            }
+            __syncwarp();
+            float sum = 0.f;
+            if (q < 4) {
+#pragma unroll 4
+                for (int i = 0; i < trips * H / 2; i++) {  // children k = 2 i, 2 i + 1 of this virtual lane, t0 before t1
+                    const float4 e = terms[i];
+                    sum += e.x;
+                    sum += e.y;
+                    sum += e.z;
+                    sum += e.w;
+                }
+            }
+            __syncwarp();
+            sum += __shfl_down_sync(0xffffffffu, sum, 2, 4);  // (s0 + s2) + (s1 + s3)
+            sum += __shfl_down_sync(0xffffffffu, sum, 1, 4);
+            sum = __shfl_sync(0xffffffffu, sum, 0, G);
+            const float res = isinf(mx) ? mx : logf(sum) + mx;
+            if (live) {
+                if (NC > 1) {
+                    if (q < NC) dsm_store_async(rcol + 4u * ((start & 3) * cs + ai), res, (start & 1) ? rbar1 : rbar0);
+                } else if (q == 0) {
+                    S0[ai] = res;
+                }
+                if (q == 0) own[r * W + start] = res;
+            }
+        }
+        // one warp waits for the column on the byte-counting barrier, the block barrier releases the others
+        if (NC > 1 && warp == kCWarps - 1) arrived = dsm_wait_column(bar, (((n - 2) - start) >> 1) & 1) && arrived;
+        __syncthreads();
+    }
+    return arrived;
+}
+
+template <int G>
+__global__ void __launch_bounds__(kCThreads, 1)
+    inside_exact_kernel(const float *__restrict__ match_all, const float *__restrict__ links,
+                        const int64_t *__restrict__ ol, const int64_t *__restrict__ tl, int L, int T, float *S, float *C,
+                        float *loss, int *status, int Mc, int Lt, int cs, int rows_cap, int lk_stride, int B, int wide,
+                        int xs, int active) {
+    extern __shared__ __align__(16) float smem[];
+    cg::cluster_group cluster = cg::this_cluster();
+    int crank = (int)cluster.block_rank();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int NC = (int)cluster.num_blocks(), b = blockIdx.x / NC;
+    if (wide >= 0) {  // sentences by decreasing cost, as in inside_cluster_kernel
+        __shared__ int s_b;
+        const int want = b < wide ? b : wide + 2 * (b - wide) + crank;
+        if (want >= B) return;
+        if (b >= wide) {
+            NC = 1;
+            crank = 0;
+        }
+        int *cost = reinterpret_cast<int *>(smem);  // [B], before the columns move in
+        for (int i = tid; i < B; i += kCThreads) {
+            const long long mi = ol[i], ni = tl[i];
+            cost[i] = lengths_ok((int)mi, (int)ni, L, T) ? (int)(mi * ni) : 0;
+        }
+        __syncthreads();
+        for (int i = tid; i < B; i += kCThreads) {
+            const int ci = cost[i];
+            int before = 0;
+            for (int j = 0; j < B; j++) before += cost[j] > ci || (cost[j] == ci && j < i);
+            if (before == want) s_b = i;
+        }
+        __syncthreads();
+        b = s_b;
+    }
+    const int ctid = crank * kCThreads + tid, cthreads = NC * kCThreads;
+    const int W = T + 2;
+    const int m = (int)ol[b], n = (int)tl[b];
+    const bool ok = lengths_ok(m, n, L, T);
+    const float *mat = match_all + (size_t)b * L * T;
+    const float *lkb = links + (size_t)b * L * 2 * L;
+    float *Sb = S + (size_t)b * Mc * W;
+    for (int i = ctid; i < Mc * W; i += cthreads) Sb[i] = neg_inf();
+    if (C) fill_leaf_table(C + (size_t)b * Lt * W * 3, mat, m, n, T, W, Lt, ok, ctid, cthreads);
+    if (!ok) {  // uniform over the cluster: nobody reaches a cluster barrier
+        if (ctid == 0) {
+            flag(status, PCFGNAT_STATUS_BAD_LENGTH);
+            if (loss) loss[b] = neg_inf();
+        }
+        return;
+    }
+    const int Mb = main_nodes_below(m), last = (m - 2) / 2;
+    const int my_rows = Mb > crank ? (Mb - crank + NC - 1) / NC : 0;  // nodes ai = crank + NC * r
+    float *col = smem;                                // [4][cs] rolling columns of the whole chain
+    float *lk0 = col + 4 * cs;                        // [rows_cap][lk_stride] links[a][0][c] by child slot, -inf from Mb on
+    float *lk1 = lk0 + (size_t)rows_cap * lk_stride;  // the same for k = 1; -inf for the first node
+    float *own = lk1 + (size_t)rows_cap * lk_stride;  // [rows_cap][W] each: table, emissions, emissions of the leaves
+    float *em0 = own + (size_t)rows_cap * W, *eml = em0 + (size_t)rows_cap * W;
+    float *scratch = smem + ((eml + (size_t)rows_cap * W - smem + 3) & ~(ptrdiff_t)3);
+    for (int i = tid; i < my_rows * W; i += kCThreads) {
+        const int r = i / W, t = i - r * W, a = 2 * (crank + NC * r) + 1;
+        em0[i] = t < T ? __ldg(mat + (size_t)a * T + t) : 0.f;
+        eml[i] = t < T && a >= 3 ? __ldg(mat + (size_t)(a - 1) * T + t) : 0.f;
+    }
+    for (int r = warp; r < my_rows; r += kCWarps) {
+        const int ai = crank + NC * r;
+        const float *row = lkb + (size_t)(2 * ai + 1) * 2 * L;
+#pragma unroll 4
+        for (int ci = ai + lane; ci < lk_stride; ci += 32) {
+            lk0[r * lk_stride + ci] = ci < Mb ? __ldg(row + 2 * ci + 1) : neg_inf();
+            lk1[r * lk_stride + ci] = ci < Mb && ai > 0 ? __ldg(row + L + 2 * ci + 1) : neg_inf();
+        }
+    }
+    __shared__ __align__(8) uint64_t col_bar[2];
+    for (int i = tid; i < 4 * cs; i += kCThreads) col[i] = neg_inf();
+    if (tid == 0) {
+        for (int i = 0; i < 2; i++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(dsm_smem_u32(&col_bar[i])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (tid == 0) col[((n - 1) & 3) * cs + last] = __ldg(mat + (size_t)(m - 1) * T + (n - 1));  // every CTA its own copy
+    // all copies initialised before anybody stores into a neighbour's; also orders the -inf fill of the global table
+    if (NC > 1) cluster.sync(); else __syncthreads();
+    if (ctid == 0) Sb[(size_t)last * W + (n - 1)] = __ldg(mat + (size_t)(m - 1) * T + (n - 1));
+    const bool arrived = inside_exact_steps<G>(col, lk0, lk1, em0, eml, own, scratch, col_bar, n, Mb, my_rows, NC, crank, W,
+                                               cs, lk_stride, xs, active);
+    if (!arrived && lane == 0) flag(status, PCFGNAT_STATUS_TIMEOUT);
+    // no CTA leaves (its shared memory with it) while a peer may still send to it; every wait above is bounded
+    if (NC > 1) cluster.sync();
+    for (int i = tid; i < my_rows * (n - 1); i += kCThreads) {  // computed cells: columns 0 .. n-2
+        const int r = i / (n - 1), t = i - r * (n - 1);
+        Sb[(size_t)(crank + NC * r) * W + t] = own[r * W + t];
     }
     if (loss && ctid == 0) loss[b] = (n >= 2) ? col[0] : Sb[0];
 }
@@ -749,8 +940,48 @@ int launch_inside(const float *match_all, const float *links, const int64_t *ol,
     return PCFGNAT_ERR_UNSUPPORTED;
 }
 
+// Reference order with G lanes per node; PCFGNAT_ERR_UNSUPPORTED when the terms do not fit beside the links.
+template <int G>
+int launch_exact(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B, int L, int T,
+                 float *S, float *C, float *loss, int *status, cudaStream_t st, int nc, int wide, bool mixed) {
+    constexpr int R = 32 / G;
+    const int Mc = main_slots(L, 1), Lt = L - Mc, W = T + 2, cs = (Mc + 3) / 4 * 4;
+    const int width = mixed ? 2 : nc;  // CTAs of a cluster
+    const int rows_cap = (Mc + nc - 1) / nc;
+    // a row is read up to G - 1 children past its last one, by the warp's later nodes up to (R - 1) nc more; the rows of a
+    // warp's nodes G banks apart
+    const int pad = G + (R - 1) * width, lk_stride = (Mc + pad + width - G + 31) / 32 * 32 + G - width;
+    const int xs = ((Mc + G - 1) / G * (G / 2) + 23) / 32 * 32 + 8;
+    const size_t base = (((size_t)4 * cs + (size_t)2 * rows_cap * lk_stride + (size_t)3 * rows_cap * W) * sizeof(float) + 15) &
+                        ~(size_t)15;
+    const size_t limit = (size_t)kSmemLimit - 1024, per_warp = (size_t)R * (4 * xs + 4) * sizeof(float);
+    if (base >= limit) return PCFGNAT_ERR_UNSUPPORTED;
+    int active = (rows_cap + R - 1) / R;
+    if (active > kCWarps) active = kCWarps;
+    if ((size_t)active * per_warp > limit - base) active = (int)((limit - base) / per_warp);
+    if (active < 8 && active * R < rows_cap) return PCFGNAT_ERR_UNSUPPORTED;
+    size_t smem = base + active * per_warp;
+    if (wide >= 0 && smem < (size_t)B * sizeof(int)) smem = (size_t)B * sizeof(int);  // the costs that rank the sentences
+    const int clusters = mixed ? wide + (B - wide + 1) / 2 : B;
+    return launch_cluster(inside_exact_kernel<G>, clusters, width, smem, st, match_all, links, ol, tl, L, T, S, C, loss, status,
+                          Mc, Lt, cs, rows_cap, lk_stride, B, wide, xs, active);
+}
+
 int launch_loss_fwd_cluster(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B,
                             int L, int T, float *S, float *C, float *loss, int *status, cudaStream_t st) {
+    const int Mc = main_slots(L, 1);
+    const ClusterGeometry g = cluster_geometry(B, Mc, T + 2);
+    if (g.nc >= 1 && g.nc <= 8) {
+        const int wide = g.nc == 1 ? mixed_width_count(B, Mc) : 0;
+        const int order = wide > 0 ? wide : (long long)B * g.nc > sm_count() && B <= 256 ? B : -1;
+        // sixteen lanes while a CTA's nodes take one pass of 32 warps (a sentence of the mixed widths that has one CTA
+        // is among the cheap ones); eight for more nodes
+        const int rows = (Mc + g.nc - 1) / g.nc;
+        const bool sixteen = rows <= 64 || (wide > 0 && rows <= 96);
+        const int rc = sixteen ? launch_exact<16>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, g.nc, order, wide > 0)
+                               : launch_exact<8>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, g.nc, order, wide > 0);
+        if (rc != PCFGNAT_ERR_UNSUPPORTED) return rc;
+    }
     return launch_inside<0>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st);
 }
 

@@ -957,6 +957,34 @@ def test_copy_links_main_rows(ops, L):
         assert (dst[:, 0::2] == -7.0).all()  # rows no kernel reads keep their contents
 
 
+@pytest.mark.parametrize("B, L, T", [(1, 4, 2), (3, 34, 9), (2, 66, 20), (70, 64, 16), (74, 130, 12), (90, 160, 48),
+                                     (80, 262, 20), (150, 96, 11), (8, 514, 100), (5, 640, 30)])
+def test_reference_order_table_edges(ops, monkeypatch, B, L, T):
+    """The inside table in the reference's order, bit for bit that of the 4-lanes-per-node kernel, at chain lengths
+    around the lanes, passes and cluster widths of the kernels that the library picks: one sentence and more than the
+    GPU has SMs, cost-ordered shared clusters, odd graph lengths, infinite and NaN entries, a length out of range."""
+    monkeypatch.delenv("PCFGNAT_DP_KERNEL", raising=False)
+    monkeypatch.delenv("PCFGNAT_DP_CLUSTER_SIZE", raising=False)
+    g = torch.Generator(DEV).manual_seed(L + B)
+    match = torch.randn(B, L, T, device=DEV, generator=g) * 3 - 4
+    links = torch.randn(B, L, 2, L, device=DEV, generator=g) * 2 - 5
+    match[0, 1, 0], links[0, 1, 0, min(3, L - 1)] = float("-inf"), float("nan")
+    links[B // 2, 1:3] = float("-inf")
+    ol = torch.randint(2, L + 1, (B,), device=DEV, generator=g)
+    tl = torch.randint(1, T + 1, (B,), device=DEV, generator=g)
+    ol[-1], tl[-1] = L, T
+    if B > 2:
+        ol[1] = L + 1
+    k = ops.get_pcfg_kernel()
+    S, C = k.pcfg_loss(match, links, ol, tl, 1)
+    monkeypatch.setenv("PCFGNAT_DP_KERNEL", "rows")
+    S_rows, C_rows = k.pcfg_loss(match, links, ol, tl, 1)
+    assert np.array_equal(_bits(S.cpu().numpy()), _bits(S_rows.cpu().numpy()))
+    assert np.array_equal(_bits(C.cpu().numpy()), _bits(C_rows.cpu().numpy()))
+    assert torch.isfinite(S).any()
+    ops.read_status(DEV)
+
+
 def test_loss_stats_and_glance_select(ops):
     k = ops.get_pcfg_kernel()
     g = torch.Generator().manual_seed(11)
