@@ -350,6 +350,13 @@ int pcfgnat_links_from_scores(const float *ac, const float *bc, const float *qm,
  * callers that stage batches from host memory: it halves the bytes the largest input sends over PCIe. */
 int pcfgnat_copy_links_main_rows(void *dst, const void *src, int B, int L, int max_left, void *stream);
 
+/* Copies n (at most 16) device tensors in one launch: dst[i] <- src[i], bytes[i] each; with odd_rows[i] > 0 only the
+ * rows 1, 3, 5, ... of that many bytes (links [B][L][2][L] with an even L: its main-chain rows, 8 L bytes each).  All
+ * four arrays are HOST arrays, read before the call returns.  PCFGNAT_ERR_UNSUPPORTED, with nothing copied, when a
+ * destination overlaps another tensor of the call: such copies need an order. */
+int pcfgnat_copy_batch(int n, void *const *dst, const void *const *src, const size_t *bytes, const size_t *odd_rows,
+                       void *stream);
+
 /* Copies the rows of the real graph nodes of sentences [b0, b1) from src to dst, both [B][L][row_bytes]:
  * rows l < m_b with m_b = host_lengths[b] clamped to [0, L]; one cudaMemcpyAsync per run of adjacent rows on
  * `stream`, through the copy engine, no kernel.  A copy costs the host several microseconds, so with max_copies > 0

@@ -9,6 +9,8 @@ _lib = None
 
 c_int, c_i64, c_size, c_void = ctypes.c_int, ctypes.c_int64, ctypes.c_size_t, ctypes.c_void_p
 
+ERR_INVALID_ARGUMENT, ERR_UNSUPPORTED = -1, -2  # PCFGNAT_ERR_*
+
 # name -> (restype, argtypes); must list every symbol include/pcfgnat.h declares
 SIGNATURES = {
     "pcfgnat_version": (c_int, []),
@@ -37,6 +39,7 @@ SIGNATURES = {
     "pcfgnat_links_backward": (c_int, [c_void] * 13 + [c_int] * 6 + [c_void] * 8),
     "pcfgnat_links_from_scores": (c_int, [c_void] * 11 + [c_int] * 6 + [c_void] * 2),
     "pcfgnat_copy_links_main_rows": (c_int, [c_void] * 2 + [c_int] * 3 + [c_void]),
+    "pcfgnat_copy_batch": (c_int, [c_int] + [c_void] * 5),
     "pcfgnat_plan_real_rows": (c_int, [c_void] + [c_int] * 4 + [c_void] + [c_int]),
     "pcfgnat_copy_real_rows": (c_int, [c_void] * 3 + [c_int] * 3 + [c_size] + [c_int] + [c_void] * 2),
     "pcfgnat_stage_inputs": (c_int, [c_void] * 2 + [c_int] + [c_void] * 3 + [c_int] * 3 + [c_void]),

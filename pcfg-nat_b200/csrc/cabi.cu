@@ -434,6 +434,24 @@ int pcfgnat_copy_links_main_rows(void *dst, const void *src, int B, int L, int m
     return PCFGNAT_OK;
 }
 
+int pcfgnat_copy_batch(int n, void *const *dst, const void *const *src, const size_t *bytes, const size_t *odd_rows,
+                       void *stream) {
+    PCFGNAT_API_RANGE();
+    if (n < 0 || n > kBatchTensors || (n && (!dst || !src || !bytes || !odd_rows))) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    for (int i = 0; i < n; i++)
+        if (bytes[i] && (!dst[i] || !src[i])) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    const auto overlap = [](const void *a, size_t na, const void *b, size_t nb) {
+        const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+        return x < y + nb && y < x + na;
+    };
+    for (int i = 0; i < n; i++)
+        for (int j = 0; j < n; j++)  // one launch has no order: nothing it writes may be read or written again by it
+            if ((overlap(dst[i], bytes[i], src[j], bytes[j]) && !(i == j && dst[i] == src[i])) ||
+                (i != j && overlap(dst[i], bytes[i], dst[j], bytes[j])))
+                return PCFGNAT_ERR_UNSUPPORTED;
+    return launch_copy_batch(n, dst, src, bytes, odd_rows, static_cast<cudaStream_t>(stream));
+}
+
 int pcfgnat_plan_real_rows(const int64_t *host_lengths, int b0, int b1, int L, int max_copies, int64_t *runs,
                            int capacity) {
     if (b0 < 0 || b1 < b0 || L < 1 || max_copies < 0 || capacity < 0) return PCFGNAT_ERR_INVALID_ARGUMENT;

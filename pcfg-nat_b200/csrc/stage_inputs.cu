@@ -52,6 +52,52 @@ __global__ void __launch_bounds__(kStageThreads)
     }
 }
 
+// Several device tensors copied in one launch: the inputs of a batch into a step's buffers.  One copy call each costs
+// 2 us of device time for the smallest and the 2 us between two of them, and the strided copy of the main-chain rows
+// of the transitions runs at a fifth of the memory's rate.  A block moves 256 x 4 pieces of one tensor, 16 bytes each
+// where both addresses allow it, all four in flight.  Five inputs of 90 sentences, graph 160: 10 us, 38 us as copies;
+// of two sentences: 2 us, 23 us.
+constexpr int kBatchThreads = 256, kBatchPieces = 4;
+
+struct BatchCopy {
+    struct Tensor {
+        const char *src;
+        char *dst;
+        unsigned pieces;      // of `unit` bytes
+        unsigned unit;        // 16, 4 or 1
+        unsigned row_pieces;  // > 0: rows 1, 3, 5, ... of this many pieces; 0: everything
+        unsigned block0;      // first block of this tensor
+    } t[kBatchTensors];
+    int n;
+};
+
+template <class Unit>
+__device__ __forceinline__ void copy_pieces(const BatchCopy::Tensor &t, unsigned first) {
+    const Unit *src = reinterpret_cast<const Unit *>(t.src);
+    Unit *dst = reinterpret_cast<Unit *>(t.dst);
+    Unit v[kBatchPieces];
+    size_t at[kBatchPieces];
+#pragma unroll
+    for (int j = 0; j < kBatchPieces; j++) {
+        const unsigned i = first + j * kBatchThreads;
+        at[j] = t.row_pieces ? i + (size_t)(i / t.row_pieces + 1) * t.row_pieces : i;
+        if (i < t.pieces) v[j] = src[at[j]];
+    }
+#pragma unroll
+    for (int j = 0; j < kBatchPieces; j++)
+        if (first + j * kBatchThreads < t.pieces) dst[at[j]] = v[j];
+}
+
+__global__ void __launch_bounds__(kBatchThreads) copy_batch_kernel(const __grid_constant__ BatchCopy copy) {
+    int k = 0;
+    while (k + 1 < copy.n && blockIdx.x >= copy.t[k + 1].block0) k++;
+    const BatchCopy::Tensor &t = copy.t[k];
+    const unsigned first = (blockIdx.x - t.block0) * (kBatchThreads * kBatchPieces) + threadIdx.x;
+    if (t.unit == 16) copy_pieces<uint4>(t, first);
+    else if (t.unit == 4) copy_pieces<uint32_t>(t, first);
+    else copy_pieces<uint8_t>(t, first);
+}
+
 }  // namespace
 
 int launch_stage_inputs(const void *hidden_src, void *hidden_dst, int row_bytes, const float *links_src, float *links_dst,
@@ -60,6 +106,29 @@ int launch_stage_inputs(const void *hidden_src, void *hidden_dst, int row_bytes,
     // few CTAs: the kernel waits on the bus, not on the SMs, and shares them with whatever else runs
     stage_inputs_kernel<<<48, kStageThreads, 0, st>>>(static_cast<const uint4 *>(hidden_src), static_cast<uint4 *>(hidden_dst),
                                                       row_bytes / 16, links_src, links_dst, ol, B, L);
+    return cuda_rc(cudaGetLastError());
+}
+
+int launch_copy_batch(int n, void *const *dst, const void *const *src, const size_t *bytes, const size_t *odd_rows,
+                      cudaStream_t st) {
+    BatchCopy c = {};
+    unsigned long long blocks = 0;
+    for (int i = 0; i < n; i++) {
+        if (bytes[i] == 0 || dst[i] == src[i]) continue;
+        const uintptr_t all = reinterpret_cast<uintptr_t>(dst[i]) | reinterpret_cast<uintptr_t>(src[i]) | bytes[i] | odd_rows[i];
+        BatchCopy::Tensor &t = c.t[c.n++];
+        t.unit = all % 16 == 0 ? 16 : all % 4 == 0 ? 4 : 1;
+        t.src = static_cast<const char *>(src[i]);
+        t.dst = static_cast<char *>(dst[i]);
+        t.row_pieces = (unsigned)(odd_rows[i] / t.unit);
+        const size_t pieces = (odd_rows[i] ? bytes[i] / odd_rows[i] / 2 * odd_rows[i] : bytes[i]) / t.unit;
+        if (pieces > INT32_MAX || (t.unit < 16 && bytes[i] > (1 << 20))) return PCFGNAT_ERR_UNSUPPORTED;  // copies do better
+        t.pieces = (unsigned)pieces;
+        t.block0 = (unsigned)blocks;
+        blocks += (t.pieces + kBatchThreads * kBatchPieces - 1) / (kBatchThreads * kBatchPieces);
+    }
+    if (blocks == 0) return PCFGNAT_OK;
+    copy_batch_kernel<<<(unsigned)blocks, kBatchThreads, 0, st>>>(c);
     return cuda_rc(cudaGetLastError());
 }
 

@@ -543,6 +543,25 @@ class _Kernel:
         _cabi.check(rc, "pcfgnat_copy_links_main_rows")
 
     @staticmethod
+    def copy_batch(pairs, odd_rows_of=None):
+        """Copies every (dst, src) pair of contiguous CUDA tensors of one device, same shape and type, in one launch on
+        the current stream; of the pair whose dst is ``odd_rows_of`` (transitions [B, L, 2, L], L even) only the
+        main-chain rows.  False, with nothing copied, when the pairs overlap one another or are too many."""
+        n = len(pairs)
+        if n == 0:
+            return True
+        dst, src = ((ctypes.c_void_p * n)(*(p[i].data_ptr() for p in pairs)) for i in range(2))
+        size = (ctypes.c_size_t * n)(*(d.numel() * d.element_size() for d, _ in pairs))
+        rows = (ctypes.c_size_t * n)(*(8 * d.shape[1] if d is odd_rows_of else 0 for d, _ in pairs))
+        dev = pairs[0][0].device
+        with torch.cuda.device(dev):
+            rc = _cabi.lib().pcfgnat_copy_batch(n, dst, src, size, rows, _stream(dev))
+        if rc in (_cabi.ERR_UNSUPPORTED, _cabi.ERR_INVALID_ARGUMENT):
+            return False
+        _cabi.check(rc, "pcfgnat_copy_batch")
+        return True
+
+    @staticmethod
     def copy_real_rows(dst, src, host_lengths, b0=0, b1=None, max_copies=0):
         """Copies the rows of the real graph nodes (l < length, clamped to [0, L]) of sentences [b0, b1) of ``src``
         [B, L, ...] into ``dst`` of the same shape on the current stream with copy-engine copies, no kernel: one per

@@ -133,8 +133,16 @@ class _GraphedStep:
         if len(tensors) != len(bufs):
             raise RuntimeError(f"expected {len(bufs)} tensors")
         if not overlap:
+            # what is on the device already goes in one launch; the rest (host memory, other types or layouts) by copies
+            here = [(dst, src) for dst, src in zip(bufs, tensors)
+                    if src.device == dst.device and src.dtype == dst.dtype and src.shape == dst.shape and src.is_contiguous()
+                    and not (dst is self.links and dst.shape[1] % 2)]
+            if len(here) < 2 or not self.kernel.copy_batch(here, odd_rows_of=self.links):
+                here = []
+            done = {id(dst) for dst, _ in here}
             for dst, src in zip(bufs, tensors):
-                self._copy_in(dst, src)
+                if id(dst) not in done:
+                    self._copy_in(dst, src)
             return
         if self.copy_stream is None:
             self.copy_stream = torch.cuda.Stream(self.device)

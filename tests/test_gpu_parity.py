@@ -985,6 +985,53 @@ def test_reference_order_table_edges(ops, monkeypatch, B, L, T):
     ops.read_status(DEV)
 
 
+def test_copy_batch(ops):
+    """Tensors of one byte to several blocks, at and off 16- and 4-byte boundaries, the main-chain rows of transitions,
+    empty and self copies; overlapping pairs and more pairs than a launch takes are refused with nothing copied."""
+    k = ops.get_pcfg_kernel()
+    g = torch.Generator(DEV).manual_seed(1)
+    pool = torch.randint(0, 256, (1 << 22,), device=DEV, generator=g).to(torch.uint8)
+    pairs, at = [], 0
+    for size, off in ((1, 0), (15, 0), (4096, 0), (16384 + 16, 0), (100000, 4), (70001, 1), (360, 8), (0, 0), (1 << 20, 0)):
+        at = (at + 31) // 16 * 16 + off
+        src = pool[at:at + size]
+        pairs.append((torch.zeros(size + 16, dtype=torch.uint8, device=DEV)[off:off + size], src))
+        at += size
+    links = torch.randn(3, 10, 2, 10, device=DEV, generator=g)
+    rows = torch.full_like(links, -7.0)
+    ids = torch.arange(5, device=DEV)
+    assert k.copy_batch(pairs + [(rows, links), (ids, ids)], odd_rows_of=rows)
+    for dst, src in pairs:
+        assert torch.equal(dst, src)
+    assert torch.equal(rows[:, 1::2], links[:, 1::2]) and (rows[:, 0::2] == -7.0).all()
+    a, b = torch.zeros(64, device=DEV), torch.ones(64, device=DEV)
+    c = b.clone()
+    assert not k.copy_batch([(a, c), (c[:32], b[32:])]) and not k.copy_batch([(a, b), (a[8:], b[8:])])
+    assert not k.copy_batch([(x, y) for x, y in zip(a.split(2), b.split(2))])
+    assert (a == 0).all() and (c == 1).all() and k.copy_batch([])
+
+
+def test_step_load_from_device_tensors(pkg, ops, syn):
+    """Inputs on the device go to a step's buffers in one launch: contiguous ones together with a host tensor, a strided
+    one and one of another type, and from the step's own buffers (copies in order)."""
+    import importlib
+
+    runtime = importlib.import_module("pcfg_nat_b200.runtime")
+    b = syn.make_batch(syn.Workload("dl", batch=3, vocab=300, hidden=64, src_min=4, src_max=9), seed=2)
+    args = [b.hidden, b.links, b.output_length, b.targets, b.target_length]
+    step = runtime.LossStep(b.weight.to(DEV), b.B, b.L, b.T, DEV)
+    step.load(*args)
+    want = [t.cpu() for t in step.run()]
+    dev = [t.to(DEV) for t in args]
+    strided = torch.stack([dev[0], dev[0]], -1)[..., 0]
+    for tensors in (dev, [strided, dev[1], args[2], dev[3].int(), dev[4]],
+                    [step.hidden, step.links, step.output_length, step.targets, step.target_length]):
+        step.load(*tensors)
+        for got, ref in zip(step.run(), want):
+            assert torch.equal(got.cpu(), ref)
+    assert torch.isinf(step.links[:, 0::2]).all()
+
+
 def test_loss_stats_and_glance_select(ops):
     k = ops.get_pcfg_kernel()
     g = torch.Generator().manual_seed(11)
