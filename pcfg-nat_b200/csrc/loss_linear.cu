@@ -37,9 +37,12 @@
 // target token, out of range), the sentence is marked and recomputed by the log-space kernels in the same call
 // (loss_fwd.cu / loss_bwd.cu, which skip unmarked sentences).
 //
-// Layout: G = 8 or 16 lanes per node (a lane covers groups of four consecutive children, its part of the node's
-// matrix rows in registers), one thread-block CLUSTER per sentence, nodes dealt round-robin to the CTAs; the
-// columns are exchanged with st.async counted on alternating mbarriers exactly as in loss_cluster.cu.  Batches
+// Layout: a warp takes a BLOCK of four consecutive nodes, a lane its groups of four consecutive children for all of them
+// (its part of the nodes' matrix rows in registers); one thread-block CLUSTER per sentence, blocks dealt round-robin to
+// the CTAs; the columns are exchanged with st.async counted on alternating mbarriers as in loss_cluster.cu, a block's
+// four values in one 16-byte message per CTA where there are three CTAs and more.  Inside and outside kernel, 90
+// sentences of at most 80 nodes: 36 + 44 us, 8 sentences of 256: 111 + 152 us (43 + 50 and 165 + 216 us with eight or
+// sixteen lanes per node, a test before every load of a column, and a message per node).  Batches
 // between half and all of the SMs run clusters of two, which the costliest sentences have to themselves and the
 // others share, one CTA per sentence (pick_sentence).
 #include <cooperative_groups.h>
@@ -76,6 +79,7 @@ namespace {
 
 constexpr int kLThreads = 512;
 constexpr int kLWarps = kLThreads / 32;
+constexpr int R = 4;                               // consecutive nodes of a warp: a block
 constexpr int kMaxMixedBatch = 256;                // mixed cluster widths only up to this many sentences (mixed_width_count)
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
@@ -191,6 +195,35 @@ __device__ __forceinline__ void token_maxima(const float *__restrict__ mat, int 
     }
 }
 
+// Node r of CTA `crank` of NC: blocks of R nodes are dealt round-robin.  Rows of the last block may lie past the chain.
+__device__ __forceinline__ int node_of(int r, int crank, int NC) { return (crank + NC * (r / R)) * R + r % R; }
+
+// Four floats to 16-byte aligned shared memory of a CTA of the cluster, counted on a barrier of that CTA.
+__device__ __forceinline__ void store_async4(uint32_t cluster_addr, const float4 &v, uint32_t cluster_bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(cluster_addr),
+                 "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)),
+                 "r"(cluster_bar)
+                 : "memory");
+}
+// A block's values, node j's in lane j * LANES.
+template <int LANES>
+__device__ __forceinline__ float4 block_values(float v) {
+    return make_float4(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, LANES),
+                       __shfl_sync(0xffffffffu, v, 2 * LANES), __shfl_sync(0xffffffffu, v, 3 * LANES));
+}
+// One round of a sum over the warp that also deals out the N values: lanes with bit `BIT` keep the upper half of them.
+template <int N, int BIT>
+__device__ __forceinline__ void halve(float (&v)[N]) {
+    const bool upper = threadIdx.x & BIT;
+#pragma unroll
+    for (int j = 0; j < N / 2; j++) {
+        const float send = upper ? v[j] : v[j + N / 2], keep = upper ? v[j + N / 2] : v[j];
+        v[j] = keep + __shfl_xor_sync(0xffffffffu, send, BIT);
+    }
+}
+template <int N>
+__device__ __forceinline__ float (&lower(float (&v)[N]))[N / 2] { return reinterpret_cast<float (&)[N / 2]>(v); }
+
 __device__ __forceinline__ void bar_init(uint64_t *bars, int count) {
     for (int i = 0; i < count; i++)
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(dsm_smem_u32(&bars[i])) : "memory");
@@ -207,7 +240,7 @@ __device__ __forceinline__ void bar_expect(uint32_t bar, int bytes) {
 // frames [B][F], F = kLinearFrameHead + W:  [0] u_0[root]  [1] log Z  [2] emission-gradient mass (outside pass)
 //                     [3] != 0: an input overflowed  [4 + t] inv_t
 // shares [B][L][T]    (the match_all_grad buffer) p0_t[a] in cell [a][t], p1_t[a] in cell [a-1][t], t <= n-2
-template <int G, int TRIPS>
+template <int CHUNKS>
 __global__ void __launch_bounds__(kLThreads, 1)
     inside_linear_kernel(const float *__restrict__ match_all, const float *__restrict__ links,
                          const int64_t *__restrict__ ol, const int64_t *__restrict__ tl, int L, int T, float *Y,
@@ -244,13 +277,15 @@ __global__ void __launch_bounds__(kLThreads, 1)
     PCFGNAT_STAMP(0, 1)
     const float *mat = match_all + (size_t)b * L * T;
     const float *lkb = links + (size_t)b * L * 2 * L;
-    const int Mb = m / 2, last = (m - 2) / 2;
-    const int my_rows = Mb > crank ? (Mb - crank + NC - 1) / NC : 0;  // nodes ai = crank + NC * r
-    float *col = smem;                          // [4][cs] rolling columns of the whole chain (every CTA has a copy)
-    float *P0 = col + 4 * cs;                   // [rows_cap][cs] exp(links[a][0][c]) of this CTA's nodes, 0 for c <= a
+    const int Mb = m / 2, last = (m - 2) / 2, blocks = (Mb + R - 1) / R;
+    const int groups = blocks > crank ? (blocks - crank + NC - 1) / NC : 0, my_rows = groups * R;  // nodes node_of(r)
+    // Columns are a whole number of the lanes' trips long (zero past the chain), so that the loads of a step need no
+    // test: with one per trip they came out one behind the other, 60 to 80 cycles each.
+    constexpr int TRIPS = (CHUNKS + 3) / 4, cp = 128 * TRIPS;
+    float *col = smem;                          // [4][cp] rolling columns of the whole chain (every CTA has a copy)
+    float *P0 = col + 4 * cp;                   // [rows_cap][cs] exp(links[a][0][c]) of this CTA's nodes, 0 for c <= a
     float *P1 = P0 + (size_t)rows_cap * cs;
-    float *ownu = P1 + (size_t)rows_cap * cs;   // [rows_cap][W] u_t of this CTA's nodes
-    float *own0 = ownu + (size_t)rows_cap * W;  // its two halves
+    float *own0 = P1 + (size_t)rows_cap * cs;   // [rows_cap][W] the two halves of u_t of this CTA's nodes
     float *own1 = own0 + (size_t)rows_cap * W;
     float *e0 = own1 + (size_t)rows_cap * W;    // [rows_cap][W] E0, E1
     float *e1 = e0 + (size_t)rows_cap * W;
@@ -269,9 +304,9 @@ __global__ void __launch_bounds__(kLThreads, 1)
     __syncthreads();
     bool big = false;
     for (int i = tid; i < my_rows * W; i += kLThreads) {
-        const int r = i / W, t = i - r * W, a = 2 * (crank + NC * r) + 1;
+        const int r = i / W, t = i - r * W, ai = node_of(r, crank, NC), a = 2 * ai + 1;
         float v0 = 0.f, v1 = 0.f;
-        if (t < n) {
+        if (t < n && ai < Mb) {
             const float ma = __ldg(mat + (size_t)a * T + t);
             v0 = exp_clean(ma - invs[t]);
             if (a >= 3 && t + 1 < n)
@@ -281,11 +316,11 @@ __global__ void __launch_bounds__(kLThreads, 1)
         big |= !(v0 < 1e30f) || !(v1 < 1e30f);
         e0[i] = v0;
         e1[i] = v1;
-        ownu[i] = 0.f;
+        own0[i] = own1[i] = 0.f;
     }
     for (int r = warp; r < my_rows; r += kLWarps) {
-        const int ai = crank + NC * r;
-        const float *row = lkb + (size_t)(2 * ai + 1) * 2 * L;
+        const int ai = node_of(r, crank, NC);
+        const float *row = lkb + (size_t)(2 * ai + 1) * 2 * L;  // not read past the chain: no child there
 #pragma unroll 4
         for (int ci = lane; ci < cs; ci += 32) {
             float p0 = 0.f, p1 = 0.f;
@@ -299,7 +334,7 @@ __global__ void __launch_bounds__(kLThreads, 1)
         }
     }
     if (big) s_overflow = 1;
-    for (int i = tid; i < 4 * cs; i += kLThreads) col[i] = 0.f;
+    for (int i = tid; i < 4 * cp; i += kLThreads) col[i] = 0.f;
     __syncthreads();  // E0 and E1 are formed: the per-token maxima make room for the scales
     float lmx_part = 0.f;  // this thread's part of sum_t lmx[t]
     for (int i = tid; i < W; i += kLThreads) {
@@ -318,43 +353,47 @@ __global__ void __launch_bounds__(kLThreads, 1)
     __syncthreads();
     const float base = exp_clean(__ldg(mat + (size_t)(m - 1) * T + (n - 1)) - s_lmx_last);
     if (tid == 0) {
-        col[((n - 1) & 3) * cs + last] = base;  // every CTA fills its own copy
-        if (last % NC == crank) ownu[(size_t)(last / NC) * W + (n - 1)] = base;
+        col[((n - 1) & 3) * cp + last] = base;  // every CTA fills its own copy
+        if (last / R % NC == crank) own0[(size_t)(last / R / NC * R + last % R) * W + (n - 1)] = base;
     }
     PCFGNAT_STAMP(0, 2)
     if (NC > 1) cluster.sync(); else __syncthreads();
     PCFGNAT_STAMP(0, 3)
     if (s_overflow && tid == 0) fr[3] = 1.f;  // after the reset above (ordered by the barrier)
 
-    // Step loop.  G lanes share a node (lane q of them covers the groups of four children q, q + G, ...), so a warp
-    // does 32 / G nodes at once, always the same ones: their rows of P0 and P1 stay in REGISTERS for the whole loop
-    // (TRIPS float4 each per lane), and a step reads only the two columns from shared memory.  Nodes beyond what
-    // the warps can hold that way (long chains on few CTAs) take their rows from shared memory every step.
-    // The last warp does not compute nodes unless the chain is that long: it derives the scale two steps ahead
-    // from the finished column, keeps the books of the scales, and waits for the column of the step on the
-    // byte-counting barrier; the block barrier then releases the others, so nobody else spins.
-    constexpr int R = 32 / G;  // nodes per warp
+    // Step loop.  A warp does a block of R nodes at once, always the same one, lane l the groups of four children l,
+    // l + 32 of all of them: their parts of P0 and P1 stay in REGISTERS for the whole loop, and a step reads each column
+    // once per warp (with eight lanes per node every node's lanes read it: shared memory bound the step, since a
+    // 16-byte load takes four cycles whatever its lanes share).  The R x 2 partial sums are added up over the warp
+    // by exchanging halves of them, nine shuffles.  Nodes beyond what the warps can hold that way (long chains on few CTAs)
+    // take their rows from shared memory every step.  The last warp does not compute nodes unless the chain is that
+    // long: it derives the scale two steps ahead from the finished column, keeps the books of the scales, and waits for
+    // the column of the step on the byte-counting barrier; the block barrier then releases the others, so nobody else
+    // spins.
     const int cs4 = cs >> 2;
-    const int groups = (my_rows + R - 1) / R;
-    const int q = lane % G, sub = lane / G;
+    const int half = lane >> 4, sub = (lane >> 2) & 3;  // what this lane holds after the sums: half u_t of node `sub`
     const float4 *P0v = reinterpret_cast<const float4 *>(P0), *P1v = reinterpret_cast<const float4 *>(P1);
-    const int r_own = warp * R + sub;
-    const bool live_own = r_own < my_rows;
-    float4 rp0[TRIPS], rp1[TRIPS];
+    float4 rp0[R][TRIPS], rp1[R][TRIPS];
 #pragma unroll
-    for (int i = 0; i < TRIPS; i++) {
-        const int c4 = q + G * i;
-        rp0[i] = rp1[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live_own && c4 < cs4) {
-            rp0[i] = P0v[r_own * cs4 + c4];
-            rp1[i] = P1v[r_own * cs4 + c4];
+    for (int j = 0; j < R; j++)
+#pragma unroll
+        for (int i = 0; i < TRIPS; i++) {
+            const int c4 = lane + 32 * i;
+            rp0[j][i] = rp1[j][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (warp < groups && c4 < cs4) {
+                rp0[j][i] = P0v[(warp * R + j) * cs4 + c4];
+                rp1[j][i] = P1v[(warp * R + j) * cs4 + c4];
+            }
         }
-    }
-    uint32_t rcol = 0, rbar0 = 0, rbar1 = 0;  // lane q < NC: this CTA's columns and barriers as CTA q maps them
-    if (NC > 1 && q < NC) {
-        rcol = dsm_map_to_cta(dsm_smem_u32(col), q);
-        rbar0 = dsm_map_to_cta(dsm_smem_u32(&col_bar[0]), q);
-        rbar1 = dsm_map_to_cta(dsm_smem_u32(&col_bar[1]), q);
+    // whole blocks to three CTAs and more, lane k to CTA k; node by node to two, one of a node's lanes to each: there the
+    // shuffles that put a block together cost more than the messages they save
+    const bool by_block = NC > 2;
+    const int peer = by_block ? lane : half ? 32 : lane & 3;
+    uint32_t rcol = 0, rbar0 = 0, rbar1 = 0;  // peer < NC: this CTA's columns and barriers as that CTA maps them
+    if (NC > 1 && peer < NC) {
+        rcol = dsm_map_to_cta(dsm_smem_u32(col), peer);
+        rbar0 = dsm_map_to_cta(dsm_smem_u32(&col_bar[0]), peer);
+        rbar1 = dsm_map_to_cta(dsm_smem_u32(&col_bar[1]), peer);
     }
     if (tid == 0) {
         s_timeout = 0;
@@ -370,66 +409,69 @@ __global__ void __launch_bounds__(kLThreads, 1)
 #define PCFGNAT_LAP(acc)
 #endif
     for (int t = n - 2; t >= 0; t--) {
-        const float4 *S1v = reinterpret_cast<const float4 *>(col + ((t + 1) & 3) * cs);
-        const float4 *S2v = reinterpret_cast<const float4 *>(col + ((t + 2) & 3) * cs);
-        float *S0 = col + (t & 3) * cs;
+        const float4 *S1v = reinterpret_cast<const float4 *>(col + ((t + 1) & 3) * cp);
+        const float4 *S2v = reinterpret_cast<const float4 *>(col + ((t + 2) & 3) * cp);
+        float *S0 = col + (t & 3) * cp;
         const uint32_t bar = dsm_smem_u32(&col_bar[t & 1]);
-        if (NC > 1 && tid == 0) bar_expect(bar, 4 * Mb);
+        if (NC > 1 && tid == 0) bar_expect(bar, 4 * R * blocks);
         if (warp < groups) {
             const float rho = s_rho[t & 3], rho_prev = s_rho[(t + 1) & 3];
-            const uint32_t rS0 = rcol + 4u * ((t & 3) * cs), rbar = (t & 1) ? rbar1 : rbar0;
+            const uint32_t rS0 = rcol + 4u * ((t & 3) * cp), rbar = (t & 1) ? rbar1 : rbar0;
             PCFGNAT_LAP(tA)
             for (int g = warp; g < groups; g += kLWarps) {
-                const int r = g * R + sub;
-                const bool live = r < my_rows;
-                const int rr = live ? r : 0;
-                float acc0 = 0.f, acc1 = 0.f;
-                if (g == warp) {  // this warp's resident nodes
-                    float a[TRIPS], c[TRIPS];
+                const int r = g * R + sub, block = (crank + NC * g) * R;  // this lane's node; the block's first one
+                const float et = (half ? e1 : e0)[r * W + t];
+                float acc[2 * R];
+                {
+                    float4 x[TRIPS], y[TRIPS];
 #pragma unroll
                     for (int i = 0; i < TRIPS; i++) {
-                        const int c4 = q + G * i;
-                        a[i] = c[i] = 0.f;
-                        if (c4 < cs4) {
-                            a[i] = dot4(rp0[i], S1v[c4]);
-                            c[i] = dot4(rp1[i], S2v[c4]);
+                        x[i] = S1v[lane + 32 * i];
+                        y[i] = S2v[lane + 32 * i];
+                    }
+                    if (g == warp) {  // this warp's resident nodes
+#pragma unroll
+                        for (int j = 0; j < R; j++) {
+                            acc[j] = dot4(rp0[j][0], x[0]);
+                            acc[R + j] = dot4(rp1[j][0], y[0]);
+                            if constexpr (TRIPS > 1) {
+                                acc[j] += dot4(rp0[j][1], x[1]);
+                                acc[R + j] += dot4(rp1[j][1], y[1]);
+                            }
                         }
-                    }
+                    } else {  // further nodes of a long chain: rows from shared memory
 #pragma unroll
-                    for (int i = 0; i < TRIPS; i++) {
-                        acc0 += a[i];
-                        acc1 += c[i];
-                    }
-                } else {  // further nodes of a long chain: rows from shared memory, children ci > ai only
-                    const float4 *p0 = P0v + rr * cs4, *p1 = P1v + rr * cs4;
-                    for (int c4 = q + ((crank + NC * rr + 1) >> 2) / G * G; c4 < cs4; c4 += G) {
-                        acc0 += dot4(p0[c4], S1v[c4]);
-                        acc1 += dot4(p1[c4], S2v[c4]);
+                        for (int j = 0; j < R; j++) {
+                            const float4 *p0 = P0v + (g * R + j) * cs4, *p1 = P1v + (g * R + j) * cs4;
+                            acc[j] = acc[R + j] = 0.f;
+#pragma unroll
+                            for (int i = 0; i < TRIPS; i++) {
+                                const int c4 = min(lane + 32 * i, cs4 - 1);  // past the row: times a zero of the column
+                                acc[j] += dot4(p0[c4], x[i]);
+                                acc[R + j] += dot4(p1[c4], y[i]);
+                            }
+                        }
                     }
                 }
                 PCFGNAT_LAP(tB)
+                halve<8, 16>(acc);
+                halve<4, 8>(lower(acc));
+                halve<2, 4>(lower(lower(acc)));
+                float a = acc[0];
+                a += __shfl_xor_sync(0xffffffffu, a, 2);
+                a += __shfl_xor_sync(0xffffffffu, a, 1);
                 // one scale at a time: the product of two scales can leave the range although the result does not
-                float v0 = e0[rr * W + t] * (acc0 * rho);
-                float v1 = e1[rr * W + t] * ((acc1 * rho_prev) * rho);
-#pragma unroll
-                for (int o = G / 2; o > 0; o >>= 1) {
-                    v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-                    v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+                const float v = et * ((half ? a * rho_prev : a) * rho);
+                const float u = v + __shfl_xor_sync(0xffffffffu, v, 16);  // 0 past the chain
+                if (by_block) {  // into the peers' columns, counted on their barriers of this step
+                    const float4 u4 = block_values<4>(u);
+                    if (peer < NC) store_async4(rS0 + 4u * block, u4, rbar);
+                } else if (NC > 1) {
+                    if (peer < NC) dsm_store_async(rS0 + 4u * (block + sub), u, rbar);
+                } else if ((lane & 19) == 0) {
+                    S0[block + sub] = u;
                 }
-                const float u = v0 + v1;
-                if (live) {
-                    const int ai = crank + NC * r;
-                    if (NC > 1) {  // lane q of the node sends to CTA q: into its column, counted on its barrier of this step
-                        if (q < NC) dsm_store_async(rS0 + 4u * ai, u, rbar);
-                    } else if (q == 0) {
-                        S0[ai] = u;
-                    }
-                    if (q == 0) {
-                        ownu[r * W + t] = u;
-                        own0[r * W + t] = v0;
-                        own1[r * W + t] = v1;
-                    }
-                }
+                if ((lane & 3) == 0) (half ? own1 : own0)[r * W + t] = v;
             }
         }
         PCFGNAT_LAP(tC)
@@ -471,19 +513,20 @@ __global__ void __launch_bounds__(kLThreads, 1)
 
     float *Yb = Y + (size_t)b * W * Mc;
     for (int i = tid; i < my_rows * (n - 1); i += kLThreads) {  // columns 1 .. n-1 of this CTA's nodes, normalised
-        const int r = i / (n - 1), t = 1 + (i - r * (n - 1));
-        Yb[(size_t)t * Mc + (crank + NC * r)] = ownu[(size_t)r * W + t] * invs[t];
+        const int r = i / (n - 1), t = 1 + (i - r * (n - 1)), ai = node_of(r, crank, NC);
+        if (ai < Mb) Yb[(size_t)t * Mc + ai] = (own0[(size_t)r * W + t] + own1[(size_t)r * W + t]) * invs[t];
     }
     float *sb = shares + (size_t)b * L * T;
     for (int i = tid; i < my_rows * (n - 1); i += kLThreads) {  // the halves of columns 0 .. n-2
-        const int r = i / (n - 1), t = i - r * (n - 1), a = 2 * (crank + NC * r) + 1;
+        const int r = i / (n - 1), t = i - r * (n - 1), a = 2 * node_of(r, crank, NC) + 1;
+        if (a >= m) continue;
         sb[(size_t)a * T + t] = own0[(size_t)r * W + t];
         if (a >= 3) sb[(size_t)(a - 1) * T + t] = own1[(size_t)r * W + t];
     }
     if (crank == 0) {
         for (int t = tid; t < W; t += kLThreads) fr[kLinearFrameHead + t] = invs[t];
         if (tid == 0) {
-            const float u00 = ownu[0];  // row 0 of rank 0 is the root, column 0
+            const float u00 = own0[0] + own1[0];  // row 0 of rank 0 is the root, column 0
             const float lz = u00 > 0.f ? (lg2f(u00) + s_sumlog) * kLn2 + s_lmx_sum : neg_inf();
             fr[0] = arrived ? u00 : 0.f;
             fr[1] = lz;
@@ -550,16 +593,15 @@ __device__ __forceinline__ void links_grad_dispatch(int dead, const float *x0r, 
     }
 }
 
-template <int G, int TRIPS>
+template <int CHUNKS>
 __global__ void __launch_bounds__(kLThreads, 1)
     outside_linear_kernel(const float *__restrict__ match_all, const float *__restrict__ links,
                           const int64_t *__restrict__ ol, const int64_t *__restrict__ tl, int L, int T,
                           const float *__restrict__ Y, float *O, float *frames, float *mg, float *lg, int *status, int Mc,
                           int cs, int rows_cap, int B, int wide) {
-    // groups of 32 children a lane sums in one pass over the steps of the links gradient: all the kernel's row
-    // width allows (4 G TRIPS children), in two passes when that is more than four
-    constexpr int kChunksMax = (4 * G * TRIPS + 31) / 32;
-    constexpr int kGradChunk = kChunksMax <= 4 ? kChunksMax : (kChunksMax + 1) / 2;
+    // groups of 32 children a lane sums in one pass over the steps of the links gradient: all of the row width, in two
+    // passes when that is more than four
+    constexpr int kGradChunk = CHUNKS <= 4 ? CHUNKS : (CHUNKS + 1) / 2;
     extern __shared__ float4 smem4[];
     float *smem = reinterpret_cast<float *>(smem4);
     chain_begin();
@@ -583,15 +625,16 @@ __global__ void __launch_bounds__(kLThreads, 1)
     PCFGNAT_STAMP(1, 1)
     const float *mat = match_all + (size_t)b * L * T;
     const float *lkb = links + (size_t)b * L * 2 * L;
-    const int Mb = m / 2, last = (m - 2) / 2;
-    const int my_rows = Mb > crank ? (Mb - crank + NC - 1) / NC : 0;  // nodes ci = crank + NC * r
+    const int Mb = m / 2, last = (m - 2) / 2, blocks = (Mb + R - 1) / R;
+    const int groups = blocks > crank ? (blocks - crank + NC - 1) / NC : 0, my_rows = groups * R;  // nodes node_of(r)
     float *e0 = smem;                            // [rows_cap][W] E0, E1; after the loop x0_t and x1_t inv_{t+1}
     float *e1 = e0 + (size_t)rows_cap * W;
     float *invs = e1 + (size_t)rows_cap * W;     // [W]
     float *loop_mem = smem + linear_outside_head(rows_cap, W);  // what follows is only needed by the step loop
-    float *xc0 = loop_mem;                       // [4][cs] rolling columns x0_s of the whole chain
-    float *xc1 = xc0 + 4 * cs;                   // [4][cs] x1_s
-    float *PT0 = xc1 + 4 * cs;                   // [rows_cap][cs] exp(links[a][0][c]) of this CTA's CHILDREN c, by parent
+    constexpr int TRIPS = (CHUNKS + 3) / 4, cp = 128 * TRIPS;  // column pitch: as in the inside pass
+    float *xc0 = loop_mem;                       // [4][cp] rolling columns x0_s of the whole chain
+    float *xc1 = xc0 + 4 * cp;                   // [4][cp] x1_s
+    float *PT0 = xc1 + 4 * cp;                   // [rows_cap][cs] exp(links[a][0][c]) of this CTA's CHILDREN c, by parent
     float *PT1 = PT0 + (size_t)rows_cap * cs;
     float *owno = PT1 + (size_t)rows_cap * cs;   // [rows_cap][W] o_t of this CTA's nodes
     __shared__ __align__(8) uint64_t col_bar[2];
@@ -601,9 +644,9 @@ __global__ void __launch_bounds__(kLThreads, 1)
     token_maxima(mat, m, n, T, W, invs);  // borrowed until the scales are loaded: invs[t] = lmx[t]
     __syncthreads();
     for (int i = tid; i < my_rows * W; i += kLThreads) {
-        const int r = i / W, t = i - r * W, a = 2 * (crank + NC * r) + 1;
+        const int r = i / W, t = i - r * W, ai = node_of(r, crank, NC), a = 2 * ai + 1;
         float v0 = 0.f, v1 = 0.f;
-        if (t < n) {
+        if (t < n && ai < Mb) {
             v0 = exp_clean(__ldg(mat + (size_t)a * T + t) - invs[t]);
             if (a >= 3 && t + 1 < n)
                 v1 = exp_clean((fmaxf(__ldg(mat + (size_t)(a - 1) * T + t), neg_inf()) - invs[t]) +
@@ -617,11 +660,11 @@ __global__ void __launch_bounds__(kLThreads, 1)
     const float e_term = exp_clean(__ldg(mat + (size_t)(m - 1) * T + (n - 1)) - invs[n - 1]);  // u of the terminal cell
     __syncthreads();  // the maxima are used up: invs takes the scales below
     for (int r = warp; r < my_rows; r += kLWarps) {
-        const int ci = crank + NC * r;
+        const int ci = node_of(r, crank, NC);
 #pragma unroll 4
         for (int ai = lane; ai < cs; ai += 32) {
             float p0 = 0.f, p1 = 0.f;
-            if (ai < ci) {
+            if (ai < ci && ci < Mb) {
                 const float *row = lkb + (size_t)(2 * ai + 1) * 2 * L + (2 * ci + 1);
                 p0 = exp_clean(__ldg(row));
                 if (ai >= 1) p1 = exp_clean(__ldg(row + L));
@@ -630,7 +673,7 @@ __global__ void __launch_bounds__(kLThreads, 1)
             PT1[(size_t)r * cs + ai] = p1;
         }
     }
-    for (int i = tid; i < 8 * cs; i += kLThreads) xc0[i] = 0.f;  // both column sets
+    for (int i = tid; i < 8 * cp; i += kLThreads) xc0[i] = 0.f;  // both column sets
     for (int t = tid; t < W; t += kLThreads) invs[t] = t >= 1 && t < n ? fr[kLinearFrameHead + t] : 0.f;
     if (tid == 0) bar_init(col_bar, 2);
     __syncthreads();
@@ -643,76 +686,87 @@ __global__ void __launch_bounds__(kLThreads, 1)
     if (NC > 1) cluster.sync(); else __syncthreads();
     PCFGNAT_STAMP(1, 3)
 
-    // Step loop, laid out as in the inside pass: G lanes per node, the node's rows of the transposed matrices in
+    // Step loop, laid out as in the inside pass: a block of R nodes per warp, their rows of the transposed matrices in
     // registers, the last warp waits for the columns of the step.
-    constexpr int R = 32 / G;
     const int cs4 = cs >> 2;
-    const int groups = (my_rows + R - 1) / R;
-    const int q = lane % G, sub = lane / G;
+    const int sub = lane >> 3, pass = (lane >> 2) & 1;  // after the sums: o of node `sub`, whose x0 or x1 this lane forms
     const float4 *PT0v = reinterpret_cast<const float4 *>(PT0), *PT1v = reinterpret_cast<const float4 *>(PT1);
-    const int r_own = warp * R + sub;
-    const bool live_own = r_own < my_rows;
-    float4 rp0[TRIPS], rp1[TRIPS];
+    float4 rp0[R][TRIPS], rp1[R][TRIPS];
 #pragma unroll
-    for (int i = 0; i < TRIPS; i++) {
-        const int c4 = q + G * i;
-        rp0[i] = rp1[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live_own && c4 < cs4) {
-            rp0[i] = PT0v[r_own * cs4 + c4];
-            rp1[i] = PT1v[r_own * cs4 + c4];
+    for (int j = 0; j < R; j++)
+#pragma unroll
+        for (int i = 0; i < TRIPS; i++) {
+            const int c4 = lane + 32 * i;
+            rp0[j][i] = rp1[j][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (warp < groups && c4 < cs4) {
+                rp0[j][i] = PT0v[(warp * R + j) * cs4 + c4];
+                rp1[j][i] = PT1v[(warp * R + j) * cs4 + c4];
+            }
         }
-    }
-    uint32_t rx0 = 0, rx1 = 0, rbar0 = 0, rbar1 = 0;  // lane q < NC: this CTA's columns and barriers as CTA q maps them
-    if (NC > 1 && q < NC) {
-        rx0 = dsm_map_to_cta(dsm_smem_u32(xc0), q);
-        rx1 = dsm_map_to_cta(dsm_smem_u32(xc1), q);
-        rbar0 = dsm_map_to_cta(dsm_smem_u32(&col_bar[0]), q);
-        rbar1 = dsm_map_to_cta(dsm_smem_u32(&col_bar[1]), q);
+    const bool by_block = NC > 2;  // as in the inside pass
+    const int peer = by_block ? lane : lane & 3;
+    uint32_t rx0 = 0, rx1 = 0, rbar0 = 0, rbar1 = 0;
+    if (NC > 1 && peer < NC) {
+        rx0 = dsm_map_to_cta(dsm_smem_u32(xc0), peer);
+        rx1 = dsm_map_to_cta(dsm_smem_u32(xc1), peer);
+        rbar0 = dsm_map_to_cta(dsm_smem_u32(&col_bar[0]), peer);
+        rbar1 = dsm_map_to_cta(dsm_smem_u32(&col_bar[1]), peer);
     }
     if (tid == 0) s_timeout = s_range = 0;
     __syncthreads();
     for (int s = 0; s <= n - 2; s++) {  // step s forms column s + 1
-        const float4 *X0v = reinterpret_cast<const float4 *>(xc0 + (s & 3) * cs);
-        const float4 *X1v = reinterpret_cast<const float4 *>(xc1 + ((s + 3) & 3) * cs);  // column s - 1 (all zero at s = 0)
-        float *D0 = xc0 + ((s + 1) & 3) * cs, *D1 = xc1 + ((s + 1) & 3) * cs;
+        const float4 *X0v = reinterpret_cast<const float4 *>(xc0 + (s & 3) * cp);
+        const float4 *X1v = reinterpret_cast<const float4 *>(xc1 + ((s + 3) & 3) * cp);  // column s - 1 (all zero at s = 0)
+        float *D0 = xc0 + ((s + 1) & 3) * cp, *D1 = xc1 + ((s + 1) & 3) * cp;
         const uint32_t bar = dsm_smem_u32(&col_bar[s & 1]);
-        if (NC > 1 && tid == 0) bar_expect(bar, 8 * Mb);
+        if (NC > 1 && tid == 0) bar_expect(bar, 8 * R * blocks);
         if (warp < groups) {
             const float k0 = invs[s + 1], k1 = invs[s];
-            const uint32_t off = 4u * (((s + 1) & 3) * cs);
+            const uint32_t off = 4u * (((s + 1) & 3) * cp);
             const uint32_t rD0 = rx0 + off, rD1 = rx1 + off, rbar = (s & 1) ? rbar1 : rbar0;
             for (int g = warp; g < groups; g += kLWarps) {
-                const int r = g * R + sub;
-                const bool live = r < my_rows;
-                const int rr = live ? r : 0;
-                float acc0 = 0.f, acc1 = 0.f;
-                if (g == warp) {
-                    float a[TRIPS], c[TRIPS];
+                const int r = g * R + sub, block = (crank + NC * g) * R;
+                const float et = (pass ? e1 : e0)[r * W + s + 1];
+                float acc[R];
+                {
+                    float4 x[TRIPS], y[TRIPS];
 #pragma unroll
                     for (int i = 0; i < TRIPS; i++) {
-                        const int c4 = q + G * i;
-                        a[i] = c[i] = 0.f;
-                        if (c4 < cs4) {
-                            a[i] = dot4(rp0[i], X0v[c4]);
-                            c[i] = dot4(rp1[i], X1v[c4]);
+                        x[i] = X0v[lane + 32 * i];
+                        y[i] = X1v[lane + 32 * i];
+                    }
+                    float acc1[R];
+                    if (g == warp) {
+#pragma unroll
+                        for (int j = 0; j < R; j++) {
+                            acc[j] = dot4(rp0[j][0], x[0]);
+                            acc1[j] = dot4(rp1[j][0], y[0]);
+                            if constexpr (TRIPS > 1) {
+                                acc[j] += dot4(rp0[j][1], x[1]);
+                                acc1[j] += dot4(rp1[j][1], y[1]);
+                            }
+                        }
+                    } else {  // further nodes of a long chain: rows from shared memory
+#pragma unroll
+                        for (int j = 0; j < R; j++) {
+                            const float4 *p0 = PT0v + (g * R + j) * cs4, *p1 = PT1v + (g * R + j) * cs4;
+                            acc[j] = acc1[j] = 0.f;
+#pragma unroll
+                            for (int i = 0; i < TRIPS; i++) {
+                                const int c4 = min(lane + 32 * i, cs4 - 1);  // past the row: times a zero of the column
+                                acc[j] += dot4(p0[c4], x[i]);
+                                acc1[j] += dot4(p1[c4], y[i]);
+                            }
                         }
                     }
 #pragma unroll
-                    for (int i = 0; i < TRIPS; i++) {
-                        acc0 += a[i];
-                        acc1 += c[i];
-                    }
-                } else {  // further nodes of a long chain: rows from shared memory, parents ai < ci only
-                    const float4 *p0 = PT0v + rr * cs4, *p1 = PT1v + rr * cs4;
-                    const int end4 = min(cs4, (crank + NC * rr + 3) >> 2);
-                    for (int c4 = q; c4 < end4; c4 += G) {
-                        acc0 += dot4(p0[c4], X0v[c4]);
-                        acc1 += dot4(p1[c4], X1v[c4]);
-                    }
+                    for (int j = 0; j < R; j++) acc[j] = fmaf(k1, acc1[j], acc[j]);
                 }
-                float o = fmaf(k1, acc1, acc0);
+                halve<4, 16>(acc);
+                halve<2, 8>(lower(acc));
+                float o = acc[0];
 #pragma unroll
-                for (int w = G / 2; w > 0; w >>= 1) o += __shfl_xor_sync(0xffffffffu, o, w);
+                for (int w = 4; w > 0; w >>= 1) o += __shfl_xor_sync(0xffffffffu, o, w);
                 // o_{s+1}[c] = rho_s (acc0 + rho_{s-1} acc1).  o u is a posterior (<= 1): as long as o stays inside the
                 // floats, what the inside pass flushed to zero or kept as a denormal costs less than 1e-7 of posterior
                 // per cell.  An o at the edge of the range (or NaN) means the cell's inside value was below ~1e-37
@@ -721,22 +775,21 @@ __global__ void __launch_bounds__(kLThreads, 1)
                 o *= k0;
                 if (!(o < 1e37f)) {
                     o = 1e37f;
-                    if (live) s_range = 1;
+                    if (block + sub < Mb) s_range = 1;
                 }
-                if (live) {
-                    const int ci = crank + NC * r;
-                    const float n0 = o * e0[r * W + s + 1], n1 = o * e1[r * W + s + 1];
-                    if (NC > 1) {
-                        if (q < NC) {
-                            dsm_store_async(rD0 + 4u * ci, n0, rbar);
-                            dsm_store_async(rD1 + 4u * ci, n1, rbar);
-                        }
-                    } else if (q == 0) {
-                        D0[ci] = n0;
-                        D1[ci] = n1;
+                const float x = o * et;  // 0 past the chain
+                if (by_block) {
+                    const float4 n0 = block_values<8>(x), n1 = block_values<8>(__shfl_xor_sync(0xffffffffu, x, 4));
+                    if (peer < NC) {
+                        store_async4(rD0 + 4u * block, n0, rbar);
+                        store_async4(rD1 + 4u * block, n1, rbar);
                     }
-                    if (q == 0) owno[r * W + s + 1] = o;
+                } else if (NC > 1) {
+                    if (peer < NC) dsm_store_async((pass ? rD1 : rD0) + 4u * (block + sub), x, rbar);
+                } else if ((lane & 3) == 0) {
+                    (pass ? D1 : D0)[block + sub] = x;
                 }
+                if ((lane & 7) == 0) owno[r * W + s + 1] = o;
             }
         }
         if (NC > 1 && warp == kLWarps - 1 && !dsm_wait_column(bar, (s >> 1) & 1)) s_timeout = 1;
@@ -751,8 +804,8 @@ __global__ void __launch_bounds__(kLThreads, 1)
     // ---- o table to global memory (the emission gradients of a node need it from whichever CTA sweeps the cell)
     float *Ob = O + (size_t)b * Mc * W;
     for (int i = tid; i < my_rows * n; i += kLThreads) {
-        const int r = i / n, t = i - r * n;
-        Ob[(size_t)(crank + NC * r) * W + t] = owno[(size_t)r * W + t];
+        const int r = i / n, t = i - r * n, ai = node_of(r, crank, NC);
+        if (ai < Mb) Ob[(size_t)ai * W + t] = owno[(size_t)r * W + t];
     }
     // x0_t and x1_t inv_{t+1} of this CTA's nodes, now as PARENTS, in place of E0 / E1
     for (int i = tid; i < my_rows * W; i += kLThreads) {
@@ -778,7 +831,8 @@ __global__ void __launch_bounds__(kLThreads, 1)
     __syncthreads();
     PCFGNAT_STAMP(1, 12)
     for (int r = warp; r < my_rows; r += kLWarps) {
-        const int ai = crank + NC * r, a = 2 * ai + 1;
+        const int ai = node_of(r, crank, NC), a = 2 * ai + 1;
+        if (ai >= Mb) continue;
         const float *x0r = e0 + r * W, *x1r = e1 + r * W;
         float *row = lgb + (size_t)a * 2 * L;
         const float *lrow = lkb + (size_t)a * 2 * L;
@@ -901,6 +955,12 @@ __global__ void __launch_bounds__(kLThreads, 1)
     PCFGNAT_ACC(1, 9, NC)
 }
 
+// Groups of 32 children: enough for the chain, one of the instantiated numbers.
+int linear_chunks(int cs) {
+    const int chunks = (cs + 31) / 32;
+    return chunks <= 4 ? chunks : chunks <= 6 ? 6 : 8;
+}
+
 struct LinearGeometry {
     int nc, cs, rows_cap;
     int wide;                 // -1: cluster k takes sentence k; else the sentences are taken by cost (pick_sentence)
@@ -916,6 +976,7 @@ LinearGeometry linear_geometry(int B, int Mc, int W) {
     LinearGeometry g;
     g.cs = (Mc + 3) / 4 * 4;
     g.wide = -1;
+    const size_t cp = linear_chunks(g.cs) <= 4 ? 128 : 256;  // column pitch
     int nc = 1;
     while (nc < 8 && (long long)B * nc * 2 <= sms && Mc > 8 * nc) nc *= 2;
     if (const char *v = getenv("PCFGNAT_DP_CLUSTER_SIZE")) {
@@ -924,11 +985,11 @@ LinearGeometry linear_geometry(int B, int Mc, int W) {
     }
     for (;; nc *= 2) {
         g.nc = nc;
-        g.rows_cap = (Mc + nc - 1) / nc;
+        g.rows_cap = ((Mc + R - 1) / R + nc - 1) / nc * R;
         const size_t mat = (size_t)2 * g.rows_cap * g.cs, own = (size_t)g.rows_cap * W;
-        g.smem_in = ((size_t)4 * g.cs + mat + 5 * own + W) * sizeof(float);
+        g.smem_in = (4 * cp + mat + 4 * own + W) * sizeof(float);
         // the step loop's columns, matrices and o table, later overlaid by the y table of the gradient sums
-        const size_t loop_mem = (size_t)8 * g.cs + mat + own, y_table = (size_t)W * g.cs;
+        const size_t loop_mem = 8 * cp + mat + own, y_table = (size_t)W * g.cs;
         g.smem_out = ((size_t)linear_outside_head(g.rows_cap, W) + (loop_mem > y_table ? loop_mem : y_table)) * sizeof(float);
         if (g.smem_in <= (size_t)kSmemLimit - 1024 && g.smem_out <= (size_t)kSmemLimit - 1024) break;
         if (nc >= 16) {
@@ -980,16 +1041,16 @@ int launch_linear_cluster(Kernel kernel, int clusters, int nc, size_t smem, cuda
     return cuda_rc(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
-template <int G, int TRIPS>
+template <int CHUNKS>
 int launch_linear(const LinearGeometry &g, const float *match_all, const float *links, const int64_t *ol, const int64_t *tl,
                   int B, int L, int T, float *Y, float *O, float *frames, float *loss, float *mg, float *lg, int *status,
                   cudaStream_t st) {
     const int Mc = main_slots(L, 1);
     const int nc = g.launch_nc, clusters = g.clusters;
-    int rc = launch_linear_cluster(inside_linear_kernel<G, TRIPS>, clusters, nc, g.smem_in, st, match_all, links, ol, tl, L, T,
+    int rc = launch_linear_cluster(inside_linear_kernel<CHUNKS>, clusters, nc, g.smem_in, st, match_all, links, ol, tl, L, T,
                                    Y, frames, loss, mg, status, Mc, g.cs, g.rows_cap, B, g.wide);
     if (rc) return rc;
-    return launch_linear_cluster(outside_linear_kernel<G, TRIPS>, clusters, nc, g.smem_out, st, match_all, links, ol, tl, L, T,
+    return launch_linear_cluster(outside_linear_kernel<CHUNKS>, clusters, nc, g.smem_out, st, match_all, links, ol, tl, L, T,
                                  (const float *)Y, O, frames, mg, lg, status, Mc, g.cs, g.rows_cap, B, g.wide);
 }
 
@@ -1018,16 +1079,18 @@ int launch_loss_linear(const float *match_all, const float *links, const int64_t
     if (Mc > 256) return PCFGNAT_ERR_UNSUPPORTED;
     const LinearGeometry g = linear_geometry(B, Mc, T + 2);
     if (g.nc == 0) return PCFGNAT_ERR_UNSUPPORTED;
-    // lanes per node and float4 per lane so that a node's row of g.cs / 4 groups of four children fits the lanes' registers
-    const int cs4 = g.cs / 4;
-#define PCFGNAT_LINEAR_CASE(G_, TRIPS_) \
-    return launch_linear<G_, TRIPS_>(g, match_all, links, ol, tl, B, L, T, Y, O, frames, loss, mg, lg, status, st)
-    if (cs4 <= 8) PCFGNAT_LINEAR_CASE(8, 1);
-    if (cs4 <= 16) PCFGNAT_LINEAR_CASE(8, 2);
-    if (cs4 <= 24) PCFGNAT_LINEAR_CASE(8, 3);
-    if (cs4 <= 32) PCFGNAT_LINEAR_CASE(8, 4);
-    if (cs4 <= 48) PCFGNAT_LINEAR_CASE(16, 3);
-    PCFGNAT_LINEAR_CASE(16, 4);
+    // float4 per lane so that a node's row of g.cs / 4 groups of four children fits the lanes' registers
+#define PCFGNAT_LINEAR_CASE(N_) \
+    case N_: return launch_linear<N_>(g, match_all, links, ol, tl, B, L, T, Y, O, frames, loss, mg, lg, status, st)
+    switch (linear_chunks(g.cs)) {
+        PCFGNAT_LINEAR_CASE(1);
+        PCFGNAT_LINEAR_CASE(2);
+        PCFGNAT_LINEAR_CASE(3);
+        PCFGNAT_LINEAR_CASE(4);
+        PCFGNAT_LINEAR_CASE(6);
+        PCFGNAT_LINEAR_CASE(8);
+        default: return PCFGNAT_ERR_UNSUPPORTED;
+    }
 #undef PCFGNAT_LINEAR_CASE
 }
 
