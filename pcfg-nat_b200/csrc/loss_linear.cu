@@ -41,7 +41,7 @@
 // (its part of the nodes' matrix rows in registers); one thread-block CLUSTER per sentence, blocks dealt round-robin to
 // the CTAs; the columns are exchanged with st.async counted on alternating mbarriers as in loss_cluster.cu, a block's
 // four values in one 16-byte message per CTA where there are three CTAs and more.  Inside and outside kernel, 90
-// sentences of at most 80 nodes: 36 + 44 us, 8 sentences of 256: 111 + 152 us (43 + 50 and 165 + 216 us with eight or
+// sentences of at most 80 nodes: 36 + 44 us, 8 sentences of 256: 104 + 147 us (43 + 50 and 165 + 216 us with eight or
 // sixteen lanes per node, a test before every load of a column, and a message per node).  Batches
 // between half and all of the SMs run clusters of two, which the costliest sentences have to themselves and the
 // others share, one CTA per sentence (pick_sentence).
@@ -365,8 +365,7 @@ __global__ void __launch_bounds__(kLThreads, 1)
     // l + 32 of all of them: their parts of P0 and P1 stay in REGISTERS for the whole loop, and a step reads each column
     // once per warp (with eight lanes per node every node's lanes read it: shared memory bound the step, since a
     // 16-byte load takes four cycles whatever its lanes share).  The R x 2 partial sums are added up over the warp
-    // by exchanging halves of them, nine shuffles.  Nodes beyond what the warps can hold that way (long chains on few CTAs)
-    // take their rows from shared memory every step.  The last warp does not compute nodes unless the chain is that
+    // by exchanging halves of them, nine shuffles.  The last warp does not compute nodes unless the chain is that
     // long: it derives the scale two steps ahead from the finished column, keeps the books of the scales, and waits for
     // the column of the step on the byte-counting barrier; the block barrier then releases the others, so nobody else
     // spins.
@@ -418,61 +417,67 @@ __global__ void __launch_bounds__(kLThreads, 1)
             const float rho = s_rho[t & 3], rho_prev = s_rho[(t + 1) & 3];
             const uint32_t rS0 = rcol + 4u * ((t & 3) * cp), rbar = (t & 1) ? rbar1 : rbar0;
             PCFGNAT_LAP(tA)
-            for (int g = warp; g < groups; g += kLWarps) {
-                const int r = g * R + sub, block = (crank + NC * g) * R;  // this lane's node; the block's first one
-                const float et = (half ? e1 : e0)[r * W + t];
-                float acc[2 * R];
-                {
-                    float4 x[TRIPS], y[TRIPS];
+            float4 x[TRIPS], y[TRIPS];
 #pragma unroll
-                    for (int i = 0; i < TRIPS; i++) {
-                        x[i] = S1v[lane + 32 * i];
-                        y[i] = S2v[lane + 32 * i];
-                    }
-                    if (g == warp) {  // this warp's resident nodes
-#pragma unroll
-                        for (int j = 0; j < R; j++) {
-                            acc[j] = dot4(rp0[j][0], x[0]);
-                            acc[R + j] = dot4(rp1[j][0], y[0]);
-                            if constexpr (TRIPS > 1) {
-                                acc[j] += dot4(rp0[j][1], x[1]);
-                                acc[R + j] += dot4(rp1[j][1], y[1]);
-                            }
-                        }
-                    } else {  // further nodes of a long chain: rows from shared memory
-#pragma unroll
-                        for (int j = 0; j < R; j++) {
-                            const float4 *p0 = P0v + (g * R + j) * cs4, *p1 = P1v + (g * R + j) * cs4;
-                            acc[j] = acc[R + j] = 0.f;
-#pragma unroll
-                            for (int i = 0; i < TRIPS; i++) {
-                                const int c4 = min(lane + 32 * i, cs4 - 1);  // past the row: times a zero of the column
-                                acc[j] += dot4(p0[c4], x[i]);
-                                acc[R + j] += dot4(p1[c4], y[i]);
-                            }
-                        }
-                    }
-                }
-                PCFGNAT_LAP(tB)
-                halve<8, 16>(acc);
-                halve<4, 8>(lower(acc));
-                halve<2, 4>(lower(lower(acc)));
-                float a = acc[0];
-                a += __shfl_xor_sync(0xffffffffu, a, 2);
-                a += __shfl_xor_sync(0xffffffffu, a, 1);
-                // one scale at a time: the product of two scales can leave the range although the result does not
-                const float v = et * ((half ? a * rho_prev : a) * rho);
-                const float u = v + __shfl_xor_sync(0xffffffffu, v, 16);  // 0 past the chain
-                if (by_block) {  // into the peers' columns, counted on their barriers of this step
-                    const float4 u4 = block_values<4>(u);
-                    if (peer < NC) store_async4(rS0 + 4u * block, u4, rbar);
-                } else if (NC > 1) {
-                    if (peer < NC) dsm_store_async(rS0 + 4u * (block + sub), u, rbar);
-                } else if ((lane & 19) == 0) {
-                    S0[block + sub] = u;
-                }
-                if ((lane & 3) == 0) (half ? own1 : own0)[r * W + t] = v;
+            for (int i = 0; i < TRIPS; i++) {
+                x[i] = S1v[lane + 32 * i];
+                y[i] = S2v[lane + 32 * i];
             }
+            const int r = warp * R + sub, block = (crank + NC * warp) * R;  // this lane's node; the block's first one
+            const float et = (half ? e1 : e0)[r * W + t];
+            float acc[2 * R];
+#pragma unroll
+            for (int j = 0; j < R; j++) {
+                acc[j] = dot4(rp0[j][0], x[0]);
+                acc[R + j] = dot4(rp1[j][0], y[0]);
+                if constexpr (TRIPS > 1) {
+                    acc[j] += dot4(rp0[j][1], x[1]);
+                    acc[R + j] += dot4(rp1[j][1], y[1]);
+                }
+            }
+            // nodes beyond what the warps hold, one at a time and spread over all warps, rows from shared memory
+            for (int rx = kLWarps * R + warp; rx < my_rows; rx += kLWarps) {
+                const float4 *p0 = P0v + rx * cs4, *p1 = P1v + rx * cs4;
+                const float ex = (half ? e1 : e0)[rx * W + t];
+                float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+                for (int i = 0; i < TRIPS; i++) {
+                    const int c4 = min(lane + 32 * i, cs4 - 1);  // past the row: times a zero of the column
+                    a0 += dot4(p0[c4], x[i]);
+                    a1 += dot4(p1[c4], y[i]);
+                }
+                float a = (half ? a1 : a0) + __shfl_xor_sync(0xffffffffu, half ? a0 : a1, 16);
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+                const float v = ex * ((half ? a * rho_prev : a) * rho);
+                const float u = v + __shfl_xor_sync(0xffffffffu, v, 16);
+                const int ai = node_of(rx, crank, NC);
+                if (NC > 1) {
+                    if (lane < NC) dsm_store_async(rS0 + 4u * ai, u, rbar);
+                } else if (lane == 0) {
+                    S0[ai] = u;
+                }
+                if ((lane & 15) == 0) (half ? own1 : own0)[rx * W + t] = v;
+            }
+            PCFGNAT_LAP(tB)
+            halve<8, 16>(acc);
+            halve<4, 8>(lower(acc));
+            halve<2, 4>(lower(lower(acc)));
+            float a = acc[0];
+            a += __shfl_xor_sync(0xffffffffu, a, 2);
+            a += __shfl_xor_sync(0xffffffffu, a, 1);
+            // one scale at a time: the product of two scales can leave the range although the result does not
+            const float v = et * ((half ? a * rho_prev : a) * rho);
+            const float u = v + __shfl_xor_sync(0xffffffffu, v, 16);  // 0 past the chain
+            if (by_block) {  // into the peers' columns, counted on their barriers of this step
+                const float4 u4 = block_values<4>(u);
+                if (peer < NC) store_async4(rS0 + 4u * block, u4, rbar);
+            } else if (NC > 1) {
+                if (peer < NC) dsm_store_async(rS0 + 4u * (block + sub), u, rbar);
+            } else if ((lane & 19) == 0) {
+                S0[block + sub] = u;
+            }
+            if ((lane & 3) == 0) (half ? own1 : own0)[r * W + t] = v;
         }
         PCFGNAT_LAP(tC)
         if (warp == kLWarps - 1) {
@@ -724,73 +729,77 @@ __global__ void __launch_bounds__(kLThreads, 1)
             const float k0 = invs[s + 1], k1 = invs[s];
             const uint32_t off = 4u * (((s + 1) & 3) * cp);
             const uint32_t rD0 = rx0 + off, rD1 = rx1 + off, rbar = (s & 1) ? rbar1 : rbar0;
-            for (int g = warp; g < groups; g += kLWarps) {
-                const int r = g * R + sub, block = (crank + NC * g) * R;
-                const float et = (pass ? e1 : e0)[r * W + s + 1];
-                float acc[R];
-                {
-                    float4 x[TRIPS], y[TRIPS];
+            float4 x[TRIPS], y[TRIPS];
 #pragma unroll
-                    for (int i = 0; i < TRIPS; i++) {
-                        x[i] = X0v[lane + 32 * i];
-                        y[i] = X1v[lane + 32 * i];
-                    }
-                    float acc1[R];
-                    if (g == warp) {
-#pragma unroll
-                        for (int j = 0; j < R; j++) {
-                            acc[j] = dot4(rp0[j][0], x[0]);
-                            acc1[j] = dot4(rp1[j][0], y[0]);
-                            if constexpr (TRIPS > 1) {
-                                acc[j] += dot4(rp0[j][1], x[1]);
-                                acc1[j] += dot4(rp1[j][1], y[1]);
-                            }
-                        }
-                    } else {  // further nodes of a long chain: rows from shared memory
-#pragma unroll
-                        for (int j = 0; j < R; j++) {
-                            const float4 *p0 = PT0v + (g * R + j) * cs4, *p1 = PT1v + (g * R + j) * cs4;
-                            acc[j] = acc1[j] = 0.f;
-#pragma unroll
-                            for (int i = 0; i < TRIPS; i++) {
-                                const int c4 = min(lane + 32 * i, cs4 - 1);  // past the row: times a zero of the column
-                                acc[j] += dot4(p0[c4], x[i]);
-                                acc1[j] += dot4(p1[c4], y[i]);
-                            }
-                        }
-                    }
-#pragma unroll
-                    for (int j = 0; j < R; j++) acc[j] = fmaf(k1, acc1[j], acc[j]);
-                }
-                halve<4, 16>(acc);
-                halve<2, 8>(lower(acc));
-                float o = acc[0];
-#pragma unroll
-                for (int w = 4; w > 0; w >>= 1) o += __shfl_xor_sync(0xffffffffu, o, w);
-                // o_{s+1}[c] = rho_s (acc0 + rho_{s-1} acc1).  o u is a posterior (<= 1): as long as o stays inside the
-                // floats, what the inside pass flushed to zero or kept as a denormal costs less than 1e-7 of posterior
-                // per cell.  An o at the edge of the range (or NaN) means the cell's inside value was below ~1e-37
-                // while it still carries mass: the sentence goes to the log-space kernels.  Clamped so that the
-                // products below stay finite until then.
-                o *= k0;
-                if (!(o < 1e37f)) {
-                    o = 1e37f;
-                    if (block + sub < Mb) s_range = 1;
-                }
-                const float x = o * et;  // 0 past the chain
-                if (by_block) {
-                    const float4 n0 = block_values<8>(x), n1 = block_values<8>(__shfl_xor_sync(0xffffffffu, x, 4));
-                    if (peer < NC) {
-                        store_async4(rD0 + 4u * block, n0, rbar);
-                        store_async4(rD1 + 4u * block, n1, rbar);
-                    }
-                } else if (NC > 1) {
-                    if (peer < NC) dsm_store_async((pass ? rD1 : rD0) + 4u * (block + sub), x, rbar);
-                } else if ((lane & 3) == 0) {
-                    (pass ? D1 : D0)[block + sub] = x;
-                }
-                if ((lane & 7) == 0) owno[r * W + s + 1] = o;
+            for (int i = 0; i < TRIPS; i++) {
+                x[i] = X0v[lane + 32 * i];
+                y[i] = X1v[lane + 32 * i];
             }
+            // o_{s+1}[c] = rho_s (acc0 + rho_{s-1} acc1).  o u is a posterior (<= 1): as long as o stays inside the
+            // floats, what the inside pass flushed to zero or kept as a denormal costs less than 1e-7 of posterior
+            // per cell.  An o at the edge of the range (or NaN) means the cell's inside value was below ~1e-37
+            // while it still carries mass: the sentence goes to the log-space kernels.  Clamped so that the
+            // products below stay finite until then.
+            auto in_range = [&](float o, int node) {
+                if (o < 1e37f) return o;
+                if (node < Mb) s_range = 1;
+                return 1e37f;
+            };
+            const int r = warp * R + sub, block = (crank + NC * warp) * R;
+            const float et = (pass ? e1 : e0)[r * W + s + 1];
+            float acc[R];
+#pragma unroll
+            for (int j = 0; j < R; j++) {
+                float a0 = dot4(rp0[j][0], x[0]), a1 = dot4(rp1[j][0], y[0]);
+                if constexpr (TRIPS > 1) {
+                    a0 += dot4(rp0[j][1], x[1]);
+                    a1 += dot4(rp1[j][1], y[1]);
+                }
+                acc[j] = fmaf(k1, a1, a0);
+            }
+            // nodes beyond what the warps hold, as in the inside pass
+            for (int rx = kLWarps * R + warp; rx < my_rows; rx += kLWarps) {
+                const float4 *p0 = PT0v + rx * cs4, *p1 = PT1v + rx * cs4;
+                const float ex0 = e0[rx * W + s + 1], ex1 = e1[rx * W + s + 1];
+                float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+                for (int i = 0; i < TRIPS; i++) {
+                    const int c4 = min(lane + 32 * i, cs4 - 1);
+                    a0 += dot4(p0[c4], x[i]);
+                    a1 += dot4(p1[c4], y[i]);
+                }
+                const int ci = node_of(rx, crank, NC);
+                const float o = in_range(warp_sum(fmaf(k1, a1, a0)) * k0, ci);
+                if (NC > 1) {
+                    if (lane < NC) {
+                        dsm_store_async(rD0 + 4u * ci, o * ex0, rbar);
+                        dsm_store_async(rD1 + 4u * ci, o * ex1, rbar);
+                    }
+                } else if (lane == 0) {
+                    D0[ci] = o * ex0;
+                    D1[ci] = o * ex1;
+                }
+                if (lane == 0) owno[rx * W + s + 1] = o;
+            }
+            halve<4, 16>(acc);
+            halve<2, 8>(lower(acc));
+            float o = acc[0];
+#pragma unroll
+            for (int w = 4; w > 0; w >>= 1) o += __shfl_xor_sync(0xffffffffu, o, w);
+            o = in_range(o * k0, block + sub);
+            const float x01 = o * et;  // 0 past the chain
+            if (by_block) {
+                const float4 n0 = block_values<8>(x01), n1 = block_values<8>(__shfl_xor_sync(0xffffffffu, x01, 4));
+                if (peer < NC) {
+                    store_async4(rD0 + 4u * block, n0, rbar);
+                    store_async4(rD1 + 4u * block, n1, rbar);
+                }
+            } else if (NC > 1) {
+                if (peer < NC) dsm_store_async((pass ? rD1 : rD0) + 4u * (block + sub), x01, rbar);
+            } else if ((lane & 3) == 0) {
+                (pass ? D1 : D0)[block + sub] = x01;
+            }
+            if ((lane & 7) == 0) owno[r * W + s + 1] = o;
         }
         if (NC > 1 && warp == kLWarps - 1 && !dsm_wait_column(bar, (s >> 1) & 1)) s_timeout = 1;
         __syncthreads();
@@ -978,7 +987,9 @@ LinearGeometry linear_geometry(int B, int Mc, int W) {
     g.wide = -1;
     const size_t cp = linear_chunks(g.cs) <= 4 ? 128 : 256;  // column pitch
     int nc = 1;
-    while (nc < 8 && (long long)B * nc * 2 <= sms && Mc > 8 * nc) nc *= 2;
+    // up to 32 nodes on one CTA: eight warps hold them, and the exchange of a column costs a step more than the second
+    // CTA saves in staging and in the sums at the end (two sentences of 16 nodes: 7.5 + 9.4 us against 8.2 + 11.3 us)
+    while (nc < 8 && (long long)B * nc * 2 <= sms && Mc > 8 * nc && Mc > 32) nc *= 2;
     if (const char *v = getenv("PCFGNAT_DP_CLUSTER_SIZE")) {
         const int want = atoi(v);
         if (want == 1 || want == 2 || want == 4 || want == 8 || want == 16) nc = want;
