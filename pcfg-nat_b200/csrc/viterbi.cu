@@ -41,6 +41,7 @@ namespace {
 
 constexpr int kVitThreads = 1024;
 constexpr int kVitWarps = kVitThreads / 32;
+constexpr int kVitActive = 16;  // warps a length's nodes are shared out to
 
 // Monotone map float -> unsigned (no NaN reaches it); -0 is mapped like +0 so that, as under the
 // reference's '>', neither beats the other.
@@ -87,30 +88,29 @@ __device__ __forceinline__ void viterbi_node(int id, int Mb, int lane, int prio,
 }
 
 // The same for a group of G lanes (G = 4, 8, 16 or 32, the groups of a warp side by side): lane q of the group scans
-// children ci = id + q + G i, so that its reference thread (ci - id) & 3 = q & 3 is still one per lane, and the group
-// settles on (largest value, smallest key) with a butterfly of shuffles.  The lanes of a group without a node
-// (live = false) go through the shuffles with -inf.
-template <class K0, class K1>
-__device__ __forceinline__ void viterbi_node_group(bool live, int id, int Mb, int q, int G, float oa, const float *S1,
-                                                   const float *S2, K0 k0, K1 k1, float &best, int &key) {
+// children ci = id + q + G i, i < trips, so that its reference thread (ci - id) & 3 = q & 3 is still one per lane, and the
+// group settles on (largest value, smallest key) with a butterfly of shuffles.  The rows r0, r1 (from the lane's first
+// child on) hold -inf past the chain, so no child is tested and the loads of four trips are in flight together.
+// A lane remembers the trip of its best, the key is made at the end.
+__device__ __forceinline__ void viterbi_node_group(int id, int trips, int q, int G, float oa, const float *r0, const float *r1,
+                                                   const float *s1, const float *s2, float &best, int &key) {
     best = neg_inf();
-    key = INT_MAX;
-    if (live) {
-        const int x = q & 3, prio = ((x & 1) << 1) | (x >> 1);
-        for (int ci = id + q; ci < Mb; ci += G) {
-            const int kk = (prio << 24) | (ci << 1);
-            const float t0 = (k0(ci) + S1[ci]) + oa;
-            if (t0 > best) {
-                best = t0;
-                key = kk;
-            }
-            const float t1 = (k1(ci) + S2[ci]) + oa;
-            if (t1 > best) {
-                best = t1;
-                key = kk | 1;
-            }
+    int at = -1;
+#pragma unroll 4
+    for (int i = 0; i < trips; i++) {
+        const float t0 = (r0[G * i] + s1[G * i]) + oa;
+        const float t1 = (r1[G * i] + s2[G * i]) + oa;
+        if (t0 > best) {
+            best = t0;
+            at = 2 * i;
+        }
+        if (t1 > best) {
+            best = t1;
+            at = 2 * i + 1;
         }
     }
+    const int x = q & 3, prio = ((x & 1) << 1) | (x >> 1);
+    key = at < 0 ? INT_MAX : (prio << 24) | ((id + q + G * (at >> 1)) << 1) | (at & 1);
     for (int o = G >> 1; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, best, o);
         const int ok = __shfl_xor_sync(0xffffffffu, key, o);
@@ -131,6 +131,9 @@ __device__ __forceinline__ void viterbi_store(float best, int key, int a, int Q,
     Rb[o] = bc;
     Mtb[o] = bj;
 }
+
+// How far past the chain's last child the G lanes of a node read, when 32 / G nodes NC apart share a warp's trips.
+__host__ __device__ inline int viterbi_overshoot(int G, int NC) { return G - 1 + NC * (32 / G - 1); }
 
 __global__ void __launch_bounds__(kVitThreads, 1)
     viterbi_cluster_kernel(const float *__restrict__ ob_lprob, const float *__restrict__ links,
@@ -193,14 +196,17 @@ __global__ void __launch_bounds__(kVitThreads, 1)
     // the loop would make every cluster barrier (a release) wait for it to reach L2
     float *own_v = lk1 + (size_t)rows_cap * lk_stride;       // [rows_cap][Q]
     int *own_k = reinterpret_cast<int *>(own_v + (size_t)rows_cap * Q);  // [rows_cap][Q]
+    float *s_oa = reinterpret_cast<float *>(own_k + (size_t)rows_cap * Q);  // [rows_cap] ob of this CTA's nodes
 
     for (int r = warp; r < my_rows; r += kVitWarps) {
         const int id = crank + NC * r;
         const float *row = lkb + (size_t)(2 * id + 1) * 2 * L;
         const float olf = id >= 1 ? __ldg(ob + 2 * id) : neg_inf();  // C[a-1][1] = ob[a-1] (pcfg_viterbi.cu:203-205)
-        for (int ci = id + lane; ci < Mb; ci += 32) {
-            lk0[r * lk_stride + ci] = __ldg(row + 2 * ci + 1) + 0.f;
-            lk1[r * lk_stride + ci] = __ldg(row + L + 2 * ci + 1) + olf;
+        if (lane == 0) s_oa[r] = __ldg(ob + 2 * id + 1);
+#pragma unroll 4
+        for (int ci = id + lane; ci < lk_stride; ci += 32) {
+            lk0[r * lk_stride + ci] = ci < Mb ? __ldg(row + 2 * ci + 1) + 0.f : neg_inf();
+            lk1[r * lk_stride + ci] = ci < Mb ? __ldg(row + L + 2 * ci + 1) + olf : neg_inf();
         }
     }
     __shared__ __align__(8) uint64_t col_bar[2];
@@ -220,10 +226,12 @@ __global__ void __launch_bounds__(kVitThreads, 1)
     if (NC > 1) cluster.sync(); else __syncthreads();
     if (ctid == 0) Sb[(size_t)(m - 1) * Q + 1] = __ldg(ob + (m - 1));
 
-    // G lanes share a node, as few as still let the warps take all of this CTA's nodes in one pass (a second pass
-    // costs a step more than the longer scan per lane does); lane q < NC of a group also sends the result to CTA q
+    // G lanes share a node, as few as still let half the warps take all of this CTA's nodes in one pass: the kernel is
+    // bound by instruction issue, and a node's fixed costs are paid per warp (58 lengths, 60 nodes per CTA: 83 us with 16
+    // warps and G = 8, 100 us with 32 and G = 16, 86 us with 8 and G = 4; a second pass costs more than either).  Lane
+    // q < NC of a group also sends the result to CTA q
     int G = 32;
-    while ((32 / G) * kVitWarps < my_rows && (G >> 1) >= 4 && (G >> 1) >= NC) G >>= 1;
+    while (((32 / G) * kVitActive < my_rows || Mb + viterbi_overshoot(G, NC) > lk_stride) && (G >> 1) >= 4 && (G >> 1) >= NC) G >>= 1;
     const int RW = 32 / G, q = lane % G, sub = lane / G;  // RW nodes per warp
     const uint32_t rcol = NC > 1 && q < NC ? dsm_map_to_cta(dsm_smem_u32(col), q) : 0;  // this CTA's columns as CTA q maps them
     const uint32_t rbar0 = NC > 1 && q < NC ? dsm_map_to_cta(dsm_smem_u32(&col_bar[0]), q) : 0;
@@ -240,12 +248,12 @@ __global__ void __launch_bounds__(kVitThreads, 1)
         for (int r0w = warp * RW; r0w < my_rows; r0w += kVitWarps * RW) {
             const int r = r0w + sub;
             const bool live = r < my_rows;
-            const int rr = live ? r : 0, id = crank + NC * rr;
-            const float *r0 = lk0 + rr * lk_stride, *r1 = lk1 + rr * lk_stride;
+            const int rr = live ? r : r0w, id = crank + NC * rr;
+            const int trips = (Mb - (crank + NC * r0w) + G - 1) / G;  // of the warp's first node, which has most children
+            const float *r0 = lk0 + rr * lk_stride + id + q, *r1 = lk1 + rr * lk_stride + id + q;
             float best;
             int key;
-            viterbi_node_group(live, id, Mb, q, G, __ldg(ob + 2 * id + 1), S1, S2, [&](int ci) { return r0[ci]; },
-                               [&](int ci) { return r1[ci]; }, best, key);
+            viterbi_node_group(id, trips, q, G, s_oa[rr], r0, r1, S1 + id + q, S2 + id + q, best, key);
             if (live) {
                 if (NC > 1) {  // into every CTA's column, counted on that CTA's barrier of this length
                     if (q < NC) dsm_store_async(rcol + 4u * ((len & 3) * cs + id), best, (len & 1) ? rbar1 : rbar0);
@@ -419,7 +427,6 @@ int launch_viterbi(const float *ob, const float *links, const int64_t *ol, int B
     if (L < 8) return PCFGNAT_ERR_INVALID_ARGUMENT;  // column 1 of an [L][L/4] table must exist
     const int Mc = main_slots(L, 1), Q = L / 4;
     const int cs = (Mc + 3) / 4 * 4;
-    const int lk_stride = (Mc + 31) / 32 * 32 + 1;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // Cluster size: as many CTAs per sentence (up to 8) as still lets all sentences run at once; more when
@@ -438,7 +445,18 @@ int launch_viterbi(const float *ob, const float *links, const int64_t *ol, int B
     if (dp_kernel_choice() == kDpRows) nc = 32;  // skips the loop below
     for (; nc <= 16; nc *= 2) {
         const int rows_cap = (Mc + nc - 1) / nc;  // also right for mixed widths: nc is 1 there, every CTA may hold a chain
-        const size_t smem = ((size_t)4 * cs + (size_t)2 * rows_cap * lk_stride + (size_t)2 * rows_cap * Q) * sizeof(float);
+        // rows long enough for the lanes a full chain takes (shorter ones take more where they fit), and with the rows of a
+        // warp's nodes in different banks where there is room for that
+        const int width = wide >= 0 && nc == 1 ? 2 : nc;
+        int G = 32;
+        while ((32 / G) * kVitActive < rows_cap && (G >> 1) >= 4 && (G >> 1) >= width) G >>= 1;
+        const int least = Mc + viterbi_overshoot(G, width);
+        int lk_stride = (least + width - G % 32 + 31) / 32 * 32 + G % 32 - width;
+        const auto bytes = [&] {
+            return ((size_t)4 * cs + (size_t)2 * rows_cap * lk_stride + (size_t)2 * rows_cap * Q + rows_cap) * sizeof(float);
+        };
+        if (bytes() > (size_t)kSmemLimit - 1024) lk_stride = least | 1;
+        const size_t smem = bytes();
         if (smem > (size_t)kSmemLimit - 1024) continue;
         if (ensure_dynamic_smem(viterbi_cluster_kernel, smem) != cudaSuccess) return PCFGNAT_ERR_CUDA;
         if (nc > 8 && cudaFuncSetAttribute(viterbi_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=

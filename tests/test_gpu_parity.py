@@ -252,6 +252,45 @@ def test_viterbi_tie_breaking(vit_kernel, ops, syn):
     assert (np.isfinite(So).sum() > 100)
 
 
+@pytest.mark.parametrize("B, L", [(1, 8), (1, 140), (3, 66), (60, 130), (100, 66), (100, 256), (150, 34), (40, 262), (5, 515)])
+def test_viterbi_table_and_trace_edges(ops, syn, monkeypatch, B, L):
+    """Tables bit for bit those of the kernel that reads the transitions from global memory, and the back-trace the
+    host restatement's, at the numbers of lanes per node, cluster sizes and shared clusters that the library picks, with
+    ties, infinite and NaN transitions, short sentences and a length out of range."""
+    import importlib
+
+    monkeypatch.delenv("PCFGNAT_DP_KERNEL", raising=False)
+    monkeypatch.delenv("PCFGNAT_DP_CLUSTER_SIZE", raising=False)
+    g = torch.Generator(DEV).manual_seed(L * 3 + B)
+    ob = -torch.randint(1, 6, (B, L), device=DEV, generator=g).float() / 4
+    links = -torch.randint(1, 8, (B, L, 2, L), device=DEV, generator=g).float() / 4
+    at = torch.arange(L, device=DEV)
+    links.masked_fill_((at[None, :] <= at[:, None])[None, :, None, :], float("-inf"))
+    links[0, 1, 0, 3:5], links[B // 2, 3] = float("nan"), float("-inf")
+    ol = torch.randint(2, L + 1, (B,), device=DEV, generator=g)
+    ol[0], ol[-1] = 2 if B > 2 else L, L
+    if B > 3:
+        ol[1] = L + 1
+    k = ops.get_pcfg_kernel()
+    got = k.pcfg_viterbi(ob, links, ol, 1)
+    monkeypatch.setenv("PCFGNAT_DP_KERNEL", "rows")
+    want = k.pcfg_viterbi(ob, links, ol, 1)
+    assert np.array_equal(_bits(got[0].cpu().numpy()), _bits(want[0].cpu().numpy()))
+    assert all(torch.equal(x, y) for x, y in zip(got[1:], want[1:])) and torch.isfinite(got[0]).any()
+    ok = ol <= L
+    S, R, Lt, Mt = (t[ok] for t in got)
+    lm = importlib.import_module("pcfg_nat_b200.support_tree").get_mask(L, 1)[0].long()
+    tok = torch.randint(1, 9, (int(ok.sum()), L), device=DEV, generator=g)
+    pen = torch.arange(L // 4, device=DEV).float()
+    ops.read_status(DEV)
+    out, cnt, pred = k.viterbi_decode_device(S, pen, ol[ok], Lt, R, Mt, tok, lm.to(DEV), 1)
+    host = [t.cpu().numpy() for t in (pred, ol[ok], Lt, R, Mt, tok)]
+    for i in range(len(pred)):
+        row = oracle.viterbi_decoding(*[t[i:i + 1] for t in host], lm.numpy(), 1)[0].astype(np.int64)
+        assert int(cnt[i]) == len(row) and out[i].cpu().tolist() == row.tolist() + [1] * (L - len(row))
+    assert ops.read_status(DEV) == 0
+
+
 @pytest.mark.parametrize("name", ["ref_viterbi_ragged.npz", "ref_viterbi_mid.npz"])
 def test_viterbi_against_reference_golden(vit_kernel, ops, name):
     g = _g(name)
