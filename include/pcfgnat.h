@@ -350,6 +350,12 @@ int pcfgnat_links_from_scores(const float *ac, const float *bc, const float *qm,
  * callers that stage batches from host memory: it halves the bytes the largest input sends over PCIe. */
 int pcfgnat_copy_links_main_rows(void *dst, const void *src, int B, int L, int max_left, void *stream);
 
+/* Rows of H elements (a multiple of 8, 16-byte aligned) around pcfgnat_proj_backward_gemms.  to_bf16 != 0: dst [n][H] bf16
+ * = src [other_rows][H] f16 at rows index[i] (int64; NULL: row i).  Else: dst [other_rows][H] f16 at rows index[i] = src [n][H]
+ * f32, the other rows untouched.  An index out of range gives zeros / is skipped. */
+int pcfgnat_convert_rows(const void *src, const int64_t *index, int64_t n, int H, int64_t other_rows, int to_bf16, void *dst,
+                         void *stream);
+
 /* Copies n (at most 16) device tensors in one launch: dst[i] <- src[i], bytes[i] each; with odd_rows[i] > 0 only the
  * rows 1, 3, 5, ... of that many bytes (links [B][L][2][L] with an even L: its main-chain rows, 8 L bytes each).  All
  * four arrays are HOST arrays, read before the call returns.  PCFGNAT_ERR_UNSUPPORTED, with nothing copied, when a

@@ -39,6 +39,7 @@ SIGNATURES = {
     "pcfgnat_links_backward": (c_int, [c_void] * 13 + [c_int] * 6 + [c_void] * 8),
     "pcfgnat_links_from_scores": (c_int, [c_void] * 11 + [c_int] * 6 + [c_void] * 2),
     "pcfgnat_copy_links_main_rows": (c_int, [c_void] * 2 + [c_int] * 3 + [c_void]),
+    "pcfgnat_convert_rows": (c_int, [c_void] * 2 + [c_i64, c_int, c_i64, c_int] + [c_void] * 2),
     "pcfgnat_copy_batch": (c_int, [c_int] + [c_void] * 5),
     "pcfgnat_plan_real_rows": (c_int, [c_void] + [c_int] * 4 + [c_void] + [c_int]),
     "pcfgnat_copy_real_rows": (c_int, [c_void] * 3 + [c_int] * 3 + [c_size] + [c_int] + [c_void] * 2),

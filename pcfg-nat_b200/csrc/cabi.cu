@@ -434,6 +434,13 @@ int pcfgnat_copy_links_main_rows(void *dst, const void *src, int B, int L, int m
     return PCFGNAT_OK;
 }
 
+int pcfgnat_convert_rows(const void *src, const int64_t *index, int64_t n, int H, int64_t other_rows, int to_bf16, void *dst,
+                         void *stream) {
+    PCFGNAT_API_RANGE();
+    if (n < 0 || H < 1 || other_rows < 0 || (n && (!src || !dst))) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    return launch_convert_rows(src, index, n, H, other_rows, to_bf16, dst, static_cast<cudaStream_t>(stream));
+}
+
 int pcfgnat_copy_batch(int n, void *const *dst, const void *const *src, const size_t *bytes, const size_t *odd_rows,
                        void *stream) {
     PCFGNAT_API_RANGE();

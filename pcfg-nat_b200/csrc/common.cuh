@@ -205,6 +205,8 @@ int launch_glance_select(const int64_t *path, const int64_t *pred, const int64_t
                          int64_t *glance_num, uint8_t *keep, int64_t *glat_prev, cudaStream_t st);
 int launch_force_emit(const float *match, const uint8_t *matchmask, const uint8_t *keep, int B, int L, int T, float *out,
                       cudaStream_t st);
+int launch_convert_rows(const void *src, const int64_t *index, long long n, int H, long long other_rows, int to_bf16, void *dst,
+                        cudaStream_t st);
 int launch_force_emit_grad(const float *grad, const uint8_t *keep, int B, int L, int T, float *out, cudaStream_t st);
 
 size_t proj_workspace_bytes(int B, int L, int T, int V);

@@ -543,6 +543,37 @@ class _Kernel:
         _cabi.check(rc, "pcfgnat_copy_links_main_rows")
 
     @staticmethod
+    def rows_to_bf16(src, index=None):
+        """bf16 copy of the rows ``index`` (int64; all of them without) of a [rows, H] tensor, in one pass."""
+        if src.dtype != torch.float16 or not src.is_cuda or src.shape[1] % 8 or src.data_ptr() % 16 or not src.is_contiguous():
+            return (src if index is None else src.index_select(0, index)).to(torch.bfloat16).contiguous()
+        index = index.contiguous() if index is not None else None
+        n = src.shape[0] if index is None else index.shape[0]
+        with torch.cuda.device(src.device):
+            out = torch.empty((n, src.shape[1]), dtype=torch.bfloat16, device=src.device)
+            rc = _cabi.lib().pcfgnat_convert_rows(src.data_ptr(), None if index is None else index.data_ptr(), n, src.shape[1],
+                                                  src.shape[0], 1, out.data_ptr(), _stream(src.device))
+        _cabi.check(rc, "pcfgnat_convert_rows")
+        return out
+
+    @staticmethod
+    def rows_from_f32(src, dst, index=None):
+        """Writes the float32 rows [n, H] into the rows ``index`` (int64; the first n without) of ``dst`` [rows, H]."""
+        if dst.dtype != torch.float16 or src.shape[1] % 8 or dst.data_ptr() % 16 or src.data_ptr() % 16 or \
+                not (src.is_contiguous() and dst.is_contiguous()) or src.dtype != torch.float32:
+            if index is None:
+                dst[:src.shape[0]].copy_(src)
+            else:
+                dst.index_copy_(0, index, src.to(dst.dtype))
+            return dst
+        index = index.contiguous() if index is not None else None
+        with torch.cuda.device(dst.device):
+            rc = _cabi.lib().pcfgnat_convert_rows(src.data_ptr(), None if index is None else index.data_ptr(), src.shape[0],
+                                                  src.shape[1], dst.shape[0], 0, dst.data_ptr(), _stream(dst.device))
+        _cabi.check(rc, "pcfgnat_convert_rows")
+        return dst
+
+    @staticmethod
     def copy_batch(pairs, odd_rows_of=None):
         """Copies every (dst, src) pair of contiguous CUDA tensors of one device, same shape and type, in one launch on
         the current stream; of the pair whose dst is ``odd_rows_of`` (transitions [B, L, 2, L], L even) only the
@@ -996,6 +1027,10 @@ class DagLogsoftmaxGatherFunc(Function):
 dag_logsoftmax_gather_inplace = DagLogsoftmaxGatherFunc.apply
 
 
+def _bf16(t):
+    return get_pcfg_kernel().rows_to_bf16(t) if t.dtype == torch.float16 else t.to(torch.bfloat16).contiguous()
+
+
 def proj_backward_products(dlogits, weight, rows):
     """(dlogits @ weight, dlogits.T @ rows) in float32 from bf16 d-logits [n, V], the projection weight [V, H] and the
     decoder states of the same n rows [n, H] (either may be None: that product is skipped).  On this library's
@@ -1005,8 +1040,7 @@ def proj_backward_products(dlogits, weight, rows):
     H = (weight if weight is not None else rows).shape[1]
     if V % 8 == 0 and H % 8 == 0:
         return get_pcfg_kernel().proj_backward_gemms(
-            dlogits, weight.to(torch.bfloat16).contiguous() if weight is not None else None,
-            rows.to(torch.bfloat16).contiguous() if rows is not None else None,
+            dlogits, _bf16(weight) if weight is not None else None, _bf16(rows) if rows is not None else None,
             want_rows=weight is not None, want_weight=rows is not None)
     d_rows = (dlogits @ weight.to(torch.bfloat16)).float() if weight is not None else None
     d_weight = (dlogits.t() @ rows.to(torch.bfloat16)).float() if rows is not None else None
@@ -1043,14 +1077,14 @@ class ProjLogsoftmaxGatherFunc(Function):
             idx = None
         else:  # the real graph nodes only
             dl, idx = k.proj_dlogits(hidden, weight, targets, ol, tl, lse, grad_match.contiguous(), n_rows=ctx.n_rows)
-            rows = hidden.reshape(B * L, H).index_select(0, idx) if need_w else None
+            rows = k.rows_to_bf16(hidden.reshape(B * L, H), idx) if need_w else None
         d_rows, d_weight = proj_backward_products(dl, weight if need_h else None, rows if need_w else None)
         if need_h:
             if idx is None:
                 d_hidden = d_rows.to(hidden.dtype).view(B, L, H)
             else:
                 d_hidden = torch.zeros((B * L, H), dtype=hidden.dtype, device=hidden.device)
-                d_hidden.index_copy_(0, idx, d_rows.to(hidden.dtype))
+                k.rows_from_f32(d_rows, d_hidden, idx)
                 d_hidden = d_hidden.view(B, L, H)
         if need_w:
             d_weight = d_weight.to(weight.dtype)

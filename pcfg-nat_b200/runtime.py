@@ -420,10 +420,10 @@ class LossStep(_GraphedStep):
             return out
         n = self.n_rows if self.n_rows is not None else int(self.output_length.clamp(min=0, max=self.L).sum())
         dl, idx = self.dlogits[:n], self.row_index[:n]
-        rows = self.hidden.view(self.B * self.L, self.H).index_select(0, idx)
+        rows = self.kernel.rows_to_bf16(self.hidden.view(self.B * self.L, self.H), idx)
         d_rows, d_weight = ops.proj_backward_products(dl, self.weight_bf16, rows)
         self.d_hidden.zero_()
-        self.d_hidden.index_copy_(0, idx, d_rows.to(torch.float16))
+        self.kernel.rows_from_f32(d_rows, self.d_hidden, idx)
         d_weight = d_weight.to(torch.float16)
         self._ev_ran.record(torch.cuda.current_stream(self.device))  # the GEMMs still read the step's buffers
         return (*out, self.d_hidden.view(self.B, self.L, self.H), d_weight)

@@ -1024,6 +1024,28 @@ def test_reference_order_table_edges(ops, monkeypatch, B, L, T):
     ops.read_status(DEV)
 
 
+@pytest.mark.parametrize("H", [8, 64, 520, 12])
+def test_convert_rows(ops, H):
+    """Gather to bf16 and scatter from float32 with the roundings of torch's conversions, with infinities, NaN and
+    denormals; a row length that the kernels do not take goes through torch."""
+    k = ops.get_pcfg_kernel()
+    g = torch.Generator(DEV).manual_seed(H)
+    src = torch.randn(301, H, device=DEV, generator=g).half()
+    src[5, 0], src[6, 1], src[7, 2], src[8, 3] = float("inf"), float("-inf"), float("nan"), 6e-8
+    index = torch.randperm(301, device=DEV, generator=g)[:123]
+    bits = lambda t: t.view(torch.int16)  # noqa: E731
+    assert torch.equal(bits(k.rows_to_bf16(src)), bits(src.to(torch.bfloat16)))
+    assert torch.equal(bits(k.rows_to_bf16(src, index)), bits(src[index].to(torch.bfloat16)))
+    grad = torch.randn(123, H, device=DEV, generator=g) * 1e5
+    grad[0, 0] = 1e-9
+    want = torch.full((301, H), -2.0, dtype=torch.float16, device=DEV)
+    got = k.rows_from_f32(grad, want.clone(), index)
+    want[index] = grad.half()
+    assert torch.equal(bits(got), bits(want))
+    assert torch.equal(bits(k.rows_from_f32(grad, torch.zeros(123, H, dtype=torch.float16, device=DEV))), bits(grad.half()))
+    assert k.rows_to_bf16(src[:0]).shape == (0, H)
+
+
 def test_copy_batch(ops):
     """Tensors of one byte to several blocks, at and off 16- and 4-byte boundaries, the main-chain rows of transitions,
     empty and self copies; overlapping pairs and more pairs than a launch takes are refused with nothing copied."""
