@@ -309,7 +309,7 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" 
 // and columns lie 16 apart.  A block makes the same tile of `heads` heads, one after the other, the next chunk (or
 // head) in flight while this one is multiplied.  A tile without a cell that anybody reads (children at or below the
 // parents, padding: six tiles in ten of a ragged batch) is left alone; the test looks at a quarter of the tile's pairs
-// at a time, so that a tile in use rarely pays for more than that.  90 sentences, M = 161, 8 x 64 features: 180 us; 296 us with a block per
+// at a time, so that a tile in use rarely pays for more than that.  90 sentences, M = 161, 8 x 64 features: 172 us; 296 us with a block per
 // head and nothing in flight, 384 us as 64 x 64 tiles of 4 x 4 outputs, every tile formed.
 constexpr int kScoreRows = 128, kScoreCols = 64, kScoreK = 32, kScorePitch = kScoreK + 4;
 constexpr int kScoreStage = (kScoreRows + kScoreCols) * kScorePitch;  // floats; two of them
@@ -320,18 +320,24 @@ __global__ void __launch_bounds__(256, 2)
     const int groups = (H + heads - 1) / heads, b = blockIdx.z / groups, h0 = (blockIdx.z - b * groups) * heads;
     const int r0 = blockIdx.y * kScoreRows, c0 = blockIdx.x * kScoreCols, tid = threadIdx.x;
     if (masks.nonpad != nullptr) {
+        __shared__ int s_row[kScoreRows], s_col[kScoreCols];  // node of a row or column; -1: nobody's, -2: every node's
         const uint8_t *np = masks.nonpad + (size_t)b * masks.L;
+        if (tid < kScoreRows) {
+            const int row = r0 + tid;
+            // row M is the left option "none", which every node shares
+            s_row[tid] = row > 2 * M ? -1 : row == M ? -2 : masks.nodes[row < M ? row : row - M - 1];
+        } else if (tid < kScoreRows + kScoreCols) {
+            const int s = c0 + tid - kScoreRows, c = s < M ? masks.nodes[s] : -1;
+            s_col[tid - kScoreRows] = c >= 0 && np[c] && masks.main_chain[c] ? c : -1;
+        }
+        __syncthreads();
         bool needed = false;
         for (int part = 0; part < 4 && !needed; part++) {  // rows part, part + 4, ... of the tile
             bool mine = false;
 #pragma unroll
-            for (int i = tid; i < kScoreRows / 4 * kScoreCols; i += 256) {
-                const int row = r0 + part + i / kScoreCols * 4, s = c0 + i % kScoreCols;
-                if (row > 2 * M || s >= M) continue;
-                const int c = masks.nodes[s];
-                if (!np[c] || !masks.main_chain[c]) continue;
-                // row M is the left option "none", which every node shares
-                mine |= row == M || !masks.right_mask[(size_t)masks.nodes[row < M ? row : row - M - 1] * masks.L + c];
+            for (int i = 0; i < kScoreRows / 4 * kScoreCols / 256; i++) {
+                const int at = tid + 256 * i, a = s_row[part + at / kScoreCols * 4], c = s_col[at % kScoreCols];
+                if (a != -1 && c >= 0) mine |= a == -2 || !__ldg(masks.right_mask + (size_t)a * masks.L + c);
             }
             needed = __syncthreads_or(mine);
         }
@@ -539,8 +545,8 @@ __global__ void __launch_bounds__(256)
 // shared-memory loads per 32 FMAs, and no shape is too large for it.  The X matrices are zero wherever a child is not
 // admissible (all children at or below the parent, padding): a chunk whose X are all zero is skipped, unless the
 // features beside it are not finite (0 x inf stays NaN).  90 sentences, M = 161, 8 x 64 features: 284 us (366 us
-// without the next chunk in flight); 3 095 us
-// with one thread per output reading its operands from global memory, as it was.
+// without the next chunk in flight); 3 095 us with one thread per output reading its operands from global memory, as
+// it was.
 constexpr int kFgThreads = 256, kFgTile = 64, kFgChunk = 32, kFgPitch = kFgChunk + 4;
 constexpr int kFgStage = 4 * kFgChunk * kFgTile;  // floats of one chunk: role 1, the larger of the two; two of them
 constexpr size_t kFgSmem = (2 * kFgStage + 4 * kFgTile) * sizeof(float);
