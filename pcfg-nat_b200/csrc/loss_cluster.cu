@@ -18,6 +18,9 @@
 // order with shuffles and every lane keeps the running sum of its virtual lane: the same additions
 // in the same order.  Lanes 0..3 are then combined (s0 + s2) + (s1 + s3).  max is order-free.
 //
+// inside_exact_kernel further below keeps that order with half or a quarter of a warp per node; it takes the shapes whose
+// terms fit shared memory beside the links.
+//
 // inside_cluster_kernel<TRIPS > 0> is the inside pass for callers that never see the table (the fused
 // forward + backward): same layout, but every lane keeps its own partial sum of exponentials and the warp
 // is reduced with a shuffle tree, exp and log are the hardware ex2 / lg2 approximations.  The table then

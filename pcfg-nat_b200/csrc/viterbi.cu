@@ -9,16 +9,16 @@
 //     t1 = ((links[a][1][c] + ob[a-1]) + S[c][len-2]) + ob[a]          (j = 1, leaf a-1)
 // The reference gives node id four threads x = 0..3; thread x scans c_id = id + x + 4k in increasing
 // k, t0 before t1, under strict '>', and the four are merged with shfl_down 2 then 1 under strict
-// '>'.  A maximum is order-free except for ties, so here a whole warp owns the node (lane l scans
-// c_id = id + l + 32 i, which is reference thread x = l & 3) and the reference's choice among equal
+// '>'.  A maximum is order-free except for ties, so here G = 4 to 32 lanes own the node (lane q scans
+// c_id = id + q + G i, which is reference thread x = q & 3) and the reference's choice among equal
 // values is reproduced by an explicit tie key: thread priority 0 > 2 > 1 > 3, then the smaller c,
 // then j = 0 before j = 1.  Values and backpointers are bit-exact.  Tables are indexed by node id;
 // R, Lt hold node ids (Lt = 0 for "no left child"), Mt holds j.
 //
 // viterbi_cluster_kernel spreads the nodes of a sentence over the CTAs of a thread-block cluster
 // (one cluster per sentence, sized so that the batch fills the GPU): every CTA keeps the rolling
-// columns of the whole chain, a warp that finishes a node stores its value into every CTA's copy
-// through distributed shared memory, and the cluster meets at a hardware barrier once per length.
+// columns of the whole chain, and the lanes that finish a node send its value into every CTA's copy with
+// st.async, counted on a barrier of the receiving CTA.
 // viterbi_global_kernel (one CTA per sentence, links read from global memory) takes the shapes
 // whose links do not fit the cluster's shared memory.
 //
