@@ -501,12 +501,13 @@ __device__ __forceinline__ bool inside_exact_steps(float *col, const float *lk0,
     return arrived;
 }
 
-template <int G>
+// Sixteen lanes per node while a CTA's nodes take one pass of 32 warps that way, eight for more.
+constexpr int kExactRows16 = 2 * kCWarps;
 __global__ void __launch_bounds__(kCThreads, 1)
     inside_exact_kernel(const float *__restrict__ match_all, const float *__restrict__ links,
                         const int64_t *__restrict__ ol, const int64_t *__restrict__ tl, int L, int T, float *S, float *C,
                         float *loss, int *status, int Mc, int Lt, int cs, int rows_cap, int lk_stride, int B, int wide,
-                        int xs, int active) {
+                        int xs, int slots) {
     extern __shared__ __align__(16) float smem[];
     cg::cluster_group cluster = cg::this_cluster();
     int crank = (int)cluster.block_rank();
@@ -585,8 +586,12 @@ __global__ void __launch_bounds__(kCThreads, 1)
     // all copies initialised before anybody stores into a neighbour's; also orders the -inf fill of the global table
     if (NC > 1) cluster.sync(); else __syncthreads();
     if (ctid == 0) Sb[(size_t)last * W + (n - 1)] = __ldg(mat + (size_t)(m - 1) * T + (n - 1));
-    const bool arrived = inside_exact_steps<G>(col, lk0, lk1, em0, eml, own, scratch, col_bar, n, Mb, my_rows, NC, crank, W,
-                                               cs, lk_stride, xs, active);
+    const bool arrived =
+        my_rows <= kExactRows16
+            ? inside_exact_steps<16>(col, lk0, lk1, em0, eml, own, scratch, col_bar, n, Mb, my_rows, NC, crank, W, cs, lk_stride,
+                                     xs, min(kCWarps, slots / 2))
+            : inside_exact_steps<8>(col, lk0, lk1, em0, eml, own, scratch, col_bar, n, Mb, my_rows, NC, crank, W, cs, lk_stride,
+                                    xs, min(kCWarps, slots / 4));
     if (!arrived && lane == 0) flag(status, PCFGNAT_STATUS_TIMEOUT);
     // no CTA leaves (its shared memory with it) while a peer may still send to it; every wait above is bounded
     if (NC > 1) cluster.sync();
@@ -943,46 +948,45 @@ int launch_inside(const float *match_all, const float *links, const int64_t *ol,
     return PCFGNAT_ERR_UNSUPPORTED;
 }
 
-// Reference order with G lanes per node; PCFGNAT_ERR_UNSUPPORTED when the terms do not fit beside the links.
-template <int G>
+// Reference order with 16 or 8 lanes per node; PCFGNAT_ERR_UNSUPPORTED when the terms do not fit beside the links.
 int launch_exact(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B, int L, int T,
                  float *S, float *C, float *loss, int *status, cudaStream_t st, int nc, int wide, bool mixed) {
-    constexpr int R = 32 / G;
     const int Mc = main_slots(L, 1), Lt = L - Mc, W = T + 2, cs = (Mc + 3) / 4 * 4;
     const int width = mixed ? 2 : nc;  // CTAs of a cluster
-    const int rows_cap = (Mc + nc - 1) / nc;
-    // a row is read up to G - 1 children past its last one, by the warp's later nodes up to (R - 1) nc more; the rows of a
-    // warp's nodes G banks apart
-    const int pad = G + (R - 1) * width, lk_stride = (Mc + pad + width - G + 31) / 32 * 32 + G - width;
-    const int xs = ((Mc + G - 1) / G * (G / 2) + 23) / 32 * 32 + 8;
+    const int rows_cap = (Mc + nc - 1) / nc, G = rows_cap <= kExactRows16 ? 16 : 8;
+    // a row is read up to G - 1 children past its last one, by the warp's later nodes up to (32 / G - 1) CTA counts more;
+    // the rows of a warp's nodes G banks apart
+    const int pad = G == 16 ? 16 + width : (8 + 3 * width > 16 + width ? 8 + 3 * width : 16 + width);
+    const int lk_stride = (Mc + pad + width - G + 31) / 32 * 32 + G - width;
+    const int xs = ((Mc + 15) / 16 * 8 + 23) / 32 * 32 + 8;  // what sixteen lanes need is enough for eight
     const size_t base = (((size_t)4 * cs + (size_t)2 * rows_cap * lk_stride + (size_t)3 * rows_cap * W) * sizeof(float) + 15) &
                         ~(size_t)15;
-    const size_t limit = (size_t)kSmemLimit - 1024, per_warp = (size_t)R * (4 * xs + 4) * sizeof(float);
+    const size_t limit = (size_t)kSmemLimit - 1024, per_node = (size_t)(4 * xs + 4) * sizeof(float);
     if (base >= limit) return PCFGNAT_ERR_UNSUPPORTED;
-    int active = (rows_cap + R - 1) / R;
-    if (active > kCWarps) active = kCWarps;
-    if ((size_t)active * per_warp > limit - base) active = (int)((limit - base) / per_warp);
-    if (active < 8 && active * R < rows_cap) return PCFGNAT_ERR_UNSUPPORTED;
-    size_t smem = base + active * per_warp;
+    // nodes in flight: all of a CTA's, as far as the warps and the room go (whole warps of either kind)
+    int slots = (rows_cap + 3) / 4 * 4;
+    if (slots > 4 * kCWarps) slots = 4 * kCWarps;
+    if ((size_t)slots * per_node > limit - base) slots = (int)((limit - base) / per_node) / 4 * 4;
+    if (slots < 32 && slots < rows_cap) return PCFGNAT_ERR_UNSUPPORTED;
+    size_t smem = base + slots * per_node;
     if (wide >= 0 && smem < (size_t)B * sizeof(int)) smem = (size_t)B * sizeof(int);  // the costs that rank the sentences
     const int clusters = mixed ? wide + (B - wide + 1) / 2 : B;
-    return launch_cluster(inside_exact_kernel<G>, clusters, width, smem, st, match_all, links, ol, tl, L, T, S, C, loss, status,
-                          Mc, Lt, cs, rows_cap, lk_stride, B, wide, xs, active);
+    return launch_cluster(inside_exact_kernel, clusters, width, smem, st, match_all, links, ol, tl, L, T, S, C, loss, status,
+                          Mc, Lt, cs, rows_cap, lk_stride, B, wide, xs, slots);
 }
 
 int launch_loss_fwd_cluster(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B,
                             int L, int T, float *S, float *C, float *loss, int *status, cudaStream_t st) {
     const int Mc = main_slots(L, 1);
     const ClusterGeometry g = cluster_geometry(B, Mc, T + 2);
-    if (g.nc >= 1 && g.nc <= 8) {
+    // Where a warp has a node to itself in every step (up to 32 nodes per CTA) the fewer trips of all its lanes are
+    // worth more: 8 sentences of 80 nodes on eight CTAs each 56 us against 66 with sixteen lanes per node, 16 of 128 213
+    // against 246; from 32 nodes on it turns: 32 of 128 on four CTAs 146 against 140, 45 of 80 on two 111 against 81.
+    const int rows = g.nc >= 1 ? (Mc + g.nc - 1) / g.nc : 0;
+    if (rows >= kCWarps && g.nc <= 8) {
         const int wide = g.nc == 1 ? mixed_width_count(B, Mc) : 0;
         const int order = wide > 0 ? wide : (long long)B * g.nc > sm_count() && B <= 256 ? B : -1;
-        // sixteen lanes while a CTA's nodes take one pass of 32 warps (a sentence of the mixed widths that has one CTA
-        // is among the cheap ones); eight for more nodes
-        const int rows = (Mc + g.nc - 1) / g.nc;
-        const bool sixteen = rows <= 64 || (wide > 0 && rows <= 96);
-        const int rc = sixteen ? launch_exact<16>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, g.nc, order, wide > 0)
-                               : launch_exact<8>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, g.nc, order, wide > 0);
+        const int rc = launch_exact(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, g.nc, order, wide > 0);
         if (rc != PCFGNAT_ERR_UNSUPPORTED) return rc;
     }
     return launch_inside<0>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st);
