@@ -111,6 +111,10 @@ __device__ __forceinline__ void viterbi_node_group(int id, int trips, int q, int
     }
     const int x = q & 3, prio = ((x & 1) << 1) | (x >> 1);
     key = at < 0 ? INT_MAX : (prio << 24) | ((id + q + G * (at >> 1)) << 1) | (at & 1);
+    if (G == 32) {  // a whole warp: two integer reductions instead of five rounds of two shuffles
+        warp_argmax(best, key, threadIdx.x & 31);
+        return;
+    }
     for (int o = G >> 1; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, best, o);
         const int ok = __shfl_xor_sync(0xffffffffu, key, o);
