@@ -62,6 +62,10 @@ __global__ void __launch_bounds__(kLookThreads)
     const bool fits = given >= 0 && given <= L;
     const int length = fits ? (int)given : 0;
     int *words = cluster.map_shared_rank(s_node, 0);
+    // Another CTA's shared memory exists once that CTA has started: the cluster meets before the first store into it.
+    // The barrier is split, so that a warp's first node is scanned meanwhile.
+    cluster.barrier_arrive();
+    bool met = false;  // uniform over the warp
     for (int a = 1 + rank * kLookWarps + warp; a < length; a += nc * kLookWarps) {
         const float *row = lkb + (size_t)a * 2 * L;
         const float left0 = lookahead ? obb[0] : 0.f, left1 = lookahead ? obb[a - 1] : 0.f;
@@ -94,6 +98,8 @@ __global__ void __launch_bounds__(kLookThreads)
                 key = ok;
             }
         }
+        if (!met) cluster.barrier_wait();
+        met = true;
         if (lane == 0) {
             if (key == INT_MAX) key = 0;
             const int k = key >= L, left = k ? a - 1 : 0;
@@ -104,7 +110,8 @@ __global__ void __launch_bounds__(kLookThreads)
             words[a] = word;
         }
     }
-    cluster.sync();
+    if (!met) cluster.barrier_wait();  // a warp without a node
+    cluster.sync();                    // the words are there
     if (rank != 0) return;
     int64_t *o = out + (size_t)b * cap;
     if (tid == 0) {

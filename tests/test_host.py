@@ -201,3 +201,42 @@ def test_plan_of_the_real_row_copies(pkg):
             assert len(runs) == k and int(sent.sum() - real.sum()) == sum(gaps[: len(free) - k])
         else:
             assert runs == free
+
+
+def _bodies(source, keyword):
+    """(name, body) of the functions of a .cu file whose declaration has ``keyword``, comments left out."""
+    source = re.sub(r"//[^\n]*", "", source)
+    for m in re.finditer(keyword, source):
+        brace, end = source.find("{", m.end()), source.find(";", m.end())
+        if brace < 0 or 0 <= end < brace:
+            continue  # a declaration
+        depth, at = 1, brace + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(source[at], 0)
+            at += 1
+        names = re.findall(r"(\w+)\s*\(", re.sub(r"__launch_bounds__\([^)]*\)", "", source[m.end():brace]))
+        if names:  # else a table of constants
+            yield names[0], source[brace:at]
+
+
+def test_kernels_meet_before_they_touch_a_peers_shared_memory():
+    """The shared memory of another block of a cluster may be accessed only once that block runs: every kernel with
+    remote stores has a barrier of the cluster before the first one."""
+    csrc = os.path.join(ROOT, "pcfg-nat_b200", "csrc")
+    remote = r"\b(?:dsm_store_async|store_async4|mbar_arrive_cluster)\s*\("
+    barrier = r"cluster\.sync\(\)|barrier_wait\(|cluster_sync_all\(\)"
+    seen = set()
+    for file in sorted(f for f in os.listdir(csrc) if f.endswith(".cu")):
+        source = open(os.path.join(csrc, file)).read()
+        callees = [name for name, body in _bodies(source, "__device__") if re.search(remote, body)]
+        for name, body in _bodies(source, "__global__"):
+            uses = [m.start() for m in re.finditer("|".join([remote] + [rf"\b{c}\s*[<(]" for c in callees]), body)]
+            for pointer in re.findall(r"(\w+) = cluster\.map_shared_rank", body):
+                uses += [m.start() for m in re.finditer(rf"\b{pointer}\[", body)]
+            if not uses:
+                continue
+            seen.add(name)
+            met = re.search(barrier, body)
+            assert met and met.start() < min(uses), f"{file}: {name}"
+    assert {"lookahead_decode_kernel", "viterbi_cluster_kernel", "inside_cluster_kernel", "inside_exact_kernel",
+            "outside_cluster_kernel", "inside_linear_kernel", "outside_linear_kernel", "proj_kernel"} <= seen, seen
