@@ -704,7 +704,9 @@ class _Kernel:
             raise RuntimeError("tree masks must cover prelen nodes")
         nonpad = prev_output_tokens.to(dev).ne(pad_index).to(torch.uint8).contiguous()
         # main-chain nodes: the only ones that have, or are, right children -> compact score matrices
-        if chain is None:
+        if chain is None and mc.is_inference():  # no version counter that would tell of a change: nothing is kept
+            chain = _Kernel.main_chain_slots(mc)
+        elif chain is None:
             key = (mc.data_ptr(), mc._version, L)
             cached = _main_chain_cache.get(key)
             if cached is None:

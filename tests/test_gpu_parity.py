@@ -1221,6 +1221,31 @@ def test_extract_links_and_gradient_at_tile_edges(pkg, ops, L, heads, dim, dtype
         assert err <= (2e-5 if x.dtype == torch.float32 else 1e-3) * y.grad.abs().max(), (tuple(x.shape), float(err))
 
 
+def test_extract_links_under_inference_mode(pkg, ops):
+    """Inference tensors have no version counter: masks made inside the mode (bool or host masks are converted there)
+    work, one that is changed in place there is read again, and a mask from outside the mode works in it."""
+    import importlib
+
+    L, heads, dim = 18, 2, 8
+    masks = importlib.import_module("pcfg_nat_b200.support_tree").get_mask(L, 1)
+    g = torch.Generator().manual_seed(3)
+    feats = [torch.randn(2, L, heads, dim, generator=g).to(DEV) for _ in range(3)] + [torch.randn(2, L, heads, generator=g).to(DEV)]
+    prev = torch.full((2, L), 3, device=DEV)
+    u8 = [m.to(DEV).ne(0).to(torch.uint8) for m in masks]
+    k = ops.get_pcfg_kernel()
+    want = k.extract_links(*feats, prev, 1, *u8)
+    shorter = u8[2].clone()
+    shorter[L - 3:] = 0
+    want_shorter = k.extract_links(*feats, prev, 1, u8[0], u8[1], shorter)
+    assert not torch.equal(want, want_shorter)
+    with torch.inference_mode():
+        inside = [m.to(DEV).ne(0).to(torch.uint8) for m in masks]
+        for given in ([m.bool() for m in masks], [m.to(DEV).bool() for m in masks], u8, inside):
+            assert torch.equal(k.extract_links(*feats, prev, 1, *given), want)
+        inside[2][L - 3:] = 0
+        assert torch.equal(k.extract_links(*feats, prev, 1, *inside), want_shorter)
+
+
 def test_decode_step_from_link_features(pkg, ops, syn):
     """DecodeStep fed with the projected link features gives what extract_links + the transition-fed step give."""
     import importlib
