@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(256)
     }
     auto term = [&](int h, int k, int s) { return (row.logit(h, k, s) - s_lse[h]) + s_lg[h]; };
     const float *grow = links_grad + ((size_t)b * p.L + a) * 2 * p.L;
-    // w of an admissible cell, or G itself (rare) below the floor of the mixture
+    // w of an admissible cell, or G itself (rare) below the floor of the mixture and where w leaves the floats
     auto weigh = [&](int k, int s, bool &rare) {
         rare = false;
         const float G = grow[(size_t)k * p.L + p.nodes[s]];
@@ -464,8 +464,9 @@ __global__ void __launch_bounds__(256)
         float sum = 0.f;
 #pragma unroll 8
         for (int h = 0; h < H; h++) sum = fmaf(row.exp_at(h, k, s), s_c[h], sum);
-        rare = !(sum > kMixtureFloor);
-        return rare ? G : G / sum;
+        const float w = G / sum;
+        rare = !(sum > kMixtureFloor && fabsf(w) < CUDART_INF_F);
+        return rare ? G : w;
     };
     if constexpr (KEEP > 0) {
         const int span = row.hi - row.lo;
@@ -477,7 +478,7 @@ __global__ void __launch_bounds__(256)
         }
         __syncthreads();
     }
-    // d lp of a cell: w e c, or formed from the log-probabilities where the sum is too small (-inf cells: nothing)
+    // d lp of a cell: w e c, or formed from the log-probabilities where that is out of range (-inf cells: nothing)
     auto share = [&](int h, int k, int s, float e) {
         float w;
         bool rare;

@@ -1246,6 +1246,39 @@ def test_extract_links_under_inference_mode(pkg, ops):
         assert torch.equal(k.extract_links(*feats, prev, 1, *inside), want_shorter)
 
 
+def _links_and_float64(pkg, ops, leaves, length, G_of):
+    """(links, gradients of the leaves, both again by autograd in float64): G_of(float64 links) weighs the finite cells."""
+    import importlib
+
+    L = leaves[0].shape[1]
+    masks = importlib.import_module("pcfg_nat_b200.support_tree").get_mask(L, 1)
+    prev = torch.where(torch.arange(L)[None, :] < length[:, None], 3, 1)
+    ref = [t.double().requires_grad_() for t in leaves]
+    want = pyref.extract_links(*ref, prev, 1, *masks, dtype=torch.float64, floor=-1e30)
+    ok = want > -1e29
+    G = G_of(want.detach()).float() * ok
+    torch.where(ok, want, 0.0).mul(G).sum().backward()
+    ours = [t.to(DEV).requires_grad_() for t in leaves]
+    links = ops.get_pcfg_kernel().extract_links(*ours, prev.to(DEV), 1, *masks)
+    (torch.where(ok.to(DEV), links, 0.0) * G.to(DEV)).sum().backward()
+    assert torch.equal(torch.isfinite(links).cpu(), ok)
+    return links.detach().cpu().double()[ok], [t.grad.cpu().double() for t in ours], want.detach()[ok], [t.grad for t in ref]
+
+
+@pytest.mark.parametrize("heads", [1, 2])
+def test_links_gradient_of_improbable_cells_with_large_weights(pkg, ops, heads):
+    """Gradients of 1e12 at transitions of e-69 to e-61, where gradient / probability leaves the floats.  Logits of up to 100
+    in float32 (spacing 8e-6, a handful of roundings) put 1e-4 on a probability."""
+    g = torch.Generator().manual_seed(heads)
+    leaves = [4 * torch.randn(2, 40, heads, 8, generator=g) for _ in range(3)] + [torch.randn(2, 40, heads, generator=g)]
+    weights = lambda want: torch.where((want > -69) & (want < -61), 1e12, 0.0)  # noqa: E731
+    got, grads, want, ref = _links_and_float64(pkg, ops, leaves, torch.tensor([40, 31]), weights)
+    assert int((weights(want) > 0).sum()) > 3
+    torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-4)
+    for x, y in zip(grads, ref):
+        assert (x - y).abs().max() <= 1e-4 * y.abs().max(), tuple(x.shape)
+
+
 def test_decode_step_from_link_features(pkg, ops, syn):
     """DecodeStep fed with the projected link features gives what extract_links + the transition-fed step give."""
     import importlib
