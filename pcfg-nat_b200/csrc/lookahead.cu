@@ -68,7 +68,9 @@ __global__ void __launch_bounds__(kLookThreads)
     bool met = false;  // uniform over the warp
     for (int a = 1 + rank * kLookWarps + warp; a < length; a += nc * kLookWarps) {
         const float *row = lkb + (size_t)a * 2 * L;
-        const float left0 = lookahead ? obb[0] : 0.f, left1 = lookahead ? obb[a - 1] : 0.f;
+        // products and sums rounded one by one, as the reference's element-wise operators do it: fused, a near-tie may
+        // go to another child
+        const float left0 = lookahead ? __fmul_rn(obb[0], beta) : 0.f, left1 = lookahead ? __fmul_rn(obb[a - 1], beta) : 0.f;
         float best = neg_inf();
         int key = INT_MAX;
         for (int i0 = lane; i0 < 2 * L; i0 += 8 * 32) {  // a lane sees its candidates in increasing index order
@@ -82,7 +84,7 @@ __global__ void __launch_bounds__(kLookThreads)
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 const int i = i0 + 32 * j;
-                const float x = lookahead ? fmaf(i >= L ? left1 : left0, beta, fmaf(o[j], beta, v[j])) : v[j];
+                const float x = lookahead ? __fadd_rn(__fadd_rn(v[j], __fmul_rn(o[j], beta)), i >= L ? left1 : left0) : v[j];
                 if (x > best || (key == INT_MAX && !isnan(x))) {  // strict: the first maximum stays; -inf counts as a value
                     best = x;
                     key = i;

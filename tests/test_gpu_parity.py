@@ -1654,6 +1654,34 @@ def test_lookahead_decode_cluster_edges(pkg, ops, L):
     assert ops.read_status(DEV) != 0 and int(cnt[4]) == 0 and (out[4] == 1).all()
 
 
+def test_lookahead_decode_near_ties(pkg, ops):
+    """Two candidates per node whose scores differ by the last bit or not at all, with a beta that is not a power of two:
+    the choice is the one of separately rounded products and sums, not of fused ones."""
+    import importlib
+
+    B, L, beta = 64, 34, 0.7
+    lm = importlib.import_module("pcfg_nat_b200.support_tree").get_mask(L, 1)[0]
+    g = torch.Generator().manual_seed(5)
+    ob = torch.randn(B, L, generator=g) * 3 - 6
+    links = torch.full((B, L, 2, L), float("-inf"))
+    fused_differs = 0
+    for a in range(1, L - 4, 2):
+        c1, c2 = a + 2, a + 4
+        links[:, a, 0, c1] = torch.randn(B, generator=g) - 4
+        links[:, a, 0, c2] = (links[:, a, 0, c1] + ob[:, c1] * beta) - ob[:, c2] * beta
+        exact = [(links[:, a, 0, c].double() + ob[:, c].double() * torch.tensor(beta).double()).float() for c in (c1, c2)]
+        split = [links[:, a, 0, c] + ob[:, c] * beta for c in (c1, c2)]
+        fused_differs += int(((exact[1] > exact[0]) != (split[1] > split[0])).sum())
+    assert fused_differs > 50
+    tok = torch.arange(L).expand(B, L) + 4
+    ol = torch.full((B,), L)
+    out, cnt = ops.get_pcfg_kernel().lookahead_decode_device(links.to(DEV), ob.to(DEV), tok.to(DEV), ol.to(DEV), lm.to(DEV), 1,
+                                                             beta, "lookahead")
+    rows = pyref.lookahead_decode(links, ob, tok, ol, lm.bool(), 1, beta)
+    for i, r in enumerate(rows):
+        assert int(cnt[i]) == len(r) and out[i].cpu().tolist() == r + [1] * (L - len(r))
+
+
 def test_loss_step_from_link_features_matches_autograd_chain(pkg, ops, syn):
     """LossStep fed with the projected link features (transitions formed and differentiated inside the step) against
     the operators chained by autograd: extract_links -> cuda_pcfg_loss -> backward."""
