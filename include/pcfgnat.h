@@ -172,7 +172,9 @@ int pcfgnat_logsoftmax_gather(void *logits, int dtype, const int64_t *select_idx
 /* Its backward, in place: probs [rows][V] (the softmax probabilities the forward left) becomes the gradient of the
  * logits, -probs * sum_s grad_selected[s] + scatter(grad_selected); replaces the torch operators of
  * DagLogsoftmaxGatherFunc.backward (fs_plugins/custom_ops/pcfg_loss.py:168-180).  grad_selected [rows][slen] f32
- * contiguous; select_idx as above; an index out of range is skipped and flagged. */
+ * contiguous; select_idx as above; an index out of range is skipped and flagged.  slen <= 256: formed in float32 and
+ * rounded to the storage type once, always the same.  More columns are added to the rounded products one by one,
+ * atomically in the storage type: the order, and with it the last bits of repeated columns, may vary. */
 int pcfgnat_logsoftmax_gather_backward(void *probs, int dtype, const float *grad_selected, const int64_t *select_idx,
                                        int64_t stride_b, int64_t stride_l, int64_t stride_s, int64_t rows,
                                        int64_t rows_per_batch, int V, int slen, int *status, void *stream);

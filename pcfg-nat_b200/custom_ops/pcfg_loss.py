@@ -266,7 +266,8 @@ class _Kernel:
     @staticmethod
     def logsoftmax_gather_backward(probs, select_idx, grad_selected):
         """Turns the softmax probabilities [B, L, V] that ``logsoftmax_gather`` left into the gradient of the logits, in
-        place: -probs * sum(grad) + scatter(grad), formed in float32 (pcfg_loss.py:168-180)."""
+        place: -probs * sum(grad) + scatter(grad) (pcfg_loss.py:168-180).  Up to 256 columns are formed in float32 and
+        rounded once; more are added one by one in the type of ``probs``, in no fixed order, as scatter_add_ does."""
         _require_cuda()
         B, L, V = probs.shape
         if not probs.is_contiguous() or probs.dtype not in (torch.float32, torch.float16):
@@ -992,6 +993,9 @@ class CUDAPCFGViterbiFunc(Function):
 cuda_pcfg_viterbi = CUDAPCFGViterbiFunc.apply
 
 
+_GRAD_COLUMNS = 256  # selected columns up to which pcfgnat_logsoftmax_gather_backward adds in a fixed order
+
+
 class DagLogsoftmaxGatherFunc(Function):
     """log-softmax + gather with the logits buffer reused for the backward: forward overwrites
     ``word_ins_out`` with softmax probabilities when it needs a gradient; backward turns that
@@ -1019,7 +1023,10 @@ class DagLogsoftmaxGatherFunc(Function):
         ctx.has_backward = True
         probs, idx = ctx.saved_tensors
         # d logits = -p * sum_s g_s + scatter(g): done in the saved buffer
-        if torch.is_grad_enabled() and grad_output.requires_grad:  # create_graph: operators autograd can follow
+        # as torch's operators where autograd has to follow them (create_graph), and where the kernel would add atomically
+        # although the program asks for deterministic algorithms
+        if torch.is_grad_enabled() and grad_output.requires_grad or \
+                idx.shape[-1] > _GRAD_COLUMNS and torch.are_deterministic_algorithms_enabled():
             probs.mul_(grad_output.sum(-1, keepdim=True).neg_().to(probs.dtype))
             probs.scatter_add_(-1, idx, grad_output.to(probs.dtype))
             return probs, None

@@ -427,6 +427,32 @@ def test_logsoftmax_gather_backward(ops, dtype, V, slen):
         torch.testing.assert_close(got[1, 0].cpu().double(), want[1, 0], rtol=4 * eps, atol=4 * eps)
 
 
+@pytest.mark.parametrize("slen", [256, 257, 600])
+def test_logsoftmax_gather_backward_deterministic(ops, slen):
+    """Under torch's deterministic algorithms the gradient repeats itself bit for bit whatever the number of columns;
+    repeated columns in half precision, whose sum depends on the order."""
+    g = torch.Generator().manual_seed(slen)
+    B, L, V = 2, 64, 1000
+    logits = (3 * torch.randn(B, L, V, generator=g)).half()
+    idx = torch.randint(0, 5, (B, L, slen), generator=g).to(DEV)
+    grad = (torch.randn(B, L, slen, generator=g) * torch.logspace(-3, 2, slen)).to(DEV)
+    probs = torch.softmax(logits.to(DEV).double(), -1)
+    want = (probs * -grad.double().sum(-1, keepdim=True)).scatter_add_(-1, idx, grad.double())
+
+    def once():
+        x = logits.to(DEV).requires_grad_()
+        return torch.autograd.grad((ops.dag_logsoftmax_gather_inplace(x * 1, idx)[1] * grad).sum(), x)[0]
+
+    torch.use_deterministic_algorithms(True)
+    try:
+        first = once()
+        assert all(torch.equal(once(), first) for _ in range(8))
+    finally:
+        torch.use_deterministic_algorithms(False)
+    # at most slen + 2 roundings, each of half a unit (2^-11) of at most the row's sum of magnitudes
+    assert ((first.double() - want).abs() <= (slen + 2) * 2 ** -11 * grad.abs().double().sum(-1, keepdim=True)).all()
+
+
 def test_fused_loss_many_sentences_mixed_cluster_widths(ops, syn, monkeypatch):
     """More sentences than half the SMs: the fused forward + backward runs its passes as cost-ordered clusters
     of two, which the costliest sentences have to themselves and the others share, one CTA each.  Loss and gradients against the oracle, with an
