@@ -590,9 +590,12 @@ __global__ void __launch_bounds__(kFgThreads, 2)
                                const int *__restrict__ nodes, int M, int L, int H, int D, int vec, float *__restrict__ dq,
                                float *__restrict__ dkl, float *__restrict__ dkr) {
     extern __shared__ __align__(16) float s_tiles[];
-    const int role = blockIdx.x & 1, r0 = (blockIdx.x >> 1) * kFgTile, d0 = blockIdx.y * kFgTile;
-    const size_t bh = blockIdx.z;
-    const int b = blockIdx.z / H, h = blockIdx.z - b * H;
+    // blocks by (sentence, head), tile of d, tile of rows, role: along x, which alone takes more than 65 535
+    const unsigned per_d = 2 * ((M + kFgTile - 1) / kFgTile), d_tiles = (D + kFgTile - 1) / kFgTile;
+    const unsigned at_d = blockIdx.x / per_d, at_r = blockIdx.x - at_d * per_d;
+    const int role = at_r & 1, r0 = (at_r >> 1) * kFgTile, d0 = at_d % d_tiles * kFgTile;
+    const size_t bh = at_d / d_tiles;
+    const int b = (int)bh / H, h = (int)bh - b * H;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const float *x0 = X0 + bh * M * M, *x1 = X1 + bh * M * M;
     const float *q = qm + bh * M * D, *kl = klm + bh * (M + 1) * D, *kr = krm + bh * M * D;
@@ -796,9 +799,10 @@ int launch_links_backward(const float *links_grad, const float *ac, const float 
     if (cudaGetLastError() != cudaSuccess) return PCFGNAT_ERR_CUDA;
     if (M == 0) return PCFGNAT_OK;
     const int vec = D % 4 == 0 && on_16_bytes({qm, klm, krm});
-    const dim3 grid(2 * ((M + kFgTile - 1) / kFgTile), (D + kFgTile - 1) / kFgTile, B * H);
+    const long long grid = 2ll * ((M + kFgTile - 1) / kFgTile) * ((D + kFgTile - 1) / kFgTile) * B * H;
+    if (grid > INT32_MAX) return PCFGNAT_ERR_TOO_LARGE;
     if (ensure_dynamic_smem(links_features_grad_kernel, kFgSmem) != cudaSuccess) return PCFGNAT_ERR_CUDA;
-    links_features_grad_kernel<<<grid, kFgThreads, kFgSmem, st>>>(X0, X1, dab, qm, klm, krm, nodes, M, L, H, D, vec, dq, dkl, dkr);
+    links_features_grad_kernel<<<(unsigned)grid, kFgThreads, kFgSmem, st>>>(X0, X1, dab, qm, klm, krm, nodes, M, L, H, D, vec, dq, dkl, dkr);
     return cuda_rc(cudaGetLastError());
 }
 

@@ -1305,6 +1305,29 @@ def test_links_gradient_of_improbable_cells_with_large_weights(pkg, ops, heads):
         assert (x - y).abs().max() <= 1e-4 * y.abs().max(), tuple(x.shape)
 
 
+def test_links_gradient_of_many_sentences(ops):
+    """More (sentence, head) pairs than a grid's second or third dimension takes: the sentences repeat, and so do their
+    transitions and gradients."""
+    import importlib
+
+    B, L, heads, dim, few = 16400, 4, 4, 4, 50
+    masks = [m.to(DEV) for m in importlib.import_module("pcfg_nat_b200.support_tree").get_mask(L, 1)]
+    g = torch.Generator(DEV).manual_seed(1)
+    base = [torch.randn(few, L, heads, dim, device=DEV, generator=g) for _ in range(3)] + \
+        [torch.randn(few, L, heads, device=DEV, generator=g)]
+    G = torch.randn(few, L, 2, L, device=DEV, generator=g)
+    k = ops.get_pcfg_kernel()
+
+    def chain(n):
+        leaves = [t.repeat(n, *[1] * (t.dim() - 1)).requires_grad_() for t in base]
+        links = k.extract_links(*leaves, torch.full((n * few, L), 3, device=DEV), 1, *masks)
+        loss = (torch.where(torch.isfinite(links), links, 0.0) * G.repeat(n, 1, 1, 1)).sum()
+        return torch.autograd.grad(loss, leaves)
+
+    for one, many in zip(chain(1), chain(B // few)):
+        assert torch.equal(many, one.repeat(B // few, *[1] * (one.dim() - 1))) and one.abs().sum() > 0
+
+
 def test_decode_step_from_link_features(pkg, ops, syn):
     """DecodeStep fed with the projected link features gives what extract_links + the transition-fed step give."""
     import importlib
