@@ -158,6 +158,7 @@ int launch_loss_linear(const float *match_all, const float *links, const int64_t
                        int T, float *Y, float *O, float *frames, float *loss, float *mg, float *lg, int *status,
                        cudaStream_t st);
 int mixed_width_count(int B, int Mc);
+int sm_count();  // of the current device
 
 int launch_loss_fwd_balanced(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B,
                              int L, int T, float *S, float *C, float *loss, int *status, cudaStream_t st);

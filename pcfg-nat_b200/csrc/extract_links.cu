@@ -16,7 +16,9 @@
 //   links_gather_kernel        packs the features of the M main-chain nodes (and of their left options) as the
 //                              float32 operands of the GEMMs:  qm, krm [B][H][M][D], klm [B][H][M+1][D];
 //   links_scores_kernel        ac [B][H][M][M] = qm krm^T,  bc [B][H][M+1][M] = klm krm^T, unscaled (small batched
-//                              float32 products, one block per sentence, head and 128 x 64 tile);
+//                              float32 products, one block per sentence, 128 x 64 tile and up to four heads).  Tiles
+//                              without an admissible (node, right child) pair are left unwritten when the masks are
+//                              given: ac and bc are defined at admissible pairs only;
 //   links_from_scores_kernel   one block per (sentence, node) does the rest.
 // Backward (training): links_grad [B][L][2][L] ->
 //   links_scores_grad_kernel   one block per (sentence, node): the row's forward quantities once more, then the
@@ -771,7 +773,7 @@ int launch_links_scores(const float *qm, const float *klm, const float *krm, con
     // up to four heads per block (the test for tiles in use and the first chunk's latency are paid once), as long as
     // there are four blocks for every place on the GPU: tiles that are not in use leave at once
     int heads = 4;
-    while (heads > 1 && (long long)tiles.x * tiles.y * B * ((H + heads - 1) / heads) < 4 * 2 * 148) heads /= 2;
+    while (heads > 1 && (long long)tiles.x * tiles.y * B * ((H + heads - 1) / heads) < 4ll * 2 * sm_count()) heads /= 2;
     const size_t smem = 2 * kScoreStage * sizeof(float);
     if (ensure_dynamic_smem(links_scores_kernel, smem) != cudaSuccess) return PCFGNAT_ERR_CUDA;
     links_scores_kernel<<<dim3(tiles.x, tiles.y, B * ((H + heads - 1) / heads)), 256, smem, st>>>(

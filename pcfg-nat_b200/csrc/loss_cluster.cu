@@ -886,15 +886,15 @@ int launch_cluster(Kernel kernel, int B, int nc, size_t smem, cudaStream_t st, A
 
 }  // namespace
 
-// Number of sentences that get both CTAs of a cluster of two when the batch has more sentences than half the
-// SMs (so that one cluster size for all would leave SMs idle or sentences waiting), or 0 when that mode does not
-// apply: the SMs left over once every sentence has one.
-static int sm_count() {
+int sm_count() {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return sms;
 }
 
+// Number of sentences that get both CTAs of a cluster of two when the batch has more sentences than half the
+// SMs (so that one cluster size for all would leave SMs idle or sentences waiting), or 0 when that mode does not
+// apply: the SMs left over once every sentence has one.
 int mixed_width_count(int B, int Mc) {
     const int sms = sm_count();
     if (B * 2 <= sms || B >= sms || B > 256 || Mc <= 16 || getenv("PCFGNAT_DP_CLUSTER_SIZE")) return 0;
