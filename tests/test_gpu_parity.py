@@ -1222,7 +1222,7 @@ def test_extract_links_backward_against_reference_autograd(ops, case, dtype):
                                                   (322, 8, 64, torch.float16)])
 def test_extract_links_and_gradient_at_tile_edges(pkg, ops, L, heads, dim, dtype):
     """Transitions and feature gradients at node and feature counts around the tiles of the product kernels, against
-    autograd in float64: float32 sums of up to 322 terms, 1e-5 of the largest entry (half precision: its rounding)."""
+    autograd in float64: float32 sums of up to 322 terms, 2e-5 of the largest entry (half precision: its rounding)."""
     import importlib
 
     lm, rm, mc = importlib.import_module("pcfg_nat_b200.support_tree").get_mask(L, 1)
@@ -1303,6 +1303,79 @@ def test_links_gradient_of_improbable_cells_with_large_weights(pkg, ops, heads):
     torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-4)
     for x, y in zip(grads, ref):
         assert (x - y).abs().max() <= 1e-4 * y.abs().max(), tuple(x.shape)
+
+
+@pytest.mark.parametrize("heads, scale", [(1, 4.0), (2, 4.0), (8, 5.0)])
+def test_links_of_improbable_cells(pkg, ops, heads, scale):
+    """Transitions below the probability (1e-30) under which the mixture is formed from log-probabilities, and their
+    gradient.  Logits of up to 150 in float32 (spacing 1.5e-5, a handful of roundings): 1e-4."""
+    g = torch.Generator().manual_seed(heads)
+    leaves = [scale * torch.randn(2, 40, heads, 8, generator=g) for _ in range(3)] + [torch.randn(2, 40, heads, generator=g)]
+    got, grads, want, ref = _links_and_float64(pkg, ops, leaves, torch.tensor([40, 31]),
+                                               lambda want: torch.randn(want.shape, generator=g))
+    assert int((want < -69.1).sum()) > 3
+    torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-4)
+    for x, y in zip(grads, ref):
+        assert (x - y).abs().max() <= 1e-4 * y.abs().max(), tuple(x.shape)
+
+
+def test_links_with_rows_beyond_shared_memory(pkg, ops):
+    """Rows whose exponentials (32 heads x 162 nodes), and rows whose weights (3 725 nodes) stay out of shared memory: the
+    same transitions and gradients, against float64.  The long graph's sentences fill its first nodes only, so that it
+    has to give what a short graph gives."""
+    import importlib
+
+    g = torch.Generator().manual_seed(7)
+    leaves = [torch.randn(1, 324, 32, 4, generator=g) for _ in range(3)] + [torch.randn(1, 324, 32, generator=g)]
+    got, grads, want, ref = _links_and_float64(pkg, ops, leaves, torch.tensor([324]),
+                                               lambda want: torch.randn(want.shape, generator=g))
+    torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-4)
+    for x, y in zip(grads, ref):
+        assert (x - y).abs().max() <= 2e-5 * y.abs().max(), tuple(x.shape)
+
+    L, short, heads = 7450, 140, 2
+    masks = importlib.import_module("pcfg_nat_b200.support_tree").get_mask(L, 1)
+    masks = [m.to(DEV).ne(0).to(torch.uint8) for m in masks]
+    leaves = [torch.randn(2, short, heads, 8, generator=g) for _ in range(3)] + [torch.randn(2, short, heads, generator=g)]
+    length = torch.tensor([short, 77])
+    G = torch.randn(2, short, 2, short, generator=g)
+    got, grads, want, ref = _links_and_float64(pkg, ops, leaves, length, lambda want: G)
+    padded = [torch.cat([t, torch.zeros(2, L - short, *t.shape[2:])], 1).to(DEV).requires_grad_() for t in leaves]
+    prev = torch.where(torch.arange(L)[None, :] < length[:, None], 3, 1).to(DEV)
+    links = ops.get_pcfg_kernel().extract_links(*padded, prev, 1, *masks)
+    part = links[:, :short, :, :short]
+    finite = torch.isfinite(part)
+    assert int(torch.isfinite(links).sum()) == int(finite.sum())
+    torch.testing.assert_close(part.detach()[finite].cpu().double(), want, rtol=1e-5, atol=1e-4)
+    (torch.where(finite, part, 0.0) * G.to(DEV)).sum().backward()
+    for x, y in zip(padded, ref):
+        assert (x.grad[:, :short].cpu().double() - y).abs().max() <= 2e-5 * y.abs().max(), tuple(x.shape)
+        assert (x.grad[:, short:] == 0).all()
+
+
+def test_links_with_an_infinite_logit(pkg, ops):
+    """A head with a logit of +inf counts nothing in its row; the others keep their part and their gradients."""
+    import importlib
+
+    L, heads, dim = 20, 2, 4
+    masks = importlib.import_module("pcfg_nat_b200.support_tree").get_mask(L, 1)
+    g = torch.Generator().manual_seed(2)
+    leaves = [torch.randn(1, L, heads, dim, generator=g) for _ in range(3)] + [torch.randn(1, L, heads, generator=g)]
+    leaves[0][0, 3, 0], leaves[2][0, 7, 0] = 1e20, 1e20  # node 3, child 7: the product of head 0 is +inf
+    ours = [t.to(DEV).requires_grad_() for t in leaves]
+    links = ops.get_pcfg_kernel().extract_links(*ours, torch.full((1, L), 3, device=DEV), 1, *masks)
+    ref = [t[..., 1:, :].double().requires_grad_() for t in leaves[:3]] + [torch.zeros(1, L, 1).double()]
+    want = pyref.extract_links(*ref, torch.full((1, L), 3), 1, *masks, dtype=torch.float64, floor=-1e30)[0, 3]
+    ok = want > -1e29
+    want = want + torch.log_softmax(leaves[3][0, 3].double(), 0)[1]
+    assert torch.equal(torch.isfinite(links[0, 3]).cpu(), ok)
+    torch.testing.assert_close(links[0, 3].detach().cpu()[ok].double(), want.detach()[ok], rtol=1e-5, atol=1e-5)
+    G = torch.randn(2, L, generator=g) * ok
+    (torch.where(ok, want, 0.0) * G).sum().backward()
+    (torch.where(ok.to(DEV), links[0, 3], 0.0) * G.to(DEV)).sum().backward()
+    for x, y in zip(ours[:3], ref[:3]):
+        err = (x.grad[..., 1:, :].cpu().double() - y.grad).abs().max()
+        assert err <= 2e-5 * y.grad.abs().max(), (tuple(x.shape), float(err))
 
 
 def test_links_gradient_of_many_sentences(ops):
