@@ -970,6 +970,9 @@ int linear_chunks(int cs) {
     return chunks <= 4 ? chunks : chunks <= 6 ? 6 : 8;
 }
 
+// Shared memory of a launch beside what the kernels declare themselves (1 088 and 1 120 bytes, most of it pick_sentence's).
+constexpr size_t kLinearSmem = (size_t)kSmemLimit - 1152;
+
 struct LinearGeometry {
     int nc, cs, rows_cap;
     int wide;                 // -1: cluster k takes sentence k; else the sentences are taken by cost (pick_sentence)
@@ -1002,7 +1005,7 @@ LinearGeometry linear_geometry(int B, int Mc, int W) {
         // the step loop's columns, matrices and o table, later overlaid by the y table of the gradient sums
         const size_t loop_mem = 8 * cp + mat + own, y_table = (size_t)W * g.cs;
         g.smem_out = ((size_t)linear_outside_head(g.rows_cap, W) + (loop_mem > y_table ? loop_mem : y_table)) * sizeof(float);
-        if (g.smem_in <= (size_t)kSmemLimit - 1024 && g.smem_out <= (size_t)kSmemLimit - 1024) break;
+        if (g.smem_in <= kLinearSmem && g.smem_out <= kLinearSmem) break;
         if (nc >= 16) {
             g.nc = 0;
             break;

@@ -1676,6 +1676,29 @@ def test_linear_space_loss_hands_unusual_sentences_to_the_log_space_kernels(ops,
         assert torch.equal(mg[i].nan_to_num(7.0), mg2[i].nan_to_num(7.0)) and torch.equal(lg[i].nan_to_num(7.0), lg2[i].nan_to_num(7.0))
 
 
+@pytest.mark.parametrize("B, L, T", [(20, 314, 238), (1, 322, 304), (2, 384, 238)])
+def test_linear_space_loss_at_the_limit_of_shared_memory(ops, monkeypatch, B, L, T):
+    """Shapes whose tables come within a hundred bytes of the shared memory that the kernels' own variables leave."""
+    monkeypatch.delenv("PCFGNAT_DP_KERNEL", raising=False)
+    monkeypatch.delenv("PCFGNAT_LINEAR_DP", raising=False)
+    g = torch.Generator(DEV).manual_seed(L)
+    match = torch.randn(B, L, T, device=DEV, generator=g) - 6
+    links = torch.randn(B, L, 2, L, device=DEV, generator=g)
+    at = torch.arange(L, device=DEV)
+    allowed = (at[:, None] % 2 == 1) & (at[None, :] % 2 == 1) & (at[None, :] > at[:, None])
+    links.masked_fill_(~allowed[None, :, None, :], float("-inf"))
+    links = torch.log_softmax(links.flatten(2), -1).nan_to_num(nan=float("-inf"), neginf=float("-inf")).view_as(links)
+    ol, tl = torch.full((B,), L, device=DEV), torch.full((B,), T, device=DEV)
+    ops.read_status(DEV)
+    got = _fused(ops, match, links, ol, tl)
+    assert ops.read_status(DEV) & ~16 == 0  # PCFGNAT_STATUS_RECOMPUTED
+    monkeypatch.setenv("PCFGNAT_LINEAR_DP", "0")
+    want = _fused(ops, match, links, ol, tl)
+    torch.testing.assert_close(got[0], want[0], rtol=1e-5, atol=0)
+    for x, y in zip(got[1:], want[1:]):
+        torch.testing.assert_close(x, y, rtol=1e-3, atol=2e-6)
+
+
 def test_pipelined_steps_overlap_copies_without_mixing_batches(pkg, ops, syn):
     """Two step objects in turn (copies of the next batch while the current one is computed): different batches
     through the pipeline come out exactly as through a single step object, in order."""
