@@ -90,7 +90,8 @@ __device__ __forceinline__ void viterbi_node(int id, int Mb, int lane, int prio,
 // The same for a group of G lanes (G = 4, 8, 16 or 32, the groups of a warp side by side): lane q of the group scans
 // children ci = id + q + G i, i < trips, so that its reference thread (ci - id) & 3 = q & 3 is still one per lane, and the
 // group settles on (largest value, smallest key) with a butterfly of shuffles.  The rows r0, r1 (from the lane's first
-// child on) hold -inf past the chain, so no child is tested and the loads of four trips are in flight together.
+// child on) hold -inf past the chain (or the lane's trips end with it), so no child is tested and the loads of four
+// trips are in flight together.
 // A lane remembers the trip of its best, the key is made at the end.
 __device__ __forceinline__ void viterbi_node_group(int id, int trips, int q, int G, float oa, const float *r0, const float *r1,
                                                    const float *s1, const float *s2, float &best, int &key) {
@@ -142,7 +143,7 @@ __host__ __device__ inline int viterbi_overshoot(int G, int NC) { return G - 1 +
 __global__ void __launch_bounds__(kVitThreads, 1)
     viterbi_cluster_kernel(const float *__restrict__ ob_lprob, const float *__restrict__ links,
                            const int64_t *__restrict__ ol, int L, float *S, int64_t *R, int64_t *Lt, int64_t *Mt,
-                           int *status, int Mc, int cs, int rows_cap, int lk_stride, int B, int wide) {
+                           int *status, int Mc, int cs, int rows_cap, int lk_stride, bool tight, int B, int wide) {
     extern __shared__ float smem[];
     cg::cluster_group cluster = cg::this_cluster();
     int crank = (int)cluster.block_rank();  // below: the rank among the CTAs that work on this sentence
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(kVitThreads, 1)
     // warps and G = 8, 100 us with 32 and G = 16, 86 us with 8 and G = 4; a second pass costs more than either).  Lane
     // q < NC of a group also sends the result to CTA q
     int G = 32;
-    while (((32 / G) * kVitActive < my_rows || Mb + viterbi_overshoot(G, NC) > lk_stride) && (G >> 1) >= 4 && (G >> 1) >= NC) G >>= 1;
+    while (((32 / G) * kVitActive < my_rows || (!tight && Mb + viterbi_overshoot(G, NC) > lk_stride)) && (G >> 1) >= 4 && (G >> 1) >= NC) G >>= 1;
     const int RW = 32 / G, q = lane % G, sub = lane / G;  // RW nodes per warp
     const uint32_t rcol = NC > 1 && q < NC ? dsm_map_to_cta(dsm_smem_u32(col), q) : 0;  // this CTA's columns as CTA q maps them
     const uint32_t rbar0 = NC > 1 && q < NC ? dsm_map_to_cta(dsm_smem_u32(&col_bar[0]), q) : 0;
@@ -253,7 +254,8 @@ __global__ void __launch_bounds__(kVitThreads, 1)
             const int r = r0w + sub;
             const bool live = r < my_rows;
             const int rr = live ? r : r0w, id = crank + NC * rr;
-            const int trips = (Mb - (crank + NC * r0w) + G - 1) / G;  // of the warp's first node, which has most children
+            // those of the warp's first node, which has most children; in rows without padding every lane's own
+            const int trips = (Mb - (tight ? id + q : crank + NC * r0w) + G - 1) / G;
             const float *r0 = lk0 + rr * lk_stride + id + q, *r1 = lk1 + rr * lk_stride + id + q;
             float best;
             int key;
@@ -487,6 +489,32 @@ int launch_trace(const float *S, const float *penalty, int64_t *pred_out, const 
 
 }  // namespace
 
+// How a CTA of n that share a sentence lays out its nodes' rows; smem 0: they do not fit.
+struct VitRows {
+    int cap, stride;
+    bool tight;
+    size_t smem;
+};
+
+static VitRows viterbi_rows(int Mc, int Q, int cs, int n, int width) {
+    VitRows r;
+    r.cap = (Mc + n - 1) / n;  // also right for mixed widths: n is 1 there, every CTA may hold a chain
+    // rows long enough for the lanes a full chain takes (shorter ones take more where they fit), and with the rows of a
+    // warp's nodes in different banks where there is room for that
+    int G = 32;
+    while ((32 / G) * kVitActive < r.cap && (G >> 1) >= 4 && (G >> 1) >= width) G >>= 1;
+    const int least = Mc + viterbi_overshoot(G, width);
+    const int strides[3] = {(least + width - G % 32 + 31) / 32 * 32 + G % 32 - width, least | 1, (Mc + 31) / 32 * 32 + 1};
+    for (int i = 0; i < 3; i++) {  // the last without room for what lanes read past the chain: there they stop at its end
+        r.stride = strides[i];
+        r.tight = i == 2;
+        r.smem = ((size_t)4 * cs + (size_t)2 * r.cap * r.stride + (size_t)2 * r.cap * Q + r.cap) * sizeof(float);
+        if (r.smem <= (size_t)kSmemLimit - 1024) return r;
+    }
+    r.smem = 0;
+    return r;
+}
+
 int launch_viterbi(const float *ob, const float *links, const int64_t *ol, int B, int L, float *S, int64_t *R,
                    int64_t *Lt, int64_t *Mt, int *status, cudaStream_t st) {
     if (B == 0) return PCFGNAT_OK;
@@ -509,51 +537,53 @@ int launch_viterbi(const float *ob, const float *links, const int64_t *ol, int B
     int wide = -1;
     if (nc == 1 && B * 2 > sms && B < sms && B <= 256 && Mc > 16 && !getenv("PCFGNAT_DP_CLUSTER_SIZE")) wide = sms - B;
     if (dp_kernel_choice() == kDpRows) nc = 32;  // skips the loop below
-    for (; nc <= 16; nc *= 2) {
-        const int rows_cap = (Mc + nc - 1) / nc;  // also right for mixed widths: nc is 1 there, every CTA may hold a chain
-        // rows long enough for the lanes a full chain takes (shorter ones take more where they fit), and with the rows of a
-        // warp's nodes in different banks where there is room for that
-        const int width = wide >= 0 && nc == 1 ? 2 : nc;
-        int G = 32;
-        while ((32 / G) * kVitActive < rows_cap && (G >> 1) >= 4 && (G >> 1) >= width) G >>= 1;
-        const int least = Mc + viterbi_overshoot(G, width);
-        int lk_stride = (least + width - G % 32 + 31) / 32 * 32 + G % 32 - width;
-        const auto bytes = [&] {
-            return ((size_t)4 * cs + (size_t)2 * rows_cap * lk_stride + (size_t)2 * rows_cap * Q + rows_cap) * sizeof(float);
-        };
-        if (bytes() > (size_t)kSmemLimit - 1024) lk_stride = least | 1;
-        const size_t smem = bytes();
-        if (smem > (size_t)kSmemLimit - 1024) continue;
-        if (ensure_dynamic_smem(viterbi_cluster_kernel, smem) != cudaSuccess) return PCFGNAT_ERR_CUDA;
-        if (nc > 8 && cudaFuncSetAttribute(viterbi_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                          cudaSuccess) {
-            cudaGetLastError();
-            break;
-        }
-        cudaLaunchConfig_t cfg = {};
-        // mixed widths only while one CTA holds a chain; a grid larger than the GPU takes the sentences by
-        // decreasing length (wide = B), so that the clusters that wait for a place get the shortest
-        const bool mixed = wide >= 0 && nc == 1;
-        const int order = mixed ? wide : ((long long)B * nc > sms && B <= 256 ? B : -1);
-        const int launch_nc = mixed ? 2 : nc;
-        cfg.gridDim = dim3((unsigned)((mixed ? wide + (B - wide + 1) / 2 : B) * launch_nc));
-        cfg.blockDim = dim3(kVitThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
+    // mixed widths only while one CTA holds a chain; a grid larger than the GPU takes the sentences by
+    // decreasing length (wide = B), so that the clusters that wait for a place get the shortest
+    const auto mixed = [&](int n) { return wide >= 0 && n == 1; };
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.blockDim = dim3(kVitThreads);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    // the launch with n CTAs per sentence; returns the clusters that run at once, 0 where there is no such launch
+    const auto configure = [&](int n, const VitRows &rows) {
+        const int launch_nc = mixed(n) ? 2 : n;
+        cfg.gridDim = dim3((unsigned)((mixed(n) ? wide + (B - wide + 1) / 2 : B) * launch_nc));
+        cfg.dynamicSmemBytes = rows.smem;
         attr[0].val.clusterDim.x = (unsigned)launch_nc;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int max_clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&max_clusters, viterbi_cluster_kernel, &cfg) != cudaSuccess || max_clusters < 1) {
+        int clusters = 0;
+        if (ensure_dynamic_smem(viterbi_cluster_kernel, rows.smem) != cudaSuccess ||
+            (n > 8 && cudaFuncSetAttribute(viterbi_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+            cudaOccupancyMaxActiveClusters(&clusters, viterbi_cluster_kernel, &cfg) != cudaSuccess) {
             cudaGetLastError();
-            continue;  // this cluster size cannot be scheduled here: try the next one
+            return 0;
         }
-        return cuda_rc(cudaLaunchKernelEx(&cfg, viterbi_cluster_kernel, ob, links, ol, L, S, R, Lt, Mt, status, Mc, cs,
-                                          rows_cap, lk_stride, B, order));
+        return clusters;
+    };
+    for (; nc <= 16; nc *= 2) {
+        VitRows rows = viterbi_rows(Mc, Q, cs, nc, mixed(nc) ? 2 : nc);
+        if (rows.smem == 0) continue;
+        int clusters = configure(nc, rows);
+        if (clusters < 1) continue;  // this cluster size cannot be scheduled here: try the next one
+        if (rows.tight && nc < 16) {
+            // Twice the CTAs have room for the padding and take two thirds of the time per wave: graph 380, two CTAs 230,
+            // four 145 us; 532, four and eight: 338 and 221; 760, eight and sixteen: 444 and 302.  64 sentences of 380 are
+            // one wave of two (231 us) or two of four (289), 90 are two (457) or three (430), 32 of 532 one (338) or three (654).
+            const VitRows more_rows = viterbi_rows(Mc, Q, cs, 2 * nc, 2 * nc);
+            const int more = more_rows.smem ? configure(2 * nc, more_rows) : 0;
+            if (more > 0 && 2 * ((B + more - 1) / more) <= 3 * ((B + clusters - 1) / clusters)) {
+                nc *= 2;
+                rows = more_rows;
+            } else {
+                configure(nc, rows);
+            }
+        }
+        const int order = mixed(nc) ? wide : ((long long)B * nc > sms && B <= 256 ? B : -1);
+        return cuda_rc(cudaLaunchKernelEx(&cfg, viterbi_cluster_kernel, ob, links, ol, L, S, R, Lt, Mt, status, Mc, cs, rows.cap,
+                                          rows.stride, rows.tight, B, order));
     }
     const size_t smem_cols = (size_t)3 * cs * sizeof(float);
     if (smem_cols > (size_t)kSmemLimit - 1024) return PCFGNAT_ERR_TOO_LARGE;

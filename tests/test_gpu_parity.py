@@ -252,7 +252,8 @@ def test_viterbi_tie_breaking(vit_kernel, ops, syn):
     assert (np.isfinite(So).sum() > 100)
 
 
-@pytest.mark.parametrize("B, L", [(1, 8), (1, 140), (3, 66), (60, 130), (100, 66), (100, 256), (150, 34), (40, 262), (5, 515)])
+@pytest.mark.parametrize("B, L", [(1, 8), (1, 140), (3, 66), (60, 130), (100, 66), (100, 256), (150, 34), (40, 262), (5, 515),
+                                  (40, 379), (38, 384), (20, 531), (5, 768), (1, 1060)])
 def test_viterbi_table_and_trace_edges(ops, syn, monkeypatch, B, L):
     """Tables bit for bit those of the kernel that reads the transitions from global memory, and the back-trace the
     host restatement's, at the numbers of lanes per node, cluster sizes and shared clusters that the library picks, with
