@@ -114,7 +114,7 @@ def table_shapes(B, L, T, max_left):
     return (B, Mc, T + 2), (B, L - Mc, T + 2, max_left + 2)
 
 
-_main_chain_cache = {}  # (address and version of the main-chain mask, prelen) -> mask, node list, slots
+_main_chain_cache = {}  # (address and version of the main-chain mask, prelen) -> mask, (node list, slots), their stream
 
 
 class _Kernel:
@@ -708,12 +708,16 @@ class _Kernel:
         if chain is None and mc.is_inference():  # no version counter that would tell of a change: nothing is kept
             chain = _Kernel.main_chain_slots(mc)
         elif chain is None:
-            key = (mc.data_ptr(), mc._version, L)
+            key, stream = (mc.data_ptr(), mc._version, L), torch.cuda.current_stream(dev)
             cached = _main_chain_cache.get(key)
             if cached is None:
-                cached = (mc, _Kernel.main_chain_slots(mc))  # keeps mc alive: its address is part of the key
+                cached = (mc, _Kernel.main_chain_slots(mc), stream)  # keeps mc alive: its address is part of the key
+                stream.synchronize()  # any stream may read them from here on
                 _main_chain_cache.clear()
                 _main_chain_cache[key] = cached
+            elif cached[2] != stream:  # another call may drop them from the cache before this one's kernels have run
+                for t in cached[1]:
+                    t.record_stream(stream)
             chain = cached[1]
         nodes, slot_of = chain
         M = nodes.numel()

@@ -1273,6 +1273,32 @@ def test_extract_links_under_inference_mode(pkg, ops):
         assert torch.equal(k.extract_links(*feats, prev, 1, *inside), want_shorter)
 
 
+def test_extract_links_on_another_stream_than_the_first(pkg, ops):
+    """The node lists that a mask's first call leaves for later ones: a call on another stream reads them when its turn
+    comes, also if a call with another mask has taken their place and their memory was handed out again by then."""
+    import importlib
+
+    get_mask, k = importlib.import_module("pcfg_nat_b200.support_tree").get_mask, ops.get_pcfg_kernel()
+    g = torch.Generator(DEV).manual_seed(4)
+
+    def inputs(L):
+        masks = [m.to(DEV).ne(0).to(torch.uint8) for m in get_mask(L, 1)]
+        feats = [torch.randn(2, L, 2, 8, device=DEV, generator=g) for _ in range(3)]
+        return [*feats, torch.randn(2, L, 2, device=DEV, generator=g), torch.full((2, L), 3, device=DEV), 1, *masks]
+
+    first, second = inputs(60), inputs(30)
+    want = k.extract_links(*first)
+    side = torch.cuda.Stream(DEV)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)  # a tenth of a second
+        got = k.extract_links(*first)
+    k.extract_links(*second)
+    filler = [torch.zeros(n, dtype=torch.int32, device=DEV) for n in (30, 60) for _ in range(64)]
+    torch.cuda.synchronize()
+    assert torch.equal(got, want), len(filler)
+
+
 def _links_and_float64(pkg, ops, leaves, length, G_of):
     """(links, gradients of the leaves, both again by autograd in float64): G_of(float64 links) weighs the finite cells."""
     import importlib
