@@ -114,6 +114,11 @@ def table_shapes(B, L, T, max_left):
     return (B, Mc, T + 2), (B, L - Mc, T + 2, max_left + 2)
 
 
+def _row_index_ok(index, device):
+    """Whether the row kernels can take ``index`` as it is; torch's operators convert or refuse what they cannot."""
+    return index is None or index.dim() == 1 and index.dtype == torch.int64 and index.device == device
+
+
 _main_chain_cache = {}  # (address and version of the main-chain mask, prelen) -> mask, (node list, slots), their stream
 
 
@@ -546,7 +551,8 @@ class _Kernel:
     @staticmethod
     def rows_to_bf16(src, index=None):
         """bf16 copy of the rows ``index`` (int64; all of them without) of a [rows, H] tensor, in one pass."""
-        if src.dtype != torch.float16 or not src.is_cuda or src.shape[1] % 8 or src.data_ptr() % 16 or not src.is_contiguous():
+        if src.dtype != torch.float16 or not src.is_cuda or src.shape[1] % 8 or src.data_ptr() % 16 or \
+                not src.is_contiguous() or not _row_index_ok(index, src.device):
             return (src if index is None else src.index_select(0, index)).to(torch.bfloat16).contiguous()
         index = index.contiguous() if index is not None else None
         n = src.shape[0] if index is None else index.shape[0]
@@ -561,7 +567,9 @@ class _Kernel:
     def rows_from_f32(src, dst, index=None):
         """Writes the float32 rows [n, H] into the rows ``index`` (int64; the first n without) of ``dst`` [rows, H]."""
         if dst.dtype != torch.float16 or src.shape[1] % 8 or dst.data_ptr() % 16 or src.data_ptr() % 16 or \
-                not (src.is_contiguous() and dst.is_contiguous()) or src.dtype != torch.float32:
+                not (src.is_contiguous() and dst.is_contiguous()) or src.dtype != torch.float32 or src.device != dst.device or \
+                src.shape[1] != dst.shape[1] or src.shape[0] != (src if index is None else index).shape[0] or \
+                src.shape[0] > dst.shape[0] and index is None or not _row_index_ok(index, dst.device):
             if index is None:
                 dst[:src.shape[0]].copy_(src)
             else:

@@ -1073,6 +1073,20 @@ def test_convert_rows(ops, H):
     assert k.rows_to_bf16(src[:0]).shape == (0, H)
 
 
+def test_convert_rows_checks_its_index(ops):
+    """What torch's index operators converted or refused still is: 32-bit indices, rows that do not match."""
+    k = ops.get_pcfg_kernel()
+    src = torch.randn(20, 16, device=DEV).half()
+    index = torch.tensor([3, 0, 19], device=DEV)
+    assert torch.equal(k.rows_to_bf16(src, index.int()), src[index].to(torch.bfloat16))
+    dst, grad = torch.zeros(20, 16, dtype=torch.float16, device=DEV), torch.randn(3, 16, device=DEV)
+    for args in ((grad, dst, index[:2]), (grad[:, :8].contiguous(), dst, index), (grad, dst, index.int()),
+                 (torch.randn(21, 16, device=DEV), dst)):
+        with pytest.raises((RuntimeError, IndexError)):
+            k.rows_from_f32(*args)
+    assert (dst == 0).all()
+
+
 def test_copy_batch(ops):
     """Tensors of one byte to several blocks, at and off 16- and 4-byte boundaries, the main-chain rows of transitions,
     empty and self copies; overlapping pairs and more pairs than a launch takes are refused with nothing copied."""
