@@ -50,8 +50,8 @@ __global__ void __launch_bounds__(kLookThreads)
     lookahead_decode_kernel(const float *__restrict__ links, const float *__restrict__ ob, const int64_t *__restrict__ tokens,
                             const int64_t *__restrict__ ol, const int64_t *__restrict__ mask, int mask_dim, float beta,
                             int lookahead, int64_t pad, int L, int cap, int64_t *out, int64_t *cnt, int *status) {
-    extern __shared__ int s_node[];  // first CTA: [L] words of the nodes, then [L] the walk's stack
-    __shared__ int s_kept;
+    // first CTA: [L] words of the nodes, then [L] the walk's stack; node 0 has none, its word takes the number of tokens
+    extern __shared__ int s_node[];
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), nc = (int)cluster.num_blocks();
     const int b = blockIdx.x / nc;
@@ -146,11 +146,11 @@ __global__ void __launch_bounds__(kLookThreads)
             now = word & kLookChild;
         }
         if (bad) flag(status, PCFGNAT_STATUS_BAD_TRACE);
-        s_kept = count < cap ? count : cap;
-        cnt[b] = s_kept;
+        s_node[0] = count < cap ? count : cap;
+        cnt[b] = s_node[0];
     }
     __syncthreads();
-    const int kept = s_kept;
+    const int kept = s_node[0];
     for (int i = tid; i < cap; i += kLookThreads) o[i] = i < kept ? tokens[(size_t)b * L + o[i]] : pad;
 }
 

@@ -1840,6 +1840,20 @@ def test_lookahead_decode_cluster_edges(pkg, ops, L):
     assert ops.read_status(DEV) != 0 and int(cnt[4]) == 0 and (out[4] == 1).all()
 
 
+def test_lookahead_decode_longest_graph(ops):
+    """The largest graph whose words and stack fit a CTA's shared memory: 29 056 nodes."""
+    L = 29056
+    links = torch.full((1, L, 2, L), float("-inf"), device=DEV)
+    chain = torch.tensor([1, 9, 20001, L - 1], device=DEV)
+    links[0, chain[:-1], 0, chain[1:]] = -1.0
+    mask = torch.zeros(L, L, dtype=torch.int64, device=DEV)  # every node may descend to node 0, which emits nothing
+    tok = torch.arange(L, device=DEV)[None] + 4
+    ops.read_status(DEV)
+    out, cnt = ops.get_pcfg_kernel().lookahead_decode_device(links, torch.zeros(1, L, device=DEV), tok,
+                                                             torch.tensor([L], device=DEV), mask, 1, 1.0, "greedy")
+    assert out[0, :int(cnt[0])].tolist() == [5, 13, 20005, L + 3] and ops.read_status(DEV) == 0
+
+
 def test_lookahead_decode_near_ties(pkg, ops):
     """Two candidates per node whose scores differ by the last bit or not at all, with a beta that is not a power of two:
     the choice is the one of separately rounded products and sums, not of fused ones."""
