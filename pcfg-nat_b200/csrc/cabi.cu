@@ -37,7 +37,11 @@ cudaError_t ensure_dynamic_smem_for(const void *kernel, size_t bytes) {
     }
     if (slot && slot->fn == kernel && dev >= 0 && dev < kDevs && slot->bytes[dev] >= (int)bytes) return cudaSuccess;
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess && slot && dev >= 0 && dev < kDevs) {
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // the caller reports it; the check after the next launch must not find it
+        return e;
+    }
+    if (slot && dev >= 0 && dev < kDevs) {
         slot->fn = kernel;
         slot->bytes[dev] = (int)bytes;
     }

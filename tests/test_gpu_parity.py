@@ -1854,6 +1854,18 @@ def test_lookahead_decode_longest_graph(ops):
     assert out[0, :int(cnt[0])].tolist() == [5, 13, 20005, L + 3] and ops.read_status(DEV) == 0
 
 
+def test_a_refused_shape_leaves_no_error_behind(ops):
+    """A graph too large for the shared memory is refused, and the next launches find no error of its."""
+    L = 29064
+    k = ops.get_pcfg_kernel()
+    links = torch.zeros(1, L, 2, L, device=DEV)
+    tok = torch.zeros(1, L, dtype=torch.int64, device=DEV)
+    with pytest.raises(RuntimeError, match="too large"):
+        k.lookahead_decode_device(links, None, tok, torch.tensor([L], device=DEV), torch.zeros(8, 8, device=DEV), 1, 1.0, "greedy")
+    rows = torch.ones(2, 8, dtype=torch.float16, device=DEV)
+    assert (k.rows_to_bf16(rows) == 1).all()
+
+
 def test_lookahead_decode_near_ties(pkg, ops):
     """Two candidates per node whose scores differ by the last bit or not at all, with a beta that is not a power of two:
     the choice is the one of separately rounded products and sums, not of fused ones."""
