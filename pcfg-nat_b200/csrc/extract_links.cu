@@ -251,7 +251,7 @@ __device__ __forceinline__ float mixture_terms(int H, LogProb term, float &sum) 
 }
 
 // One block per (sentence, node).  A cell takes one exponential per head, one FMA per head and one logarithm.  Bound by
-// latency (a row is a few hundred cells behind five barriers): rows of nodes that are not on the main chain, and
+// its instructions (64 % of the issue slots) and the five barriers of a row of a few hundred cells: rows of nodes that are not on the main chain, and
 // slots outside the admissible range, cost nothing but their -inf.  90 sentences, M = 161, eight heads: 136 us; 190 us
 // with two exponentials per cell and head, each from scores read again.  Against float64 the transitions are off by
 // 2.3e-7 (rms; 2.8e-7 before).

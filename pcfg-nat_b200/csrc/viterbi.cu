@@ -231,8 +231,8 @@ __global__ void __launch_bounds__(kVitThreads, 1)
     if (NC > 1) cluster.sync(); else __syncthreads();
     if (ctid == 0) Sb[(size_t)(m - 1) * Q + 1] = __ldg(ob + (m - 1));
 
-    // G lanes share a node, as few as still let half the warps take all of this CTA's nodes in one pass: the kernel is
-    // bound by instruction issue, and a node's fixed costs are paid per warp (58 lengths, 60 nodes per CTA: 83 us with 16
+    // G lanes share a node, as few as still let half the warps take all of this CTA's nodes in one pass: a length is a chain
+    // of the scan, the arg-max and the exchange, and a node's fixed costs are paid per warp (58 lengths, 60 nodes per CTA: 83 us with 16
     // warps and G = 8, 100 us with 32 and G = 16, 86 us with 8 and G = 4; a second pass costs more than either).  Lane
     // q < NC of a group also sends the result to CTA q
     int G = 32;
