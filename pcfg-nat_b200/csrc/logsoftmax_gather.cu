@@ -403,12 +403,15 @@ int launch_typed(T *logits, const int64_t *sel, int64_t sb, int64_t sl, int64_t 
 // (what DagLogsoftmaxGatherFunc.backward of the reference does with mul_ and scatter_add_, custom_ops/pcfg_loss.py:168-180),
 // formed in float32 and rounded to the storage type once.  HBM bound: one read and one write of [rows][V], a block
 // per row, 16-byte pieces between the row's first and last 16-byte boundary, four loads in flight per thread; the
-// blocks of an SM cover each other's two barriers.  The selected columns are worked out before the row is overwritten
-// (a column that is selected several times is added up, in order, by the first thread that names it) and stored after
-// it.  More columns than threads are added to the rounded products atomically in the storage type, in no fixed order, as
-// torch's scatter_add_ adds them.  [14 400, 40 000] half precision: 392 us, 0.91 of the
-// measured copy bandwidth; 1 331 us as torch's broadcast multiplication and scatter.
-constexpr int kGradThreads = 256;
+// blocks of an SM cover each other's two barriers.  The selected columns and the row's first pieces are read together,
+// before anything is written; a column that is selected several times is added up, in order, by the first thread that
+// names it, and stored after the row.  More than kGradColumns columns are added to the rounded products atomically in
+// the storage type, in no fixed order, as torch's scatter_add_ adds them.  [4 096, 40 000] half precision, 48 columns: 111 us, 0.92
+// of the measured copy bandwidth; 398 us as torch's broadcast multiplication and scatter.
+// Rows of up to 8 KB take blocks of 64 threads: such a row is over before 256 threads have looked its columns up, and
+// four times as many rows of an SM are in flight.  [20 000, 1 000] half, 20 columns: 28 us, 77 us with 256 threads, 57 us as
+// torch's operators; [5 000, 1 000] float, 76 columns: 19, 50 and 26 us.
+constexpr int kGradColumns = 256, kGradSmallRow = 8192;
 
 __device__ __forceinline__ void atomic_add_to(float *p, float g) { atomicAdd(p, g); }
 __device__ __forceinline__ void atomic_add_to(__half *p, float g) { atomicAdd(p, __float2half(g)); }
@@ -421,68 +424,99 @@ __device__ __forceinline__ uint4 scaled(uint4 v, float scale) {
     return v;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kGradThreads)
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS)
     logsoftmax_gather_grad_kernel(T *probs, const float *__restrict__ grad, const int64_t *__restrict__ sel, int64_t sb,
-                                  int64_t sl, int64_t ss, int64_t rpb, int V, int slen, int *status) {
-    __shared__ int s_sel[kGradThreads];
-    __shared__ float s_g[kGradThreads];
-    constexpr int kVec = 16 / sizeof(T);
+                                  int64_t sl, int64_t ss, unsigned rpb, int V, int slen, int *status) {
+    __shared__ __align__(16) int s_sel[kGradColumns];
+    __shared__ float s_g[kGradColumns];
+    constexpr int kVec = 16 / sizeof(T), kCols = kGradColumns / THREADS;
     const int tid = threadIdx.x, lane = tid & 31;
-    const int64_t r = blockIdx.x;
+    const unsigned r = blockIdx.x;
     T *row = probs + (size_t)r * V;
     const float *g = grad + (size_t)r * slen;
-    const int64_t *srow = sel + (r / rpb) * sb + (r % rpb) * sl;
-    float sum = 0.f;
-    for (int s = lane; s < slen; s += 32) sum += __ldg(g + s);  // every warp for itself: no barrier
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    const float scale = -sum;
-    int col = -1;     // the column this thread answers for, and its new value
-    float val = 0.f;
-    if (slen <= kGradThreads) {
-        if (tid < slen) {
-            const int64_t v = srow[(int64_t)tid * ss];
-            if (v >= 0 && v < V) col = (int)v;
-            else flag(status, PCFGNAT_STATUS_BAD_INDEX);
-            s_sel[tid] = col;
-            s_g[tid] = __ldg(g + tid);
-        }
-        __syncthreads();
-        if (col >= 0) {
-            for (int s = 0; s < slen; s++) {
-                if (s_sel[s] != col) continue;
-                if (s < tid) {  // an earlier thread has this column
-                    col = -1;
-                    break;
-                }
-                val += s_g[s];
-            }
-        }
-        if (col >= 0) val = fmaf(to_f<T>(row[col]), scale, val);
-        __syncthreads();  // the selected probabilities are read
-    }
+    const int64_t *srow = sel + (int64_t)(r / rpb) * sb + (int64_t)(r % rpb) * sl;
     const int head = min(V, (int)((16 - (reinterpret_cast<uintptr_t>(row) & 15)) % 16 / sizeof(T)));
     const int n_vec = (V - head) / kVec, tail = head + n_vec * kVec;
     uint4 *body = reinterpret_cast<uint4 *>(row + head);
-    int i = tid;
-    for (; i + 3 * kGradThreads < n_vec; i += 4 * kGradThreads) {
-        uint4 v[4];
+    uint4 v[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) v[j] = body[i + j * kGradThreads];
+    for (int j = 0; j < 4; j++)
+        if (tid + j * THREADS < n_vec) v[j] = body[tid + j * THREADS];
+    const bool listed = slen <= kGradColumns;
+    int col[kCols];     // the columns this thread answers for, and their probabilities
+    float own[kCols];
+    if (listed) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) body[i + j * kGradThreads] = scaled<T>(v[j], scale);
+        for (int j = 0; j < kCols; j++) {
+            const int s = tid + j * THREADS;
+            col[j] = -1;
+            own[j] = 0.f;
+            if (s < slen) {
+                const int64_t at = srow[(int64_t)s * ss];
+                if (at >= 0 && at < V) {
+                    col[j] = (int)at;
+                    own[j] = to_f<T>(row[at]);
+                } else {
+                    flag(status, PCFGNAT_STATUS_BAD_INDEX);
+                }
+                s_g[s] = __ldg(g + s);
+            }
+            s_sel[s] = col[j];
+        }
+        __syncthreads();  // and nobody writes the row before the selected probabilities are read
     }
-    for (; i < n_vec; i += kGradThreads) body[i] = scaled<T>(body[i], scale);
+    float sum = 0.f;
+    for (int s = lane; s < slen; s += 32) sum += listed ? s_g[s] : __ldg(g + s);  // every warp for itself
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float scale = -sum;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (tid + j * THREADS < n_vec) body[tid + j * THREADS] = scaled<T>(v[j], scale);
+    int i = tid + 4 * THREADS;
+    for (; i + 3 * THREADS < n_vec; i += 4 * THREADS) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = body[i + j * THREADS];
+#pragma unroll
+        for (int j = 0; j < 4; j++) body[i + j * THREADS] = scaled<T>(v[j], scale);
+    }
+    for (; i < n_vec; i += THREADS) body[i] = scaled<T>(body[i], scale);
     if (tid < head) row[tid] = from_f<T>(to_f<T>(row[tid]) * scale);
     if (tail + tid < V) row[tail + tid] = from_f<T>(to_f<T>(row[tail + tid]) * scale);
+    if (listed) {
+#pragma unroll
+        for (int j = 0; j < kCols; j++) {
+            if (col[j] < 0) continue;
+            float val = 0.f;
+            for (int s = 0; s < slen; s += 4) {
+                const int4 c = *reinterpret_cast<const int4 *>(s_sel + s);
+                const int at[4] = {c.x, c.y, c.z, c.w};
+                if (at[0] != col[j] && at[1] != col[j] && at[2] != col[j] && at[3] != col[j]) continue;
+                bool earlier = false;  // a thread with an earlier place has this column
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    if (at[e] != col[j]) continue;
+                    earlier |= s + e < tid + j * THREADS;
+                    val += s_g[s + e];
+                }
+                if (earlier) {
+                    col[j] = -1;
+                    break;
+                }
+            }
+            own[j] = fmaf(own[j], scale, val);
+        }
+    }
     __syncthreads();
-    if (slen <= kGradThreads) {
-        if (col >= 0) row[col] = from_f<T>(val);
+    if (listed) {
+#pragma unroll
+        for (int j = 0; j < kCols; j++)
+            if (col[j] >= 0) row[col[j]] = from_f<T>(own[j]);
     } else {
-        for (int s = tid; s < slen; s += kGradThreads) {
-            const int64_t v = srow[(int64_t)s * ss];
-            if (v >= 0 && v < V) atomic_add_to(row + v, __ldg(g + s));
+        for (int s = tid; s < slen; s += THREADS) {
+            const int64_t at = srow[(int64_t)s * ss];
+            if (at >= 0 && at < V) atomic_add_to(row + at, __ldg(g + s));
             else flag(status, PCFGNAT_STATUS_BAD_INDEX);
         }
     }
@@ -492,7 +526,11 @@ template <typename T>
 int launch_grad_typed(T *probs, const float *grad, const int64_t *sel, int64_t sb, int64_t sl, int64_t ss, int64_t rows,
                       int64_t rpb, int V, int slen, int *status, cudaStream_t st) {
     if (rows > INT32_MAX) return PCFGNAT_ERR_TOO_LARGE;
-    logsoftmax_gather_grad_kernel<T><<<(unsigned)rows, kGradThreads, 0, st>>>(probs, grad, sel, sb, sl, ss, rpb, V, slen, status);
+    const unsigned per = rpb < rows ? (unsigned)rpb : (unsigned)rows;
+    if ((size_t)V * sizeof(T) <= kGradSmallRow)
+        logsoftmax_gather_grad_kernel<T, 64><<<(unsigned)rows, 64, 0, st>>>(probs, grad, sel, sb, sl, ss, per, V, slen, status);
+    else
+        logsoftmax_gather_grad_kernel<T, 256><<<(unsigned)rows, 256, 0, st>>>(probs, grad, sel, sb, sl, ss, per, V, slen, status);
     return cuda_rc(cudaGetLastError());
 }
 

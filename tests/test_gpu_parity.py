@@ -428,6 +428,26 @@ def test_logsoftmax_gather_backward(ops, dtype, V, slen):
         torch.testing.assert_close(got[1, 0].cpu().double(), want[1, 0], rtol=4 * eps, atol=4 * eps)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("V, slen", [(33, 1), (1000, 63), (2048, 64), (2049, 65), (3001, 129), (4096, 256), (4100, 255), (4104, 65)])
+def test_logsoftmax_gather_backward_block_sizes(ops, dtype, V, slen):
+    """Rows and column counts on both sides of the blocks' sizes, all columns repeated.  An entry is a product and sums of at
+    most slen terms in float32 (half a unit, 2^-24, of the magnitudes each), rounded to the storage type once."""
+    g = torch.Generator().manual_seed(V + slen)
+    probs = torch.softmax(3 * torch.randn(3, 7, V, generator=g), -1).to(dtype)
+    idx = torch.randint(0, max(1, slen // 3), (3, 7, slen), generator=g) * 31 % V
+    grad = torch.randn(3, 7, slen, generator=g)
+    exact = probs.double() * -grad.double().sum(-1, keepdim=True)
+    exact.scatter_add_(-1, idx, grad.double())
+    size = probs.double() * grad.double().abs().sum(-1, keepdim=True)
+    size.scatter_add_(-1, idx, grad.double().abs())
+    bound = (slen + 3) * 2.0 ** -24 * size + (2.0 ** -11 * exact.abs() + 2.0 ** -25 if dtype == torch.float16 else 0.0)
+    got = ops.get_pcfg_kernel().logsoftmax_gather_backward(probs.to(DEV), idx.to(DEV), grad.to(DEV)).cpu()
+    assert ((got.double() - exact).abs() <= bound).all()
+    again = ops.get_pcfg_kernel().logsoftmax_gather_backward(probs.to(DEV), idx.to(DEV), grad.to(DEV)).cpu()
+    assert torch.equal(got, again)
+
+
 @pytest.mark.parametrize("slen", [256, 257, 600])
 def test_logsoftmax_gather_backward_deterministic(ops, slen):
     """Under torch's deterministic algorithms the gradient repeats itself bit for bit whatever the number of columns;
