@@ -313,31 +313,36 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" 
 // parents, padding: six tiles in ten of a ragged batch) is left alone; the test looks at a quarter of the tile's pairs
 // at a time, so that a tile in use rarely pays for more than that.  90 sentences, M = 161, 8 x 64 features: 172 us; 296 us with a block per
 // head and nothing in flight, 384 us as 64 x 64 tiles of 4 x 4 outputs, every tile formed.
-constexpr int kScoreRows = 128, kScoreCols = 64, kScoreK = 32, kScorePitch = kScoreK + 4;
-constexpr int kScoreStage = (kScoreRows + kScoreCols) * kScorePitch;  // floats; two of them
-__global__ void __launch_bounds__(256, 2)
+// ROWS: 128, or 64 for chains of at most 31 nodes, whose rows fit one tile of either (128 sentences of 29 nodes, 8 x 64
+// features: 27 us, 41 us with 128 rows; of 12 nodes 26 and 39 us), and where 128 would leave SMs without a block (2
+// sentences of 65 nodes: 8.4 and 11.8 us).
+constexpr int kScoreCols = 64, kScoreK = 32, kScorePitch = kScoreK + 4;
+template <int ROWS>
+constexpr int kScoreStage = (ROWS + kScoreCols) * kScorePitch;  // floats; two of them
+template <int ROWS>
+__global__ void __launch_bounds__(256, ROWS == 128 ? 2 : 3)
     links_scores_kernel(const float *__restrict__ qm, const float *__restrict__ klm, const float *__restrict__ krm, int M,
                         int H, int D, int heads, int vec, ScoreMasks masks, float *__restrict__ ac, float *__restrict__ bc) {
     extern __shared__ __align__(16) float s_tiles[];
     const int groups = (H + heads - 1) / heads, b = blockIdx.z / groups, h0 = (blockIdx.z - b * groups) * heads;
-    const int r0 = blockIdx.y * kScoreRows, c0 = blockIdx.x * kScoreCols, tid = threadIdx.x;
+    const int r0 = blockIdx.y * ROWS, c0 = blockIdx.x * kScoreCols, tid = threadIdx.x;
     if (masks.nonpad != nullptr) {
-        __shared__ int s_row[kScoreRows], s_col[kScoreCols];  // node of a row or column; -1: nobody's, -2: every node's
+        __shared__ int s_row[ROWS], s_col[kScoreCols];  // node of a row or column; -1: nobody's, -2: every node's
         const uint8_t *np = masks.nonpad + (size_t)b * masks.L;
-        if (tid < kScoreRows) {
+        if (tid < ROWS) {
             const int row = r0 + tid;
             // row M is the left option "none", which every node shares
             s_row[tid] = row > 2 * M ? -1 : row == M ? -2 : masks.nodes[row < M ? row : row - M - 1];
-        } else if (tid < kScoreRows + kScoreCols) {
-            const int s = c0 + tid - kScoreRows, c = s < M ? masks.nodes[s] : -1;
-            s_col[tid - kScoreRows] = c >= 0 && np[c] && masks.main_chain[c] ? c : -1;
+        } else if (tid < ROWS + kScoreCols) {
+            const int s = c0 + tid - ROWS, c = s < M ? masks.nodes[s] : -1;
+            s_col[tid - ROWS] = c >= 0 && np[c] && masks.main_chain[c] ? c : -1;
         }
         __syncthreads();
         bool needed = false;
         for (int part = 0; part < 4 && !needed; part++) {  // rows part, part + 4, ... of the tile
             bool mine = false;
 #pragma unroll
-            for (int i = 0; i < kScoreRows / 4 * kScoreCols / 256; i++) {
+            for (int i = 0; i < ROWS / 4 * kScoreCols / 256; i++) {
                 const int at = tid + 256 * i, a = s_row[part + at / kScoreCols * 4], c = s_col[at % kScoreCols];
                 if (a != -1 && c >= 0) mine |= a == -2 || !__ldg(masks.right_mask + (size_t)a * masks.L + c);
             }
@@ -350,17 +355,17 @@ __global__ void __launch_bounds__(256, 2)
     auto stage = [&](int step) {
         const size_t bh = (size_t)b * H + h0 + step / chunks;
         const int k0 = step % chunks * kScoreK;
-        float *tile = s_tiles + (step & 1) * kScoreStage;  // rows of A, then rows of krm
+        float *tile = s_tiles + (step & 1) * kScoreStage<ROWS>;  // rows of A, then rows of krm
         auto source = [&](int r, bool &in) {
-            in = r < kScoreRows ? r0 + r <= 2 * M : c0 + r - kScoreRows < M;
+            in = r < ROWS ? r0 + r <= 2 * M : c0 + r - ROWS < M;
             if (!in) return krm;
             const int row = r0 + r;
-            return r >= kScoreRows ? krm + (bh * M + c0 + r - kScoreRows) * D
+            return r >= ROWS ? krm + (bh * M + c0 + r - ROWS) * D
                                    : row < M ? qm + (bh * M + row) * D : klm + (bh * (M + 1) + row - M) * D;
         };
         if (vec) {
 #pragma unroll
-            for (int i = tid; i < (kScoreRows + kScoreCols) * (kScoreK / 4); i += 256) {
+            for (int i = tid; i < (ROWS + kScoreCols) * (kScoreK / 4); i += 256) {
                 const int r = i / (kScoreK / 4), k = i % (kScoreK / 4) * 4;
                 bool in;
                 const float *src = source(r, in);
@@ -368,7 +373,7 @@ __global__ void __launch_bounds__(256, 2)
                 copy_async16(tile + r * kScorePitch + k, in ? src + k0 + k : krm, in);
             }
         } else {
-            for (int i = tid; i < (kScoreRows + kScoreCols) * kScoreK; i += 256) {
+            for (int i = tid; i < (ROWS + kScoreCols) * kScoreK; i += 256) {
                 const int r = i / kScoreK, k = i % kScoreK;
                 bool in;
                 const float *src = source(r, in);
@@ -378,20 +383,20 @@ __global__ void __launch_bounds__(256, 2)
         }
         copy_commit();
     };
-    float acc[8][4] = {};
+    float acc[ROWS / 16][4] = {};
     stage(0);
     for (int step = 0; step < steps; step++) {
         copy_wait();
         __syncthreads();  // this chunk is there, and nobody reads the other buffer any more
         if (step + 1 < steps) stage(step + 1);
-        const float *sa = s_tiles + (step & 1) * kScoreStage, *sb = sa + kScoreRows * kScorePitch;
+        const float *sa = s_tiles + (step & 1) * kScoreStage<ROWS>, *sb = sa + ROWS * kScorePitch;
 #pragma unroll 2
         for (int k = 0; k < kScoreK; k += 4) {
             float4 b4[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) b4[j] = *reinterpret_cast<const float4 *>(sb + (tx + 16 * j) * kScorePitch + k);
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
+            for (int i = 0; i < ROWS / 16; i++) {
                 const float4 a4 = *reinterpret_cast<const float4 *>(sa + (ty + 16 * i) * kScorePitch + k);
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
@@ -405,7 +410,7 @@ __global__ void __launch_bounds__(256, 2)
         if ((step + 1) % chunks == 0) {
             const size_t bh = (size_t)b * H + h0 + step / chunks;
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
+            for (int i = 0; i < ROWS / 16; i++) {
                 const int row = r0 + ty + 16 * i;
                 float *out = row < M ? ac + (bh * M + row) * M : bc + (bh * (M + 1) + (row - M)) * M;
 #pragma unroll
@@ -542,7 +547,7 @@ __global__ void __launch_bounds__(256)
 // and scattered to the nodes: dq[nodes[a]], dkr[nodes[s]], dkl[nodes[a] - 1] and dkl[0] (which also takes row 1 of the
 // first main-chain node, whose left option 1 is node 0 again).  dq, dkl, dkr [B][L][H][D] f32 were zero-filled.
 //
-// Four float32 matrix products, M x M x D each, per (sentence, head).  A block makes 64 rows x 64 columns of d of the
+// Four float32 matrix products, M x M x D each, per (sentence, head).  A block makes ROWS rows x 64 columns of d of the
 // parents' two products (role 0) or of the children's two (role 1), 4 x 4 outputs of both per thread, the summed index
 // walked in chunks of 32 through shared memory (the next chunk in flight while this one is multiplied): three 16-byte
 // shared-memory loads per 32 FMAs, and no shape is too large for it.  The X matrices are zero wherever a child is not
@@ -550,24 +555,28 @@ __global__ void __launch_bounds__(256)
 // features beside it are not finite (0 x inf stays NaN).  90 sentences, M = 161, 8 x 64 features: 284 us (366 us
 // without the next chunk in flight); 3 095 us with one thread per output reading its operands from global memory, as
 // it was.
-constexpr int kFgThreads = 256, kFgTile = 64, kFgChunk = 32, kFgPitch = kFgChunk + 4;
-constexpr int kFgStage = 4 * kFgChunk * kFgTile;  // floats of one chunk: role 1, the larger of the two; two of them
-constexpr size_t kFgSmem = (2 * kFgStage + 4 * kFgTile) * sizeof(float);
+// ROWS: rows of a tile, 64, or 32 or 16 where the chain has no more nodes (128 sentences of 29 nodes: 34 us, 54 us with 64
+// rows; of 12 nodes: 20 and 51 us); four threads per row.
+constexpr int kFgTile = 64, kFgChunk = 32, kFgPitch = kFgChunk + 4;
+constexpr int fg_stage(int rows) { return 2 * kFgChunk * (rows + kFgTile); }  // floats of a chunk: role 1, the larger one
+constexpr int fg_stages(int rows) { return rows > kFgChunk ? 2 : 1; }         // chains up to 32 nodes are one chunk
+constexpr size_t fg_smem(int rows) { return (fg_stages(rows) * fg_stage(rows) + 4 * rows) * sizeof(float); }
 
 __device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) < CUDART_INF_F); }
 
 // rows r0 .. r0 + 31 (< rows), columns d0 .. d0 + 63 (< D) of src [rows][D] into dst [32][64], zero outside
+template <int THREADS>
 __device__ __forceinline__ void stage_features(const float *__restrict__ src, int r0, int rows, int d0, int D, bool vec,
                                                float *dst) {
     if (vec) {
 #pragma unroll
-        for (int i = threadIdx.x; i < kFgChunk * kFgTile / 4; i += kFgThreads) {
+        for (int i = threadIdx.x; i < kFgChunk * kFgTile / 4; i += THREADS) {
             const int r = r0 + i / (kFgTile / 4), d = d0 + i % (kFgTile / 4) * 4;
             const bool in = r < rows && d < D;
             copy_async16(dst + 4 * i, in ? src + (size_t)r * D + d : src, in);
         }
     } else {
-        for (int i = threadIdx.x; i < kFgChunk * kFgTile; i += kFgThreads) {
+        for (int i = threadIdx.x; i < kFgChunk * kFgTile; i += THREADS) {
             const int r = r0 + i / kFgTile, d = d0 + i % kFgTile;
             const bool in = r < rows && d < D;
             copy_async4(dst + i, in ? src + (size_t)r * D + d : src, in);
@@ -575,27 +584,30 @@ __device__ __forceinline__ void stage_features(const float *__restrict__ src, in
     }
 }
 // whether what this thread staged there has an infinity or a NaN
+template <int THREADS>
 __device__ __forceinline__ bool staged_not_finite(const float *dst, bool vec) {
     bool odd = false;
 #pragma unroll
-    for (int j = 0; j < kFgChunk * kFgTile / kFgThreads; j++)
-        odd |= not_finite(vec ? dst[4 * (threadIdx.x + j / 4 * kFgThreads) + j % 4] : dst[threadIdx.x + j * kFgThreads]);
+    for (int j = 0; j < kFgChunk * kFgTile / THREADS; j++)
+        odd |= not_finite(vec ? dst[4 * (threadIdx.x + j / 4 * THREADS) + j % 4] : dst[threadIdx.x + j * THREADS]);
     return odd;
 }
 
 __device__ __forceinline__ float part(const float4 &v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
 
 // vec: D a multiple of 4 and the feature matrices on 16-byte boundaries
-__global__ void __launch_bounds__(kFgThreads, 2)
+template <int ROWS>
+__global__ void __launch_bounds__(4 * ROWS, 2 * (64 / ROWS))
     links_features_grad_kernel(const float *__restrict__ X0, const float *__restrict__ X1, const float *__restrict__ dab,
                                const float *__restrict__ qm, const float *__restrict__ klm, const float *__restrict__ krm,
                                const int *__restrict__ nodes, int M, int L, int H, int D, int vec, float *__restrict__ dq,
                                float *__restrict__ dkl, float *__restrict__ dkr) {
     extern __shared__ __align__(16) float s_tiles[];
+    constexpr int THREADS = 4 * ROWS, STAGE = fg_stage(ROWS);
     // blocks by (sentence, head), tile of d, tile of rows, role: along x, which alone takes more than 65 535
-    const unsigned per_d = 2 * ((M + kFgTile - 1) / kFgTile), d_tiles = (D + kFgTile - 1) / kFgTile;
+    const unsigned per_d = 2 * ((M + ROWS - 1) / ROWS), d_tiles = (D + kFgTile - 1) / kFgTile;
     const unsigned at_d = blockIdx.x / per_d, at_r = blockIdx.x - at_d * per_d;
-    const int role = at_r & 1, r0 = (at_r >> 1) * kFgTile, d0 = at_d % d_tiles * kFgTile;
+    const int role = at_r & 1, r0 = (at_r >> 1) * ROWS, d0 = at_d % d_tiles * kFgTile;
     const size_t bh = at_d / d_tiles;
     const int b = (int)bh / H, h = (int)bh - b * H;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -605,28 +617,28 @@ __global__ void __launch_bounds__(kFgThreads, 2)
     float acc0[4][4] = {}, acc1[4][4] = {};
     const int chunks = (M + kFgChunk - 1) / kFgChunk;
     if (role == 0) {  // rows are parents a; summed over the children s
-        constexpr int kX1 = kFgTile * kFgPitch, kK = 2 * kX1;  // X0, X1 [64][36] and krm [32][64] in a stage
+        constexpr int kX1 = ROWS * kFgPitch, kK = 2 * kX1;  // X0, X1 [ROWS][36] and krm [32][64] in a stage
         auto stage = [&](int step) {
             const int s0 = step * kFgChunk;
-            float *tile = s_tiles + (step & 1) * kFgStage;
+            float *tile = s_tiles + (step & 1) * STAGE;
 #pragma unroll
-            for (int i = tid; i < kFgTile * kFgChunk; i += kFgThreads) {
+            for (int i = tid; i < ROWS * kFgChunk; i += THREADS) {
                 const int r = i / kFgChunk, s = i % kFgChunk;
                 const bool in = r0 + r < M && s0 + s < M;
                 const size_t at = in ? (size_t)(r0 + r) * M + s0 + s : 0;
                 copy_async4(tile + r * kFgPitch + s, x0 + at, in);
                 copy_async4(tile + kX1 + r * kFgPitch + s, x1 + at, in);
             }
-            stage_features(kr, s0, M, d0, D, vec, tile + kK);
+            stage_features<THREADS>(kr, s0, M, d0, D, vec, tile + kK);
             copy_commit();
         };
         stage(0);
         for (int step = 0; step < chunks; step++) {
-            const float *sx0 = s_tiles + (step & 1) * kFgStage, *sx1 = sx0 + kX1, *sk = sx0 + kK;
+            const float *sx0 = s_tiles + (step & 1) * STAGE, *sx1 = sx0 + kX1, *sk = sx0 + kK;
             copy_wait();
-            bool work = staged_not_finite(sk, vec);  // a thread looks at what it copied itself: no barrier in between
+            bool work = staged_not_finite<THREADS>(sk, vec);  // a thread looks at what it copied itself: no barrier in between
 #pragma unroll
-            for (int i = tid; i < kFgTile * kFgChunk; i += kFgThreads) {
+            for (int i = tid; i < ROWS * kFgChunk; i += THREADS) {
                 const int at = i / kFgChunk * kFgPitch + i % kFgChunk;
                 work |= sx0[at] != 0.f || sx1[at] != 0.f;
             }
@@ -682,38 +694,38 @@ __global__ void __launch_bounds__(kFgThreads, 2)
         if (tid < kFgTile && d0 + tid < D) {
             float sum = 0.f;
 #pragma unroll
-            for (int i = 0; i < 16; i++) sum += red[i * kFgTile + tid];
+            for (int i = 0; i < ROWS / 4; i++) sum += red[i * kFgTile + tid];
             atomicAdd(dkl + base + d0 + tid, sum);
         }
     } else {  // rows are children s; summed over the parents a
-        constexpr int kPart = kFgChunk * kFgTile;  // X0 (then X0 + X1), X1, qm, klm, each [32][64], in a stage
-        float *sums = s_tiles + 2 * kFgStage;      // [4][64]
-        const int s_own = r0 + (tid & 63);         // the column whose X this thread stages
-        float x0sum = 0.f;                         // its sum of X0 over a = tid / 64 + 4 j
+        constexpr int kX = kFgChunk * ROWS, kPart = kFgChunk * kFgTile;  // X0 (then X0 + X1), X1 [32][ROWS], qm, klm [32][64] in a stage
+        float *sums = s_tiles + fg_stages(ROWS) * STAGE;  // [4][ROWS]
+        const int own = tid % ROWS, a_own = tid / ROWS, s_own = r0 + own;  // the column whose X this thread stages
+        float x0sum = 0.f;                                // its sum of X0 over a = a_own + 4 j
         auto stage = [&](int step) {
             const int a0 = step * kFgChunk;
-            float *tile = s_tiles + (step & 1) * kFgStage;
+            float *tile = s_tiles + (step & 1) * STAGE;
 #pragma unroll
             for (int j = 0; j < kFgChunk / 4; j++) {
-                const int a = (tid >> 6) + 4 * j;
+                const int a = a_own + 4 * j;
                 const bool in = a0 + a < M && s_own < M;
                 const size_t at = in ? (size_t)(a0 + a) * M + s_own : 0;
-                copy_async4(tile + a * kFgTile + (tid & 63), x0 + at, in);
-                copy_async4(tile + kPart + a * kFgTile + (tid & 63), x1 + at, in);
+                copy_async4(tile + a * ROWS + own, x0 + at, in);
+                copy_async4(tile + kX + a * ROWS + own, x1 + at, in);
             }
-            stage_features(q, a0, M, d0, D, vec, tile + 2 * kPart);
-            stage_features(kl + D, a0, M, d0, D, vec, tile + 3 * kPart);
+            stage_features<THREADS>(q, a0, M, d0, D, vec, tile + 2 * kX);
+            stage_features<THREADS>(kl + D, a0, M, d0, D, vec, tile + 2 * kX + kPart);
             copy_commit();
         };
         stage(0);
         for (int step = 0; step < chunks; step++) {
-            float *sxs = s_tiles + (step & 1) * kFgStage;
-            const float *sx1 = sxs + kPart, *sq = sxs + 2 * kPart, *sk = sxs + 3 * kPart;
+            float *sxs = s_tiles + (step & 1) * STAGE;
+            const float *sx1 = sxs + kX, *sq = sxs + 2 * kX, *sk = sq + kPart;
             copy_wait();
-            bool work = staged_not_finite(sq, vec) || staged_not_finite(sk, vec);
+            bool work = staged_not_finite<THREADS>(sq, vec) || staged_not_finite<THREADS>(sk, vec);
 #pragma unroll
             for (int j = 0; j < kFgChunk / 4; j++) {
-                const int at = ((tid >> 6) + 4 * j) * kFgTile + (tid & 63);
+                const int at = (a_own + 4 * j) * ROWS + own;
                 const float v0 = sxs[at], v1 = sx1[at];
                 work |= v0 != 0.f || v1 != 0.f;
                 x0sum += v0;
@@ -724,8 +736,8 @@ __global__ void __launch_bounds__(kFgThreads, 2)
             if (!work) continue;
 #pragma unroll 4
             for (int a = 0; a < kFgChunk; a++) {
-                const float4 xs = *reinterpret_cast<const float4 *>(sxs + a * kFgTile + 4 * ty);
-                const float4 xb = *reinterpret_cast<const float4 *>(sx1 + a * kFgTile + 4 * ty);
+                const float4 xs = *reinterpret_cast<const float4 *>(sxs + a * ROWS + 4 * ty);
+                const float4 xb = *reinterpret_cast<const float4 *>(sx1 + a * ROWS + 4 * ty);
                 const float4 qv = *reinterpret_cast<const float4 *>(sq + a * kFgTile + 4 * tx);
                 const float4 kv = *reinterpret_cast<const float4 *>(sk + a * kFgTile + 4 * tx);
 #pragma unroll
@@ -737,14 +749,14 @@ __global__ void __launch_bounds__(kFgThreads, 2)
                     }
             }
         }
-        sums[(tid >> 6) * kFgTile + (tid & 63)] = x0sum;
+        sums[a_own * ROWS + own] = x0sum;
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int r = r0 + 4 * ty + i;
             if (r >= M) continue;
             const int t = 4 * ty + i;
-            const float w = (sums[t] + sums[kFgTile + t]) + (sums[2 * kFgTile + t] + sums[3 * kFgTile + t]);
+            const float w = (sums[t] + sums[ROWS + t]) + (sums[2 * ROWS + t] + sums[3 * ROWS + t]);
             const size_t at = base + nodes[r] * pitch;
 #pragma unroll
             for (int c = 0; c < 4; c++) {
@@ -769,16 +781,22 @@ int launch_links_scores(const float *qm, const float *klm, const float *krm, con
                         cudaStream_t st) {
     if (B == 0 || M == 0) return PCFGNAT_OK;
     const int vec = D % 4 == 0 && on_16_bytes({qm, klm, krm});
-    const dim3 tiles((M + kScoreCols - 1) / kScoreCols, (2 * M + 1 + kScoreRows - 1) / kScoreRows);
+    const int cols = (M + kScoreCols - 1) / kScoreCols;
+    const bool small = 2 * M + 1 <= 64 || (long long)cols * ((2 * M + 1 + 127) / 128) * B * H < sm_count();
+    const int rows = small ? 64 : 128;
+    const dim3 tiles(cols, (2 * M + 1 + rows - 1) / rows);
     // up to four heads per block (the test for tiles in use and the first chunk's latency are paid once), as long as
     // there are four blocks for every place on the GPU: tiles that are not in use leave at once
     int heads = 4;
     while (heads > 1 && (long long)tiles.x * tiles.y * B * ((H + heads - 1) / heads) < 4ll * 2 * sm_count()) heads /= 2;
-    const size_t smem = 2 * kScoreStage * sizeof(float);
-    if (ensure_dynamic_smem(links_scores_kernel, smem) != cudaSuccess) return PCFGNAT_ERR_CUDA;
-    links_scores_kernel<<<dim3(tiles.x, tiles.y, B * ((H + heads - 1) / heads)), 256, smem, st>>>(
-        qm, klm, krm, M, H, D, heads, vec, ScoreMasks{nonpad, right_mask, main_chain, nodes, L}, ac, bc);
-    return cuda_rc(cudaGetLastError());
+    const auto launch = [&](auto kernel, size_t smem) {
+        if (ensure_dynamic_smem(kernel, smem) != cudaSuccess) return PCFGNAT_ERR_CUDA;
+        kernel<<<dim3(tiles.x, tiles.y, B * ((H + heads - 1) / heads)), 256, smem, st>>>(
+            qm, klm, krm, M, H, D, heads, vec, ScoreMasks{nonpad, right_mask, main_chain, nodes, L}, ac, bc);
+        return cuda_rc(cudaGetLastError());
+    };
+    return small ? launch(links_scores_kernel<64>, 2 * kScoreStage<64> * sizeof(float))
+                 : launch(links_scores_kernel<128>, 2 * kScoreStage<128> * sizeof(float));
 }
 
 int launch_links_backward(const float *links_grad, const float *ac, const float *bc, const float *qm, const float *klm,
@@ -801,11 +819,16 @@ int launch_links_backward(const float *links_grad, const float *ac, const float 
     if (cudaGetLastError() != cudaSuccess) return PCFGNAT_ERR_CUDA;
     if (M == 0) return PCFGNAT_OK;
     const int vec = D % 4 == 0 && on_16_bytes({qm, klm, krm});
-    const long long grid = 2ll * ((M + kFgTile - 1) / kFgTile) * ((D + kFgTile - 1) / kFgTile) * B * H;
-    if (grid > INT32_MAX) return PCFGNAT_ERR_TOO_LARGE;
-    if (ensure_dynamic_smem(links_features_grad_kernel, kFgSmem) != cudaSuccess) return PCFGNAT_ERR_CUDA;
-    links_features_grad_kernel<<<(unsigned)grid, kFgThreads, kFgSmem, st>>>(X0, X1, dab, qm, klm, krm, nodes, M, L, H, D, vec, dq, dkl, dkr);
-    return cuda_rc(cudaGetLastError());
+    const auto launch = [&](auto kernel, int rows) {
+        const long long grid = 2ll * ((M + rows - 1) / rows) * ((D + kFgTile - 1) / kFgTile) * B * H;
+        if (grid > INT32_MAX) return PCFGNAT_ERR_TOO_LARGE;
+        if (ensure_dynamic_smem(kernel, fg_smem(rows)) != cudaSuccess) return PCFGNAT_ERR_CUDA;
+        kernel<<<(unsigned)grid, 4 * rows, fg_smem(rows), st>>>(X0, X1, dab, qm, klm, krm, nodes, M, L, H, D, vec, dq, dkl, dkr);
+        return cuda_rc(cudaGetLastError());
+    };
+    return M <= 16   ? launch(links_features_grad_kernel<16>, 16)
+           : M <= 32 ? launch(links_features_grad_kernel<32>, 32)
+                     : launch(links_features_grad_kernel<64>, 64);
 }
 
 int launch_links_gather(const void *q, const void *kl, const void *kr, int is_half, const int *nodes, int M, int B, int L,

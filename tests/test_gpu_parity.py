@@ -1366,6 +1366,20 @@ def test_links_gradient_of_improbable_cells_with_large_weights(pkg, ops, heads):
         assert (x - y).abs().max() <= 1e-4 * y.abs().max(), tuple(x.shape)
 
 
+@pytest.mark.parametrize("B, L, heads, dim", [(3, 6, 3, 64), (2, 32, 2, 68), (2, 34, 2, 33), (40, 66, 4, 36), (20, 130, 8, 8)])
+def test_links_and_gradient_at_other_tiles(pkg, ops, B, L, heads, dim):
+    """The smaller tiles of the product kernels (up to 16, 32 and 31 nodes, and grids smaller than the GPU) and the larger
+    one with a single tile of rows, ragged sentences, against float64: float32 sums, 2e-5 of the largest entry."""
+    g = torch.Generator().manual_seed(L)
+    leaves = [torch.randn(B, L, heads, dim, generator=g) for _ in range(3)] + [torch.randn(B, L, heads, generator=g)]
+    length = torch.randint(2, L + 1, (B,), generator=g)
+    length[0] = L
+    got, grads, want, ref = _links_and_float64(pkg, ops, leaves, length, lambda want: torch.randn(want.shape, generator=g))
+    torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-4)
+    for x, y in zip(grads, ref):
+        assert (x - y).abs().max() <= 2e-5 * y.abs().max(), tuple(x.shape)
+
+
 @pytest.mark.parametrize("heads, scale", [(1, 4.0), (2, 4.0), (8, 5.0)])
 def test_links_of_improbable_cells(pkg, ops, heads, scale):
     """Transitions below the probability (1e-30) under which the mixture is formed from log-probabilities, and their
