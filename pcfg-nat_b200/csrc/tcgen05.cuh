@@ -131,8 +131,15 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t *r) {
 using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// The driver's encoder wants a context, which a thread has only after its first runtime call: the device's is bound here.
 inline EncodeTiledFn encode_tiled_fn() {
     static EncodeTiledFn fn = nullptr;
+    static thread_local bool bound = false;
+    if (!bound) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return nullptr;
+        bound = true;
+    }
     if (!fn) {
         void *p = nullptr;
         cudaDriverEntryPointQueryResult q;

@@ -1093,6 +1093,30 @@ def test_convert_rows(ops, H):
     assert k.rows_to_bf16(src[:0]).shape == (0, H)
 
 
+def test_projection_as_the_first_call_of_a_thread(ops):
+    """A thread that has made no CUDA call yet (an autograd thread, a server's worker) has no context until one is bound: the
+    tensor maps are encoded for it all the same."""
+    import threading
+
+    k = ops.get_pcfg_kernel()
+    h, w = torch.randn(2, 16, 64, device=DEV).half(), (torch.randn(96, 64, device=DEV) * 0.1).half()
+    targets = torch.randint(0, 96, (2, 5), device=DEV)
+    out = k.proj_logsoftmax_gather(h, w, targets, want_lse=True)
+    grad = torch.randn(2, 16, 5, device=DEV)
+    calls = [lambda: k.proj_logsoftmax_gather(h, w, targets)["match"],
+             lambda: k.proj_dlogits(h, w, targets, None, None, out["lse"], grad)]
+    dl, wb, rows = calls[1](), w.to(torch.bfloat16), h.view(32, 64).to(torch.bfloat16)
+    calls.append(lambda: k.proj_backward_gemms(dl, wb, rows)[1])
+    for call in calls:
+        want, got = call(), []
+        torch.cuda.synchronize()
+        thread = threading.Thread(target=lambda: got.append(call()))
+        thread.start()
+        thread.join()
+        torch.cuda.synchronize()
+        assert len(got) == 1 and torch.equal(got[0], want)
+
+
 def test_convert_rows_checks_its_index(ops):
     """What torch's index operators converted or refused still is: 32-bit indices, rows that do not match."""
     k = ops.get_pcfg_kernel()
