@@ -1049,7 +1049,10 @@ dag_logsoftmax_gather_inplace = DagLogsoftmaxGatherFunc.apply
 
 
 def _bf16(t):
-    return get_pcfg_kernel().rows_to_bf16(t) if t.dtype == torch.float16 else t.to(torch.bfloat16).contiguous()
+    # a small matrix by one operator of torch: 8 us of host time where the kernel's call takes 15, and 2 us more on the device
+    if t.dtype == torch.float16 and t.numel() >= 1 << 20:
+        return get_pcfg_kernel().rows_to_bf16(t)
+    return t.to(torch.bfloat16).contiguous()
 
 
 def proj_backward_products(dlogits, weight, rows):
