@@ -327,6 +327,23 @@ int pcfgnat_links_scores(const float *qm, const float *klm, const float *krm, in
 int pcfgnat_links_scores_masked(const float *qm, const float *klm, const float *krm, const uint8_t *nonpad,
                                 const uint8_t *right_tree_mask, const uint8_t *main_chain, const int *nodes, int M, int B,
                                 int L, int heads, int head_dim, float *ac, float *bc, void *stream);
+/* The same links without score matrices, in two launches, for half-precision features (dtype PCFGNAT_DTYPE_F16, on 16-byte
+ * boundaries) of head_dim 32 or 64, heads x head_dim up to 1024 and up to 1024 main-chain nodes; others are refused with
+ * PCFGNAT_ERR_UNSUPPORTED, as are a few long sentences, which the three launches form faster
+ * (pcfgnat_links_fused_kept_bytes is 0 for a shape that is refused).  `kept`: memory of that many bytes, 16-byte
+ * aligned; scratch, unless `training`, when it holds what pcfgnat_links_fused_backward reads (packed features, sums of the rows:
+ * the features themselves are not read again). */
+int pcfgnat_links_fused(const void *q, const void *kl, const void *kr, int dtype, const float *gate_logits,
+                        const uint8_t *nonpad, const uint8_t *left_tree_mask, const uint8_t *right_tree_mask,
+                        const uint8_t *main_chain, const int *nodes, int M, int B, int L, int heads, int head_dim, int max_left,
+                        float *links, void *kept, size_t kept_bytes, int training, void *stream);
+/* Their gradient, in three launches.  Outputs dq, dkl, dkr [B][L][heads][head_dim] of type `dtype` (PCFGNAT_DTYPE_F16 or _F32,
+ * 16-byte aligned) and dgates [B][L][heads] f32, every cell written.  `kept` is only read. */
+size_t pcfgnat_links_fused_kept_bytes(int M, int B, int heads, int head_dim, int training);
+size_t pcfgnat_links_fused_scratch_bytes(int M, int B, int heads, int head_dim);
+int pcfgnat_links_fused_backward(const float *links_grad, const void *kept, const int *slot_of, const int *nodes, int M, int B, int L,
+                                 int heads, int head_dim, int max_left, void *scratch, size_t scratch_bytes, int dtype, void *dq,
+                                 void *dkl, void *dkr, float *dgates, void *stream);
 /* Gradient of those links with respect to the link features and the gate logits (training; the reference gets it
  * from autograd through the ~30 operators of extract_links).  links_grad [B][L][2][L] f32; ac, bc, qm, klm, krm and
  * the masks as in the forward.  Scratch: X0, X1 [B][heads][M][M] and dab [B][heads][M][2] f32 (fully overwritten at

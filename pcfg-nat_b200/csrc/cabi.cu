@@ -555,6 +555,41 @@ int pcfgnat_proj_backward_gemms(const void *dlogits, const void *weight_bf16, co
                                       static_cast<cudaStream_t>(stream));
 }
 
+int pcfgnat_links_fused(const void *q, const void *kl, const void *kr, int dtype, const float *gate_logits,
+                        const uint8_t *nonpad, const uint8_t *left_tree_mask, const uint8_t *right_tree_mask,
+                        const uint8_t *main_chain, const int *nodes, int M, int B, int L, int heads, int head_dim, int max_left,
+                        float *links, void *kept, size_t kept_bytes, int training, void *stream) {
+    PCFGNAT_API_RANGE();
+    if (max_left != 1 || dtype != PCFGNAT_DTYPE_F16) return PCFGNAT_ERR_UNSUPPORTED;
+    if (B < 0 || L < 1 || M < 0 || M > L || heads < 1 || head_dim < 1) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    if (B && (!q || !kl || !kr || !gate_logits || !nonpad || !left_tree_mask || !right_tree_mask || !main_chain || !nodes || !links || !kept))
+        return PCFGNAT_ERR_INVALID_ARGUMENT;
+    if (kept_bytes < links_fused_kept_bytes(M, B, heads, head_dim, training)) return PCFGNAT_ERR_WORKSPACE;
+    return launch_links_fused(q, kl, kr, gate_logits, nonpad, left_tree_mask, right_tree_mask, main_chain, nodes, M, B, L, heads,
+                              head_dim, links, kept, training, static_cast<cudaStream_t>(stream));
+}
+
+size_t pcfgnat_links_fused_kept_bytes(int M, int B, int heads, int head_dim, int training) {
+    return M < 0 || B < 0 || heads < 1 || head_dim < 1 ? 0 : links_fused_kept_bytes(M, B, heads, head_dim, training);
+}
+
+size_t pcfgnat_links_fused_scratch_bytes(int M, int B, int heads, int head_dim) {
+    return M < 0 || B < 0 || heads < 1 || head_dim < 1 ? 0 : links_fused_scratch_bytes(M, B, heads, head_dim);
+}
+
+int pcfgnat_links_fused_backward(const float *links_grad, const void *kept, const int *slot_of, const int *nodes, int M, int B, int L,
+                                 int heads, int head_dim, int max_left, void *scratch, size_t scratch_bytes, int dtype, void *dq,
+                                 void *dkl, void *dkr, float *dgates, void *stream) {
+    PCFGNAT_API_RANGE();
+    if (max_left != 1 || (dtype != PCFGNAT_DTYPE_F16 && dtype != PCFGNAT_DTYPE_F32)) return PCFGNAT_ERR_UNSUPPORTED;
+    if (B < 0 || L < 1 || M < 0 || M > L || heads < 1 || head_dim < 1) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    if (B && (!links_grad || !kept || !slot_of || !nodes || !scratch || !dq || !dkl || !dkr || !dgates))
+        return PCFGNAT_ERR_INVALID_ARGUMENT;
+    if (scratch_bytes < links_fused_scratch_bytes(M, B, heads, head_dim)) return PCFGNAT_ERR_WORKSPACE;
+    return launch_links_fused_backward(links_grad, kept, slot_of, nodes, M, B, L, heads, head_dim, scratch,
+                                       dtype == PCFGNAT_DTYPE_F16, dq, dkl, dkr, dgates, static_cast<cudaStream_t>(stream));
+}
+
 int pcfgnat_links_gather_features(const void *q, const void *kl, const void *kr, int dtype, const int *nodes, int M,
                                   int B, int L, int heads, int head_dim, float *qm, float *klm, float *krm, void *stream) {
     PCFGNAT_API_RANGE();

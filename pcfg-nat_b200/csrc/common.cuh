@@ -215,6 +215,14 @@ int launch_proj(const void *hidden, const void *weight, const int64_t *targets, 
                 int B, int L, int T, int V, int H, float *match, float *max_lprob, int64_t *argmax, float *lse,
                 void *workspace, size_t ws_bytes, int *status, cudaStream_t st);
 
+int launch_links_fused(const void *q, const void *kl, const void *kr, const float *gates, const uint8_t *nonpad,
+                       const uint8_t *left_mask, const uint8_t *right_mask, const uint8_t *main_chain, const int *nodes, int M,
+                       int B, int L, int H, int D, float *links, void *kept, int training, cudaStream_t st);
+size_t links_fused_kept_bytes(int M, int B, int H, int D, int training);  // 0: shape not taken
+size_t links_fused_scratch_bytes(int M, int B, int H, int D);
+int launch_links_fused_backward(const float *links_grad, const void *kept, const int *slot_of, const int *nodes, int M, int B, int L,
+                                int H, int D, void *scratch, int half_out, void *dq, void *dkl, void *dkr, float *dgates,
+                                cudaStream_t st);
 int launch_links_gather(const void *q, const void *kl, const void *kr, int is_half, const int *nodes, int M, int B, int L,
                         int H, int D, float *qm, float *klm, float *krm, cudaStream_t st);
 int launch_links_scores(const float *qm, const float *klm, const float *krm, const uint8_t *nonpad, const uint8_t *right_mask,

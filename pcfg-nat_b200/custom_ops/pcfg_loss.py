@@ -681,9 +681,10 @@ class _Kernel:
 
     @staticmethod
     def _links_forward(query, key_left, key_right, gate_logits, prev_output_tokens, pad_index, left_tree_mask,
-                       right_tree_mask, main_chain, chain=None):
+                       right_tree_mask, main_chain, chain=None, keep=True):
         """Forward of ``extract_links``; returns (links, everything the backward needs).  ``chain``: the
-        ``main_chain_slots`` of main_chain where the caller keeps them (a step object, whose graph reads them)."""
+        ``main_chain_slots`` of main_chain where the caller keeps them (a step object, whose graph reads them).
+        ``keep=False``: no gradient will be asked for, nothing is kept (None)."""
         _require_cuda()
         if query.dim() != 4 or key_left.shape != query.shape or key_right.shape != query.shape:
             raise RuntimeError("query, key_left, key_right must be [batch, prelen, heads, head_dim] and agree")
@@ -730,6 +731,18 @@ class _Kernel:
         nodes, slot_of = chain
         M = nodes.numel()
         lib = _cabi.lib()
+        kept_bytes = lib.pcfgnat_links_fused_kept_bytes(M, B, H, D, int(keep)) if dt == torch.float16 else 0
+        if kept_bytes:  # a shape that the one-launch kernel takes
+            with torch.cuda.device(dev):
+                links = torch.empty((B, L, 2, L), dtype=torch.float32, device=dev)
+                kept = torch.empty(kept_bytes, dtype=torch.uint8, device=dev)
+                rc = lib.pcfgnat_links_fused(q.data_ptr(), kl.data_ptr(), kr.data_ptr(), 1, gates.data_ptr(),
+                                             nonpad.data_ptr(), lm.data_ptr(), rm.data_ptr(), mc.data_ptr(),
+                                             nodes.data_ptr(), M, B, L, H, D, 1, links.data_ptr(),
+                                             kept.data_ptr(), kept_bytes, int(keep), _stream(dev))
+            if rc != _cabi.ERR_UNSUPPORTED:  # features that are not on 16-byte boundaries
+                _cabi.check(rc, "pcfgnat_links_fused")
+                return links, dict(kept=kept, slot_of=slot_of, nodes=nodes, dims=(B, L, H, D, M)) if keep else None
         with torch.cuda.device(dev):
             qm = torch.empty((B, H, M, D), dtype=torch.float32, device=dev)
             krm = torch.empty((B, H, M, D), dtype=torch.float32, device=dev)
@@ -755,13 +768,28 @@ class _Kernel:
         return links, saved
 
     @staticmethod
-    def _links_backward(links_grad, saved):
-        """(d query, d key_left, d key_right [B, L, heads, head_dim] f32, d gate_logits [B, L, heads] f32)."""
+    def _links_backward(links_grad, saved, dtype=torch.float32):
+        """(d query, d key_left, d key_right [B, L, heads, head_dim], d gate_logits [B, L, heads] f32).  ``dtype`` of the
+        first three where the kernels can write it at once (float16, from half-precision features), else float32."""
         B, L, H, D, M = saved["dims"]
         g = _f32_cuda(links_grad, "links_grad", 4)
         if tuple(g.shape) != (B, L, 2, L):
             raise RuntimeError("links_grad must have the shape of links")
         dev = g.device
+        if "kept" in saved:
+            lib = _cabi.lib()
+            out_dtype = dtype if dtype == torch.float16 else torch.float32
+            with torch.cuda.device(dev):
+                nbytes = lib.pcfgnat_links_fused_scratch_bytes(M, B, H, D)
+                scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+                dq, dkl, dkr = (torch.empty((B, L, H, D), dtype=out_dtype, device=dev) for _ in range(3))
+                dgates = torch.empty((B, L, H), dtype=torch.float32, device=dev)
+                rc = lib.pcfgnat_links_fused_backward(g.data_ptr(), saved["kept"].data_ptr(), saved["slot_of"].data_ptr(),
+                                                      saved["nodes"].data_ptr(), M, B, L, H, D, 1, scratch.data_ptr(), nbytes,
+                                                      1 if out_dtype == torch.float16 else 0, dq.data_ptr(), dkl.data_ptr(),
+                                                      dkr.data_ptr(), dgates.data_ptr(), _stream(dev))
+            _cabi.check(rc, "pcfgnat_links_fused_backward")
+            return dq, dkl, dkr, dgates
         p = lambda name: saved[name].data_ptr()
         with torch.cuda.device(dev):
             # every main-chain node's block writes its whole row of these
@@ -785,14 +813,15 @@ class _Kernel:
                       right_tree_mask, main_chain, chain=None):
         """links [B, L, 2, L] f32 as the model's extract_links() forms them from the projected link features
         (models/...pcfg.py:140-201, max_left == 1): ``query``, ``key_left``, ``key_right`` [B, L, heads, head_dim]
-        (outputs of the three link projections, reshaped), ``gate_logits`` [B, L, heads].  Three launches: feature
-        gather, the per-head score products, and masking + joint log-softmax + head mixture + -inf rows.
+        (outputs of the three link projections, reshaped), ``gate_logits`` [B, L, heads].  Half-precision features of 32
+        or 64 per head without score matrices in memory (``pcfgnat_links_fused``); others, and a few long sentences, in
+        three launches: feature gather, the per-head score products, and masking + joint log-softmax + head mixture.
         Differentiable with respect to the four feature tensors (``ExtractLinksFunc``)."""
         if torch.is_grad_enabled() and any(t.requires_grad for t in (query, key_left, key_right, gate_logits)):
             return ExtractLinksFunc.apply(query, key_left, key_right, gate_logits, prev_output_tokens, pad_index,
                                           left_tree_mask, right_tree_mask, main_chain)
         return _Kernel._links_forward(query, key_left, key_right, gate_logits, prev_output_tokens, pad_index, left_tree_mask,
-                                      right_tree_mask, main_chain, chain)[0]
+                                      right_tree_mask, main_chain, chain, keep=False)[0]
 
     @staticmethod
     def loss_stats(sentence_loss, target_length):
@@ -1132,7 +1161,8 @@ class ExtractLinksFunc(Function):
 
     @staticmethod
     def backward(ctx, links_grad):
-        dq, dkl, dkr, dgates = _Kernel._links_backward(links_grad.contiguous(), ctx.saved)
+        dq, dkl, dkr, dgates = _Kernel._links_backward(links_grad.contiguous(), ctx.saved,
+                                                       torch.float16 if all(t == torch.float16 for t in ctx.dtypes[:3]) else torch.float32)
         out = [g.to(dt) if need else None
                for g, dt, need in zip((dq, dkl, dkr, dgates), ctx.dtypes, ctx.needs_input_grad[:4])]
         return (*out, None, None, None, None, None)

@@ -1357,6 +1357,12 @@ def test_extract_links_on_another_stream_than_the_first(pkg, ops):
     assert torch.equal(got, want), len(filler)
 
 
+def _tree_masks(L):
+    import importlib
+
+    return [m.to(DEV) for m in importlib.import_module("pcfg_nat_b200.support_tree").get_mask(L, 1)]
+
+
 def _links_and_float64(pkg, ops, leaves, length, G_of):
     """(links, gradients of the leaves, both again by autograd in float64): G_of(float64 links) weighs the finite cells."""
     import importlib
@@ -1402,6 +1408,60 @@ def test_links_and_gradient_at_other_tiles(pkg, ops, B, L, heads, dim):
     torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-4)
     for x, y in zip(grads, ref):
         assert (x - y).abs().max() <= 2e-5 * y.abs().max(), tuple(x.shape)
+
+
+@pytest.mark.parametrize("B, L, heads, dim, scale", [(2, 2, 1, 64, 1.0), (3, 3, 3, 32, 1.0), (2, 30, 9, 64, 1.0), (3, 32, 8, 64, 1.0),
+                                                     (2, 34, 32, 32, 1.0), (5, 66, 2, 64, 1.0), (1, 95, 12, 64, 1.0),
+                                                     (20, 130, 5, 32, 1.0), (64, 98, 1, 64, 1.0), (4, 94, 2, 64, 16.0)])
+def test_links_from_half_features_in_registers(pkg, ops, B, L, heads, dim, scale):
+    """The kernels without score matrices: chains of 1 to 65 nodes around their tiles of 16, more and fewer heads than a
+    block has warps, both head sizes, ragged sentences, improbable cells (scale 16: logits of up to 150 in units of log 2, spacing
+    1.5e-5, a handful of roundings: 2e-4), against autograd in float64: float32 sums, 2e-5 of the largest entry before
+    the gradients are rounded to half precision (2^-11 of each)."""
+    g = torch.Generator().manual_seed(L)
+    leaves = [(scale ** 0.5 * torch.randn(B, L, heads, dim, generator=g)).half() for _ in range(3)] + [torch.randn(B, L, heads, generator=g)]
+    length = torch.randint(2, L + 1, (B,), generator=g)
+    length[0] = L
+    k = ops.get_pcfg_kernel()
+    kept = k._links_forward(*[t.to(DEV) for t in leaves], torch.full((B, L), 3, device=DEV), 1, *_tree_masks(L))[1]
+    assert "kept" in kept  # the kernels under test
+    got, grads, want, ref = _links_and_float64(pkg, ops, leaves, length, lambda want: torch.randn(want.shape, generator=g))
+    assert scale == 1.0 or int((want < -69.1).sum()) > 3
+    torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-4 if scale == 1.0 else 2e-4)
+    for x, y, leaf in zip(grads, ref, leaves):
+        bound = (2e-5 if scale == 1.0 else 2e-4) * y.abs().max() + (y.abs() * 2.0 ** -11 if leaf.dtype == torch.float16 else 0)
+        assert ((x - y).abs() <= bound).all(), tuple(x.shape)
+
+
+def test_links_from_half_features_by_masks_and_odd_values(pkg, ops):
+    """Masks that are no tree's (random left and right children, an irregular main chain) with pads in the middle, features
+    with an infinity and a NaN, gradients of 1e12 and 1e-20: the kernels in registers against the ones over float32 scores,
+    which take the same features in float32 (sums of up to 40 terms in another order: 2e-5; a half's rounding)."""
+    B, L, heads, dim = 3, 44, 3, 32
+    g = torch.Generator().manual_seed(5)
+    left, right = (torch.rand(L, L, generator=g) < 0.5).to(torch.uint8), (torch.rand(L, L, generator=g) < 0.4).to(torch.uint8)
+    chain = (torch.rand(L, generator=g) < 0.8).to(torch.uint8)
+    left[:, 0], left[7] = 0, 1
+    prev = torch.where(torch.rand(B, L, generator=g) < 0.9, 3, 1)
+    prev[:, 0] = 3
+    feats = [torch.randn(B, L, heads, dim, generator=g).half() for _ in range(3)] + [torch.randn(B, L, heads, generator=g)]
+    feats[0][1, int(chain.nonzero()[5]), 1, 0], feats[2][2, int(chain.nonzero()[9]), 2, 3] = float("inf"), float("nan")
+    G = torch.randn(B, L, 2, L, generator=g)
+    G[0, :20] *= 1e12
+    G[0, 20:] *= 1e-20
+    masks = [m.to(DEV) for m in (left, right, chain)]
+    k = ops.get_pcfg_kernel()
+    half, kept = k._links_forward(*[t.to(DEV) for t in feats], prev.to(DEV), 1, *masks)
+    full, saved = k._links_forward(*[t.float().to(DEV) for t in feats], prev.to(DEV), 1, *masks)
+    assert "kept" in kept and "kept" not in saved
+    assert torch.equal(torch.isfinite(half), torch.isfinite(full))
+    torch.testing.assert_close(half, full, rtol=1e-5, atol=1e-4, equal_nan=True)
+    G = torch.where(torch.isfinite(full), G.to(DEV), 0)
+    for x, y in zip(k._links_backward(G, kept), k._links_backward(G, saved)):
+        assert torch.equal(torch.isfinite(x), torch.isfinite(y))
+        for b in range(B):  # sentences have scales of their own
+            part, of = x[b][torch.isfinite(y[b])], y[b][torch.isfinite(y[b])]
+            assert ((part - of).abs() <= 2e-5 * of.abs().max()).all(), (b, tuple(x.shape))
 
 
 @pytest.mark.parametrize("heads, scale", [(1, 4.0), (2, 4.0), (8, 5.0)])
