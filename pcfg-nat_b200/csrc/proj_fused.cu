@@ -194,6 +194,35 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
+// Two floats in one instruction (sm_100): each half rounded as the scalar instruction rounds it.  The epilogue's FMAs and sums go
+// two at a time and its maxima three: the tensor cores draw the card's power (1.4 GHz while they run), and what the epilogue
+// saves in instructions they get.  10 804 rows x 40 000 x 512: 332 -> 327 us a call, 354 -> 342 us in a loop of them.
+struct F2 {
+    unsigned long long bits;
+    __device__ __forceinline__ F2(float x, float y) { asm("mov.b64 %0, {%1, %2};" : "=l"(bits) : "f"(x), "f"(y)); }
+    __device__ __forceinline__ float2 get() const {
+        float2 v;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(bits));
+        return v;
+    }
+};
+__device__ __forceinline__ F2 fma2(F2 a, const F2 &b, const F2 &c) {
+    asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(a.bits) : "l"(b.bits), "l"(c.bits));
+    return a;
+}
+__device__ __forceinline__ F2 mul2(F2 a, const F2 &b) {
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(a.bits) : "l"(b.bits));
+    return a;
+}
+__device__ __forceinline__ F2 add2(F2 a, const F2 &b) {
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a.bits) : "l"(b.bits));
+    return a;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    asm("max.f32 %0, %0, %1, %2;" : "+f"(a) : "f"(b), "f"(c));
+    return a;
+}
+
 // ---------------------------------------------------------------------------------------
 // preparation: compact row list, target lists sorted by token id
 // ---------------------------------------------------------------------------------------
@@ -538,8 +567,13 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1)
                             if (col0 + i >= V) v[i] = -CUDART_INF_F;
                     }
                     if (MODE == kGradLogits) {
+                        const F2 scale(kLog2e, kLog2e), shift(row_nlse, row_nlse), factor(-row_gsum, -row_gsum);
 #pragma unroll
-                        for (int i = 0; i < 32; i++) v[i] = -row_gsum * ex2(fmaf(v[i], kLog2e, row_nlse));
+                        for (int i = 0; i < 32; i += 2) {
+                            const float2 x = fma2(F2(v[i], v[i + 1]), scale, shift).get();
+                            const float2 y = mul2(F2(ex2(x.x), ex2(x.y)), factor).get();
+                            v[i] = y.x, v[i + 1] = y.y;
+                        }
                         while (next_tok < col0 + 32) {
                             const int idx = next_tok - col0;
                             if (idx >= 0 && row_ok) {
@@ -581,14 +615,13 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1)
                         }
                         return;
                     }
-                    float w16[16];  // tree max
+                    float w11[11];  // tree max
 #pragma unroll
-                    for (int i = 0; i < 16; i++) w16[i] = fmaxf(v[i], v[i + 16]);
+                    for (int i = 0; i < 10; i++) w11[i] = max3(v[3 * i], v[3 * i + 1], v[3 * i + 2]);
+                    w11[10] = fmaxf(v[30], v[31]);
 #pragma unroll
-                    for (int i = 0; i < 8; i++) w16[i] = fmaxf(w16[i], w16[i + 8]);
-#pragma unroll
-                    for (int i = 0; i < 4; i++) w16[i] = fmaxf(w16[i], w16[i + 4]);
-                    const float cmax = fmaxf(fmaxf(w16[0], w16[2]), fmaxf(w16[1], w16[3]));
+                    for (int i = 0; i < 3; i++) w11[i] = max3(w11[3 * i], w11[3 * i + 1], w11[3 * i + 2]);
+                    const float cmax = max3(max3(w11[0], w11[1], w11[2]), w11[9], w11[10]);
                     if (cmax > m) {
                         const float f = ex2((m - cmax) * kLog2e);  // 0 on the first chunk (m = -inf)
                         s0 *= f, s1 *= f, s2 *= f, s3 *= f;
@@ -603,13 +636,16 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1)
                     }
                     if (m > -CUDART_INF_F) {
                         const float nm = -m * kLog2e;
+                        const F2 scale(kLog2e, kLog2e), shift(nm, nm);
+                        F2 a(s0, s1), b(s2, s3);
 #pragma unroll
                         for (int i = 0; i < 32; i += 4) {
-                            s0 += ex2(fmaf(v[i], kLog2e, nm));
-                            s1 += ex2(fmaf(v[i + 1], kLog2e, nm));
-                            s2 += ex2(fmaf(v[i + 2], kLog2e, nm));
-                            s3 += ex2(fmaf(v[i + 3], kLog2e, nm));
+                            const float2 x = fma2(F2(v[i], v[i + 1]), scale, shift).get();
+                            const float2 y = fma2(F2(v[i + 2], v[i + 3]), scale, shift).get();
+                            a = add2(a, F2(ex2(x.x), ex2(x.y)));
+                            b = add2(b, F2(ex2(y.x), ex2(y.y)));
                         }
+                        s0 = a.get().x, s1 = a.get().y, s2 = b.get().x, s3 = b.get().y;
                     }
                     while (next_tok < col0 + 32) {  // targets are sorted; those below col0 belong to the other half
                         const int idx = next_tok - col0;
