@@ -226,6 +226,13 @@ int pcfgnat_proj_dlogits_compact(const void *hidden, const void *weight, const i
                                  int64_t *row_index, int *n_rows, void *workspace, size_t workspace_bytes, int *status,
                                  void *stream);
 
+/* Both of the above (compact when row_index is given) with rows `pitch` elements apart, a multiple of 8 and at least V: an odd V
+ * then costs no more than an even one.  Cells between V and pitch are undefined. */
+int pcfgnat_proj_dlogits_pitched(const void *hidden, const void *weight, const int64_t *targets, const int64_t *output_length,
+                                 const int64_t *target_length, const float *lse, const float *grad_match, int B, int L, int T,
+                                 int V, int H, int capacity, void *dlogits, int pitch, int64_t *row_index, int *n_rows,
+                                 void *workspace, size_t workspace_bytes, int *status, void *stream);
+
 /* The two matrix products that finish the backward of the projection, on the tcgen05 tensor cores (bf16 operands,
  * float32 accumulation), in place of autograd's GEMMs of nn.Linear behind DagLogsoftmaxGatherFunc.backward
  * (fs_plugins/custom_ops/pcfg_loss.py:168-180, models/glat_decomposed_with_link_two_hands_tri_pcfg.py:237):
@@ -237,6 +244,9 @@ int pcfgnat_proj_dlogits_compact(const void *hidden, const void *weight, const i
  * of a captured graph that is replayed for batches with other row counts. */
 int pcfgnat_proj_backward_gemms(const void *dlogits, const void *weight_bf16, const void *rows_bf16, int n, int V, int H,
                                 float *d_rows, float *d_weight, int *status, void *stream);
+/* The same for d-logits whose rows are `pitch` elements apart (a multiple of 8, at least V; V may be odd then). */
+int pcfgnat_proj_backward_gemms_pitched(const void *dlogits, int pitch, const void *weight_bf16, const void *rows_bf16, int n, int V,
+                                        int H, float *d_rows, float *d_weight, int *status, void *stream);
 
 /* The three numbers the criterion's scalar loss is formed from, in one launch
  * (fs_plugins/criterions/nat_pcfg_loss.py:117-135: sentences whose loss is infinite or NaN are

@@ -32,7 +32,9 @@ SIGNATURES = {
     "pcfgnat_proj_logsoftmax_gather": (c_int, [c_void] * 5 + [c_int] * 5 + [c_void] * 5 + [c_size] + [c_void] * 2),
     "pcfgnat_proj_dlogits": (c_int, [c_void] * 7 + [c_int] * 5 + [c_void] * 2 + [c_size] + [c_void] * 2),
     "pcfgnat_proj_dlogits_compact": (c_int, [c_void] * 7 + [c_int] * 6 + [c_void] * 4 + [c_size] + [c_void] * 2),
+    "pcfgnat_proj_dlogits_pitched": (c_int, [c_void] * 7 + [c_int] * 6 + [c_void, c_int] + [c_void] * 3 + [c_size] + [c_void] * 2),
     "pcfgnat_proj_backward_gemms": (c_int, [c_void] * 3 + [c_int] * 3 + [c_void] * 4),
+    "pcfgnat_proj_backward_gemms_pitched": (c_int, [c_void, c_int] + [c_void] * 2 + [c_int] * 3 + [c_void] * 4),
     "pcfgnat_links_fused": (c_int, [c_void] * 3 + [c_int] + [c_void] * 6 + [c_int] * 6 + [c_void] * 2 + [c_size, c_int, c_void]),
     "pcfgnat_links_fused_kept_bytes": (c_size, [c_int] * 5),
     "pcfgnat_links_fused_scratch_bytes": (c_size, [c_int] * 4),

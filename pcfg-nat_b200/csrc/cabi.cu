@@ -526,7 +526,7 @@ int pcfgnat_proj_dlogits(const void *hidden, const void *weight, const int64_t *
         return PCFGNAT_ERR_INVALID_ARGUMENT;
     if (target_length != nullptr && output_length == nullptr) return PCFGNAT_ERR_INVALID_ARGUMENT;
     return launch_proj_dlogits(hidden, weight, targets, output_length, target_length, lse, grad_match, B, L, T, V, H,
-                               dlogits, workspace, workspace_bytes, status, static_cast<cudaStream_t>(stream));
+                               dlogits, V, workspace, workspace_bytes, status, static_cast<cudaStream_t>(stream));
 }
 
 int pcfgnat_proj_dlogits_compact(const void *hidden, const void *weight, const int64_t *targets,
@@ -541,8 +541,23 @@ int pcfgnat_proj_dlogits_compact(const void *hidden, const void *weight, const i
     if (B && capacity && !dlogits) return PCFGNAT_ERR_INVALID_ARGUMENT;
     if (target_length != nullptr && output_length == nullptr) return PCFGNAT_ERR_INVALID_ARGUMENT;
     return launch_proj_dlogits(hidden, weight, targets, output_length, target_length, lse, grad_match, B, L, T, V, H,
-                               dlogits, workspace, workspace_bytes, status, static_cast<cudaStream_t>(stream), capacity,
+                               dlogits, V, workspace, workspace_bytes, status, static_cast<cudaStream_t>(stream), capacity,
                                row_index, n_rows);
+}
+
+int pcfgnat_proj_dlogits_pitched(const void *hidden, const void *weight, const int64_t *targets, const int64_t *output_length,
+                                 const int64_t *target_length, const float *lse, const float *grad_match, int B, int L, int T,
+                                 int V, int H, int capacity, void *dlogits, int pitch, int64_t *row_index, int *n_rows,
+                                 void *workspace, size_t workspace_bytes, int *status, void *stream) {
+    PCFGNAT_API_RANGE();
+    if (B < 0 || L < 1 || T < 1 || V < 1 || H < 1 || capacity < 0 || pitch < V || pitch % 8) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    if ((long long)B * L > (1ll << 30)) return PCFGNAT_ERR_TOO_LARGE;
+    if (B && (!hidden || !weight || !targets || !lse || !grad_match || !workspace)) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    if (B && !dlogits && (capacity || !row_index)) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    if (target_length != nullptr && output_length == nullptr) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    return launch_proj_dlogits(hidden, weight, targets, output_length, target_length, lse, grad_match, B, L, T, V, H, dlogits,
+                               pitch, workspace, workspace_bytes, status, static_cast<cudaStream_t>(stream), capacity, row_index,
+                               n_rows);
 }
 
 int pcfgnat_proj_backward_gemms(const void *dlogits, const void *weight_bf16, const void *rows_bf16, int n, int V, int H,
@@ -551,7 +566,17 @@ int pcfgnat_proj_backward_gemms(const void *dlogits, const void *weight_bf16, co
     if (n < 0 || V < 1 || H < 1) return PCFGNAT_ERR_INVALID_ARGUMENT;
     if ((long long)n * V > (1ll << 40)) return PCFGNAT_ERR_TOO_LARGE;
     if (n && (!dlogits || (d_rows && !weight_bf16) || (d_weight && !rows_bf16))) return PCFGNAT_ERR_INVALID_ARGUMENT;
-    return launch_proj_backward_gemms(dlogits, weight_bf16, rows_bf16, n, V, H, d_rows, d_weight, status,
+    return launch_proj_backward_gemms(dlogits, weight_bf16, rows_bf16, n, V, V, H, d_rows, d_weight, status,
+                                      static_cast<cudaStream_t>(stream));
+}
+
+int pcfgnat_proj_backward_gemms_pitched(const void *dlogits, int pitch, const void *weight_bf16, const void *rows_bf16, int n, int V,
+                                        int H, float *d_rows, float *d_weight, int *status, void *stream) {
+    PCFGNAT_API_RANGE();
+    if (n < 0 || V < 1 || H < 1 || pitch < V) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    if ((long long)n * V > (1ll << 40)) return PCFGNAT_ERR_TOO_LARGE;
+    if (n && (!dlogits || (d_rows && !weight_bf16) || (d_weight && !rows_bf16))) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    return launch_proj_backward_gemms(dlogits, weight_bf16, rows_bf16, n, V, pitch, H, d_rows, d_weight, status,
                                       static_cast<cudaStream_t>(stream));
 }
 

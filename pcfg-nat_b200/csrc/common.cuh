@@ -239,9 +239,9 @@ int launch_links_from_scores(const float *ac, const float *bc, const float *qm, 
                              int D, float *links, cudaStream_t st);
 int launch_proj_dlogits(const void *hidden, const void *weight, const int64_t *targets, const int64_t *ol,
                         const int64_t *tl, const float *lse, const float *grad_match, int B, int L, int T, int V, int H,
-                        void *dlogits, void *workspace, size_t ws_bytes, int *status, cudaStream_t st, int capacity = 0,
+                        void *dlogits, int pitch, void *workspace, size_t ws_bytes, int *status, cudaStream_t st, int capacity = 0,
                         int64_t *row_index = nullptr, int *n_rows_out = nullptr);
-int launch_proj_backward_gemms(const void *dlogits, const void *weight_bf16, const void *rows_bf16, int n, int V, int H,
-                               float *d_rows, float *d_weight, int *status, cudaStream_t st);
+int launch_proj_backward_gemms(const void *dlogits, const void *weight_bf16, const void *rows_bf16, int n, int V, int pitch,
+                               int H, float *d_rows, float *d_weight, int *status, cudaStream_t st);
 
 }  // namespace pcfgnat

@@ -255,21 +255,21 @@ int launch_gemm(const void *A, bool a_mn, int lda, const void *B, bool b_mn, int
 
 }  // namespace
 
-int launch_proj_backward_gemms(const void *dlogits, const void *weight_bf16, const void *rows_bf16, int n, int V, int H,
+int launch_proj_backward_gemms(const void *dlogits, const void *weight_bf16, const void *rows_bf16, int n, int V, int pitch, int H,
                                float *d_rows, float *d_weight, int *status, cudaStream_t st) {
-    if (V % 8 || H % 8) return PCFGNAT_ERR_UNSUPPORTED;  // row pitches of 16-byte multiples for the tensor maps
+    if (pitch % 8 || H % 8) return PCFGNAT_ERR_UNSUPPORTED;  // row pitches of 16-byte multiples for the tensor maps
     if ((reinterpret_cast<uintptr_t>(dlogits) | reinterpret_cast<uintptr_t>(weight_bf16) |
          reinterpret_cast<uintptr_t>(rows_bf16) | reinterpret_cast<uintptr_t>(d_rows) |
          reinterpret_cast<uintptr_t>(d_weight)) % 16)
         return PCFGNAT_ERR_INVALID_ARGUMENT;
     if (d_rows) {
         if (cudaMemsetAsync(d_rows, 0, (size_t)n * H * sizeof(float), st) != cudaSuccess) return PCFGNAT_ERR_CUDA;
-        const int rc = launch_gemm(dlogits, false, V, weight_bf16, true, H, d_rows, n, H, V, status, st);
+        const int rc = launch_gemm(dlogits, false, pitch, weight_bf16, true, H, d_rows, n, H, V, status, st);
         if (rc != PCFGNAT_OK) return rc;
     }
     if (d_weight) {
         if (cudaMemsetAsync(d_weight, 0, (size_t)V * H * sizeof(float), st) != cudaSuccess) return PCFGNAT_ERR_CUDA;
-        const int rc = launch_gemm(dlogits, true, V, rows_bf16, true, H, d_weight, V, H, n, status, st);
+        const int rc = launch_gemm(dlogits, true, pitch, rows_bf16, true, H, d_weight, V, H, n, status, st);
         if (rc != PCFGNAT_OK) return rc;
     }
     return PCFGNAT_OK;

@@ -122,6 +122,11 @@ def _row_index_ok(index, device):
 _main_chain_cache = {}  # (address and version of the main-chain mask, prelen) -> mask, (node list, slots), their stream
 
 
+def _rows_apart(t):
+    """Whether the rows of a matrix are a multiple of 16 bytes apart in memory, as an odd vocabulary's padded d-logits are."""
+    return t.dim() == 2 and t.stride(1) == 1 and t.stride(0) >= t.shape[1] and t.stride(0) % 8 == 0
+
+
 class _Kernel:
     """Extension-level API: the functions of the reference's pybind module (pcfg_loss.cpp:75-82)."""
 
@@ -404,16 +409,71 @@ class _Kernel:
         return dl
 
     @staticmethod
+    def proj_dlogits_rows(hidden, weight, targets, output_length, target_length, lse, grad_match, n_rows=None, out=None,
+                          row_index_out=None):
+        """``proj_dlogits`` for ``proj_backward_products``: (d-logits, row_index or None), the d-logits a view [n, V] of a
+        buffer whose rows are a multiple of 16 bytes apart, which an odd vocabulary's own rows are not.  ``out``: such a
+        buffer, bfloat16 [rows, V rounded up to a multiple of 8]; ``row_index_out`` as in ``proj_dlogits``."""
+        B, L, H = hidden.shape
+        V = weight.shape[0]
+        if V % 8 == 0:
+            got = _Kernel.proj_dlogits(hidden, weight, targets, output_length, target_length, lse, grad_match, n_rows=n_rows,
+                                       out=out, row_index_out=row_index_out)
+            return got if n_rows is not None else (got, None)
+        _require_cuda()
+        if hidden.dtype != torch.float16 or weight.dtype != torch.float16 or not (hidden.is_cuda and weight.is_cuda):
+            raise RuntimeError("hidden and weight must be float16 CUDA tensors")
+        dev = hidden.device
+        hidden, weight = hidden.contiguous(), weight.contiguous()
+        targets = targets.to(device=dev, dtype=torch.int64).contiguous()
+        T = targets.shape[1]
+        lse = _f32_cuda(lse, "lse", 2)
+        g = _f32_cuda(grad_match, "grad_match", 3)
+        if tuple(lse.shape) != (B, L) or tuple(g.shape) != (B, L, T):
+            raise RuntimeError("lse must be [batch, prelen] and grad_match [batch, prelen, tarlen]")
+        if target_length is not None and output_length is None:
+            raise RuntimeError("target_length (EOS masking) needs output_length as well")
+        ol = _lengths(output_length, "output_length", B, dev) if output_length is not None else None
+        tl = _lengths(target_length, "target_length", B, dev) if target_length is not None else None
+        n = int(n_rows) if n_rows is not None else B * L
+        if n < 0 or n > B * L:
+            raise RuntimeError("n_rows must be between 0 and batch * prelen")
+        lib = _cabi.lib()
+        nbytes = lib.pcfgnat_proj_workspace_bytes(B, L, T, V)
+        pitch = (V + 7) // 8 * 8
+        ptr = lambda t: t.data_ptr() if t is not None else None
+        with torch.cuda.device(dev):
+            ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=dev)
+            dl = out if out is not None else torch.empty((n, pitch), dtype=torch.bfloat16, device=dev)
+            idx = row_index_out if row_index_out is not None or n_rows is None else torch.empty((n,), dtype=torch.int64, device=dev)
+            if dl.dtype != torch.bfloat16 or dl.dim() != 2 or dl.shape[1] != pitch or dl.shape[0] < n or not dl.is_contiguous() or \
+                    idx is not None and (idx.dtype != torch.int64 or idx.numel() < n):
+                raise RuntimeError("out must be a contiguous bfloat16 [>= n_rows, V rounded up], row_index_out int64 [>= n_rows]")
+            rc = lib.pcfgnat_proj_dlogits_pitched(hidden.data_ptr(), weight.data_ptr(), targets.data_ptr(), ptr(ol), ptr(tl),
+                                                  lse.data_ptr(), g.data_ptr(), B, L, T, V, H, n, ptr(dl), pitch, ptr(idx), None,
+                                                  ws.data_ptr(), nbytes, _status_ptr(dev), _stream(dev))
+        _cabi.check(rc, "pcfgnat_proj_dlogits_pitched")
+        return dl[:n, :V], idx if idx is None else idx[:n]
+
+    @staticmethod
     def proj_backward_gemms(dlogits, weight_bf16, rows_bf16, want_rows=True, want_weight=True):
         """The two products that finish the projection's backward, on the tensor cores: (d rows [n, H] float32 =
         dlogits [n, V] @ weight_bf16 [V, H], d weight [V, H] float32 = dlogits.T @ rows_bf16 [n, H]); None for a
         product not wanted.  All operands bfloat16 and contiguous; V and H multiples of 8."""
         _require_cuda()
+        if not dlogits.is_contiguous():
+            raise RuntimeError("dlogits must be a contiguous bfloat16 CUDA matrix")
+        return _Kernel._proj_backward_gemms(dlogits, weight_bf16, rows_bf16, want_rows, want_weight)
+
+    @staticmethod
+    def _proj_backward_gemms(dlogits, weight_bf16, rows_bf16, want_rows=True, want_weight=True):
+        """The same, of d-logits whose rows may also lie further apart than they are long (``proj_dlogits_rows``)."""
+        _require_cuda()
         dev = dlogits.device
         for t, name in ((dlogits, "dlogits"), (weight_bf16, "weight_bf16"), (rows_bf16, "rows_bf16")):
             if t is None:
                 continue
-            if not t.is_cuda or t.dtype != torch.bfloat16 or t.dim() != 2 or not t.is_contiguous():
+            if not t.is_cuda or t.dtype != torch.bfloat16 or t.dim() != 2 or not (t.is_contiguous() or t is dlogits and _rows_apart(t)):
                 raise RuntimeError(f"{name} must be a contiguous bfloat16 CUDA matrix")
         n, V = dlogits.shape
         H = (weight_bf16 if weight_bf16 is not None else rows_bf16).shape[1]
@@ -425,8 +485,9 @@ class _Kernel:
         with torch.cuda.device(dev):
             d_rows = torch.empty((n, H), dtype=torch.float32, device=dev) if want_rows else None
             d_weight = torch.empty((V, H), dtype=torch.float32, device=dev) if want_weight else None
-            rc = _cabi.lib().pcfgnat_proj_backward_gemms(dlogits.data_ptr(), ptr(weight_bf16), ptr(rows_bf16), n, V, H,
-                                                         ptr(d_rows), ptr(d_weight), _status_ptr(dev), _stream(dev))
+            rc = _cabi.lib().pcfgnat_proj_backward_gemms_pitched(dlogits.data_ptr(), V if dlogits.is_contiguous() else dlogits.stride(0),
+                                                                 ptr(weight_bf16), ptr(rows_bf16), n, V, H, ptr(d_rows),
+                                                                 ptr(d_weight), _status_ptr(dev), _stream(dev))
         _cabi.check(rc, "pcfgnat_proj_backward_gemms")
         return d_rows, d_weight
 
@@ -1087,12 +1148,14 @@ def _bf16(t):
 def proj_backward_products(dlogits, weight, rows):
     """(dlogits @ weight, dlogits.T @ rows) in float32 from bf16 d-logits [n, V], the projection weight [V, H] and the
     decoder states of the same n rows [n, H] (either may be None: that product is skipped).  On this library's
-    tensor-core kernels (``pcfgnat_proj_backward_gemms``); shapes whose V or H is not a multiple of 8 cannot be
+    tensor-core kernels (``pcfgnat_proj_backward_gemms``); d-logits whose rows are not a multiple of 16 bytes apart
+    (``proj_dlogits_rows`` makes such an odd vocabulary's), and an H that is not a multiple of 8, cannot be
     described to the tensor maps and go through torch's matmul instead."""
     V = dlogits.shape[1]
     H = (weight if weight is not None else rows).shape[1]
-    if V % 8 == 0 and H % 8 == 0:
-        return get_pcfg_kernel().proj_backward_gemms(
+    if H % 8 == 0 and (V % 8 == 0 or _rows_apart(dlogits)):
+        gemms = get_pcfg_kernel().proj_backward_gemms if V % 8 == 0 else get_pcfg_kernel()._proj_backward_gemms
+        return gemms(
             dlogits, _bf16(weight) if weight is not None else None, _bf16(rows) if rows is not None else None,
             want_rows=weight is not None, want_weight=rows is not None)
     d_rows = (dlogits @ weight.to(torch.bfloat16)).float() if weight is not None else None
@@ -1125,11 +1188,11 @@ class ProjLogsoftmaxGatherFunc(Function):
         need_h, need_w = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         V = weight.shape[0]
         if ctx.n_rows is None:  # every row of the padded tensor
-            dl = k.proj_dlogits(hidden, weight, targets, ol, tl, lse, grad_match.contiguous())
+            dl, _ = k.proj_dlogits_rows(hidden, weight, targets, ol, tl, lse, grad_match.contiguous())
             rows = hidden.reshape(B * L, H)
             idx = None
         else:  # the real graph nodes only
-            dl, idx = k.proj_dlogits(hidden, weight, targets, ol, tl, lse, grad_match.contiguous(), n_rows=ctx.n_rows)
+            dl, idx = k.proj_dlogits_rows(hidden, weight, targets, ol, tl, lse, grad_match.contiguous(), n_rows=ctx.n_rows)
             rows = k.rows_to_bf16(hidden.reshape(B * L, H), idx) if need_w else None
         d_rows, d_weight = proj_backward_products(dl, weight if need_h else None, rows if need_w else None)
         if need_h:

@@ -359,7 +359,9 @@ class LossStep(_GraphedStep):
             V = int(self.weight.shape[0])
             # d-logits of the real graph nodes only, compact; the two GEMMs run after the graph, over as many rows
             # as the batch has real nodes (a number the host knows from the lengths it loaded)
-            self.dlogits = torch.empty((B * L, V), dtype=torch.bfloat16, device=self.device)
+            # (its rows a multiple of 16 bytes apart, also where an odd vocabulary's are not that long)
+            self.dlogits_rows = torch.empty((B * L, (V + 7) // 8 * 8), dtype=torch.bfloat16, device=self.device)
+            self.dlogits = self.dlogits_rows[:, :V]
             self.row_index = torch.zeros((B * L,), dtype=torch.int64, device=self.device)
             self.d_hidden = torch.zeros((B * L, self.H), dtype=torch.float16, device=self.device)
             self.n_rows = None
@@ -403,8 +405,8 @@ class LossStep(_GraphedStep):
                  else sharding.local_loss_stats(loss, self.target_length))
         if not self.proj_backward:
             return stats, mg, lg, loss
-        self.kernel.proj_dlogits(self.hidden, self.weight, self.targets, self.output_length, self.target_length,
-                                 em["lse"], mg, n_rows=self.B * self.L, out=self.dlogits, row_index_out=self.row_index)
+        self.kernel.proj_dlogits_rows(self.hidden, self.weight, self.targets, self.output_length, self.target_length, em["lse"],
+                                      mg, n_rows=self.B * self.L, out=self.dlogits_rows, row_index_out=self.row_index)
         return stats, mg, lg, loss
 
     def load(self, *tensors, overlap=False):

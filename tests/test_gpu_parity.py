@@ -903,6 +903,51 @@ def test_projection_backward_gemms_with_no_rows(ops):
                               torch.zeros((1001, 64), dtype=torch.bfloat16, device=DEV), None, want_weight=False)
 
 
+@pytest.mark.parametrize("B, L, V, H, ragged", [(1, 3, 1001, 64, False), (3, 50, 513, 128, True), (5, 70, 2047, 64, True),
+                                                (2, 130, 4004, 512, False), (4, 64, 3999, 256, True), (2, 33, 33, 64, True)])
+def test_projection_backward_of_a_vocabulary_that_is_no_multiple_of_eight(ops, B, L, V, H, ragged):
+    """d hidden and d weight where a row of d-logits is no multiple of 16 bytes (its padding is never read), over all
+    rows and over the real nodes only, against autograd in float64: bf16 d-logits and operands (2^-8 each, rounded
+    independently), sums of up to 4004 terms: 1e-2 of the result's norm; single entries 3e-2 of the largest."""
+    g = torch.Generator(DEV).manual_seed(V)
+    hidden, weight = torch.randn(B, L, H, device=DEV, generator=g).half(), (torch.randn(V, H, device=DEV, generator=g) * 0.1).half()
+    T = 6
+    targets = torch.randint(0, V, (B, T), device=DEV, generator=g)
+    targets[0, 0] = V - 1
+    ol = torch.randint(1, L + 1, (B,), device=DEV, generator=g) if ragged else torch.full((B,), L, device=DEV)
+    grad = torch.randn(B, L, T, device=DEV, generator=g)
+    real = torch.arange(L, device=DEV)[None] < ol[:, None]
+    h64, w64 = hidden.double().requires_grad_(), weight.double().requires_grad_()
+    lp = torch.log_softmax(h64 @ w64.t(), -1).gather(2, targets[:, None].expand(-1, L, -1))
+    want = torch.autograd.grad((lp * grad * real[..., None]).sum(), (h64, w64))
+    for n_rows in (None, int(ol.sum())):
+        h, w = hidden.clone().requires_grad_(), weight.clone().requires_grad_()
+        match = ops.proj_logsoftmax_gather_with_grad(h, w, targets, ol, None, n_rows=n_rows)
+        got = torch.autograd.grad(match, (h, w), grad)
+        for x, y in zip(got, want):
+            assert torch.isfinite(x).all() and x.shape == y.shape
+            assert (x.double() - y).norm() <= 1e-2 * y.norm() and (x.double() - y).abs().max() <= 3e-2 * y.abs().max()
+        assert (got[0][~real] == 0).all()
+
+
+def test_loss_step_with_projection_backward_of_an_odd_vocabulary(pkg, ops, syn):
+    """The step object's d hidden and d weight with padded rows of d-logits, against the differentiable operator (which the
+    test above holds to float64): the same kernels over the same rows, sums by atomics in another order."""
+    import importlib
+    runtime = importlib.import_module("pcfg_nat_b200.runtime")
+    b = syn.make_batch(syn.Workload("odd", batch=4, vocab=1003, hidden=64, src_min=6, src_max=20, hidden_std=1.0), seed=3)
+    weight = b.weight.to(DEV)
+    step = runtime.LossStep(weight, b.B, b.L, b.T, DEV, use_graph=True, proj_backward=True)
+    step.load(b.hidden, b.links, b.output_length, b.targets, b.target_length)
+    stats, mg, lg, loss, d_hidden, d_weight = step.run()
+    hid, wt = b.hidden.to(DEV).requires_grad_(True), weight.clone().requires_grad_(True)
+    match = ops.proj_logsoftmax_gather_with_grad(hid, wt, b.targets.to(DEV), b.output_length.to(DEV), b.target_length.to(DEV))
+    fin = torch.isfinite(match)
+    (match[fin] * mg[fin]).sum().backward()
+    for got, want in ((d_hidden.float(), hid.grad.float()), (d_weight.float(), wt.grad.float())):
+        assert float((got - want).norm() / want.norm()) < 2e-3
+
+
 def test_copy_real_rows_sends_the_real_nodes_only(ops):
     """pcfgnat_copy_real_rows: rows l < length arrive, the others keep what they held; lengths beyond the tensor
     and below zero are clamped; full sentences next to each other go as one copy; a sentence range."""
