@@ -8,9 +8,9 @@
 // 80 KB, so two CTAs fit per SM): one HBM read, and one HBM write only when the softmax is
 // asked for.  Rows that do not fit fall back to re-reading global memory.
 //
-// Rows that are 16-byte multiples and fit shared memory run on the streaming kernel further below (bulk
-// asynchronous copies in chunks, sum of exponentials accumulated as the chunks land); the kernel here remains for
-// the other rows.
+// Rows that fit shared memory run on the streaming kernel further below (bulk asynchronous copies in chunks, sum of
+// exponentials accumulated as the chunks land); the kernel here remains for longer rows, and for short ones that are no
+// multiple of 16 bytes.
 // Like the reference this kernel uses the fast exp/log/divide intrinsics
 // (logsoftmax_gather.cu:107-148), so parity with it is by tolerance.
 #include <cuda_fp16.h>
@@ -206,8 +206,11 @@ struct Pack<__half> {
 // still holds them); with the softmax the row stays until the probabilities have been written, and each chunk is
 // refilled as soon as it has been written out.  Two CTAs per SM (when two rows fit) run out of step with one
 // another, which keeps both the exponential unit and the copy stream busy.
-// Rows of V * sizeof(T) bytes, a multiple of 16, on a 16-byte aligned base; nch * kChunkBytes >= the row.
-template <typename T>
+// nch * kChunkBytes >= the row.  EDGES: rows that are no multiple of 16 bytes, or whose base is not aligned.  What is copied is a
+// row's part between its first and its last 16-byte boundary; the up to seven entries on either side stay in registers, one a
+// thread, so that nothing of a neighbouring row is read or written.  [4 687, 31 999] half with the softmax 131 us, read-only 84;
+// [2 343, 31 999] float 121 and 74 (213, 143, 195 and 143 as the single-buffer kernel took them, element by element).
+template <typename T, bool EDGES>
 __global__ void __launch_bounds__(kStreamThreads)
     logsoftmax_gather_stream_kernel(T *logits, const int64_t *__restrict__ sel, int64_t sb, int64_t sl, int64_t ss,
                                     int64_t rows, int64_t rpb, int V, int slen, int req_grad, float *selected,
@@ -217,7 +220,14 @@ __global__ void __launch_bounds__(kStreamThreads)
     __shared__ __align__(8) uint64_t bars[kMaxChunks];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int kVec = 16 / sizeof(T);
-    const uint32_t row_bytes = (uint32_t)V * sizeof(T);
+    const auto head_of = [&](int64_t r) {  // entries before the row's first boundary
+        if (!EDGES) return 0;
+        const int n = (int)((16 - reinterpret_cast<uintptr_t>(logits + (size_t)r * V) % 16) % 16 / sizeof(T));
+        return n < V ? n : V;
+    };
+    const auto body_of = [&](int head) {  // bytes between the boundaries
+        return EDGES ? (uint32_t)(V - head) * (uint32_t)sizeof(T) / 16 * 16 : (uint32_t)V * (uint32_t)sizeof(T);
+    };
     const uint32_t base = dsm_smem_u32(smem_raw);
     const uint32_t bar0 = dsm_smem_u32(&bars[0]);
     if (tid == 0) {
@@ -225,15 +235,18 @@ __global__ void __launch_bounds__(kStreamThreads)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    auto chunk_bytes = [&](int c) {
+    auto chunk_bytes = [&](int c, uint32_t body) {
         const uint32_t off = (uint32_t)c * kChunkBytes;
-        return row_bytes - off < kChunkBytes ? row_bytes - off : kChunkBytes;
+        if (EDGES && off >= body) return 0u;
+        return body - off < kChunkBytes ? body - off : kChunkBytes;
     };
     auto fetch = [&](int64_t r, int c) {  // thread 0 only; every thread is past its reads of chunk c
-        const uint32_t bar = bar0 + 8 * c, n = chunk_bytes(c);
+        const int head = head_of(r);
+        const uint32_t bar = bar0 + 8 * c, n = chunk_bytes(c, body_of(head));
         asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(n) : "memory");
-        bulk_load(base + c * kChunkBytes, reinterpret_cast<const unsigned char *>(logits + (size_t)r * V) + (size_t)c * kChunkBytes,
-                  n, bar);
+        if (EDGES && n == 0) return;  // the row ends before
+        bulk_load(base + c * kChunkBytes,
+                  reinterpret_cast<const unsigned char *>(logits + (size_t)r * V + head) + (size_t)c * kChunkBytes, n, bar);
     };
     if (tid == 0 && (int64_t)blockIdx.x < rows)
         for (int c = 0; c < nch; c++) fetch(blockIdx.x, c);
@@ -246,6 +259,12 @@ __global__ void __launch_bounds__(kStreamThreads)
         // the logits to gather are fetched now, from global memory (the row there is rewritten only at the end of
         // this iteration), so that their latency is spent under the sweep
         T *grow = logits + (size_t)r * V;
+        const int head = head_of(r);
+        const uint32_t body = body_of(head);
+        // this thread's entry outside the body, if any
+        const int tail = EDGES ? V - head - (int)(body / sizeof(T)) : 0, edge = tid < head ? tid : V - tail + (tid - head);
+        const bool has_edge = EDGES && tid < head + tail;
+        const float x_edge = has_edge ? to_f<T>(grow[edge]) : 0.f;
         const int64_t bi = r / rpb, li = r % rpb;
         int64_t t_sel = 0;
         float x_sel = 0.f;
@@ -261,7 +280,7 @@ __global__ void __launch_bounds__(kStreamThreads)
             ok = ok && bulk_wait(bar0 + 8 * c, par);
             if (ok) {
                 const uint4 *s4 = reinterpret_cast<const uint4 *>(smem_raw + (size_t)c * kChunkBytes);
-                const int n16 = chunk_bytes(c) / 16;
+                const int n16 = chunk_bytes(c, body) / 16;
                 for (int i = tid; i < n16; i += 2 * kStreamThreads) {  // two independent 16-byte pieces at a time
                     const uint4 v0 = s4[i];
                     const uint4 v1 = i + kStreamThreads < n16 ? s4[i + kStreamThreads] : Pack<T>::lowest();
@@ -302,6 +321,15 @@ __global__ void __launch_bounds__(kStreamThreads)
             __syncthreads();
             return;
         }
+        if (has_edge) {
+            if (x_edge > m) {
+                const float scale = ex2_ftz((m - x_edge) * kLog2e);
+                sum *= scale, sum_b *= scale;
+                m = x_edge;
+                shift = -x_edge * kLog2e;
+            }
+            sum += ex2_ftz(fmaf(x_edge, kLog2e, shift));
+        }
         // (maximum, sum) of the row: within each warp, through shared memory (one barrier), across the warps
         float wm = m;
 #pragma unroll
@@ -322,7 +350,7 @@ __global__ void __launch_bounds__(kStreamThreads)
         if (early) {
             if (tid < slen) selected[(size_t)r * slen + tid] = t_sel < 0 || t_sel >= V ? CUDART_NAN_F : (x_sel - mx) - lse;
         } else {
-            const T *row = req_grad ? reinterpret_cast<const T *>(smem_raw) : grow;
+            const T *row = req_grad && !EDGES ? reinterpret_cast<const T *>(smem_raw) : grow;
             for (int s = tid; s < slen; s += kStreamThreads) {
                 int64_t t = sel[bi * sb + li * sl + (int64_t)s * ss];
                 float v;
@@ -337,10 +365,14 @@ __global__ void __launch_bounds__(kStreamThreads)
         }
         if (req_grad) {  // softmax = ex2(x * log2(e) - (mx * log2(e) + log2(sum))): the division is in the exponent
             const float shift2 = -mx * kLog2e - __log2f(sum);
+            if (EDGES) {
+                if (!early) __syncthreads();  // the gathers have read the row where it is overwritten now
+                if (has_edge) grow[edge] = from_f<T>(ex2_ftz(fmaf(x_edge, kLog2e, shift2)));
+            }
             for (int c = 0; c < nch; c++) {
                 const uint4 *s4 = reinterpret_cast<const uint4 *>(smem_raw + (size_t)c * kChunkBytes);
-                uint4 *g4 = reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(grow) + (size_t)c * kChunkBytes);
-                const int n16 = chunk_bytes(c) / 16;
+                uint4 *g4 = reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(grow + head) + (size_t)c * kChunkBytes);
+                const int n16 = chunk_bytes(c, body) / 16;
                 for (int i = tid; i < n16; i += kStreamThreads) {
                     float f[kVec];
                     Pack<T>::unpack(s4[i], f);
@@ -367,8 +399,11 @@ int launch_typed(T *logits, const int64_t *sel, int64_t sb, int64_t sl, int64_t 
     const int nch = (int)(((size_t)V * sizeof(T) + kChunkBytes - 1) / kChunkBytes);
     const size_t stream_bytes = ((size_t)V * sizeof(T) + 127) / 128 * 128;
     const char *env = getenv("PCFGNAT_LSG_STREAM");  // "0": the single-buffer kernels only
-    if (vec_ok && nch <= kMaxChunks && stream_bytes + 2048 <= (size_t)kSmemLimit && !(env && env[0] == '0')) {
-        auto k = logsoftmax_gather_stream_kernel<T>;
+    // shorter rows of this kind are faster four to an SM: 14 400 of 501 halves 124 and 149 us, of 999 halves 151 and 150, of 501
+    // floats 129 and 126
+    const bool edges_pay = (size_t)V * sizeof(T) >= 2000;
+    if ((vec_ok || edges_pay) && nch <= kMaxChunks && stream_bytes + 2048 <= (size_t)kSmemLimit && !(env && env[0] == '0')) {
+        const auto k = vec_ok ? logsoftmax_gather_stream_kernel<T, false> : logsoftmax_gather_stream_kernel<T, true>;
         e = ensure_dynamic_smem(k, stream_bytes);
         if (e != cudaSuccess) return PCFGNAT_ERR_CUDA;
         int per_sm = (int)((size_t)kSmemLimit / (stream_bytes + 2048));

@@ -948,6 +948,39 @@ def test_loss_step_with_projection_backward_of_an_odd_vocabulary(pkg, ops, syn):
         assert float((got - want).norm() / want.norm()) < 2e-3
 
 
+@pytest.mark.parametrize("V", [1001, 1007, 2051, 16384, 16387, 33001])
+@pytest.mark.parametrize("dtype, offset, columns", [(torch.float16, 0, 20), (torch.float16, 3, 600), (torch.float32, 0, 600),
+                                                    (torch.float32, 1, 20)])
+def test_logsoftmax_gather_of_unaligned_rows(ops, V, dtype, offset, columns):
+    """Rows that start and end between 16-byte boundaries (and bodies of exactly one chunk), more columns than threads, with
+    and without the softmax in place, against float64; what lies before and after the rows stays.  Fast exponentials over
+    float32 sums of up to 33 001 terms: 1e-5 of a log-probability's scale, 2e-5 of a probability (and a half's rounding)."""
+    g = torch.Generator(DEV).manual_seed(V)
+    rows = 5
+    buffer = torch.randn(offset + rows * V + 64, device=DEV, generator=g).mul_(3).to(dtype)
+    buffer[offset + V - 1], buffer[offset + 2 * V] = 30, -60000 if dtype == torch.float16 else float("-inf")
+    sel = torch.randint(0, V, (1, rows, columns), device=DEV, generator=g)
+    sel[..., 0], sel[..., 1] = 0, V - 1
+    x = buffer[offset:offset + rows * V].view(1, rows, V).double()
+    want = torch.log_softmax(x, -1)
+    for in_place in (True, False):
+        mine = buffer.clone()
+        assert mine.data_ptr() % 16 == 0
+        got = ops.get_pcfg_kernel().logsoftmax_gather(mine[offset:offset + rows * V].view(1, rows, V), sel, in_place)
+        picked = want.gather(2, sel)
+        finite = torch.isfinite(picked)
+        assert torch.equal(torch.isfinite(got), finite)
+        assert ((got.double() - picked)[finite].abs() <= 1e-5 * picked[finite].abs().clamp(min=1)).all()
+        assert torch.equal(mine[:offset], buffer[:offset]) and torch.equal(mine[offset + rows * V:], buffer[offset + rows * V:])
+        after = mine[offset:offset + rows * V].view(1, rows, V)
+        if not in_place:
+            assert torch.equal(after, buffer[offset:offset + rows * V].view(1, rows, V))
+            continue
+        p = want.exp()
+        bound = 2e-5 * p + (2.0 ** -11 * p + 2.0 ** -24 if dtype == torch.float16 else 1e-38)
+        assert ((after.double() - p).abs() <= bound).all()
+
+
 def test_copy_real_rows_sends_the_real_nodes_only(ops):
     """pcfgnat_copy_real_rows: rows l < length arrive, the others keep what they held; lengths beyond the tensor
     and below zero are clamped; full sentences next to each other go as one copy; a sentence range."""
