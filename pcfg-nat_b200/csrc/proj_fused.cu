@@ -235,7 +235,7 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 //    their original positions in sslot; ids outside [0, V) sort last as INT_MAX and raise a status bit.
 __global__ void proj_prepare_kernel(const int64_t *__restrict__ ol, const int64_t *__restrict__ targets, int B, int L,
                                     int T, int V, int *prefix, int *row_src, int *n_rows, int *stok, int *sslot,
-                                    int *status) {
+                                    int *status, int sort_smem) {
     __shared__ int warp_sum[32];
     __shared__ int before_s;
     chain_begin();
@@ -269,19 +269,26 @@ __global__ void proj_prepare_kernel(const int64_t *__restrict__ ol, const int64_
     for (int l = threadIdx.x; l < mine; l += blockDim.x) row_src[before + l] = b * L + l;
     if (!targets) return;
     const int64_t *tg = targets + (size_t)b * T;
+    // [T], unless it has no room for them (sort_smem == 0): 154 targets a sentence 5.2 us, 9.2 from global memory
+    extern __shared__ int keys[];
+    const auto key_of = [&](int s) {
+        const int64_t k = tg[s];
+        return k < 0 || k >= V ? INT_MAX : (int)k;
+    };
+    if (sort_smem) {
+        for (int s = threadIdx.x; s < T; s += blockDim.x) keys[s] = key_of(s);
+        __syncthreads();
+    }
     for (int s = threadIdx.x; s < T; s += blockDim.x) {
-        int64_t key = tg[s];
-        if (key < 0 || key >= V) {
-            flag(status, PCFGNAT_STATUS_BAD_INDEX);
-            key = INT_MAX;
-        }
+        const int key = sort_smem ? keys[s] : key_of(s);
+        if (key == INT_MAX) flag(status, PCFGNAT_STATUS_BAD_INDEX);
         int rank = 0;
+#pragma unroll 8
         for (int j = 0; j < T; j++) {
-            int64_t o = tg[j];
-            if (o < 0 || o >= V) o = INT_MAX;
+            const int o = sort_smem ? keys[j] : key_of(j);
             rank += (o < key) || (o == key && j < s);
         }
-        stok[(size_t)b * T + rank] = (int)key;
+        stok[(size_t)b * T + rank] = key;
         sslot[(size_t)b * T + rank] = s;
     }
 }
@@ -712,19 +719,21 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1)
 }
 
 // ---------------------------------------------------------------------------------------
-// merge of the per-segment partials.  Blocks [0, 8 * row_tiles) take 16 rows of one tile of 128 compact
-// rows each (the schedule is looked up once per block, one warp per row); the B blocks after them fill
-// the padding rows of one sentence each.
+// merge of the per-segment partials.  Blocks [0, kMergeSplit * row_tiles) take 16 rows of one tile of 128 compact rows each,
+// LANES lanes a row (the schedule is looked up once per block); the B blocks after them fill the padding rows of one
+// sentence each.  Bound by the latency of its chain of loads: a row's first emissions and targets are on their way before
+// its partials are merged, and as many rows as the GPU has room for are under way at once.  LANES: see launch_proj.
 // ---------------------------------------------------------------------------------------
-constexpr int kMergeSplit = 8, kMergeThreads = 32 * (BM / kMergeSplit);
-__global__ void proj_merge_kernel(const Partial *__restrict__ partials, const int *__restrict__ prefix,
-                                  const int *__restrict__ row_src, const int *__restrict__ n_rows_ptr, int ctas,
-                                  int max_seg, int row_tiles, int pair, int V, int L, int T, const int64_t *__restrict__ ol,
-                                  const int64_t *__restrict__ tl, const int64_t *__restrict__ targets, float *match,
-                                  float *max_lprob, int64_t *argmax, float *lse_out) {
+constexpr int kMergeSplit = 8, kMergeRows = BM / kMergeSplit;
+template <int LANES>
+__global__ void __launch_bounds__(kMergeRows *LANES)
+    proj_merge_kernel(const Partial *__restrict__ partials, const int *__restrict__ prefix, const int *__restrict__ row_src,
+                      const int *__restrict__ n_rows_ptr, int ctas, int max_seg, int row_tiles, int pair, int V, int L, int T,
+                      const int64_t *__restrict__ ol, const int64_t *__restrict__ tl, const int64_t *__restrict__ targets,
+                      float *match, float *max_lprob, int64_t *argmax, float *lse_out) {
     chain_begin();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
     if ((int)blockIdx.x >= kMergeSplit * row_tiles) {  // padding rows of sentence b: not projected
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
         const int b = blockIdx.x - kMergeSplit * row_tiles;
         const int len_b = prefix[b + 1] - prefix[b];
         for (int l = len_b + warp; l < L; l += n_warps) {
@@ -742,12 +751,15 @@ __global__ void proj_merge_kernel(const Partial *__restrict__ partials, const in
         }
         return;
     }
-    const int rt = blockIdx.x / kMergeSplit, part = blockIdx.x % kMergeSplit, n_rows = *n_rows_ptr;
-    if (rt * BM + part * (BM / kMergeSplit) >= n_rows) return;
+    const int rt = blockIdx.x / kMergeSplit, part = blockIdx.x % kMergeSplit, lane = threadIdx.x % LANES;
+    const int r_in = part * kMergeRows + threadIdx.x / LANES, cr = rt * BM + r_in, n_rows = *n_rows_ptr;
+    if (rt * BM + part * kMergeRows >= n_rows) return;
+    const bool on = cr < n_rows;  // the lanes of other rows take part in the exchanges
+    const int row = on ? row_src[cr] : 0;
+    // `ctas` counts schedule owners: CTAs, or CTA pairs (then a unit is two row tiles and the partials of row tile rt are in
+    // CTA 2 * owner + (rt & 1))
     __shared__ int s_glo, s_ghi, s_seg_lo;
     if (threadIdx.x == 0) {
-        // `ctas` counts schedule owners: CTAs, or CTA pairs (then a unit is two row tiles and the partials of
-        // row tile rt are in CTA 2 * owner + (rt & 1))
         const Plan plan = Plan::make(n_rows, V, ctas, max_seg, pair != 0);
         const int ut = pair ? rt >> 1 : rt;
         const long long u0 = (long long)ut * plan.n_tiles, u1 = u0 + plan.n_tiles - 1;
@@ -755,69 +767,80 @@ __global__ void proj_merge_kernel(const Partial *__restrict__ partials, const in
         s_ghi = plan.cta_of(u1);
         // only the first owner of the tile can have begun in an earlier row tile; the others start inside
         // this one, where it is their segment 0
-        s_seg_lo = ut - (int)(plan.begin(s_glo) / plan.n_tiles);
+        const long long first = plan.begin(s_glo);
+        s_seg_lo = ut - (int)(first / plan.n_tiles);
+    }
+    const int b = row / L, l = row - b * L;
+    float *out = match + (size_t)row * T;
+    const int64_t *tok_of = targets + (size_t)b * T;
+    constexpr int AHEAD = 4;  // cells a lane has in flight
+    float cell[AHEAD];
+    int64_t tok[AHEAD];
+    int eos_col = -1;
+    if (match && on) {
+#pragma unroll
+        for (int i = 0; i < AHEAD; i++) {
+            const int t = lane + i * LANES;
+            if (t < T) cell[i] = out[t], tok[i] = tok_of[t];
+        }
+        // criterion's EOS masking (criterions/nat_pcfg_loss.py:112-115)
+        if (ol && tl && l != (int)ol[b] - 1) eos_col = (int)tl[b] - 1;
     }
     __syncthreads();
     const int g_lo = s_glo, seg_lo = s_seg_lo, n_part = (s_ghi - g_lo + 1) * 2;
-    for (int r_in = part * (BM / kMergeSplit) + warp; r_in < (part + 1) * (BM / kMergeSplit); r_in += n_warps) {
-        const int cr = rt * BM + r_in;
-        if (cr >= n_rows) break;
-        const int row = row_src[cr], b = row / L, l = row - b * L;
-        // lane i merges partials i, i + 32, ...; then the lanes are combined
-        float m = -CUDART_INF_F, s = 0.f, best = -CUDART_INF_F;
-        int best_idx = INT_MAX;
-        for (int i = lane; i < n_part; i += 32) {
-            const int owner = g_lo + (i >> 1), h = i & 1, seg = (i >> 1) == 0 ? seg_lo : 0;
-            const int g = pair ? 2 * owner + (rt & 1) : owner;
-            const Partial p = partials[(((size_t)g * max_seg + seg) * 2 + h) * BM + r_in];
-            if (p.s > 0.f) {  // then p.m is finite
-                const float nm = fmaxf(m, p.m);
-                s = (s > 0.f ? s * exp2f((m - nm) * kLog2e) : 0.f) + p.s * exp2f((p.m - nm) * kLog2e);
-                m = nm;
-            }
-            // first maximum in column order: equal values are resolved by the recorded column
-            if (p.best > best || (p.best == best && p.best_idx < best_idx)) {
-                best = p.best;
-                best_idx = p.best_idx;
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float om = __shfl_xor_sync(0xffffffffu, m, o), os = __shfl_xor_sync(0xffffffffu, s, o);
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, best_idx, o);
-            const float nm = fmaxf(m, om);
-            s = (s > 0.f ? s * exp2f((m - nm) * kLog2e) : 0.f) + (os > 0.f ? os * exp2f((om - nm) * kLog2e) : 0.f);
+    // lane i merges partials i, i + LANES, ...; then the lanes are combined
+    float m = -CUDART_INF_F, s = 0.f, best = -CUDART_INF_F;
+    int best_idx = INT_MAX;
+    const auto fetch = [&](int i) {
+        const int owner = g_lo + (i >> 1), h = i & 1, seg = (i >> 1) == 0 ? seg_lo : 0;
+        const int g = pair ? 2 * owner + (rt & 1) : owner;
+        return partials[(((size_t)g * max_seg + seg) * 2 + h) * BM + r_in];
+    };
+    const auto add = [&](const Partial &p) {
+        if (p.s > 0.f) {  // then p.m is finite
+            const float nm = fmaxf(m, p.m);
+            s = (s > 0.f ? s * exp2f((m - nm) * kLog2e) : 0.f) + p.s * exp2f((p.m - nm) * kLog2e);
             m = nm;
-            if (ob > best || (ob == best && oi < best_idx)) {
-                best = ob;
-                best_idx = oi;
-            }
         }
-        if (best_idx == INT_MAX) best_idx = 0;
-        const float lse = m + log2f(s) * kLn2;
-        if (lane == 0) {
-            if (lse_out) lse_out[row] = lse;
-            if (max_lprob) max_lprob[row] = best - lse;
-            if (argmax) argmax[row] = best_idx;
+        // first maximum in column order: equal values are resolved by the recorded column
+        if (p.best > best || (p.best == best && p.best_idx < best_idx)) {
+            best = p.best;
+            best_idx = p.best_idx;
         }
-        if (match) {
-            int eos_col = -1;
-            bool keep_eos = true;
-            if (ol && tl) {  // criterion's EOS masking (criterions/nat_pcfg_loss.py:112-115)
-                eos_col = (int)tl[b] - 1;
-                keep_eos = l == (int)ol[b] - 1;
-            }
-            float *out = match + (size_t)row * T;
-            for (int t = lane; t < T; t += 32) {
-                const int64_t tok = targets[(size_t)b * T + t];
-                float v = out[t] - lse;
-                if (t == eos_col && !keep_eos) v = -CUDART_INF_F;
-                if (tok < 0 || tok >= V) v = CUDART_NAN_F;  // never gathered
-                out[t] = v;
-            }
+    };
+    for (int i = lane; i < n_part; i += LANES) add(fetch(i));
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) {
+        const float om = __shfl_xor_sync(0xffffffffu, m, o), os = __shfl_xor_sync(0xffffffffu, s, o);
+        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, best_idx, o);
+        const float nm = fmaxf(m, om);
+        s = (s > 0.f ? s * exp2f((m - nm) * kLog2e) : 0.f) + (os > 0.f ? os * exp2f((om - nm) * kLog2e) : 0.f);
+        m = nm;
+        if (ob > best || (ob == best && oi < best_idx)) {
+            best = ob;
+            best_idx = oi;
         }
     }
+    if (!on) return;
+    if (best_idx == INT_MAX) best_idx = 0;
+    const float lse = m + log2f(s) * kLn2;
+    if (lane == 0) {
+        if (lse_out) lse_out[row] = lse;
+        if (max_lprob) max_lprob[row] = best - lse;
+        if (argmax) argmax[row] = best_idx;
+    }
+    if (!match) return;
+    const auto finish = [&](int t, float x, int64_t k) {
+        float v = x - lse;
+        if (t == eos_col) v = -CUDART_INF_F;
+        if (k < 0 || k >= V) v = CUDART_NAN_F;  // never gathered
+        out[t] = v;
+    };
+#pragma unroll
+    for (int i = 0; i < AHEAD; i++)
+        if (lane + i * LANES < T) finish(lane + i * LANES, cell[i], tok[i]);
+    for (int t = lane + AHEAD * LANES; t < T; t += LANES) finish(t, out[t], tok_of[t]);
 }
 
 // [rows][K] fp16 row-major, box = 64 (K) x box_rows, 128-byte swizzle, out-of-bounds reads give zeros.
@@ -928,6 +951,9 @@ Workspace carve(void *base, int B, int L, int T, int V) {
 
 }  // namespace
 
+// a sentence's targets in shared memory while they are sorted, as long as that needs no opt-in
+static size_t sort_bytes(int T) { return T > 0 && T <= 8192 ? (size_t)T * sizeof(int) : 0; }
+
 size_t proj_workspace_bytes(int B, int L, int T, int V) { return carve(nullptr, B, L, T, V).bytes; }
 
 int launch_proj(const void *hidden, const void *weight, const int64_t *targets, const int64_t *ol, const int64_t *tl,
@@ -945,8 +971,8 @@ int launch_proj(const void *hidden, const void *weight, const int64_t *targets, 
 
     CUtensorMap map_w;
     if (!make_map(&map_w, weight, (uint64_t)V, (uint64_t)H, geo.pair ? BN / 2 : BN)) return PCFGNAT_ERR_CUDA;
-    if (launch_chain(proj_prepare_kernel, dim3(B), dim3(128), 0, st, ol, gather ? targets : nullptr, B, L, T, V, w.prefix,
-                     w.row_src, w.n_rows, w.stok, w.sslot, status) != cudaSuccess)
+    if (launch_chain(proj_prepare_kernel, dim3(B), dim3(128), sort_bytes(T), st, ol, gather ? targets : nullptr, B, L, T, V, w.prefix,
+                     w.row_src, w.n_rows, w.stok, w.sslot, status, sort_bytes(T) ? 1 : 0) != cudaSuccess)
         return PCFGNAT_ERR_CUDA;
     const size_t smem = (size_t)KC_MAX * A_CHUNK_BYTES + (size_t)NSTAGE * B_STAGE_BYTES + 1024;
     const bool want_arg = max_lprob != nullptr || argmax != nullptr;
@@ -960,10 +986,15 @@ int launch_proj(const void *hidden, const void *weight, const int64_t *targets, 
                                                            gather ? match : nullptr, w.partials, none, status);
     if (rc != PCFGNAT_OK) return rc;
     const int row_tiles = (N + BM - 1) / BM;
-    return cuda_rc(launch_chain(proj_merge_kernel, dim3(kMergeSplit * row_tiles + B), dim3(kMergeThreads), 0, st,
-                                (const Partial *)w.partials, (const int *)w.prefix, (const int *)w.row_src,
-                                (const int *)w.n_rows, geo.owners, geo.max_seg, row_tiles, geo.pair ? 1 : 0, V, L, T, ol, tl,
-                                targets, gather ? match : nullptr, max_lprob, argmax, lse));
+    const auto merge = [&](auto kernel, int lanes) {
+        return cuda_rc(launch_chain(kernel, dim3(kMergeSplit * row_tiles + B), dim3(kMergeRows * lanes), 0, st,
+                                    (const Partial *)w.partials, (const int *)w.prefix, (const int *)w.row_src,
+                                    (const int *)w.n_rows, geo.owners, geo.max_seg, row_tiles, geo.pair ? 1 : 0, V, L, T, ol, tl,
+                                    targets, gather ? match : nullptr, max_lprob, argmax, lse));
+    };
+    // few rows leave the GPU empty with eight lanes each, and have more partials: 3 600 rows with 154 targets 6.5 us with 32 lanes,
+    // 9.5 with 8; 10 804 rows with 47 targets 10.1 and 6.0, 16 384 with 76: 17.3 and 7.6, 21 788 with 48: 19.5 and 14.0
+    return row_tiles * 4 <= geo.owners ? merge(proj_merge_kernel<32>, 32) : merge(proj_merge_kernel<8>, 8);
 }
 
 // Rows of padding (l >= m_b) are not projected: their gradient rows are zero.
@@ -1008,8 +1039,8 @@ int launch_proj_dlogits(const void *hidden, const void *weight, const int64_t *t
     const Workspace w = carve(workspace, B, L, T, V);
     CUtensorMap map_w;
     if (!make_map(&map_w, weight, (uint64_t)V, (uint64_t)H, geo.pair ? BN / 2 : BN)) return PCFGNAT_ERR_CUDA;
-    if (launch_chain(proj_prepare_kernel, dim3(B), dim3(128), 0, st, ol, targets, B, L, T, V, w.prefix, w.row_src, w.n_rows,
-                     w.stok, w.sslot, status) != cudaSuccess)
+    if (launch_chain(proj_prepare_kernel, dim3(B), dim3(128), sort_bytes(T), st, ol, targets, B, L, T, V, w.prefix, w.row_src, w.n_rows,
+                     w.stok, w.sslot, status, sort_bytes(T) ? 1 : 0) != cudaSuccess)
         return PCFGNAT_ERR_CUDA;
     __nv_bfloat16 *dl = static_cast<__nv_bfloat16 *>(dlogits);
     const int compact = row_index != nullptr;
