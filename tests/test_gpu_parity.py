@@ -1913,6 +1913,38 @@ def test_linear_space_loss_hands_unusual_sentences_to_the_log_space_kernels(ops,
         assert torch.equal(mg[i].nan_to_num(7.0), mg2[i].nan_to_num(7.0)) and torch.equal(lg[i].nan_to_num(7.0), lg2[i].nan_to_num(7.0))
 
 
+@pytest.mark.parametrize("B, odd", [(1, 0), (6, 6), (90, 0), (90, 89), (160, 40)])
+def test_outside_pass_that_starts_before_the_inside_pass_has_ended(ops, syn, monkeypatch, B, odd):
+    """The outside pass stages its inputs while the inside pass is at work, and its clusters without work (odd graph lengths
+    here, or fewer sentences than clusters) leave early: repeated calls over the same buffers, and a captured one, give bit for
+    bit what a call alone gives, and the sentences handed over are those of the log-space kernels."""
+    monkeypatch.delenv("PCFGNAT_DP_KERNEL", raising=False)
+    monkeypatch.delenv("PCFGNAT_LINEAR_DP", raising=False)
+    b = syn.make_batch(syn.Workload("early", batch=B, vocab=50, hidden=8, src_min=4, src_max=24, emissions="logits"), seed=41)
+    ma, lk, tl = syn.reference_match_all(b).to(DEV), b.links.to(DEV), b.target_length.to(DEV)
+    ol = b.output_length.to(DEV)
+    ol[:odd] -= 1
+    ops.read_status(DEV)
+    want = [x.clone() for x in _fused(ops, ma, lk, ol, tl)]
+    assert bool(ops.read_status(DEV) & 16) == (odd > 0)  # PCFGNAT_STATUS_RECOMPUTED
+    k = ops.get_pcfg_kernel()
+    got = [k.pcfg_loss_fwd_bwd(ma, lk, ol, tl) for _ in range(4)]  # no synchronisation in between
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got.append(k.pcfg_loss_fwd_bwd(ma, lk, ol, tl))
+    graph.replay()
+    graph.replay()
+    torch.cuda.synchronize()
+    for out in got:
+        for x, y in zip(out, want):
+            assert torch.equal(x.nan_to_num(7.0), y.nan_to_num(7.0))
+    if odd:
+        monkeypatch.setenv("PCFGNAT_DP_KERNEL", "rows")
+        for x, y in zip(_fused(ops, ma, lk, ol, tl), want):
+            assert torch.equal(x[:odd].nan_to_num(7.0), y[:odd].nan_to_num(7.0))
+    ops.read_status(DEV)
+
+
 @pytest.mark.parametrize("B, L, T", [(20, 314, 238), (1, 322, 304), (2, 384, 238)])
 def test_linear_space_loss_at_the_limit_of_shared_memory(ops, monkeypatch, B, L, T):
     """Shapes whose tables come within a hundred bytes of the shared memory that the kernels' own variables leave."""
