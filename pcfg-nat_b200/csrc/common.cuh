@@ -165,6 +165,8 @@ int launch_loss_fwd_balanced(const float *match_all, const float *links, const i
 int launch_outside_balanced(const float *grad_output, const float *S, const float *match_all, const float *links,
                             const int64_t *ol, const int64_t *tl, int B, int L, int T, float *G, float *mg, float *lg,
                             int *status, cudaStream_t st);
+int launch_loss_fwd_exact(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B, int L, int T,
+                          float *S, float *C, float *loss, int *status, cudaStream_t st);
 int launch_loss_fwd_cluster(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B,
                             int L, int T, float *S, float *C, float *loss, int *status, cudaStream_t st);
 int launch_loss_fwd_fast(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B, int L,
@@ -187,11 +189,11 @@ int launch_outside_cluster(const float *grad_output, const float *S, const float
 bool outside_cluster_fits_grad(int B, int L, int T);
 
 // Which family of DP kernels runs the inside / outside passes.  PCFGNAT_DP_KERNEL in the environment
-// selects one for A/B runs and tests: "cluster" (default: warp per node, cluster per sentence),
+// selects one for A/B runs and tests: "cluster" (default: clusters of CTAs per sentence),
 // "balanced" (phase-balanced single CTA), "rows" (4 lanes per node, the only one without a size limit).
 // A family that cannot take a shape falls through to the next one in that order.
-// Unset (kDpAuto): clusters when cluster_kernels_pay(), else the measured-fastest single-CTA pair
-// (row-per-thread inside pass, phase-balanced outside pass).
+// Unset (kDpAuto): the inside pass as for "cluster"; the outside pass on clusters when cluster_kernels_pay(), else
+// phase-balanced.
 enum DpKernel { kDpCluster = 0, kDpBalanced = 1, kDpRows = 2, kDpAuto = 3 };
 DpKernel dp_kernel_choice();
 bool cluster_kernels_pay(int B, int L, int T);

@@ -18,8 +18,8 @@
 // order with shuffles and every lane keeps the running sum of its virtual lane: the same additions
 // in the same order.  Lanes 0..3 are then combined (s0 + s2) + (s1 + s3).  max is order-free.
 //
-// inside_exact_kernel further below keeps that order with half or a quarter of a warp per node; it takes the shapes whose
-// terms fit shared memory beside the links.
+// inside_exact_kernel further below keeps that order with 4 to 16 lanes per node and takes whatever fits it; the warp per node is
+// for the shapes between.
 //
 // inside_cluster_kernel<TRIPS > 0> is the inside pass for callers that never see the table (the fused
 // forward + backward): same layout, but every lane keeps its own partial sum of exponentials and the warp
@@ -29,6 +29,8 @@
 #include <cooperative_groups.h>
 
 #include <cstdlib>
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -412,106 +414,178 @@ __global__ void __launch_bounds__(kCThreads, 1)
 // ---------------------------------------------------------------------------------------
 // inside pass, reference order, G lanes per node
 // ---------------------------------------------------------------------------------------
-// The table of inside_cluster_kernel<0> bit for bit, for shapes whose terms fit shared memory beside the links.  With a
-// warp per node the kernel is bound by instruction issue (70 % of the cycles), and most of what it issues is not terms:
-// a node's fixed costs (emissions, the maximum, the 16 ordered shuffles per 32 children, logarithm, sending) are paid
-// by a whole warp, and the last trip of a node is mostly empty lanes.  Here G = 16 or 8 lanes take a node's children
-// c = a + q + G i, so that those costs are paid for 32 / G nodes at once; rows are staged with -inf where there is no
-// child (and for the first node's leaf), so that no term is tested; the exponentials go to the node's scratch in the
-// order in which the reference adds them, and four lanes per node, one per virtual lane x, add them up from 16-byte
-// loads.  Scratch of a node: xs floats per virtual lane, 8 modulo 32, nodes 4 xs + 4 apart: conflict-free both ways.
-// 64 sentences, M = 128, T = 76: 192 us (267 us with a warp per node); 90 sentences, M <= 80: 82 us (112 us).
-template <int G>
-__device__ __forceinline__ bool inside_exact_steps(float *col, const float *lk0, const float *lk1, const float *em0,
-                                                   const float *eml, float *own, float *scratch, uint64_t *col_bar, int n,
-                                                   int Mb, int my_rows, int NC, int crank, int W, int cs, int lk_stride,
-                                                   int xs, int active) {
-    constexpr int R = 32 / G, H = G / 4;  // nodes per warp; lanes per virtual lane
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int q = lane % G, sub = lane / G, x = q & 3;
-    float *node_scratch = scratch + (size_t)(warp * R + sub) * (4 * xs + 4) + x * xs;
-    float2 *cells = reinterpret_cast<float2 *>(node_scratch) + (q >> 2);
-    const float4 *terms = reinterpret_cast<const float4 *>(node_scratch);
-    uint32_t rcol = 0, rbar0 = 0, rbar1 = 0;  // lane q < NC: this CTA's columns and barriers as CTA q maps them
-    if (NC > 1 && q < NC) {
-        rcol = dsm_map_to_cta(dsm_smem_u32(col), q);
-        rbar0 = dsm_map_to_cta(dsm_smem_u32(&col_bar[0]), q);
-        rbar1 = dsm_map_to_cta(dsm_smem_u32(&col_bar[1]), q);
+// The table of inside_cluster_kernel<0> bit for bit.  The reference's four lanes x of a node take its children
+// c = a + x + 4 k in turn; here lane q = x + 4 h of a node's G = 4, 8 or 16 lanes takes k = h, h + G / 4, ...: with G = 4 every
+// lane adds up its own terms, beyond the h are visited in order with shuffles.  32 / G nodes share a warp's fixed costs (the
+// reduction of the maximum, logarithm, sending), all of a CTA's nodes are in one pass, a trip of 32 children at a time without a
+// test: rows are staged with -inf where there is no child and for the first node's leaf.  Both kinds of terms go as pairs: the
+// links of a child lie side by side and so do S[t + 1] and S[t + 2] in column t (a node stores its value into two columns), a
+// term costs one load of eight bytes of either and half of a packed addition.  The terms of the first 128 children stay in
+// registers between the maximum and the sum; those of further children are formed twice.
+//
+// Bound by the latency of a step on the longest row (57 % of the issue slots with eight lanes; the exponentials, expf for the
+// bits, are half of the instructions).  With the exponentials handed over through shared memory and 1024 threads before
+// (sixteen or eight lanes, a pass per 64 or 128 nodes), and a warp per node below 32 nodes: 64 sentences, M = 128, T = 76: 191
+// -> 131 us; 90 sentences, M <= 80: 84 -> 70; 16 sentences, M = 128 on eight CTAs each 213 -> 105; 160 sentences, M <= 80 (the
+// row-per-thread kernel of loss_fwd.cu before) 189 -> 79.  Terms formed twice for all children: 137 us for the first of these.
+struct Pair {
+    unsigned long long bits;
+    __device__ __forceinline__ Pair(float x, float y) { asm("mov.b64 %0, {%1, %2};" : "=l"(bits) : "f"(x), "f"(y)); }
+    __device__ __forceinline__ Pair operator+(const Pair &o) const {
+        Pair r = *this;
+        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(r.bits) : "l"(o.bits));
+        return r;
     }
+    __device__ __forceinline__ float2 get() const {
+        float2 v;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(bits));
+        return v;
+    }
+};
+
+constexpr int kExactThreads = 512;
+
+template <int G>
+struct ExactShape {
+    static constexpr int kNodes = 32 / G;  // of a warp
+    static constexpr int kTrips = 32 / G;  // taken together: 32 children of a node
+    static constexpr int kHeld = 128 / G;  // whose terms stay in registers
+    static constexpr int pad(int nc) { return (kNodes - 1) * nc + kTrips * G - 1; }  // children read past a chain's last one
+};
+
+template <int G>
+__device__ __forceinline__ bool inside_exact_steps(float2 *col, const float2 *lk, const float *em0, const float *eml, float *own,
+                                                   uint64_t *col_bar, int n, int Mb, int my_rows, int NC, int crank, int W,
+                                                   int cs, int pitch) {
+    using Shape = ExactShape<G>;
+    constexpr int R = Shape::kNodes, H = G / 4, U = Shape::kTrips, HELD = Shape::kHeld;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int q = lane % G, sub = lane / G;
+    // groups of R nodes get shorter along the chain: every other four in reverse, so that the four schedulers get alike shares
+    const int first = ((warp & 4) ? warp ^ 3 : warp) * R;
+    const bool live = first + sub < my_rows;
+    const int r = live ? first + sub : 0, ai = live ? crank + NC * r : crank + NC * first;
+    // of the warp's first node, which has most children; none in a warp without nodes
+    const int trips = first < my_rows ? (Mb - (crank + NC * first) + G - 1) / G : 0;
+    const float2 *lr = lk + r * pitch + ai + q, *sr = col + ai + q;
+    const float *em_r = em0 + r * W, *eml_r = eml + r * W;
+    float *own_r = own + r * W;
+    // lane q sends to CTA q / 2, the left halves of the pairs from the even lanes and the right halves from the odd ones
+    const int half = q & 1;
+    const uint32_t cell = dsm_smem_u32(col) + 8u * ai + 4u * half;
+    const uint32_t bar0 = dsm_smem_u32(col_bar);
     bool arrived = true;
+    float ma1 = em_r[n - 1], ma0 = em_r[max(n - 2, 0)], ml = eml_r[max(n - 2, 0)];
     for (int start = n - 2; start >= 0; start--) {
-        const float *S1 = col + ((start + 1) & 3) * cs, *S2 = col + ((start + 2) & 3) * cs;
-        float *S0 = col + (start & 3) * cs;
-        const uint32_t bar = dsm_smem_u32(&col_bar[start & 1]);
-        if (NC > 1 && tid == 0)  // this CTA expects the whole column of this step: one value per node of the chain
-            asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(4 * Mb)
+        const float2 *s = sr + (start & 3) * cs;
+        const uint32_t bar = bar0 + 8u * (start & 1);
+        if (NC > 1 && tid == 0)  // this CTA expects the whole column of this step: two copies of a value per node of the chain
+            asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(8 * Mb)
                          : "memory");
-        for (int first = warp * R; warp < active && first < my_rows; first += active * R) {  // warp-uniform
-            const bool live = first + sub < my_rows;
-            const int r = live ? first + sub : first, ai = crank + NC * r;
-            const int trips = (Mb - (crank + NC * first) + G - 1) / G;  // of the warp's first node, which has most children
-            const float ma0 = em0[r * W + start], ma1 = em0[r * W + start + 1], ml = eml[r * W + start];
-            const float *r0 = lk0 + r * lk_stride + ai + q, *r1 = lk1 + r * lk_stride + ai + q;
-            const float *s1 = S1 + ai + q, *s2 = S2 + ai + q;
+        if (first < my_rows) {  // warp-uniform
+            const Pair em(ma0, ml);
+            auto terms = [&](int i) {
+                const float2 l = lr[G * i], c = s[G * i];
+                float2 v = ((Pair(l.x, l.y) + Pair(c.x, c.y)) + em).get();
+                v.y += ma1;
+                return v;
+            };
             float mx = neg_inf();
-#pragma unroll 4
-            for (int i = 0; i < trips; i++) {  // fmaxf: NaN counts as -inf, like an absent child
-                const float a = fmaxf((r0[G * i] + s1[G * i]) + ma0, neg_inf());
-                const float b = fmaxf(((r1[G * i] + s2[G * i]) + ml) + ma1, neg_inf());
-                mx = fmaxf(mx, fmaxf(a, b));
-                cells[H * i] = make_float2(a, b);
+            float2 held[HELD];
+#pragma unroll
+            for (int k = 0; k < HELD / U; k++) {
+                if (k * U < trips) {
+#pragma unroll
+                    for (int j = 0; j < U; j++) held[k * U + j] = terms(k * U + j);
+#pragma unroll
+                    for (int j = 0; j < U; j++) mx = fmaxf(mx, fmaxf(held[k * U + j].x, held[k * U + j].y));
+                }
+            }
+#pragma unroll 1
+            for (int i = HELD; i < trips; i += U) {
+                float2 v[U];
+#pragma unroll
+                for (int j = 0; j < U; j++) v[j] = terms(i + j);
+#pragma unroll
+                for (int j = 0; j < U; j++) mx = fmaxf(mx, fmaxf(v[j].x, v[j].y));  // fmaxf: NaN counts as absent
             }
 #pragma unroll
             for (int o = G / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-#pragma unroll 4
-            for (int i = 0; i < trips; i++) {  // not looked at where mx is infinite
-                const float2 v = cells[H * i];
-                cells[H * i] = make_float2(expf(v.x - mx), expf(v.y - mx));
-            }
-            __syncwarp();
-            float sum = 0.f;
-            if (q < 4) {
-#pragma unroll 4
-                for (int i = 0; i < trips * H / 2; i++) {  // children k = 2 i, 2 i + 1 of this virtual lane, t0 before t1
-                    const float4 e = terms[i];
-                    sum += e.x;
-                    sum += e.y;
-                    sum += e.z;
-                    sum += e.w;
+            float sum;
+            const Pair shift(-mx, -mx);
+            auto add_block = [&](const float2 *v, auto clean) {
+                float2 e[U];
+#pragma unroll
+                for (int j = 0; j < U; j++) {
+                    e[j] = v[j];
+                    if (clean) e[j] = make_float2(fmaxf(e[j].x, neg_inf()), fmaxf(e[j].y, neg_inf()));
+                    e[j] = (Pair(e[j].x, e[j].y) + shift).get();
                 }
-            }
-            __syncwarp();
-            sum += __shfl_down_sync(0xffffffffu, sum, 2, 4);  // (s0 + s2) + (s1 + s3)
-            sum += __shfl_down_sync(0xffffffffu, sum, 1, 4);
-            sum = __shfl_sync(0xffffffffu, sum, 0, G);
+#pragma unroll
+                for (int j = 0; j < U; j++) e[j] = make_float2(expf(e[j].x), expf(e[j].y));
+#pragma unroll
+                for (int j = 0; j < U; j++) {
+                    sum += e[j].x;
+                    sum += e[j].y;
+#pragma unroll
+                    for (int h = 1; h < H; h++) {
+                        sum += __shfl_down_sync(0xffffffffu, e[j].x, 4 * h, G);
+                        sum += __shfl_down_sync(0xffffffffu, e[j].y, 4 * h, G);
+                    }
+                }
+            };
+            auto add_up = [&](auto clean) {  // not looked at where mx is infinite
+                sum = 0.f;
+                if (!clean) {
+#pragma unroll
+                    for (int k = 0; k < HELD / U; k++)
+                        if (k * U < trips) add_block(held + k * U, clean);
+                }
+#pragma unroll 1
+                for (int i = clean ? 0 : HELD; i < trips; i += U) {
+                    float2 v[U];
+#pragma unroll
+                    for (int j = 0; j < U; j++) v[j] = terms(i + j);
+                    add_block(v, clean);
+                }
+                sum += __shfl_down_sync(0xffffffffu, sum, 2, 4);  // (s0 + s2) + (s1 + s3)
+                sum += __shfl_down_sync(0xffffffffu, sum, 1, 4);
+                sum = __shfl_sync(0xffffffffu, sum, 0, G);
+            };
+            add_up(std::false_type());
+            if (__any_sync(0xffffffffu, isnan(sum) && !isinf(mx))) add_up(std::true_type());  // NaN counts as -inf, like an absent child
             const float res = isinf(mx) ? mx : logf(sum) + mx;
             if (live) {
+                // the left half of column start - 1's pairs and the right half of column start - 2's
+                const uint32_t to = cell + 8u * (((start - 1 - half) & 3) * cs);
                 if (NC > 1) {
-                    if (q < NC) dsm_store_async(rcol + 4u * ((start & 3) * cs + ai), res, (start & 1) ? rbar1 : rbar0);
-                } else if (q == 0) {
-                    S0[ai] = res;
+#pragma unroll 1
+                    for (int i = q >> 1; i < NC; i += G / 2) dsm_store_async(dsm_map_to_cta(to, i), res, dsm_map_to_cta(bar, i));
+                } else if (q < 2) {
+                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(to), "f"(res) : "memory");
                 }
-                if (q == 0) own[r * W + start] = res;
+                if (q == 0) own_r[start] = res;
             }
+            ma1 = ma0;
+            ma0 = em_r[max(start - 1, 0)];
+            ml = eml_r[max(start - 1, 0)];
         }
         // one warp waits for the column on the byte-counting barrier, the block barrier releases the others
-        if (NC > 1 && warp == kCWarps - 1) arrived = dsm_wait_column(bar, (((n - 2) - start) >> 1) & 1) && arrived;
+        if (NC > 1 && warp == (blockDim.x >> 5) - 1) arrived = dsm_wait_column(bar, (((n - 2) - start) >> 1) & 1) && arrived;
         __syncthreads();
     }
     return arrived;
 }
 
-// Sixteen lanes per node while a CTA's nodes take one pass of 32 warps that way, eight for more.
-constexpr int kExactRows16 = 2 * kCWarps;
-__global__ void __launch_bounds__(kCThreads, 1)
+template <int G>
+__global__ void __launch_bounds__(kExactThreads, 1)
     inside_exact_kernel(const float *__restrict__ match_all, const float *__restrict__ links,
                         const int64_t *__restrict__ ol, const int64_t *__restrict__ tl, int L, int T, float *S, float *C,
-                        float *loss, int *status, int Mc, int Lt, int cs, int rows_cap, int lk_stride, int B, int wide,
-                        int xs, int slots) {
+                        float *loss, int *status, int Mc, int Lt, int cs, int rows_cap, int pitch, int B, int wide) {
     extern __shared__ __align__(16) float smem[];
     cg::cluster_group cluster = cg::this_cluster();
     int crank = (int)cluster.block_rank();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, threads = blockDim.x, warps = threads >> 5;
     int NC = (int)cluster.num_blocks(), b = blockIdx.x / NC;
     if (wide >= 0) {  // sentences by decreasing cost, as in inside_cluster_kernel
         __shared__ int s_b;
@@ -522,12 +596,12 @@ __global__ void __launch_bounds__(kCThreads, 1)
             crank = 0;
         }
         int *cost = reinterpret_cast<int *>(smem);  // [B], before the columns move in
-        for (int i = tid; i < B; i += kCThreads) {
+        for (int i = tid; i < B; i += threads) {
             const long long mi = ol[i], ni = tl[i];
             cost[i] = lengths_ok((int)mi, (int)ni, L, T) ? (int)(mi * ni) : 0;
         }
         __syncthreads();
-        for (int i = tid; i < B; i += kCThreads) {
+        for (int i = tid; i < B; i += threads) {
             const int ci = cost[i];
             int before = 0;
             for (int j = 0; j < B; j++) before += cost[j] > ci || (cost[j] == ci && j < i);
@@ -536,7 +610,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
         __syncthreads();
         b = s_b;
     }
-    const int ctid = crank * kCThreads + tid, cthreads = NC * kCThreads;
+    const int ctid = crank * threads + tid, cthreads = NC * threads;
     const int W = T + 2;
     const int m = (int)ol[b], n = (int)tl[b];
     const bool ok = lengths_ok(m, n, L, T);
@@ -554,52 +628,49 @@ __global__ void __launch_bounds__(kCThreads, 1)
     }
     const int Mb = main_nodes_below(m), last = (m - 2) / 2;
     const int my_rows = Mb > crank ? (Mb - crank + NC - 1) / NC : 0;  // nodes ai = crank + NC * r
-    float *col = smem;                                // [4][cs] rolling columns of the whole chain
-    float *lk0 = col + 4 * cs;                        // [rows_cap][lk_stride] links[a][0][c] by child slot, -inf from Mb on
-    float *lk1 = lk0 + (size_t)rows_cap * lk_stride;  // the same for k = 1; -inf for the first node
-    float *own = lk1 + (size_t)rows_cap * lk_stride;  // [rows_cap][W] each: table, emissions, emissions of the leaves
+    // column t: (S[t + 1], S[t + 2]) of the whole chain; [4][cs], -inf from the chain's end on
+    float2 *col = reinterpret_cast<float2 *>(smem);
+    float2 *lk = col + 4 * cs;  // [rows_cap][pitch] links[a][0 and 1][c] by child slot; -inf from Mb on and for the first node's 1
+    float *own = reinterpret_cast<float *>(lk + (size_t)rows_cap * pitch);  // [rows_cap][W] each: table, emissions, leaves' emissions
     float *em0 = own + (size_t)rows_cap * W, *eml = em0 + (size_t)rows_cap * W;
-    float *scratch = smem + ((eml + (size_t)rows_cap * W - smem + 3) & ~(ptrdiff_t)3);
-    for (int i = tid; i < my_rows * W; i += kCThreads) {
+    for (int i = tid; i < my_rows * W; i += threads) {
         const int r = i / W, t = i - r * W, a = 2 * (crank + NC * r) + 1;
         em0[i] = t < T ? __ldg(mat + (size_t)a * T + t) : 0.f;
         eml[i] = t < T && a >= 3 ? __ldg(mat + (size_t)(a - 1) * T + t) : 0.f;
     }
-    for (int r = warp; r < my_rows; r += kCWarps) {
+    for (int r = warp; r < my_rows; r += warps) {
         const int ai = crank + NC * r;
         const float *row = lkb + (size_t)(2 * ai + 1) * 2 * L;
 #pragma unroll 4
-        for (int ci = ai + lane; ci < lk_stride; ci += 32) {
-            lk0[r * lk_stride + ci] = ci < Mb ? __ldg(row + 2 * ci + 1) : neg_inf();
-            lk1[r * lk_stride + ci] = ci < Mb && ai > 0 ? __ldg(row + L + 2 * ci + 1) : neg_inf();
-        }
+        for (int ci = ai + lane; ci < pitch; ci += 32)
+            lk[r * pitch + ci] = make_float2(ci < Mb ? __ldg(row + 2 * ci + 1) : neg_inf(),
+                                             ci < Mb && ai > 0 ? __ldg(row + L + 2 * ci + 1) : neg_inf());
     }
     __shared__ __align__(8) uint64_t col_bar[2];
-    for (int i = tid; i < 4 * cs; i += kCThreads) col[i] = neg_inf();
+    for (int i = tid; i < 4 * cs; i += threads) col[i] = make_float2(neg_inf(), neg_inf());
     if (tid == 0) {
         for (int i = 0; i < 2; i++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(dsm_smem_u32(&col_bar[i])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (tid == 0) col[((n - 1) & 3) * cs + last] = __ldg(mat + (size_t)(m - 1) * T + (n - 1));  // every CTA its own copy
+    if (tid == 0) {  // column n - 1, every CTA its own copy
+        const float term = __ldg(mat + (size_t)(m - 1) * T + (n - 1));
+        col[((n - 2) & 3) * cs + last].x = term;
+        col[((n - 3) & 3) * cs + last].y = term;
+    }
     // all copies initialised before anybody stores into a neighbour's; also orders the -inf fill of the global table
     if (NC > 1) cluster.sync(); else __syncthreads();
     if (ctid == 0) Sb[(size_t)last * W + (n - 1)] = __ldg(mat + (size_t)(m - 1) * T + (n - 1));
-    const bool arrived =
-        my_rows <= kExactRows16
-            ? inside_exact_steps<16>(col, lk0, lk1, em0, eml, own, scratch, col_bar, n, Mb, my_rows, NC, crank, W, cs, lk_stride,
-                                     xs, min(kCWarps, slots / 2))
-            : inside_exact_steps<8>(col, lk0, lk1, em0, eml, own, scratch, col_bar, n, Mb, my_rows, NC, crank, W, cs, lk_stride,
-                                    xs, min(kCWarps, slots / 4));
+    const bool arrived = inside_exact_steps<G>(col, lk, em0, eml, own, col_bar, n, Mb, my_rows, NC, crank, W, cs, pitch);
     if (!arrived && lane == 0) flag(status, PCFGNAT_STATUS_TIMEOUT);
     // no CTA leaves (its shared memory with it) while a peer may still send to it; every wait above is bounded
     if (NC > 1) cluster.sync();
-    for (int i = tid; i < my_rows * (n - 1); i += kCThreads) {  // computed cells: columns 0 .. n-2
+    for (int i = tid; i < my_rows * (n - 1); i += threads) {  // computed cells: columns 0 .. n-2
         const int r = i / (n - 1), t = i - r * (n - 1);
         Sb[(size_t)(crank + NC * r) * W + t] = own[r * W + t];
     }
-    if (loss && ctid == 0) loss[b] = (n >= 2) ? col[0] : Sb[0];
+    if (loss && ctid == 0) loss[b] = (n >= 2) ? own[0] : Sb[0];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -827,6 +898,11 @@ struct ClusterGeometry {
     size_t smem_in, smem_out;
 };
 
+int cluster_size_wanted(const char *v, int nc) {  // experiments: 1, 2, 4, 8 or 16
+    const int want = atoi(v);
+    return want == 1 || want == 2 || want == 4 || want == 8 || want == 16 ? want : nc;
+}
+
 // Cluster size: the largest power of two <= 16 that still lets all sentences run at once, raised if a
 // CTA's share of the links would not fit shared memory; nc = 0 when no size fits.
 ClusterGeometry cluster_geometry(int B, int Mc, int W) {
@@ -839,10 +915,7 @@ ClusterGeometry cluster_geometry(int B, int Mc, int W) {
     // measured on 8 sentences x 256 nodes: 8 CTAs per sentence 1.12 ms, 16 CTAs 1.85 ms (the barrier of a
     // 16-CTA cluster costs more than the extra SMs give), 4 CTAs 1.65 ms: stop at 8
     while (nc < 8 && (long long)B * nc * 2 <= sms && Mc > 8 * nc) nc *= 2;
-    if (const char *v = getenv("PCFGNAT_DP_CLUSTER_SIZE")) {  // experiments: 1, 2, 4, 8 or 16
-        const int want = atoi(v);
-        if (want == 1 || want == 2 || want == 4 || want == 8 || want == 16) nc = want;
-    }
+    if (const char *v = getenv("PCFGNAT_DP_CLUSTER_SIZE")) nc = cluster_size_wanted(v, nc);
     for (;; nc *= 2) {
         g.nc = nc;
         g.rows_cap = (Mc + nc - 1) / nc;
@@ -860,13 +933,13 @@ ClusterGeometry cluster_geometry(int B, int Mc, int W) {
 }
 
 template <class Kernel, class... Args>
-int launch_cluster(Kernel kernel, int B, int nc, size_t smem, cudaStream_t st, Args... args) {
+int launch_cluster(Kernel kernel, int threads, int B, int nc, size_t smem, cudaStream_t st, Args... args) {
     if (ensure_dynamic_smem(kernel, smem) != cudaSuccess) return PCFGNAT_ERR_CUDA;
     if (nc > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
         return PCFGNAT_ERR_UNSUPPORTED;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(B * nc));
-    cfg.blockDim = dim3(kCThreads);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -934,61 +1007,70 @@ int launch_inside(const float *match_all, const float *links, const int64_t *ol,
             // and the others share (see the kernel); every CTA can hold a whole chain, so the shared memory is that of one CTA
             const int wide = mixed_width_count(B, Mc);
             if (wide > 0) {
-                int rc = launch_cluster(inside_cluster_kernel<TRIPS, SHARES>, wide + (B - wide + 1) / 2, 2, g.smem_in, st, match_all, links, ol, tl,
+                int rc = launch_cluster(inside_cluster_kernel<TRIPS, SHARES>, kCThreads, wide + (B - wide + 1) / 2, 2, g.smem_in, st, match_all, links, ol, tl,
                                         L, T, S, C, loss, status, Mc, Lt, g.cs, g.rows_cap, g.lk_stride, B, wide, shares);
                 if (rc != PCFGNAT_ERR_UNSUPPORTED) return rc;
             }
         }
         // more CTAs than SMs: sentences by decreasing cost, so that the clusters that wait for a place get the cheapest
         const int ranked = (long long)B * g.nc > sm_count() && B <= 256 ? B : -1;
-        int rc = launch_cluster(inside_cluster_kernel<TRIPS, SHARES>, B, g.nc, g.smem_in, st, match_all, links, ol, tl, L,
+        int rc = launch_cluster(inside_cluster_kernel<TRIPS, SHARES>, kCThreads, B, g.nc, g.smem_in, st, match_all, links, ol, tl, L,
                                 T, S, C, loss, status, Mc, Lt, g.cs, g.rows_cap, g.lk_stride, B, ranked, shares);
         if (rc != PCFGNAT_ERR_UNSUPPORTED) return rc;
     }
     return PCFGNAT_ERR_UNSUPPORTED;
 }
 
-// Reference order with 16 or 8 lanes per node; PCFGNAT_ERR_UNSUPPORTED when the terms do not fit beside the links.
+// Reference order with G lanes per node; PCFGNAT_ERR_UNSUPPORTED when the tables or the nodes of a CTA do not fit.
+template <int G>
 int launch_exact(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B, int L, int T,
-                 float *S, float *C, float *loss, int *status, cudaStream_t st, int nc, int wide, bool mixed) {
-    const int Mc = main_slots(L, 1), Lt = L - Mc, W = T + 2, cs = (Mc + 3) / 4 * 4;
+                 float *S, float *C, float *loss, int *status, cudaStream_t st, int nc, int wide, bool mixed, bool crowded) {
+    const int Mc = main_slots(L, 1), Lt = L - Mc, W = T + 2;
     const int width = mixed ? 2 : nc;  // CTAs of a cluster
-    const int rows_cap = (Mc + nc - 1) / nc, G = rows_cap <= kExactRows16 ? 16 : 8;
-    // a row is read up to G - 1 children past its last one, by the warp's later nodes up to (32 / G - 1) CTA counts more;
-    // the rows of a warp's nodes G banks apart
-    const int pad = G == 16 ? 16 + width : (8 + 3 * width > 16 + width ? 8 + 3 * width : 16 + width);
-    const int lk_stride = (Mc + pad + width - G + 31) / 32 * 32 + G - width;
-    const int xs = ((Mc + 15) / 16 * 8 + 23) / 32 * 32 + 8;  // what sixteen lanes need is enough for eight
-    const size_t base = (((size_t)4 * cs + (size_t)2 * rows_cap * lk_stride + (size_t)3 * rows_cap * W) * sizeof(float) + 15) &
-                        ~(size_t)15;
-    const size_t limit = (size_t)kSmemLimit - 1024, per_node = (size_t)(4 * xs + 4) * sizeof(float);
-    if (base >= limit) return PCFGNAT_ERR_UNSUPPORTED;
-    // nodes in flight: all of a CTA's, as far as the warps and the room go (whole warps of either kind)
-    int slots = (rows_cap + 3) / 4 * 4;
-    if (slots > 4 * kCWarps) slots = 4 * kCWarps;
-    if ((size_t)slots * per_node > limit - base) slots = (int)((limit - base) / per_node) / 4 * 4;
-    if (slots < 32 && slots < rows_cap) return PCFGNAT_ERR_UNSUPPORTED;
-    size_t smem = base + slots * per_node;
+    const int rows_cap = (Mc + nc - 1) / nc;
+    const int cs = Mc + ExactShape<G>::pad(width);
+    // the eight-byte cells that a half-warp reads for its nodes in distinct banks, on a CTA that has a sentence to itself
+    int pitch = cs;
+    while (G < 16 && (pitch + nc) % 16 != G) pitch++;
+    size_t smem = ((size_t)4 * cs + (size_t)rows_cap * pitch) * sizeof(float2) + (size_t)3 * rows_cap * W * sizeof(float);
     if (wide >= 0 && smem < (size_t)B * sizeof(int)) smem = (size_t)B * sizeof(int);  // the costs that rank the sentences
+    int threads = (rows_cap + ExactShape<G>::kNodes - 1) / ExactShape<G>::kNodes * 32;  // all nodes in one pass
+    if (smem > (size_t)kSmemLimit - 1024 || threads > kExactThreads) return PCFGNAT_ERR_UNSUPPORTED;
+    const int least = crowded ? 128 : 256;  // fewer take longer to stage the links
+    threads = threads <= least ? least : (threads + 127) / 128 * 128;
     const int clusters = mixed ? wide + (B - wide + 1) / 2 : B;
-    return launch_cluster(inside_exact_kernel, clusters, width, smem, st, match_all, links, ol, tl, L, T, S, C, loss, status,
-                          Mc, Lt, cs, rows_cap, lk_stride, B, wide, xs, slots);
+    return launch_cluster(inside_exact_kernel<G>, threads, clusters, width, smem, st, match_all, links, ol, tl, L, T, S, C, loss,
+                          status, Mc, Lt, cs, rows_cap, pitch, B, wide);
+}
+
+// Inside pass in the reference's order on as many CTAs per sentence as leave all sentences on the GPU at once, on more where
+// the tables need the room.  PCFGNAT_ERR_UNSUPPORTED: they do not fit sixteen CTAs either.
+int launch_loss_fwd_exact(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B, int L, int T,
+                          float *S, float *C, float *loss, int *status, cudaStream_t st) {
+    const int Mc = main_slots(L, 1);
+    int nc = 1;
+    while (nc < 8 && (long long)B * nc * 2 <= sm_count() && Mc > 8 * nc) nc *= 2;
+    if (const char *v = getenv("PCFGNAT_DP_CLUSTER_SIZE")) nc = cluster_size_wanted(v, nc);
+    for (; nc <= 16; nc *= 2) {
+        const int wide = nc == 1 ? mixed_width_count(B, Mc) : 0;
+        const bool crowded = (long long)B * nc > sm_count();
+        const int order = wide > 0 ? wide : crowded && B <= 256 ? B : -1;
+        const int rows = (Mc + nc - 1) / nc;
+        // Fewer lanes per node share more of the fixed costs, more lanes shorten the longest row.  Where every CTA has an SM to
+        // itself: 24 nodes of 96 on a CTA (24 sentences) 76 / 70 / 68 us with 4 / 8 / 16 lanes, 48 nodes (100 sentences)
+        // 37 / 34.5 / -, 64 of 128 (56 sentences) 128 / 133 / -.  With more CTAs than SMs the four-lane blocks, smaller, share
+        // SMs: 300 sentences of 32 nodes 22 / 22 / 33 us, of 64 nodes 58 / 82 / -.
+        const int rc = crowded || rows > 48
+                           ? launch_exact<4>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, nc, order, wide > 0, crowded)
+                       : rows > 32 ? launch_exact<8>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, nc, order, wide > 0, crowded)
+                                   : launch_exact<16>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, nc, order, wide > 0, crowded);
+        if (rc != PCFGNAT_ERR_UNSUPPORTED) return rc;
+    }
+    return PCFGNAT_ERR_UNSUPPORTED;
 }
 
 int launch_loss_fwd_cluster(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B,
                             int L, int T, float *S, float *C, float *loss, int *status, cudaStream_t st) {
-    const int Mc = main_slots(L, 1);
-    const ClusterGeometry g = cluster_geometry(B, Mc, T + 2);
-    // Where a warp has a node to itself in every step (up to 32 nodes per CTA) the fewer trips of all its lanes are
-    // worth more: 8 sentences of 80 nodes on eight CTAs each 56 us against 66 with sixteen lanes per node, 16 of 128 213
-    // against 246; from 32 nodes on it turns: 32 of 128 on four CTAs 146 against 140, 45 of 80 on two 111 against 81.
-    const int rows = g.nc >= 1 ? (Mc + g.nc - 1) / g.nc : 0;
-    if (rows >= kCWarps && g.nc <= 8) {
-        const int wide = g.nc == 1 ? mixed_width_count(B, Mc) : 0;
-        const int order = wide > 0 ? wide : (long long)B * g.nc > sm_count() && B <= 256 ? B : -1;
-        const int rc = launch_exact(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, g.nc, order, wide > 0);
-        if (rc != PCFGNAT_ERR_UNSUPPORTED) return rc;
-    }
     return launch_inside<0>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st);
 }
 
@@ -1032,14 +1114,14 @@ int launch_outside_cluster(const float *grad_output, const float *S, const float
     ClusterGeometry g = cluster_geometry(B, Mc, T + 2);
     if (mg && lg) {
         if (!outside_cluster_fits_grad(B, L, T)) return PCFGNAT_ERR_UNSUPPORTED;
-        return launch_cluster(outside_cluster_kernel<true>, B, g.nc, outside_grad_smem(g, T), st, grad_output, S, match_all,
+        return launch_cluster(outside_cluster_kernel<true>, kCThreads, B, g.nc, outside_grad_smem(g, T), st, grad_output, S, match_all,
                               links, ol, tl, L, T, G, mg, lg, status, Mc, g.cs, g.rows_cap, g.lk_stride);
     }
     for (; g.nc >= 1; g.nc /= 2) {
         g.rows_cap = (Mc + g.nc - 1) / g.nc;
         g.smem_out = ((size_t)8 * g.cs + (size_t)2 * g.rows_cap * g.lk_stride + (size_t)2 * g.rows_cap * (T + 2)) * sizeof(float);
         if (g.smem_out > (size_t)kSmemLimit - 1024) break;
-        int rc = launch_cluster(outside_cluster_kernel<false>, B, g.nc, g.smem_out, st, grad_output, S, match_all, links, ol,
+        int rc = launch_cluster(outside_cluster_kernel<false>, kCThreads, B, g.nc, g.smem_out, st, grad_output, S, match_all, links, ol,
                                 tl, L, T, G, nullptr, nullptr, status, Mc, g.cs, g.rows_cap, g.lk_stride);
         if (rc != PCFGNAT_ERR_UNSUPPORTED) return rc;
     }

@@ -216,13 +216,19 @@ __global__ void __launch_bounds__(kMaxRows *kLanes)
 int launch_loss_fwd(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B, int L,
                     int T, float *S, float *C, float *loss, int *status, cudaStream_t st) {
     if (B == 0) return PCFGNAT_OK;
-    // Kernel families, all producing bit-identical tables: warp-per-node clusters (loss_cluster.cu; chosen
-    // when few sentences leave several SMs per sentence, or the chain is long), phase-balanced single CTA
+    // Kernel families, all producing bit-identical tables: 4 to 16 lanes per node on clusters (loss_cluster.cu), a warp per node
+    // on clusters where few sentences leave several SMs per sentence or the chain is long, phase-balanced single CTA
     // (loss_balanced.cu, on request only: measured slower here) and the row-per-thread kernel below, which
     // has no size limit because it can read links from global memory.
     const DpKernel choice = dp_kernel_choice();
-    if (choice == kDpCluster || (choice == kDpAuto && (cluster_kernels_pay(B, L, T) || inside_mixed_widths_pay(B, L, T)))) {
-        const int rc = launch_loss_fwd_cluster(match_all, links, ol, tl, B, L, T, S, C, loss, status, st);
+    if (choice == kDpCluster || choice == kDpAuto) {
+        const bool pays = choice == kDpCluster || cluster_kernels_pay(B, L, T);
+        int rc = PCFGNAT_ERR_UNSUPPORTED;
+        // of batches with one CTA per sentence the shortest chains stay with the kernel below, which fits more sentences on an
+        // SM: 1000 of 16 nodes 18.6 us against 27.4, 128 of 12 nodes 18.1 against 18.5, but 128 of 20 nodes 20.3 against 19.1
+        if (pays || main_slots(L, 1) > 16) rc = launch_loss_fwd_exact(match_all, links, ol, tl, B, L, T, S, C, loss, status, st);
+        if (rc == PCFGNAT_ERR_UNSUPPORTED && (pays || inside_mixed_widths_pay(B, L, T)))
+            rc = launch_loss_fwd_cluster(match_all, links, ol, tl, B, L, T, S, C, loss, status, st);
         if (rc != PCFGNAT_ERR_UNSUPPORTED) return rc;
     }
     if (choice == kDpBalanced) {

@@ -549,6 +549,43 @@ def test_fused_loss_model_graph_size(ops, syn, monkeypatch, batch):
     assert ops.read_status(DEV) == 0
 
 
+@pytest.mark.parametrize("B, L, T", [(1, 2, 1), (3, 8, 5), (4, 64, 30), (20, 162, 40), (5, 515, 70), (3, 780, 200), (30, 260, 60),
+                                     (60, 98, 31), (60, 255, 76), (50, 330, 100), (80, 36, 12), (100, 33, 10), (100, 129, 40),
+                                     (100, 256, 76), (90, 280, 20), (150, 30, 9), (200, 66, 20), (260, 130, 30), (300, 40, 12)])
+def test_inside_table_edges(ops, monkeypatch, B, L, T):
+    """Tables bit for bit those of the kernel with a thread row per node, at the numbers of lanes per node, cluster sizes and
+    shared clusters that the library picks, chains beyond the terms held in registers included; with NaN and infinite transitions
+    and emissions, sentences without a finite term, odd, short and out-of-range lengths, one target token."""
+    for name in ("PCFGNAT_DP_KERNEL", "PCFGNAT_DP_CLUSTER_SIZE"):
+        monkeypatch.delenv(name, raising=False)
+    g = torch.Generator(DEV).manual_seed(L * 3 + B)
+    match = 2 * torch.randn(B, L, T, device=DEV, generator=g) - 6
+    links = torch.randn(B, L, 2, L, device=DEV, generator=g) - 4
+    at = torch.arange(L, device=DEV)
+    links.masked_fill_((at[None, :] <= at[:, None])[None, :, None, :], float("-inf"))
+    ol = torch.randint(max(2, L // 4), L + 1, (B,), device=DEV, generator=g)
+    tl = torch.randint(1, T + 1, (B,), device=DEV, generator=g)
+    ol[0], tl[0], ol[-1], tl[-1] = L, T, L, max(1, T - 1)
+    if B > 3:
+        links[1].masked_fill_(torch.rand(L, 2, L, device=DEV, generator=g) < 0.05, float("nan"))
+        match[1].masked_fill_(torch.rand(L, T, device=DEV, generator=g) < 0.02, float("nan"))
+        links[2].masked_fill_(torch.rand(L, 2, L, device=DEV, generator=g) < 0.6, float("-inf"))
+        match[2, :, T // 2:] = float("-inf")
+        links[3, L // 2, 0, -3:] = float("inf")
+    if B > 4:
+        tl[2], tl[4], ol[B // 2], tl[B // 2 + 1] = T, 1, L + 1, 0
+    k = ops.get_pcfg_kernel()
+    ops.read_status(DEV)
+    S, C = k.pcfg_loss(match, links, ol, tl, 1)
+    status = ops.read_status(DEV)
+    monkeypatch.setenv("PCFGNAT_DP_KERNEL", "rows")
+    want_S, want_C = k.pcfg_loss(match, links, ol, tl, 1)
+    assert status == ops.read_status(DEV) == (B > 4)  # PCFGNAT_STATUS_BAD_LENGTH
+    assert np.array_equal(_bits(S.cpu().numpy()), _bits(want_S.cpu().numpy()))
+    assert np.array_equal(_bits(C.cpu().numpy()), _bits(want_C.cpu().numpy()))
+    assert torch.isfinite(S).any()
+
+
 @pytest.mark.parametrize("batch", [97, 6])  # one CTA per sentence; a cluster of CTAs per sentence
 @pytest.mark.parametrize("L_even", [True, False])
 def test_outside_pass_with_fused_gradients_matches_the_gradient_kernel(ops, syn, monkeypatch, L_even, batch):
