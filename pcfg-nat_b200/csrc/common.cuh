@@ -44,6 +44,22 @@ __device__ __forceinline__ float fast_exp(float x) {
     return y;
 }
 
+// Two floats that are added at once, each rounded as by itself.
+struct Pair {
+    unsigned long long bits;
+    __device__ __forceinline__ Pair(float x, float y) { asm("mov.b64 %0, {%1, %2};" : "=l"(bits) : "f"(x), "f"(y)); }
+    __device__ __forceinline__ Pair operator+(const Pair &o) const {
+        Pair r = *this;
+        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(r.bits) : "l"(o.bits));
+        return r;
+    }
+    __device__ __forceinline__ float2 get() const {
+        float2 v;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(bits));
+        return v;
+    }
+};
+
 // ---- column exchange without a cluster barrier: a finished node is sent to every CTA of the cluster with
 // st.async, which also counts its bytes on a barrier in the receiving CTA; a CTA starts the next step when its
 // own barrier has seen the whole column.  Two barriers alternate by step (a CTA can be at most one step

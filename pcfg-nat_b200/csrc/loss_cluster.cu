@@ -428,21 +428,6 @@ __global__ void __launch_bounds__(kCThreads, 1)
 // (sixteen or eight lanes, a pass per 64 or 128 nodes), and a warp per node below 32 nodes: 64 sentences, M = 128, T = 76: 191
 // -> 131 us; 90 sentences, M <= 80: 84 -> 70; 16 sentences, M = 128 on eight CTAs each 213 -> 105; 160 sentences, M <= 80 (the
 // row-per-thread kernel of loss_fwd.cu before) 189 -> 79.  Terms formed twice for all children: 137 us for the first of these.
-struct Pair {
-    unsigned long long bits;
-    __device__ __forceinline__ Pair(float x, float y) { asm("mov.b64 %0, {%1, %2};" : "=l"(bits) : "f"(x), "f"(y)); }
-    __device__ __forceinline__ Pair operator+(const Pair &o) const {
-        Pair r = *this;
-        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(r.bits) : "l"(o.bits));
-        return r;
-    }
-    __device__ __forceinline__ float2 get() const {
-        float2 v;
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(bits));
-        return v;
-    }
-};
-
 constexpr int kExactThreads = 512;
 
 template <int G>

@@ -9,7 +9,7 @@
 //     t1 = ((links[a][1][c] + ob[a-1]) + S[c][len-2]) + ob[a]          (j = 1, leaf a-1)
 // The reference gives node id four threads x = 0..3; thread x scans c_id = id + x + 4k in increasing
 // k, t0 before t1, under strict '>', and the four are merged with shfl_down 2 then 1 under strict
-// '>'.  A maximum is order-free except for ties, so here G = 4 to 32 lanes own the node (lane q scans
+// '>'.  A maximum is order-free except for ties, so here G = 4 to 16 lanes own the node (lane q scans
 // c_id = id + q + G i, which is reference thread x = q & 3) and the reference's choice among equal
 // values is reproduced by an explicit tie key: thread priority 0 > 2 > 1 > 3, then the smaller c,
 // then j = 0 before j = 1.  Values and backpointers are bit-exact.  Tables are indexed by node id;
@@ -39,9 +39,7 @@ namespace pcfgnat {
 
 namespace {
 
-constexpr int kVitThreads = 1024;
-constexpr int kVitWarps = kVitThreads / 32;
-constexpr int kVitActive = 16;  // warps a length's nodes are shared out to
+constexpr int kVitThreads = 512;
 
 // Monotone map float -> unsigned (no NaN reaches it); -0 is mapped like +0 so that, as under the
 // reference's '>', neither beats the other.
@@ -87,45 +85,6 @@ __device__ __forceinline__ void viterbi_node(int id, int Mb, int lane, int prio,
     warp_argmax(best, key, lane);
 }
 
-// The same for a group of G lanes (G = 4, 8, 16 or 32, the groups of a warp side by side): lane q of the group scans
-// children ci = id + q + G i, i < trips, so that its reference thread (ci - id) & 3 = q & 3 is still one per lane, and the
-// group settles on (largest value, smallest key) with a butterfly of shuffles.  The rows r0, r1 (from the lane's first
-// child on) hold -inf past the chain (or the lane's trips end with it), so no child is tested and the loads of four
-// trips are in flight together.
-// A lane remembers the trip of its best, the key is made at the end.
-__device__ __forceinline__ void viterbi_node_group(int id, int trips, int q, int G, float oa, const float *r0, const float *r1,
-                                                   const float *s1, const float *s2, float &best, int &key) {
-    best = neg_inf();
-    int at = -1;
-#pragma unroll 4
-    for (int i = 0; i < trips; i++) {
-        const float t0 = (r0[G * i] + s1[G * i]) + oa;
-        const float t1 = (r1[G * i] + s2[G * i]) + oa;
-        if (t0 > best) {
-            best = t0;
-            at = 2 * i;
-        }
-        if (t1 > best) {
-            best = t1;
-            at = 2 * i + 1;
-        }
-    }
-    const int x = q & 3, prio = ((x & 1) << 1) | (x >> 1);
-    key = at < 0 ? INT_MAX : (prio << 24) | ((id + q + G * (at >> 1)) << 1) | (at & 1);
-    if (G == 32) {  // a whole warp: two integer reductions instead of five rounds of two shuffles
-        warp_argmax(best, key, threadIdx.x & 31);
-        return;
-    }
-    for (int o = G >> 1; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int ok = __shfl_xor_sync(0xffffffffu, key, o);
-        if (ov > best || (ov == best && ok < key)) {  // -0 and +0 compare equal, as under the reference's '>'
-            best = ov;
-            key = ok;
-        }
-    }
-}
-
 __device__ __forceinline__ void viterbi_store(float best, int key, int a, int Q, int len, float *Sb, int64_t *Rb,
                                               int64_t *Lb, int64_t *Mtb) {
     if (isinf(best)) return;  // cell stays at its initial value (pcfg_viterbi.cu:113-121)
@@ -137,17 +96,159 @@ __device__ __forceinline__ void viterbi_store(float best, int key, int a, int Q,
     Mtb[o] = bj;
 }
 
-// How far past the chain's last child the G lanes of a node read, when 32 / G nodes NC apart share a warp's trips.
-__host__ __device__ inline int viterbi_overshoot(int G, int NC) { return G - 1 + NC * (32 / G - 1); }
+// Lanes per node: as few as let a block's warps take all of its nodes in one pass.  60 nodes on 16 warps: 76 / 69 / 94 us with
+// 4 / 8 / 16 lanes (64 sentences of 120 nodes); 16 nodes: 141 / 103 / 93, and 101 with 32 (16 sentences of 128).
+__host__ __device__ inline int viterbi_lanes(int rows, int warps) {
+    int G = 16;
+    while ((32 / G) * warps < rows && G > 4) G >>= 1;
+    return G;
+}
+// How far past the chain's last child they read, 32 children at a time, when 32 / G nodes NC apart share a warp's trips.
+__host__ __device__ constexpr int viterbi_overshoot(int G, int NC) { return 31 + NC * (32 / G - 1); }
+
+// The lengths of a sentence, G lanes per node: lane q takes children id + q + G i, so that its reference thread
+// (ci - id) & 3 = q & 3 is one per lane, blocks of 32 children without a test: the columns hold -inf past the chain, and
+// whatever lies behind a node's row gives -inf or NaN with it, which never wins.  Both kinds of terms go as pairs: a child's
+// links lie side by side and so do S[len - 1] and S[len - 2] in column len (a node stores its value into two columns).  Peers wait
+// for the value alone: the maximum is sent, and which term it was, with the reference's order of ties, is looked up in the held
+// terms while it is on its way (the terms of a node's first 128 children; of further ones value and term are carried
+// together).
+//
+// Bound by the latency of a length (loads, the chain of maxima, shuffles, exchange and barrier).  With value and key carried
+// through every comparison, 1024 threads and one load and addition per term before: 64 sentences of up to 120 nodes 82 -> 68 us,
+// 24 of 128 74 -> 57, 56 of up to 160 144 -> 119, one of 256 on eight CTAs 175 -> 141.
+template <int G>
+__device__ __forceinline__ bool viterbi_lengths(float2 *col, const float2 *lk, const float *s_oa, float *own_v, uint16_t *own_k,
+                                                uint64_t *col_bar, int n_len, int Mb, int my_rows, int NC, int crank, int Q,
+                                                int cs, int pitch) {
+    constexpr int R = 32 / G, U = 32 / G, HELD = 128 / G;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    const int q = lane % G, sub = lane / G;
+    const int prio = ((q & 1) << 1) | ((q >> 1) & 1);
+    const int half = q & 1;  // lane q sends to CTA q / 2: the left halves of the pairs if even, the right halves if odd
+    const uint32_t bar0 = dsm_smem_u32(col_bar), cells = dsm_smem_u32(col) + 4u * half;
+    bool arrived = true;
+    for (int len = 2; len < n_len; len++) {
+        const float2 *pairs = col + (len & 3) * cs;
+        const uint32_t bar = bar0 + 8u * (len & 1);
+        if (NC > 1 && tid == 0)  // this CTA expects the whole column of this length: two copies of a value per node of the chain
+            asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(8 * Mb)
+                         : "memory");
+        for (int first = warp * R; first < my_rows; first += warps * R) {  // warp-uniform
+            const bool live = first + sub < my_rows;
+            const int r = live ? first + sub : first, id = crank + NC * r;
+            const int trips = (Mb - (crank + NC * first) + G - 1) / G;  // of the warp's first node, which has most children
+            const float oa = s_oa[r];
+            const Pair both(oa, oa);
+            const float2 *lr = lk + r * pitch + id + q, *sr = pairs + id + q;
+            // t0 = ((links[a][0][c] + 0) + S[c][len-1]) + ob[a], t1 = ((links[a][1][c] + ob[a-1]) + S[c][len-2]) + ob[a]
+            auto terms = [&](int i) {
+                const float2 l = lr[G * i], c = sr[G * i];
+                return ((Pair(l.x, l.y) + Pair(c.x, c.y)) + both).get();
+            };
+            float2 held[HELD];
+            float best = neg_inf();
+#pragma unroll
+            for (int k = 0; k < HELD / U; k++) {
+                if (k * U >= trips) break;
+#pragma unroll
+                for (int j = 0; j < U; j++) held[k * U + j] = terms(k * U + j);
+#pragma unroll
+                for (int j = 0; j < U; j++) best = fmaxf(best, fmaxf(held[k * U + j].x, held[k * U + j].y));  // NaN never wins
+            }
+            float far = neg_inf();  // further children: value and trip together
+            int far_at = INT_MAX;
+#pragma unroll 1
+            for (int i = HELD; i < trips; i += U) {
+                float2 t[U];
+#pragma unroll
+                for (int j = 0; j < U; j++) t[j] = terms(i + j);
+#pragma unroll
+                for (int j = 0; j < U; j++) {
+                    if (t[j].x > far) {
+                        far = t[j].x;
+                        far_at = 2 * (i + j);
+                    }
+                    if (t[j].y > far) {
+                        far = t[j].y;
+                        far_at = 2 * (i + j) + 1;
+                    }
+                }
+            }
+            best = fmaxf(best, far);
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+            int key = INT_MAX;
+            const bool zero = __any_sync(0xffffffffu, best == 0.f);
+            if (zero) {  // -0 and +0 compare equal: the value is the one that comes first
+                best = neg_inf();
+#pragma unroll 1
+                for (int i = 0; i < trips; i++) {
+                    const float2 t = terms(i);
+                    const int kk = (prio << 24) | ((id + q + G * i) << 1);
+                    if (t.x > best) {
+                        best = t.x;
+                        key = kk;
+                    }
+                    if (t.y > best) {
+                        best = t.y;
+                        key = kk | 1;
+                    }
+                }
+                for (int o = G / 2; o > 0; o >>= 1) {
+                    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+                    const int ok = __shfl_xor_sync(0xffffffffu, key, o);
+                    if (ov > best || (ov == best && ok < key)) {
+                        best = ov;
+                        key = ok;
+                    }
+                }
+            }
+            if (live) {  // the left half of column len + 1's pairs and the right half of column len + 2's
+                const uint32_t to = cells + 8u * (((len + 1 + half) & 3) * cs + id);
+                if (NC > 1) {
+#pragma unroll 1
+                    for (int i = q >> 1; i < NC; i += G / 2) dsm_store_async(dsm_map_to_cta(to, i), best, dsm_map_to_cta(bar, i));
+                } else if (q < 2) {
+                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(to), "f"(best) : "memory");
+                }
+            }
+            if (!zero) {  // which term it was, while the value is on its way
+                int at = far == best ? far_at : INT_MAX;
+#pragma unroll
+                for (int k = HELD / U - 1; k >= 0; k--) {
+                    if (k * U < trips) {
+#pragma unroll
+                        for (int j = U - 1; j >= 0; j--) {
+                            const int i = k * U + j;
+                            at = held[i].x == best ? 2 * i : held[i].y == best ? 2 * i + 1 : at;
+                        }
+                    }
+                }
+                if (at != INT_MAX) key = (prio << 24) | ((id + q + G * (at >> 1)) << 1) | (at & 1);
+#pragma unroll
+                for (int o = G / 2; o > 0; o >>= 1) key = min(key, __shfl_xor_sync(0xffffffffu, key, o));
+            }
+            if (live && q == 0) {
+                own_v[r * Q + len] = best;
+                own_k[r * Q + len] = (uint16_t)key;
+            }
+        }
+        // one warp waits for the column on the byte-counting barrier, the block barrier releases the others
+        if (NC > 1 && warp == warps - 1) arrived = dsm_wait_column(bar, ((len - 2) >> 1) & 1) && arrived;
+        __syncthreads();
+    }
+    return arrived;
+}
 
 __global__ void __launch_bounds__(kVitThreads, 1)
     viterbi_cluster_kernel(const float *__restrict__ ob_lprob, const float *__restrict__ links,
                            const int64_t *__restrict__ ol, int L, float *S, int64_t *R, int64_t *Lt, int64_t *Mt,
-                           int *status, int Mc, int cs, int rows_cap, int lk_stride, bool tight, int B, int wide) {
+                           int *status, int Mc, int cs, int rows_cap, int pitch, int B, int wide) {
     extern __shared__ float smem[];
     cg::cluster_group cluster = cg::this_cluster();
     int crank = (int)cluster.block_rank();  // below: the rank among the CTAs that work on this sentence
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, threads = blockDim.x, warps = threads >> 5;
     // wide < 0: every sentence gets the whole cluster.  wide >= 0 (more sentences than half the SMs; clusters of
     // two): the sentences are taken in order of decreasing graph length, the `wide` longest get a cluster each and
     // the others share clusters, one CTA per sentence, so that the grid is one CTA per SM and every sentence
@@ -163,7 +264,7 @@ __global__ void __launch_bounds__(kVitThreads, 1)
             NC = 1;
             crank = 0;
         }
-        for (int i = tid; i < B; i += kVitThreads) {
+        for (int i = tid; i < B; i += threads) {
             const long long mi = ol[i], ci = (mi >= 2 && mi <= L) ? mi : 0;
             int before = 0;
             for (int j = 0; j < B; j++) {
@@ -175,7 +276,7 @@ __global__ void __launch_bounds__(kVitThreads, 1)
         __syncthreads();
         b = s_b;
     }
-    const int ctid = crank * kVitThreads + tid, cthreads = NC * kVitThreads;  // thread index inside the cluster
+    const int ctid = crank * threads + tid, cthreads = NC * threads;  // thread index inside the cluster
     const int Q = L / 4;
     const int m = (int)ol[b];
     const float *ob = ob_lprob + (size_t)b * L;
@@ -194,100 +295,58 @@ __global__ void __launch_bounds__(kVitThreads, 1)
     }
     const int Mb = main_nodes_below(m);
     const int my_rows = Mb > crank ? (Mb - crank + NC - 1) / NC : 0;  // nodes id = crank + NC * r
-    float *col = smem;                // [4][cs] rolling S columns of the whole chain (replicated per CTA)
-    float *lk0 = col + 4 * cs;        // [rows_cap][lk_stride] links[a][0][c] + 0 of this CTA's nodes, by child slot
-    float *lk1 = lk0 + (size_t)rows_cap * lk_stride;  // links[a][1][c] + ob[a-1]
+    // column len: (S[len - 1], S[len - 2]) of the whole chain, replicated per CTA
+    float2 *col = reinterpret_cast<float2 *>(smem);  // [4][cs]
+    float2 *lk = col + 4 * cs;  // [rows_cap][pitch] (links[a][0][c] + 0, links[a][1][c] + ob[a-1]) of this CTA's nodes, by child slot
     // results of this CTA's nodes, flushed to global memory after the last length: a global store inside
     // the loop would make every cluster barrier (a release) wait for it to reach L2
-    float *own_v = lk1 + (size_t)rows_cap * lk_stride;       // [rows_cap][Q]
-    int *own_k = reinterpret_cast<int *>(own_v + (size_t)rows_cap * Q);  // [rows_cap][Q]
-    float *s_oa = reinterpret_cast<float *>(own_k + (size_t)rows_cap * Q);  // [rows_cap] ob of this CTA's nodes
+    float *own_v = reinterpret_cast<float *>(lk + (size_t)rows_cap * pitch + cs - Mc);  // [rows_cap][Q]
+    float *s_oa = own_v + (size_t)rows_cap * Q;                        // [rows_cap] ob of this CTA's nodes
+    uint16_t *own_k = reinterpret_cast<uint16_t *>(s_oa + rows_cap);  // [rows_cap][Q] child slot and kind, (c << 1) | j
 
-    for (int r = warp; r < my_rows; r += kVitWarps) {
+    for (int r = warp; r < my_rows; r += warps) {
         const int id = crank + NC * r;
         const float *row = lkb + (size_t)(2 * id + 1) * 2 * L;
         const float olf = id >= 1 ? __ldg(ob + 2 * id) : neg_inf();  // C[a-1][1] = ob[a-1] (pcfg_viterbi.cu:203-205)
         if (lane == 0) s_oa[r] = __ldg(ob + 2 * id + 1);
 #pragma unroll 4
-        for (int ci = id + lane; ci < lk_stride; ci += 32) {
-            lk0[r * lk_stride + ci] = ci < Mb ? __ldg(row + 2 * ci + 1) + 0.f : neg_inf();
-            lk1[r * lk_stride + ci] = ci < Mb ? __ldg(row + L + 2 * ci + 1) + olf : neg_inf();
-        }
+        for (int ci = id + lane; ci < pitch; ci += 32)
+            lk[r * pitch + ci] = make_float2(ci < Mb ? __ldg(row + 2 * ci + 1) + 0.f : neg_inf(),
+                                             ci < Mb ? __ldg(row + L + 2 * ci + 1) + olf : neg_inf());
     }
     __shared__ __align__(8) uint64_t col_bar[2];
-    __shared__ int s_timeout;
-    for (int i = tid; i < 4 * cs; i += kVitThreads) col[i] = neg_inf();  // lengths 0 and 1; slots >= Mb for good
+    for (int i = tid; i < 4 * cs; i += threads) col[i] = make_float2(neg_inf(), neg_inf());  // slots >= Mb for good
     if (tid == 0) {
-        s_timeout = 0;
         for (int i = 0; i < 2; i++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(dsm_smem_u32(&col_bar[i])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     // S[m-1][1] = ob[m-1] (pcfg_viterbi.cu:58); it feeds the recurrence only if m-1 is a main-chain node
-    if (tid == 0 && ((m - 1) & 1)) col[1 * cs + (m - 2) / 2] = __ldg(ob + (m - 1));  // every CTA fills its own copy
+    if (tid == 0 && ((m - 1) & 1))  // every CTA fills its own copy
+        col[2 * cs + (m - 2) / 2].x = col[3 * cs + (m - 2) / 2].y = __ldg(ob + (m - 1));
     // all copies initialised before anybody stores into a neighbour's; also orders the initial fill of the
     // global tables (done by threads of any CTA of the cluster) before the cells written below
     if (NC > 1) cluster.sync(); else __syncthreads();
     if (ctid == 0) Sb[(size_t)(m - 1) * Q + 1] = __ldg(ob + (m - 1));
 
-    // G lanes share a node, as few as still let half the warps take all of this CTA's nodes in one pass: a length is a chain
-    // of the scan, the arg-max and the exchange, and a node's fixed costs are paid per warp (58 lengths, 60 nodes per CTA: 83 us with 16
-    // warps and G = 8, 100 us with 32 and G = 16, 86 us with 8 and G = 4; a second pass costs more than either).  Lane
-    // q < NC of a group also sends the result to CTA q
-    int G = 32;
-    while (((32 / G) * kVitActive < my_rows || (!tight && Mb + viterbi_overshoot(G, NC) > lk_stride)) && (G >> 1) >= 4 && (G >> 1) >= NC) G >>= 1;
-    const int RW = 32 / G, q = lane % G, sub = lane / G;  // RW nodes per warp
-    const uint32_t rcol = NC > 1 && q < NC ? dsm_map_to_cta(dsm_smem_u32(col), q) : 0;  // this CTA's columns as CTA q maps them
-    const uint32_t rbar0 = NC > 1 && q < NC ? dsm_map_to_cta(dsm_smem_u32(&col_bar[0]), q) : 0;
-    const uint32_t rbar1 = NC > 1 && q < NC ? dsm_map_to_cta(dsm_smem_u32(&col_bar[1]), q) : 0;
     const int n_len = m / 4;
-    for (int len = 2; len < n_len; len++) {
-        const float *S1 = col + ((len - 1) & 3) * cs;
-        const float *S2 = col + ((len - 2) & 3) * cs;
-        float *S0 = col + (len & 3) * cs;
-        const uint32_t bar = dsm_smem_u32(&col_bar[len & 1]);
-        if (NC > 1 && tid == 0)  // this CTA expects the whole column of this length: one value per node of the chain
-            asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(4 * Mb)
-                         : "memory");
-        for (int r0w = warp * RW; r0w < my_rows; r0w += kVitWarps * RW) {
-            const int r = r0w + sub;
-            const bool live = r < my_rows;
-            const int rr = live ? r : r0w, id = crank + NC * rr;
-            // those of the warp's first node, which has most children; in rows without padding every lane's own
-            const int trips = (Mb - (tight ? id + q : crank + NC * r0w) + G - 1) / G;
-            const float *r0 = lk0 + rr * lk_stride + id + q, *r1 = lk1 + rr * lk_stride + id + q;
-            float best;
-            int key;
-            viterbi_node_group(id, trips, q, G, s_oa[rr], r0, r1, S1 + id + q, S2 + id + q, best, key);
-            if (live) {
-                if (NC > 1) {  // into every CTA's column, counted on that CTA's barrier of this length
-                    if (q < NC) dsm_store_async(rcol + 4u * ((len & 3) * cs + id), best, (len & 1) ? rbar1 : rbar0);
-                } else if (q == 0) {
-                    S0[id] = best;
-                }
-                if (q == 0) {
-                    own_v[r * Q + len] = best;
-                    own_k[r * Q + len] = key;
-                }
-            }
-        }
-        // one warp waits for the column on the byte-counting barrier, the block barrier releases the others: 32 warps
-        // polling the same barrier get in each other's way
-        if (NC > 1 && warp == kVitWarps - 1 && !dsm_wait_column(bar, ((len - 2) >> 1) & 1)) s_timeout = 1;
-        __syncthreads();
-    }
-    if (s_timeout && tid == 0) flag(status, PCFGNAT_STATUS_TIMEOUT);
+    const int G = viterbi_lanes(my_rows, warps);  // no fewer than the launch made room for
+#define PCFGNAT_VITERBI_CASE(G_) \
+    viterbi_lengths<G_>(col, lk, s_oa, own_v, own_k, col_bar, n_len, Mb, my_rows, NC, crank, Q, cs, pitch)
+    const bool arrived = G == 4 ? PCFGNAT_VITERBI_CASE(4) : G == 8 ? PCFGNAT_VITERBI_CASE(8) : PCFGNAT_VITERBI_CASE(16);
+#undef PCFGNAT_VITERBI_CASE
+    if (!arrived && lane == 0) flag(status, PCFGNAT_STATUS_TIMEOUT);
     // no CTA leaves (its shared memory with it) while a peer may still send to it: the last column has arrived
     // everywhere once every CTA has passed its last wait
     if (NC > 1) cluster.sync();
-    for (int i = tid; i < my_rows * (n_len - 2); i += kVitThreads) {  // computed cells: lengths 2 .. n_len-1
+    for (int i = tid; i < my_rows * (n_len - 2); i += threads) {  // computed cells: lengths 2 .. n_len-1
         const int r = i / (n_len - 2), len = 2 + i - r * (n_len - 2);
         viterbi_store(own_v[r * Q + len], own_k[r * Q + len], 2 * (crank + NC * r) + 1, Q, len, Sb, Rb, Lb, Mtb);
     }
 }
 
-__global__ void __launch_bounds__(kVitThreads)
+__global__ void __launch_bounds__(1024)
     viterbi_global_kernel(const float *__restrict__ ob_lprob, const float *__restrict__ links,
                           const int64_t *__restrict__ ol, int L, float *S, int64_t *R, int64_t *Lt, int64_t *Mt,
                           int *status, int Mc, int cs) {
@@ -491,24 +550,27 @@ int launch_trace(const float *S, const float *penalty, int64_t *pred_out, const 
 
 // How a CTA of n that share a sentence lays out its nodes' rows; smem 0: they do not fit.
 struct VitRows {
-    int cap, stride;
-    bool tight;
+    int cap, stride, cs;
     size_t smem;
 };
 
-static VitRows viterbi_rows(int Mc, int Q, int cs, int n, int width) {
+// Warps of a block; with more CTAs than SMs no more than the nodes need, so that CTAs share SMs: 1000 sentences of 16 nodes
+// 49 -> 24 us, 300 of 64 105 -> 78.
+static int viterbi_warps(int rows, bool crowded) {
+    const int least = (rows + 31) / 32 * 4;
+    return crowded && least < kVitThreads / 32 ? least : kVitThreads / 32;
+}
+
+static VitRows viterbi_rows(int Mc, int Q, int n, int width, bool crowded) {
     VitRows r;
     r.cap = (Mc + n - 1) / n;  // also right for mixed widths: n is 1 there, every CTA may hold a chain
-    // rows long enough for the lanes a full chain takes (shorter ones take more where they fit), and with the rows of a
-    // warp's nodes in different banks where there is room for that
-    int G = 32;
-    while ((32 / G) * kVitActive < r.cap && (G >> 1) >= 4 && (G >> 1) >= width) G >>= 1;
-    const int least = Mc + viterbi_overshoot(G, width);
-    const int strides[3] = {(least + width - G % 32 + 31) / 32 * 32 + G % 32 - width, least | 1, (Mc + 31) / 32 * 32 + 1};
-    for (int i = 0; i < 3; i++) {  // the last without room for what lanes read past the chain: there they stop at its end
-        r.stride = strides[i];
-        r.tight = i == 2;
-        r.smem = ((size_t)4 * cs + (size_t)2 * r.cap * r.stride + (size_t)2 * r.cap * Q + r.cap) * sizeof(float);
+    const int G = viterbi_lanes(r.cap, viterbi_warps(r.cap, crowded));
+    r.cs = Mc + viterbi_overshoot(G, width);
+    for (int banks = 1; banks >= 0; banks--) {  // the rows that a half-warp reads in different banks where there is room for that
+        r.stride = Mc;
+        while (banks && G < 16 && (r.stride + n) % 16 != G) r.stride++;
+        r.smem = ((size_t)4 * r.cs + (size_t)r.cap * r.stride + r.cs - Mc) * sizeof(float2) +
+                 (size_t)r.cap * ((Q + 1) * sizeof(float) + Q * sizeof(uint16_t));
         if (r.smem <= (size_t)kSmemLimit - 1024) return r;
     }
     r.smem = 0;
@@ -540,11 +602,11 @@ int launch_viterbi(const float *ob, const float *links, const int64_t *ol, int B
     // mixed widths only while one CTA holds a chain; a grid larger than the GPU takes the sentences by
     // decreasing length (wide = B), so that the clusters that wait for a place get the shortest
     const auto mixed = [&](int n) { return wide >= 0 && n == 1; };
+    const auto crowded = [&](int n) { return !mixed(n) && (long long)B * n > sms; };
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(kVitThreads);
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
@@ -553,6 +615,7 @@ int launch_viterbi(const float *ob, const float *links, const int64_t *ol, int B
         const int launch_nc = mixed(n) ? 2 : n;
         cfg.gridDim = dim3((unsigned)((mixed(n) ? wide + (B - wide + 1) / 2 : B) * launch_nc));
         cfg.dynamicSmemBytes = rows.smem;
+        cfg.blockDim = dim3(32 * viterbi_warps(rows.cap, crowded(n)));
         attr[0].val.clusterDim.x = (unsigned)launch_nc;
         int clusters = 0;
         if (ensure_dynamic_smem(viterbi_cluster_kernel, rows.smem) != cudaSuccess ||
@@ -563,32 +626,24 @@ int launch_viterbi(const float *ob, const float *links, const int64_t *ol, int B
         }
         return clusters;
     };
+    // Sixteen CTAs where a chain is long and all sentences still run at once: one sentence of 257 nodes 175 -> 156 us, five of
+    // 380 348 -> 281, but nine of 300, for whose clusters there is no room, 226 -> 352.
+    if (nc == 8 && Mc > 256) {
+        const VitRows rows = viterbi_rows(Mc, Q, 16, 16, crowded(16));
+        if (rows.smem && configure(16, rows) >= B) nc = 16;
+    }
     for (; nc <= 16; nc *= 2) {
-        VitRows rows = viterbi_rows(Mc, Q, cs, nc, mixed(nc) ? 2 : nc);
+        const VitRows rows = viterbi_rows(Mc, Q, nc, mixed(nc) ? 2 : nc, crowded(nc));
         if (rows.smem == 0) continue;
-        int clusters = configure(nc, rows);
-        if (clusters < 1) continue;  // this cluster size cannot be scheduled here: try the next one
-        if (rows.tight && nc < 16) {
-            // Twice the CTAs have room for the padding and take two thirds of the time per wave: graph 380, two CTAs 230,
-            // four 145 us; 532, four and eight: 338 and 221; 760, eight and sixteen: 444 and 302.  64 sentences of 380 are
-            // one wave of two (231 us) or two of four (289), 90 are two (457) or three (430), 32 of 532 one (338) or three (654).
-            const VitRows more_rows = viterbi_rows(Mc, Q, cs, 2 * nc, 2 * nc);
-            const int more = more_rows.smem ? configure(2 * nc, more_rows) : 0;
-            if (more > 0 && 2 * ((B + more - 1) / more) <= 3 * ((B + clusters - 1) / clusters)) {
-                nc *= 2;
-                rows = more_rows;
-            } else {
-                configure(nc, rows);
-            }
-        }
-        const int order = mixed(nc) ? wide : ((long long)B * nc > sms && B <= 256 ? B : -1);
-        return cuda_rc(cudaLaunchKernelEx(&cfg, viterbi_cluster_kernel, ob, links, ol, L, S, R, Lt, Mt, status, Mc, cs, rows.cap,
-                                          rows.stride, rows.tight, B, order));
+        if (configure(nc, rows) < 1) continue;  // this cluster size cannot be scheduled here: try the next one
+        const int order = mixed(nc) ? wide : (crowded(nc) && B <= 256 ? B : -1);
+        return cuda_rc(cudaLaunchKernelEx(&cfg, viterbi_cluster_kernel, ob, links, ol, L, S, R, Lt, Mt, status, Mc, rows.cs, rows.cap,
+                                          rows.stride, B, order));
     }
     const size_t smem_cols = (size_t)3 * cs * sizeof(float);
     if (smem_cols > (size_t)kSmemLimit - 1024) return PCFGNAT_ERR_TOO_LARGE;
     if (ensure_dynamic_smem(viterbi_global_kernel, smem_cols) != cudaSuccess) return PCFGNAT_ERR_CUDA;
-    const int warps = Mc < 4 ? 4 : (Mc > kVitWarps ? kVitWarps : Mc);
+    const int warps = Mc < 4 ? 4 : (Mc > 32 ? 32 : Mc);
     viterbi_global_kernel<<<B, 32 * warps, smem_cols, st>>>(ob, links, ol, L, S, R, Lt, Mt, status, Mc, cs);
     return cuda_rc(cudaGetLastError());
 }

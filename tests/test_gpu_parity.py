@@ -292,6 +292,31 @@ def test_viterbi_table_and_trace_edges(ops, syn, monkeypatch, B, L):
     assert ops.read_status(DEV) == 0
 
 
+@pytest.mark.parametrize("B, L", [(2, 36), (9, 514), (9, 600), (40, 98), (70, 150), (260, 70), (600, 34)])
+def test_viterbi_signed_zeros_and_crowded_grids(ops, monkeypatch, B, L):
+    """Values that compare equal but differ in their bits (-0 and +0, of which the first in the reference's order is kept), few
+    distinct values, chains beyond the terms held in registers and grids larger than the GPU: tables bit for bit those of the
+    kernel that reads the transitions from global memory."""
+    monkeypatch.delenv("PCFGNAT_DP_KERNEL", raising=False)
+    monkeypatch.delenv("PCFGNAT_DP_CLUSTER_SIZE", raising=False)
+    g = torch.Generator(DEV).manual_seed(L + B)
+    signed = lambda *shape: torch.randint(0, 2, shape, device=DEV, generator=g).float() * -0.0  # noqa: E731
+    ob, links = signed(B, L), signed(B, L, 2, L)
+    ob = torch.where(torch.rand(B, L, device=DEV, generator=g) < 0.3, -0.25, ob)
+    links = torch.where(torch.rand(B, L, 2, L, device=DEV, generator=g) < 0.5, -0.5, links)
+    at = torch.arange(L, device=DEV)
+    links.masked_fill_((at[None, :] <= at[:, None])[None, :, None, :], float("-inf"))
+    ol = torch.randint(max(2, L // 2), L + 1, (B,), device=DEV, generator=g)
+    ol[0] = L
+    k = ops.get_pcfg_kernel()
+    got = k.pcfg_viterbi(ob, links, ol, 1)
+    monkeypatch.setenv("PCFGNAT_DP_KERNEL", "rows")
+    want = k.pcfg_viterbi(ob, links, ol, 1)
+    assert np.array_equal(_bits(got[0].cpu().numpy()), _bits(want[0].cpu().numpy()))
+    assert all(torch.equal(x, y) for x, y in zip(got[1:], want[1:])) and bool((got[0] == 0).any())
+    assert ops.read_status(DEV) == 0
+
+
 @pytest.mark.parametrize("name", ["ref_viterbi_ragged.npz", "ref_viterbi_mid.npz"])
 def test_viterbi_against_reference_golden(vit_kernel, ops, name):
     g = _g(name)
