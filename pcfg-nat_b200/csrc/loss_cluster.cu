@@ -426,8 +426,9 @@ __global__ void __launch_bounds__(kCThreads, 1)
 // Bound by the latency of a step on the longest row (57 % of the issue slots with eight lanes; the exponentials, expf for the
 // bits, are half of the instructions).  With the exponentials handed over through shared memory and 1024 threads before
 // (sixteen or eight lanes, a pass per 64 or 128 nodes), and a warp per node below 32 nodes: 64 sentences, M = 128, T = 76: 191
-// -> 131 us; 90 sentences, M <= 80: 84 -> 70; 16 sentences, M = 128 on eight CTAs each 213 -> 105; 160 sentences, M <= 80 (the
-// row-per-thread kernel of loss_fwd.cu before) 189 -> 79.  Terms formed twice for all children: 137 us for the first of these.
+// -> 123 us; 90 sentences, M <= 80: 84 -> 64; 16 sentences, M = 128 on eight CTAs each 213 -> 96; 160 sentences, M <= 80 (the
+// row-per-thread kernel of loss_fwd.cu before) 189 -> 75.  For the first of these: terms formed twice for all children 137 us, a
+// test of its own for each block of children behind the row's end, instead of one way out, 131.
 constexpr int kExactThreads = 512;
 
 template <int G>
@@ -479,12 +480,11 @@ __device__ __forceinline__ bool inside_exact_steps(float2 *col, const float2 *lk
             float2 held[HELD];
 #pragma unroll
             for (int k = 0; k < HELD / U; k++) {
-                if (k * U < trips) {
+                if (k * U >= trips) break;
 #pragma unroll
-                    for (int j = 0; j < U; j++) held[k * U + j] = terms(k * U + j);
+                for (int j = 0; j < U; j++) held[k * U + j] = terms(k * U + j);
 #pragma unroll
-                    for (int j = 0; j < U; j++) mx = fmaxf(mx, fmaxf(held[k * U + j].x, held[k * U + j].y));
-                }
+                for (int j = 0; j < U; j++) mx = fmaxf(mx, fmaxf(held[k * U + j].x, held[k * U + j].y));
             }
 #pragma unroll 1
             for (int i = HELD; i < trips; i += U) {
@@ -523,8 +523,10 @@ __device__ __forceinline__ bool inside_exact_steps(float2 *col, const float2 *lk
                 sum = 0.f;
                 if (!clean) {
 #pragma unroll
-                    for (int k = 0; k < HELD / U; k++)
-                        if (k * U < trips) add_block(held + k * U, clean);
+                    for (int k = 0; k < HELD / U; k++) {
+                        if (k * U >= trips) break;
+                        add_block(held + k * U, clean);
+                    }
                 }
 #pragma unroll 1
                 for (int i = clean ? 0 : HELD; i < trips; i += U) {
