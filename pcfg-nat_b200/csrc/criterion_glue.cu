@@ -150,13 +150,19 @@ __global__ void loss_stats_exchange_kernel(const float *__restrict__ loss, const
 //   glat_prev[l] = keep[l] ? oracle[l] : prev[l]
 // For the two counting strategies the reference then draws rand < keep_prob with keep_prob in {0, 1}: the same
 // mask, so no second draw.
-__global__ void glance_select_kernel(const int64_t *__restrict__ path, const int64_t *__restrict__ pred,
-                                     const int64_t *__restrict__ tgt, const int64_t *__restrict__ prev,
-                                     const int64_t *__restrict__ tl, const float *__restrict__ noise,
-                                     const float *__restrict__ uniform, int strategy, float context_p, int L, int T,
-                                     uint8_t *matchmask, int64_t *oracle, int64_t *same_num, int64_t *glance_num,
-                                     uint8_t *keep, int64_t *glat_prev) {
+//
+// Bound by latency, one sentence per block.  The T x L match mask is most of what is written: a warp takes a row at a time, from a
+// copy of the alignment in shared memory and in words of four cells where the rows allow it (a division and a read of the
+// alignment per cell, 256 threads and one thread per node's rank before: 12.0 -> 7.0 us for 64 sentences, L = 256, T = 76).
+constexpr int kSelectThreads = 1024;
+__global__ void __launch_bounds__(kSelectThreads)
+    glance_select_kernel(const int64_t *__restrict__ path, const int64_t *__restrict__ pred, const int64_t *__restrict__ tgt, const
+                         int64_t *__restrict__ prev, const int64_t *__restrict__ tl, const float *__restrict__ noise, const float
+                         *__restrict__ uniform, int strategy, float context_p, int L, int T, int staged, uint8_t *matchmask, int64_t
+                         *oracle, int64_t *same_num, int64_t *glance_num, uint8_t *keep, int64_t *glat_prev) {
     extern __shared__ float sm_noise[];  // [L]
+    // [L] target position of a node, -1: none (staged == 0: no room, graphs of more than 28 000 nodes)
+    int *aligned_to = reinterpret_cast<int *>(sm_noise + L);
     __shared__ float scratch[32];
     const int b = blockIdx.x;
     const int64_t *pb = path + (size_t)b * L;
@@ -165,17 +171,31 @@ __global__ void glance_select_kernel(const int64_t *__restrict__ path, const int
         const int64_t raw = pb[l];
         const bool aligned = raw >= 0;
         const int p = (raw >= 0 && raw < T) ? (int)raw : -1;
+        if (staged) aligned_to[l] = p;
         const int64_t o = tgt[(size_t)b * T + (p < 0 ? 0 : p)];
         oracle[(size_t)b * L + l] = o;
         if (aligned && pred[(size_t)b * L + l] == o) same += 1.f;
         if (strategy == PCFGNAT_GLANCE_FRACTION) sm_noise[l] = aligned ? 1.f : 0.f;
         else sm_noise[l] = aligned ? noise[(size_t)b * L + l] : -100.f;
     }
-    for (int i = threadIdx.x; i < T * L; i += blockDim.x) {
-        const int t = i / L, l = i - t * L;
-        matchmask[(size_t)b * T * L + i] = pb[l] == t;
+    same = block_sum(same, scratch);  // exact: a count below 2^24; its barriers also publish sm_noise and aligned_to
+    auto hit = [&](int l, int t) { return staged ? aligned_to[l] == t : pb[l] == t; };
+    const bool words = (L & 3) == 0 && (reinterpret_cast<uintptr_t>(matchmask) & 3) == 0;
+    for (int t = threadIdx.x >> 5; t < T; t += kSelectThreads / 32) {
+        uint8_t *row = matchmask + ((size_t)b * T + t) * L;
+        if (words) {
+            for (int l = 4 * (threadIdx.x & 31); l < L; l += 128) {
+                uchar4 v;
+                v.x = hit(l, t);
+                v.y = hit(l + 1, t);
+                v.z = hit(l + 2, t);
+                v.w = hit(l + 3, t);
+                *reinterpret_cast<uchar4 *>(row + l) = v;
+            }
+        } else {
+            for (int l = threadIdx.x & 31; l < L; l += 32) row[l] = hit(l, t);
+        }
     }
-    same = block_sum(same, scratch);  // exact: a count below 2^24; its barriers also publish sm_noise
     const int64_t n = tl[b];
     const int64_t same_i = (int64_t)same;
     if (strategy == PCFGNAT_GLANCE_FRACTION) {
@@ -200,10 +220,14 @@ __global__ void glance_select_kernel(const int64_t *__restrict__ path, const int
         same_num[b] = same_i;
         glance_num[b] = k;
     }
-    for (int l = threadIdx.x; l < L; l += blockDim.x) {
-        const float mine = sm_noise[l];
+    for (int l0 = 0; l0 < L; l0 += kSelectThreads / 4) {  // four lanes per node
+        const int l = l0 + threadIdx.x / 4;
+        const float mine = sm_noise[l < L ? l : 0];
         int larger = 0;
-        for (int j = 0; j < L; j++) larger += sm_noise[j] > mine;
+        for (int j = threadIdx.x & 3; j < L; j += 4) larger += sm_noise[j] > mine;
+        larger += __shfl_xor_sync(0xffffffffu, larger, 1);
+        larger += __shfl_xor_sync(0xffffffffu, larger, 2);
+        if (l >= L || (threadIdx.x & 3)) continue;
         const bool kp = k != 0 && larger < (k < 1 ? 1 : k);  // a negative k indexes the sorted list at 0, as torch's clip does
         keep[(size_t)b * L + l] = kp;
         glat_prev[(size_t)b * L + l] = kp ? oracle[(size_t)b * L + l] : prev[(size_t)b * L + l];
@@ -249,10 +273,11 @@ int launch_glance_select(const int64_t *path, const int64_t *pred, const int64_t
                          int B, int L, int T, uint8_t *matchmask, int64_t *oracle, int64_t *same_num,
                          int64_t *glance_num, uint8_t *keep, int64_t *glat_prev, cudaStream_t st) {
     if (B == 0) return PCFGNAT_OK;
-    const size_t smem = (size_t)L * sizeof(float);
+    const int staged = (size_t)L * (sizeof(float) + sizeof(int)) <= (size_t)kSmemLimit - 1024;
+    const size_t smem = (size_t)L * (staged ? sizeof(float) + sizeof(int) : sizeof(float));
     if (smem > 48 * 1024 && ensure_dynamic_smem(glance_select_kernel, smem) != cudaSuccess) return PCFGNAT_ERR_TOO_LARGE;
-    glance_select_kernel<<<B, 256, smem, st>>>(path, pred, tgt, prev, tl, noise, uniform, strategy, context_p, L, T,
-                                               matchmask, oracle, same_num, glance_num, keep, glat_prev);
+    glance_select_kernel<<<B, kSelectThreads, smem, st>>>(path, pred, tgt, prev, tl, noise, uniform, strategy, context_p, L, T,
+                                                          staged, matchmask, oracle, same_num, glance_num, keep, glat_prev);
     return cuda_rc(cudaGetLastError());
 }
 

@@ -1349,6 +1349,28 @@ def test_loss_stats_and_glance_select(ops):
             assert torch.equal(got[key].cpu(), val), (key, B, L, T)
 
 
+@pytest.mark.parametrize("B, L, T", [(1, 2, 1), (3, 41, 12), (2, 255, 33), (2, 256, 31), (4, 130, 64), (2, 1030, 40), (1, 29500, 3)])
+@pytest.mark.parametrize("strategy", ["number-random", "cmlm", None])
+def test_glance_select_sizes(ops, B, L, T, strategy):
+    """Rows of the match mask in words and in bytes, more nodes than threads, and graphs whose alignment has no room in shared
+    memory: every output against the torch restatement (positions past the target and ties included)."""
+    g = torch.Generator().manual_seed(L)
+    tlen = torch.randint(1, T + 1, (B,), generator=g)
+    path = torch.randint(-1, T + 2, (B, L), generator=g)
+    path[torch.rand(B, L, generator=g) < 0.4] = -1
+    tgt, pred = torch.randint(4, 9, (B, T), generator=g), torch.randint(4, 9, (B, L), generator=g)
+    prev = torch.randint(1, 4, (B, L), generator=g)
+    noise = torch.randn(B, L, generator=g)
+    noise[:, ::3] = noise[:, :1].clone()
+    uniform = torch.rand((B, L) if strategy is None else (B,), generator=g)
+    k = ops.get_pcfg_kernel()
+    d = lambda t: t.to(DEV)  # noqa: E731
+    got = k.glance_select(d(path), d(pred), d(tgt), d(prev), d(tlen), d(noise), 0.5, strategy, d(uniform))
+    want = pyref.glance_select(path, pred, tgt, prev, tlen, noise, 0.5, strategy, uniform)
+    for key, val in want.items():
+        assert torch.equal(got[key].cpu(), val), key
+
+
 @pytest.mark.parametrize("case", ["small", "mid"])
 def test_extract_links_against_reference_model(ops, case):
     """links from the projected link features against the reference model's own extract_links (run on the CPU
