@@ -227,7 +227,8 @@ int pcfgnat_proj_dlogits_compact(const void *hidden, const void *weight, const i
                                  void *stream);
 
 /* Both of the above (compact when row_index is given) with rows `pitch` elements apart, a multiple of 8 and at least V: an odd V
- * then costs no more than an even one.  Cells between V and pitch are undefined. */
+ * then costs no more than an even one.  Cells between V and pitch are undefined.  capacity: rows that dlogits holds; without
+ * row_index all B * L of them are written, and fewer are refused. */
 int pcfgnat_proj_dlogits_pitched(const void *hidden, const void *weight, const int64_t *targets, const int64_t *output_length,
                                  const int64_t *target_length, const float *lse, const float *grad_match, int B, int L, int T,
                                  int V, int H, int capacity, void *dlogits, int pitch, int64_t *row_index, int *n_rows,

@@ -554,6 +554,7 @@ int pcfgnat_proj_dlogits_pitched(const void *hidden, const void *weight, const i
     if ((long long)B * L > (1ll << 30)) return PCFGNAT_ERR_TOO_LARGE;
     if (B && (!hidden || !weight || !targets || !lse || !grad_match || !workspace)) return PCFGNAT_ERR_INVALID_ARGUMENT;
     if (B && !dlogits && (capacity || !row_index)) return PCFGNAT_ERR_INVALID_ARGUMENT;
+    if (!row_index && capacity < (long long)B * L) return PCFGNAT_ERR_INVALID_ARGUMENT;  // padded order writes every row
     if (target_length != nullptr && output_length == nullptr) return PCFGNAT_ERR_INVALID_ARGUMENT;
     return launch_proj_dlogits(hidden, weight, targets, output_length, target_length, lse, grad_match, B, L, T, V, H, dlogits,
                                pitch, workspace, workspace_bytes, status, static_cast<cudaStream_t>(stream), capacity, row_index,

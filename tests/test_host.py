@@ -37,6 +37,18 @@ def test_library_exports_every_declared_symbol(pkg):
     assert l.pcfgnat_loss_fwd_bwd(1, 1, 1, 1, 1, 32, 10, 1, 1, 8, 1, 1, 1, None, None) == -4
 
 
+@pytest.mark.parametrize("capacity, row_index, rc", [(23, None, -1), (0, None, -1), (24, None, -4), (0, 16, -4)])
+def test_pitched_dlogits_in_padded_order_need_room_for_every_row(pkg, capacity, row_index, rc):
+    """Without row_index the 3 x 8 rows are all written: a smaller buffer is refused (-1).  What passes is stopped by a workspace
+    of no bytes (-4), before any CUDA call."""
+    import importlib
+
+    l = importlib.import_module("pcfg_nat_b200._cabi").lib()
+    at = 16
+    assert l.pcfgnat_proj_dlogits_pitched(at, at, at, None, None, at, at, 3, 8, 4, 33, 64, capacity, at, 40, row_index, None, at, 0,
+                                          None, None) == rc
+
+
 @pytest.mark.skipif(torch.cuda.is_available(), reason="checks the no-GPU behaviour")
 def test_operators_refuse_to_run_without_cuda(ops):
     with pytest.raises(RuntimeError, match="You need GPU"):
