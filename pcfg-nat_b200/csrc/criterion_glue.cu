@@ -275,7 +275,8 @@ int launch_glance_select(const int64_t *path, const int64_t *pred, const int64_t
     if (B == 0) return PCFGNAT_OK;
     const int staged = (size_t)L * (sizeof(float) + sizeof(int)) <= (size_t)kSmemLimit - 1024;
     const size_t smem = (size_t)L * (staged ? sizeof(float) + sizeof(int) : sizeof(float));
-    if (smem > 48 * 1024 && ensure_dynamic_smem(glance_select_kernel, smem) != cudaSuccess) return PCFGNAT_ERR_TOO_LARGE;
+    // what a launch may ask for without opting in is 48 KB with the kernel's own 128 bytes (6 129 to 6 144 nodes are between)
+    if (smem > 47 * 1024 && ensure_dynamic_smem(glance_select_kernel, smem) != cudaSuccess) return PCFGNAT_ERR_TOO_LARGE;
     glance_select_kernel<<<B, kSelectThreads, smem, st>>>(path, pred, tgt, prev, tl, noise, uniform, strategy, context_p, L, T,
                                                           staged, matchmask, oracle, same_num, glance_num, keep, glat_prev);
     return cuda_rc(cudaGetLastError());

@@ -1371,6 +1371,31 @@ def test_glance_select_sizes(ops, B, L, T, strategy):
         assert torch.equal(got[key].cpu(), val), key
 
 
+def test_glance_select_just_below_48_kb_of_shared_memory():
+    """6 140 nodes ask for 49 120 bytes beside the kernel's own 128, in a process of their own: an earlier call for a longer graph
+    raises the kernel's limit for good."""
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+
+    program = """
+import sys; sys.path.insert(0, "tests")
+import torch, _pyref as pyref, __graft_entry__ as entry
+entry.load_package()
+from pcfg_nat_b200.custom_ops import pcfg_loss as ops
+B, L, T = 2, 6140, 3
+g = torch.Generator().manual_seed(1)
+args = [torch.randint(-1, T, (B, L), generator=g), torch.randint(4, 9, (B, L), generator=g), torch.randint(4, 9, (B, T), generator=g),
+        torch.ones(B, L, dtype=torch.long), torch.tensor([3, 2]), torch.randn(B, L, generator=g)]
+got = ops.get_pcfg_kernel().glance_select(*[t.cuda() for t in args], 0.5, "number-random", None)
+for key, val in pyref.glance_select(*args, 0.5, "number-random", None).items():
+    assert torch.equal(got[key].cpu(), val), key
+"""
+    r = subprocess.run([sys.executable, "-c", program], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+
+
 @pytest.mark.parametrize("case", ["small", "mid"])
 def test_extract_links_against_reference_model(ops, case):
     """links from the projected link features against the reference model's own extract_links (run on the CPU
