@@ -485,9 +485,10 @@ class _Kernel:
         with torch.cuda.device(dev):
             d_rows = torch.empty((n, H), dtype=torch.float32, device=dev) if want_rows else None
             d_weight = torch.empty((V, H), dtype=torch.float32, device=dev) if want_weight else None
-            rc = _cabi.lib().pcfgnat_proj_backward_gemms_pitched(dlogits.data_ptr(), V if dlogits.is_contiguous() else dlogits.stride(0),
-                                                                 ptr(weight_bf16), ptr(rows_bf16), n, V, H, ptr(d_rows),
-                                                                 ptr(d_weight), _status_ptr(dev), _stream(dev))
+            # (torch calls a slice of one row or none contiguous, whatever its stride)
+            pitch = dlogits.stride(0) if _rows_apart(dlogits) else V
+            rc = _cabi.lib().pcfgnat_proj_backward_gemms_pitched(dlogits.data_ptr(), pitch, ptr(weight_bf16), ptr(rows_bf16), n, V, H,
+                                                                 ptr(d_rows), ptr(d_weight), _status_ptr(dev), _stream(dev))
         _cabi.check(rc, "pcfgnat_proj_backward_gemms")
         return d_rows, d_weight
 

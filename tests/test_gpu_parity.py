@@ -1010,6 +1010,34 @@ def test_loss_step_with_projection_backward_of_an_odd_vocabulary(pkg, ops, syn):
         assert float((got - want).norm() / want.norm()) < 2e-3
 
 
+@pytest.mark.parametrize("V", [33, 513, 1001])
+def test_projection_backward_of_an_odd_vocabulary_and_one_row(pkg, ops, V):
+    """One real row, as n_rows and as the whole tensor, and a step whose batch has one real node or none; bounds of the test of
+    more rows."""
+    import importlib
+    runtime = importlib.import_module("pcfg_nat_b200.runtime")
+    B, L, H, T = 2, 6, 64, 3
+    g = torch.Generator(DEV).manual_seed(V)
+    hidden, weight = torch.randn(B, L, H, device=DEV, generator=g).half(), (torch.randn(V, H, device=DEV, generator=g) * 0.1).half()
+    targets, grad = torch.randint(0, V, (B, T), device=DEV, generator=g), torch.randn(B, L, T, device=DEV, generator=g)
+    one = torch.tensor([1, 0], device=DEV)
+    cases = [(hidden, targets, grad, one, 1), (hidden[:1, :1], targets[:1], grad[:1, :1], None, None)]
+    for hid, tgt, gr, ol, n_rows in cases:
+        h64, w64 = hid.double().requires_grad_(), weight.double().requires_grad_()
+        lp = torch.log_softmax(h64 @ w64.t(), -1).gather(2, tgt[:, None].expand(-1, hid.shape[1], -1))
+        want = torch.autograd.grad((lp * gr)[0, 0].sum(), (h64, w64))
+        h, w = hid.clone().requires_grad_(), weight.clone().requires_grad_()
+        got = torch.autograd.grad(ops.proj_logsoftmax_gather_with_grad(h, w, tgt, ol, None, n_rows=n_rows), (h, w), gr)
+        for x, y in zip(got, want):
+            assert (x.double() - y).norm() <= 1e-2 * y.norm() and (x.double() - y).abs().max() <= 3e-2 * y.abs().max()
+    step = runtime.LossStep(weight, B, L, T, DEV, use_graph=False, proj_backward=True)
+    for real in (1, 0):
+        step.load(hidden, torch.full((B, L, 2, L), float("-inf"), device=DEV), real * one, targets, torch.ones(B, dtype=torch.long, device=DEV))
+        d_hidden, d_weight = step.run()[-2:]
+        assert (d_hidden[1] == 0).all() and (d_hidden[0, real:] == 0).all() and (real or (d_weight == 0).all())
+    ops.read_status(DEV)
+
+
 @pytest.mark.parametrize("V", [1001, 1007, 2051, 16384, 16387, 33001])
 @pytest.mark.parametrize("dtype, offset, columns", [(torch.float16, 0, 20), (torch.float16, 3, 600), (torch.float32, 0, 600),
                                                     (torch.float32, 1, 20)])
