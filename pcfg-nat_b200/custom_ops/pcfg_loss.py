@@ -122,11 +122,6 @@ def _row_index_ok(index, device):
 _main_chain_cache = {}  # (address and version of the main-chain mask, prelen) -> mask, (node list, slots), their stream
 
 
-def _rows_apart(t):
-    """Whether the rows of a matrix are a multiple of 16 bytes apart in memory, as an odd vocabulary's padded d-logits are."""
-    return t.dim() == 2 and t.stride(1) == 1 and t.stride(0) >= t.shape[1] and t.stride(0) % 8 == 0
-
-
 class _Kernel:
     """Extension-level API: the functions of the reference's pybind module (pcfg_loss.cpp:75-82)."""
 
@@ -411,7 +406,7 @@ class _Kernel:
     @staticmethod
     def proj_dlogits_rows(hidden, weight, targets, output_length, target_length, lse, grad_match, n_rows=None, out=None,
                           row_index_out=None):
-        """``proj_dlogits`` for ``proj_backward_products``: (d-logits, row_index or None), the d-logits a view [n, V] of a
+        """``proj_dlogits`` for ``products_of_rows``: (d-logits, row_index or None), the d-logits a view [n, V] of a
         buffer whose rows are a multiple of 16 bytes apart, which an odd vocabulary's own rows are not.  ``out``: such a
         buffer, bfloat16 [rows, V rounded up to a multiple of 8]; ``row_index_out`` as in ``proj_dlogits``."""
         B, L, H = hidden.shape
@@ -463,19 +458,21 @@ class _Kernel:
         _require_cuda()
         if not dlogits.is_contiguous():
             raise RuntimeError("dlogits must be a contiguous bfloat16 CUDA matrix")
-        return _Kernel._proj_backward_gemms(dlogits, weight_bf16, rows_bf16, want_rows, want_weight)
+        return _Kernel._proj_backward_gemms(dlogits, dlogits.shape[1], weight_bf16, rows_bf16, want_rows, want_weight)
 
     @staticmethod
-    def _proj_backward_gemms(dlogits, weight_bf16, rows_bf16, want_rows=True, want_weight=True):
-        """The same, of d-logits whose rows may also lie further apart than they are long (``proj_dlogits_rows``)."""
+    def _proj_backward_gemms(dlogits, pitch, weight_bf16, rows_bf16, want_rows=True, want_weight=True):
+        """The same, of d-logits whose rows are ``pitch`` elements apart."""
         _require_cuda()
         dev = dlogits.device
         for t, name in ((dlogits, "dlogits"), (weight_bf16, "weight_bf16"), (rows_bf16, "rows_bf16")):
             if t is None:
                 continue
-            if not t.is_cuda or t.dtype != torch.bfloat16 or t.dim() != 2 or not (t.is_contiguous() or t is dlogits and _rows_apart(t)):
+            if not t.is_cuda or t.dtype != torch.bfloat16 or t.dim() != 2 or not (t is dlogits or t.is_contiguous()):
                 raise RuntimeError(f"{name} must be a contiguous bfloat16 CUDA matrix")
         n, V = dlogits.shape
+        if n > 1 and dlogits.stride(0) != pitch or V > 1 and dlogits.stride(1) != 1:
+            raise RuntimeError(f"the rows of dlogits must be {pitch} elements apart")
         H = (weight_bf16 if weight_bf16 is not None else rows_bf16).shape[1]
         if want_rows and (weight_bf16 is None or tuple(weight_bf16.shape) != (V, H)):
             raise RuntimeError("weight_bf16 must be [V, H]")
@@ -485,8 +482,6 @@ class _Kernel:
         with torch.cuda.device(dev):
             d_rows = torch.empty((n, H), dtype=torch.float32, device=dev) if want_rows else None
             d_weight = torch.empty((V, H), dtype=torch.float32, device=dev) if want_weight else None
-            # (torch calls a slice of one row or none contiguous, whatever its stride)
-            pitch = dlogits.stride(0) if _rows_apart(dlogits) else V
             rc = _cabi.lib().pcfgnat_proj_backward_gemms_pitched(dlogits.data_ptr(), pitch, ptr(weight_bf16), ptr(rows_bf16), n, V, H,
                                                                  ptr(d_rows), ptr(d_weight), _status_ptr(dev), _stream(dev))
         _cabi.check(rc, "pcfgnat_proj_backward_gemms")
@@ -1149,14 +1144,13 @@ def _bf16(t):
 def proj_backward_products(dlogits, weight, rows):
     """(dlogits @ weight, dlogits.T @ rows) in float32 from bf16 d-logits [n, V], the projection weight [V, H] and the
     decoder states of the same n rows [n, H] (either may be None: that product is skipped).  On this library's
-    tensor-core kernels (``pcfgnat_proj_backward_gemms``); d-logits whose rows are not a multiple of 16 bytes apart
-    (``proj_dlogits_rows`` makes such an odd vocabulary's), and an H that is not a multiple of 8, cannot be
-    described to the tensor maps and go through torch's matmul instead."""
+    tensor-core kernels (``pcfgnat_proj_backward_gemms``); shapes whose V or H is not a multiple of 8 cannot be
+    described to the tensor maps and go through torch's matmul instead (an odd vocabulary's d-logits from
+    ``proj_dlogits_rows`` can: ``products_of_rows``)."""
     V = dlogits.shape[1]
     H = (weight if weight is not None else rows).shape[1]
-    if H % 8 == 0 and (V % 8 == 0 or _rows_apart(dlogits)):
-        gemms = get_pcfg_kernel().proj_backward_gemms if V % 8 == 0 else get_pcfg_kernel()._proj_backward_gemms
-        return gemms(
+    if V % 8 == 0 and H % 8 == 0:
+        return get_pcfg_kernel().proj_backward_gemms(
             dlogits, _bf16(weight) if weight is not None else None, _bf16(rows) if rows is not None else None,
             want_rows=weight is not None, want_weight=rows is not None)
     d_rows = (dlogits @ weight.to(torch.bfloat16)).float() if weight is not None else None
@@ -1164,11 +1158,22 @@ def proj_backward_products(dlogits, weight, rows):
     return d_rows, d_weight
 
 
+def products_of_rows(dlogits, weight, rows):
+    """``proj_backward_products`` of what ``proj_dlogits_rows`` returned, or of its first rows: they lie V rounded up to a
+    multiple of 8 apart, on a 16-byte boundary, so that the tensor maps can describe an odd vocabulary's too."""
+    H = (weight if weight is not None else rows).shape[1]
+    if H % 8:
+        return proj_backward_products(dlogits, weight, rows)
+    return get_pcfg_kernel()._proj_backward_gemms(
+        dlogits, (dlogits.shape[1] + 7) // 8 * 8, _bf16(weight) if weight is not None else None,
+        _bf16(rows) if rows is not None else None, want_rows=weight is not None, want_weight=rows is not None)
+
+
 class ProjLogsoftmaxGatherFunc(Function):
     """match = log_softmax(hidden @ weight.T)[targets] with a backward that never holds a [B, L, V] tensor of
     the forward: the forward keeps only the per-row log-sum-exp; the backward recomputes the logits on the
     tensor cores into d loss / d logits (bf16, the only [B * L, V] buffer, alive during the backward only) and
-    finishes with this library's two tensor-core products (``proj_backward_products``).  Stands in for output_projection + DagLogsoftmaxGatherFunc
+    finishes with this library's two tensor-core products (``products_of_rows``).  Stands in for output_projection + DagLogsoftmaxGatherFunc
     (models/...pcfg.py:237, custom_ops/pcfg_loss.py:160-180), whose forward overwrites the float32 logits with
     the softmax to keep them for the backward."""
 
@@ -1195,7 +1200,7 @@ class ProjLogsoftmaxGatherFunc(Function):
         else:  # the real graph nodes only
             dl, idx = k.proj_dlogits_rows(hidden, weight, targets, ol, tl, lse, grad_match.contiguous(), n_rows=ctx.n_rows)
             rows = k.rows_to_bf16(hidden.reshape(B * L, H), idx) if need_w else None
-        d_rows, d_weight = proj_backward_products(dl, weight if need_h else None, rows if need_w else None)
+        d_rows, d_weight = products_of_rows(dl, weight if need_h else None, rows if need_w else None)
         if need_h:
             if idx is None:
                 d_hidden = d_rows.to(hidden.dtype).view(B, L, H)

@@ -423,7 +423,7 @@ class LossStep(_GraphedStep):
         n = self.n_rows if self.n_rows is not None else int(self.output_length.clamp(min=0, max=self.L).sum())
         dl, idx = self.dlogits[:n], self.row_index[:n]
         rows = self.kernel.rows_to_bf16(self.hidden.view(self.B * self.L, self.H), idx)
-        d_rows, d_weight = ops.proj_backward_products(dl, self.weight_bf16, rows)
+        d_rows, d_weight = ops.products_of_rows(dl, self.weight_bf16, rows)
         self.d_hidden.zero_()
         self.kernel.rows_from_f32(d_rows, self.d_hidden, idx)
         d_weight = d_weight.to(torch.float16)

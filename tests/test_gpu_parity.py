@@ -1038,6 +1038,20 @@ def test_projection_backward_of_an_odd_vocabulary_and_one_row(pkg, ops, V):
     ops.read_status(DEV)
 
 
+@pytest.mark.parametrize("n, V, pitch, offset", [(5, 33, 40, 0), (5, 33, 40, 3), (1, 1001, 1008, 1), (4, 999, 999, 0), (3, 64, 64, 0)])
+def test_projection_backward_products_of_any_view(ops, n, V, pitch, offset):
+    """The public products take d-logits of any V, pitch and offset.  Odd vocabularies go through torch's matmul, which may round
+    partial sums and the result to bf16: 2^-9 of each part twice, and a part is no larger than the sum of its terms' magnitudes."""
+    g = torch.Generator(DEV).manual_seed(V)
+    buffer = torch.randn(offset + n * pitch, device=DEV, generator=g).to(torch.bfloat16)
+    dlogits = buffer[offset:].view(n, pitch)[:, :V]
+    weight, rows = torch.randn(V, 64, device=DEV, generator=g).half(), torch.randn(n, 64, device=DEV, generator=g).half()
+    got = ops.proj_backward_products(dlogits, weight, rows)
+    left, right = (dlogits.double(), weight.bfloat16().double()), (dlogits.double().t(), rows.bfloat16().double())
+    for x, (a, b) in zip(got, (left, right)):
+        assert x.dtype == torch.float32 and ((x.double() - a @ b).abs() <= 2.0 ** -8 * (a.abs() @ b.abs())).all()
+
+
 @pytest.mark.parametrize("V", [1001, 1007, 2051, 16384, 16387, 33001])
 @pytest.mark.parametrize("dtype, offset, columns", [(torch.float16, 0, 20), (torch.float16, 3, 600), (torch.float32, 0, 600),
                                                     (torch.float32, 1, 20)])
