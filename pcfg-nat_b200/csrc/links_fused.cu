@@ -21,9 +21,11 @@
 // The scores are 0.5 GFLOP a pass on a training batch; what costs is what is done per cell (one exponential, a dozen instructions
 // a pass), for which the registers of mma's accumulators are the right place: tcgen05 would put them into tensor memory, 128
 // nodes a tile, more than most sentences have to give to an SM.  The tensor cores cut sums off where an FMA rounds them: chains
-// of two instructions are started from zero and added up by the FMA pipe.  Logits are kept in units of log 2, so that an
-// exponential is one ex2.  Against float64 (8 x 64 features, graphs of 162 to 514 nodes) the transitions are off by 2.1e-7 (rms;
-// 2.5e-7 with the float32 kernels), the gradients by 1.6e-7 to 2.9e-7 of their norm (2.2e-7 to 2.7e-7).
+// of two or three instructions are started from zero and added up by the FMA pipe.  Logits are kept in units of log 2, so that an
+// exponential is one ex2.  Against float64 (8 x 64 features, graphs of 162 to 514 nodes) the transitions are off by 2.0e-7 to
+// 2.3e-7 (rms; 2.3e-7 to 2.5e-7 with the float32 kernels), the gradients by 1.5e-7 to 2.0e-7 of their norm (2.0e-7 to 2.7e-7) and
+// every row of them (a node and head) by 1.9e-7 of its own norm in the median, also where the rows of links_grad are 1e12
+// apart (2.3e-7).
 // All five are bound by the issue of their instructions and the latency between them (45 % of the slots, 8 to 16 warps an
 // SM).  90 sentences, M = 161, 8 x 64 features: 33 + 60 us forward, 357 us with extract_links.cu's three; 13 + 100 + 59 us
 // backward, 643 us with its two, 33 of zero fills and 41 of conversions, which these need none of.
@@ -680,7 +682,6 @@ struct Weights {        // of the cells: [B][tiles][tiles][kCells], written at a
     float *w;
     float2 *rare;       // written where w is marked
     float *gs, *back;   // [B][tiles][H][16] Gs, Gs / sum e
-    float *bound;       // [B][H][16 tiles]: no |X| of the node and head is larger
     float *none_part;   // [B][H][tiles][D]: d kl[0] (left option 0) of the tile's nodes
 };
 
@@ -691,32 +692,57 @@ __device__ __noinline__ float rare_share(const float2 *rare, float term) {
     return !isinf(zg.x) && term > neg_inf() ? zg.y * ex2(term - zg.x) : 0.f;
 }
 
-// ---- X as an operand: scaled by a power of two into the halves' range and split in two, 22 bits in all
-struct Split {
-    float up, down;  // the scale and its inverse
-    // most: no |X| is larger.  |X0 + X1| <= 2 most < 2^(exponent + 2), scaled below 2^14
-    __device__ __forceinline__ explicit Split(float most) {
-        const int exponent = most > 0.f ? (int)(__float_as_uint(most) >> 23) - 127 : 0;
-        const int shift = min(12 - exponent, 100);
-        up = __uint_as_float((uint32_t)(127 + shift) << 23);
-        down = __uint_as_float((uint32_t)(127 - shift) << 23);
+// ---- X of a step as two operands of 16 rows and 16 columns: d[half][4 * operand + 2 * row + cell] is what a lane has of row g (0) or
+// g + 8 (1), columns 8 * half + 2 j + cell.  Each row of an operand goes by a power of two of its own into the halves' range and is
+// split in three: all 24 bits of whatever is above 2^-16 of the row's largest, 2^-40 of that below.  (One scale for 16 nodes or
+// a whole chain, and two halves, before: 22 bits, and nothing below 2^-38 of the largest of all.)
+struct Operands {
+    uint32_t part[2][3][4];  // [operand][largest to smallest][register]
+    float down[2][2];        // [operand][row]: undoes the scale
+    __device__ __forceinline__ explicit Operands(const float (&d)[2][8]) {
+        float up[2][2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            uint32_t top[2];  // of the lane, then of the quad: the upper halves of the floats suffice
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int x = 4 * k + 2 * r;
+                top[k] = __float_as_uint(fmaxf(fmaxf(fabsf(d[0][x]), fabsf(d[0][x + 1])), fmaxf(fabsf(d[1][x]), fabsf(d[1][x + 1]))));
+            }
+            uint32_t both = __byte_perm(top[0], top[1], 0x7632);
+            both = __vmaxu2(both, __shfl_xor_sync(0xffffffffu, both, 1));
+            both = __vmaxu2(both, __shfl_xor_sync(0xffffffffu, both, 2));
+#pragma unroll
+            for (int k = 0; k < 2; k++) {  // the largest to 2^14 .. 2^15; both scales are normal floats
+                const int exponent = (int)(both >> (k ? 23 : 7) & 0xff), shift = min(141 - exponent, 126);
+                up[k][r] = __uint_as_float((uint32_t)(127 + shift) << 23);
+                down[k][r] = __uint_as_float((uint32_t)(127 - shift) << 23);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                float x = d[i >> 1][4 * k + 2 * (i & 1)] * up[k][i & 1], y = d[i >> 1][4 * k + 2 * (i & 1) + 1] * up[k][i & 1];
+#pragma unroll
+                for (int p = 0; p < 3; p++) {
+                    const __half2 h = __floats2half2_rn(x, y);
+                    part[k][p][i] = *reinterpret_cast<const uint32_t *>(&h);
+                    const float2 back = __half22float2(h);
+                    x -= back.x, y -= back.y;
+                }
+            }
     }
-    __device__ __forceinline__ void operator()(float x, float y, uint32_t &hi, uint32_t &lo) const {
-        x *= up, y *= up;
-        const __half2 big = __floats2half2_rn(x, y);
-        const float2 back = __half22float2(big);
-        const __half2 small = __floats2half2_rn(x - back.x, y - back.y);
-        hi = *reinterpret_cast<const uint32_t *>(&big);
-        lo = *reinterpret_cast<const uint32_t *>(&small);
+    // acc += operand k . f, the tensor cores' part from zero
+    __device__ __forceinline__ void add_product(float (&acc)[4], int k, uint32_t f0, uint32_t f1) const {
+        float sum[4];
+        mma_zero(sum, part[k][2][0], part[k][2][1], part[k][2][2], part[k][2][3], f0, f1);
+#pragma unroll
+        for (int p = 1; p >= 0; p--) mma_add(sum, part[k][p][0], part[k][p][1], part[k][p][2], part[k][p][3], f0, f1);
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[i] = fmaf(sum[i], down[k][i >> 1], acc[i]);
     }
 };
-// the largest finite one of a warp's values: a row with an infinite gradient has none to be exact about
-__device__ __forceinline__ float warp_finite_max(float x) {
-    x = x < CUDART_INF_F ? x : 0.f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
-    return x;
-}
 // 16 x 16 of a tile, transposed: the second operand of two neighbouring column tiles
 __device__ __forceinline__ void load_transposed(uint32_t address, uint32_t (&r)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -728,15 +754,6 @@ template <int D>
 __device__ __forceinline__ uint32_t transposed_base(const __half *tile, int lane) {
     return dsm_smem_u32(tile + (lane & 15) * kPitch<D> + (lane >> 4) * 8);
 }
-// acc += (hi + lo) . f, the tensor cores' part from zero
-__device__ __forceinline__ void add_product(float (&acc)[4], const uint32_t (&hi)[4], const uint32_t (&lo)[4], uint32_t f0, uint32_t f1) {
-    float sum[4];
-    mma_zero(sum, lo[0], lo[1], lo[2], lo[3], f0, f1);
-    mma_add(sum, hi[0], hi[1], hi[2], hi[3], f0, f1);
-#pragma unroll
-    for (int i = 0; i < 4; i++) acc[i] += sum[i];
-}
-
 template <class T>
 __device__ __forceinline__ void store2(T *p, float x, float y) {
     if constexpr (sizeof(T) == 2) *reinterpret_cast<__half2 *>(p) = __floats2half2_rn(x, y);
@@ -865,11 +882,12 @@ __global__ void __launch_bounds__(32 * kParentWarps, 3)
     };
     // ---- Gs
     children.list = lists, children.n = used;
-    float sum[2] = {0.f, 0.f}, most[2] = {0.f, 0.f};
+    float sum[2] = {0.f, 0.f};
     children.walk(h, one_head, [&](int t, int, int, const __half *step) {
         const uint32_t row_ok[2] = {step_masks(step)[0], step_masks(step)[8]}, bits[2] = {row_ok[0] >> (2 * j), row_ok[1] >> (2 * j)};
         const bool full = all_admitted(row_ok[0], row_ok[1]);
         const size_t at = tile_cells + (size_t)t * kCells + cells_at(g, j);
+        float part[2] = {0.f, 0.f};  // short chains: a row has up to 2048 cells
 #pragma unroll
         for (int half = 0; half < 2; half++) {
             float w[8], v[8], share[8];
@@ -891,31 +909,24 @@ __global__ void __launch_bounds__(32 * kParentWarps, 3)
                     if (!admitted(bits, half, x)) share[x] = 0.f;
                     else if (marked(w[x])) share[x] = rare_share(wt.rare + at + cell_at(half, x), rare_term(v[x], x >> 1 & 1));
 #pragma unroll
-            for (int x = 0; x < 8; x++) {
-                sum[x >> 1 & 1] += share[x];
-                most[x >> 1 & 1] = fmaxf(most[x >> 1 & 1], fabsf(share[x]));
-            }
+            for (int r = 0; r < 2; r++) part[r] += (share[2 * r] + share[2 * r + 1]) + (share[4 + 2 * r] + share[5 + 2 * r]);
         }
+#pragma unroll
+        for (int r = 0; r < 2; r++) sum[r] += part[r];
     });
-    float back[2], bound[2];
+    float back[2];
 #pragma unroll
     for (int r = 0; r < 2; r++) {
 #pragma unroll
-        for (int o = 1; o < 4; o *= 2) {
-            sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
-            most[r] = fmaxf(most[r], __shfl_xor_sync(0xffffffffu, most[r], o));
-        }
+        for (int o = 1; o < 4; o *= 2) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
         // a block without an admitted child, and nodes past the chain, have no sums from the forward
         const bool on = used > 0 && r0 + g + 8 * r < M;
         back[r] = !on ? 0.f : (r ? p1.z : p0.z) < CUDART_INF_F ? sum[r] * __ldg(&stat[8 * r].more).x : CUDART_NAN_F;
-        bound[r] = on ? most[r] + fabsf(back[r]) : 0.f;
         if (j == 0) {
             wt.gs[(((size_t)b * c.tiles + rt) * H + h) * kTile + g + 8 * r] = on ? sum[r] : 0.f;
             wt.back[(((size_t)b * c.tiles + rt) * H + h) * kTile + g + 8 * r] = back[r];
-            wt.bound[bh * P + r0 + g + 8 * r] = bound[r];
         }
     }
-    const Split split(warp_finite_max(fmaxf(bound[0] < CUDART_INF_F ? bound[0] : 0.f, bound[1] < CUDART_INF_F ? bound[1] : 0.f)));
 
     // ---- X times the children's features; tiles with a feature that zeros don't cancel take part
     children.list = lists + kListBytes;
@@ -925,10 +936,11 @@ __global__ void __launch_bounds__(32 * kParentWarps, 3)
         const uint32_t row_ok[2] = {step_masks(step)[0], step_masks(step)[8]}, bits[2] = {row_ok[0] >> (2 * j), row_ok[1] >> (2 * j)};
         const bool full = all_admitted(row_ok[0], row_ok[1]);
         const size_t at = tile_cells + (size_t)t * kCells + cells_at(g, j);
-        uint32_t hi[2][4], lo[2][4];  // [option]: X as the first operand, 16 nodes x 16 children
+        float X[2][8];  // [half of the children]: 4 * option + 2 * row + cell
 #pragma unroll
         for (int half = 0; half < 2; half++) {
-            float w[8], d[8];
+            float w[8];
+            float(&d)[8] = X[half];
             bool rare = false;
 #pragma unroll
             for (int x = 0; x < 8; x += 2) {
@@ -950,11 +962,9 @@ __global__ void __launch_bounds__(32 * kParentWarps, 3)
 #pragma unroll
                 for (int x = 0; x < 8; x++) d[x] = ex2(d[x]) * fmaf(w[x], gate[x >> 1 & 1], -back[x >> 1 & 1]);
 #pragma unroll
-            for (int x = 0; x < 8; x += 2) {
-                dab[x >> 1 & 1][x >> 2] += d[x] + d[x + 1];
-                split(d[x], d[x + 1], hi[x >> 2][2 * half + (x >> 1 & 1)], lo[x >> 2][2 * half + (x >> 1 & 1)]);
-            }
+            for (int x = 0; x < 8; x += 2) dab[x >> 1 & 1][x >> 2] += d[x] + d[x + 1];
         }
+        const Operands operands(X);
         const uint32_t base = transposed_base<D>(step, lane);
 #pragma unroll
         for (int m = 0; m < N; m += 2) {
@@ -963,10 +973,9 @@ __global__ void __launch_bounds__(32 * kParentWarps, 3)
 #pragma unroll
             for (int y = 0; y < 2; y++)
 #pragma unroll
-                for (int k = 0; k < 2; k++) add_product(acc[k][m + y], hi[k], lo[k], f[2 * y], f[2 * y + 1]);
+                for (int k = 0; k < 2; k++) operands.add_product(acc[k][m + y], k, f[2 * y], f[2 * y + 1]);
         }
     });
-    const float down = split.down * scale;
 #pragma unroll
     for (int r = 0; r < 2; r++)
 #pragma unroll
@@ -993,8 +1002,8 @@ __global__ void __launch_bounds__(32 * kParentWarps, 3)
         for (int r = 0; r < 2; r++) {
             if (!is_row[r]) continue;
             const float2 qv = half2_at(own + (g + 8 * r) * PITCH + 8 * m + 2 * j), kv = half2_at(own + (kTile + g + 8 * r) * PITCH + 8 * m + 2 * j);
-            const float x0[2] = {acc[0][m][2 * r] * down, acc[0][m][2 * r + 1] * down};
-            const float x1[2] = {acc[1][m][2 * r] * down, acc[1][m][2 * r + 1] * down};
+            const float x0[2] = {acc[0][m][2 * r] * scale, acc[0][m][2 * r + 1] * scale};
+            const float x1[2] = {acc[1][m][2 * r] * scale, acc[1][m][2 * r + 1] * scale};
             store2(q_out[r] + 8 * m, dab[r][0] * none0.x + dab[r][1] * kv.x + (x0[0] + x1[0]),
                    dab[r][0] * none0.y + dab[r][1] * kv.y + (x0[1] + x1[1]));
             const float l0 = dab[r][1] * qv.x + x1[0], l1 = dab[r][1] * qv.y + x1[1];
@@ -1076,12 +1085,6 @@ __global__ void __launch_bounds__(32 * kChildWarps)
         copy_commit();
     };
     load(0, 0);
-    float most = 0.f;
-    for (int i = lane; i < P; i += 32) {
-        const float x = __ldg(wt.bound + bh * P + i);
-        if (x < CUDART_INF_F) most = fmaxf(most, x);
-    }
-    const Split split(warp_finite_max(most));
     const __half *mine = in.child + (((size_t)b * c.tiles + ct) * H + h) * kChildBlock<D>;
     Frag<KS> c0, c1;
     c0.template load<true>(mine + g * D, j);
@@ -1105,10 +1108,11 @@ __global__ void __launch_bounds__(32 * kChildWarps)
         for (int m = 0; m < 2; m++) on[m] = *reinterpret_cast<const uint32_t *>(masks + 8 * m + 2 * j);
         const auto admits = [&](int x) { return on[x >> 3] >> (16 * (x & 1) + g + (x & 2 ? 8 : 0)) & 1; };
         const bool full = __all_sync(0xffffffffu, (on[0] & on[1]) == 0xffffffffu);
-        uint32_t hi[2][4], lo[2][4];  // X0 + X1 and X1, 16 children x 16 parents
+        float X[2][8];  // [half of the parents]: X0 + X1 and X1 of 16 children
 #pragma unroll
         for (int half = 0; half < 2; half++) {
-            float vq[4], vk[4], d[8];
+            float vq[4], vk[4];
+            float(&d)[8] = X[half];
             Frag<KS> f;
             f.load(sq + (8 * half + g) * PITCH, j);
             products(c0, c1, f, vq);
@@ -1149,13 +1153,11 @@ __global__ void __launch_bounds__(32 * kChildWarps)
                     }
             }
 #pragma unroll
-            for (int r = 0; r < 2; r++) {
-                const float *x0 = d + 2 * r, *x1 = x0 + 4;
-                x0sum[r] += x0[0] + x0[1];
-                split(x0[0] + x1[0], x0[1] + x1[1], hi[0][2 * half + r], lo[0][2 * half + r]);
-                split(x1[0], x1[1], hi[1][2 * half + r], lo[1][2 * half + r]);
-            }
+            for (int r = 0; r < 2; r++) x0sum[r] += d[2 * r] + d[2 * r + 1];
+#pragma unroll
+            for (int x = 0; x < 4; x++) d[x] += d[4 + x];
         }
+        const Operands operands(X);
 #pragma unroll
         for (int k = 0; k < 2; k++) {
             const uint32_t from = transposed_base<D>(k ? sk : sq, lane);
@@ -1164,12 +1166,11 @@ __global__ void __launch_bounds__(32 * kChildWarps)
                 uint32_t f[4];
                 load_transposed(from + 16 * m, f);
 #pragma unroll
-                for (int y = 0; y < 2; y++) add_product(acc[m + y], hi[k], lo[k], f[2 * y], f[2 * y + 1]);
+                for (int y = 0; y < 2; y++) operands.add_product(acc[m + y], k, f[2 * y], f[2 * y + 1]);
             }
         }
         __syncwarp();
     }
-    const float down = split.down * scale;
 #pragma unroll
     for (int r = 0; r < 2; r++) {
         x0sum[r] *= scale;
@@ -1180,7 +1181,7 @@ __global__ void __launch_bounds__(32 * kChildWarps)
 #pragma unroll
         for (int m = 0; m < N; m++) {
             const float2 none0 = half2_at(in.kl0 + (size_t)b * HD + h * D + 8 * m + 2 * j);
-            store2(to + 8 * m, fmaf(x0sum[r], none0.x, acc[m][2 * r] * down), fmaf(x0sum[r], none0.y, acc[m][2 * r + 1] * down));
+            store2(to + 8 * m, fmaf(x0sum[r], none0.x, acc[m][2 * r] * scale), fmaf(x0sum[r], none0.y, acc[m][2 * r + 1] * scale));
         }
     }
 }
@@ -1228,7 +1229,6 @@ size_t carve_weights(void *base, int M, int B, int H, int D, Weights &w) {
     w.rare = c.take<float2>(cells);
     w.gs = c.take<float>(blocks * kTile);
     w.back = c.take<float>(blocks * kTile);
-    w.bound = c.take<float>(blocks * kTile);
     w.none_part = c.take<float>(blocks * D);
     return c.used;
 }

@@ -1693,6 +1693,31 @@ def test_links_from_half_features_by_masks_and_odd_values(pkg, ops):
             assert ((part - of).abs() <= 2e-5 * of.abs().max()).all(), (b, tuple(x.shape))
 
 
+@pytest.mark.parametrize("B, L, heads, dim, by", [(4, 66, 3, 64, "rows"), (4, 66, 3, 64, "cells"), (33, 98, 2, 32, "rows"), (3, 34, 9, 64, "rows")])
+def test_links_gradient_of_rows_of_different_sizes(pkg, ops, B, L, heads, dim, by):
+    """links_grad rows (or cells) that are up to 1e24 apart, some 1e-12 and less: the feature gradients of every (node, head) against
+    autograd in float64, by that row's own size.  Logits of up to 16 in units of log 2 (spacing 2e-6, a handful of roundings) put
+    1e-5 on a probability; what a row's cells cancel of one another, two digits at most: 1e-3."""
+    g = torch.Generator().manual_seed(L)
+    leaves = [torch.randn(B, L, heads, dim, generator=g).half() for _ in range(3)] + [torch.randn(B, L, heads, generator=g)]
+    length = torch.randint(L // 2, L + 1, (B,), generator=g)
+    length[0] = L
+    prev = torch.where(torch.arange(L)[None, :] < length[:, None], 3, 1)
+    masks = _tree_masks(L)
+    ref = [t.double().requires_grad_() for t in leaves]
+    want = pyref.extract_links(*ref, prev, 1, *[m.cpu() for m in masks], dtype=torch.float64, floor=-1e30)
+    ok = want > -1e29
+    size = torch.rand((B, L, 1, 1) if by == "rows" else (B, L, 2, L), generator=g)
+    G = torch.randn(B, L, 2, L, generator=g) * ok * 10 ** (24 * size - 12)
+    torch.where(ok, want, 0.0).mul(G).sum().backward()
+    k = ops.get_pcfg_kernel()
+    _, saved = k._links_forward(*[t.to(DEV) for t in leaves], prev.to(DEV), 1, *[m.ne(0).to(torch.uint8) for m in masks])
+    assert "kept" in saved  # the kernels under test
+    for got, leaf in zip(k._links_backward(G.to(DEV), saved), ref[:3]):
+        got, y = got.cpu().double(), leaf.grad
+        assert ((got - y).norm(dim=-1) <= 1e-3 * y.norm(dim=-1)).all()
+
+
 @pytest.mark.parametrize("heads, scale", [(1, 4.0), (2, 4.0), (8, 5.0)])
 def test_links_of_improbable_cells(pkg, ops, heads, scale):
     """Transitions below the probability (1e-30) under which the mixture is formed from log-probabilities, and their
