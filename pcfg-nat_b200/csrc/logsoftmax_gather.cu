@@ -154,6 +154,12 @@ __device__ __forceinline__ float ex2_ftz(float x) {
     return y;
 }
 
+__device__ __forceinline__ float ex2(float x) {  // below 2^-126 too
+    float y;
+    asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // 16 bytes of a row at a time: the maximum is taken in the storage type (packed halves stay packed), the
 // exponentials in float32.
 template <typename T>
@@ -208,8 +214,8 @@ struct Pack<__half> {
 // another, which keeps both the exponential unit and the copy stream busy.
 // nch * kChunkBytes >= the row.  EDGES: rows that are no multiple of 16 bytes, or whose base is not aligned.  What is copied is a
 // row's part between its first and its last 16-byte boundary; the up to seven entries on either side stay in registers, one a
-// thread, so that nothing of a neighbouring row is read or written.  [4 687, 31 999] half with the softmax 131 us, read-only 84;
-// [2 343, 31 999] float 121 and 74 (213, 143, 195 and 143 as the single-buffer kernel took them, element by element).
+// thread, so that nothing of a neighbouring row is read or written.  [4 687, 31 999] half with the softmax 153 us, read-only 97;
+// [2 343, 31 999] float 130 and 86 (225, 157, 206 and 154 as the single-buffer kernel takes them, element by element).
 template <typename T, bool EDGES>
 __global__ void __launch_bounds__(kStreamThreads)
     logsoftmax_gather_stream_kernel(T *logits, const int64_t *__restrict__ sel, int64_t sb, int64_t sl, int64_t ss,
@@ -251,6 +257,9 @@ __global__ void __launch_bounds__(kStreamThreads)
     if (tid == 0 && (int64_t)blockIdx.x < rows)
         for (int c = 0; c < nch; c++) fetch(blockIdx.x, c);
     const float kLog2e = 1.4426950408889634f;
+    // Terms are ex2(x * log2(e) + shift), shift = -m * log2(e) rounded: half an ulp of m * log2(e) in the exponent, the same for all
+    // of a thread's terms.  EDGES: rest is what was rounded away, and goes into the sum where m changes and at the end.
+    const auto rest_of = [&](float m, float shift) { return EDGES && fabsf(m) < CUDART_INF_F ? fmaf(-m, kLog2e, -shift) : 0.f; };
     const bool early = slen <= kStreamThreads;
     uint32_t par = 0;  // every barrier completes one phase per row
     for (int64_t r = blockIdx.x; r < rows; r += gridDim.x, par ^= 1) {
@@ -273,7 +282,7 @@ __global__ void __launch_bounds__(kStreamThreads)
             if (t_sel < 0 || t_sel >= V) flag(status, PCFGNAT_STATUS_BAD_INDEX);
             else x_sel = to_f<T>(grow[t_sel]);
         }
-        float m = -CUDART_INF_F, sum = 0.f, sum_b = 0.f, shift = 0.f;  // shift = -m * log2(e), 0 while m is still -inf
+        float m = -CUDART_INF_F, sum = 0.f, sum_b = 0.f, shift = 0.f, rest = 0.f;  // 0 while m is still -inf
         bool ok = true;
         int failed_at = nch;
         for (int c = 0; c < nch; c++) {
@@ -286,10 +295,11 @@ __global__ void __launch_bounds__(kStreamThreads)
                     const uint4 v1 = i + kStreamThreads < n16 ? s4[i + kStreamThreads] : Pack<T>::lowest();
                     const float vm = fmaxf(Pack<T>::max_of(v0), Pack<T>::max_of(v1));
                     if (vm > m) {
-                        const float scale = ex2_ftz((m - vm) * kLog2e);  // m == -inf: the sums are 0 and stay 0
+                        const float to = -vm * kLog2e, left = rest_of(vm, to);
+                        const float scale = ex2_ftz((m - vm) * kLog2e + (rest - left));  // m == -inf: the sums are 0 and stay 0
                         sum *= scale, sum_b *= scale;
                         m = vm;
-                        shift = -vm * kLog2e;
+                        shift = to, rest = left;
                     }
                     float f0[kVec], f1[kVec];
                     Pack<T>::unpack(v0, f0);
@@ -323,10 +333,10 @@ __global__ void __launch_bounds__(kStreamThreads)
         }
         if (has_edge) {
             if (x_edge > m) {
-                const float scale = ex2_ftz((m - x_edge) * kLog2e);
+                const float to = -x_edge * kLog2e, left = rest_of(x_edge, to), scale = ex2_ftz((m - x_edge) * kLog2e + (rest - left));
                 sum *= scale, sum_b *= scale;
                 m = x_edge;
-                shift = -x_edge * kLog2e;
+                shift = to, rest = left;
             }
             sum += ex2_ftz(fmaf(x_edge, kLog2e, shift));
         }
@@ -334,7 +344,7 @@ __global__ void __launch_bounds__(kStreamThreads)
         float wm = m;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffu, wm, o));
-        float ws = m == -CUDART_INF_F ? 0.f : (sum + sum_b) * ex2_ftz((m - wm) * kLog2e);  // a thread without entries
+        float ws = m == -CUDART_INF_F ? 0.f : (sum + sum_b) * ex2_ftz((m - wm) * kLog2e + rest);  // a thread without entries
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
         if (lane == 0) red[par][warp] = make_float2(wm, ws);
@@ -363,11 +373,18 @@ __global__ void __launch_bounds__(kStreamThreads)
                 selected[(size_t)r * slen + s] = v;
             }
         }
-        if (req_grad) {  // softmax = ex2(x * log2(e) - (mx * log2(e) + log2(sum))): the division is in the exponent
-            const float shift2 = -mx * kLog2e - __log2f(sum);
+        if (req_grad) {
+            // softmax = ex2(x * log2(e) - (mx * log2(e) + log2(sum))): the division is in the exponent; EDGES: a factor of its own, with
+            // what the shift lacks
+            const float back = -mx * kLog2e, shift2 = EDGES ? back : back - __log2f(sum);
+            const float factor = EDGES ? ex2_ftz(rest_of(mx, back)) / sum : 1.f;
+            const auto probability = [&](float x) {
+                const float arg = fmaf(x, kLog2e, shift2);
+                return !EDGES ? ex2_ftz(arg) : (sizeof(T) == 4 ? ex2(arg) : ex2_ftz(arg)) * factor;
+            };
             if (EDGES) {
                 if (!early) __syncthreads();  // the gathers have read the row where it is overwritten now
-                if (has_edge) grow[edge] = from_f<T>(ex2_ftz(fmaf(x_edge, kLog2e, shift2)));
+                if (has_edge) grow[edge] = from_f<T>(probability(x_edge));
             }
             for (int c = 0; c < nch; c++) {
                 const uint4 *s4 = reinterpret_cast<const uint4 *>(smem_raw + (size_t)c * kChunkBytes);
@@ -377,7 +394,7 @@ __global__ void __launch_bounds__(kStreamThreads)
                     float f[kVec];
                     Pack<T>::unpack(s4[i], f);
 #pragma unroll
-                    for (int k = 0; k < kVec; k++) f[k] = ex2_ftz(fmaf(f[k], kLog2e, shift2));
+                    for (int k = 0; k < kVec; k++) f[k] = probability(f[k]);
                     g4[i] = Pack<T>::pack(f);
                 }
                 __syncthreads();  // the gathers and this sweep have read chunk c
@@ -399,9 +416,9 @@ int launch_typed(T *logits, const int64_t *sel, int64_t sb, int64_t sl, int64_t 
     const int nch = (int)(((size_t)V * sizeof(T) + kChunkBytes - 1) / kChunkBytes);
     const size_t stream_bytes = ((size_t)V * sizeof(T) + 127) / 128 * 128;
     const char *env = getenv("PCFGNAT_LSG_STREAM");  // "0": the single-buffer kernels only
-    // shorter rows of this kind are faster four to an SM: 14 400 of 501 halves 124 and 149 us, of 999 halves 151 and 150, of 501
-    // floats 129 and 126
-    const bool edges_pay = (size_t)V * sizeof(T) >= 2000;
+    // shorter rows of this kind are faster four to an SM.  14 400 rows, here and there (us): with the softmax 1 501 halves 169 and 165,
+    // 2 001 172 and 179, 501 floats 137 and 132, 601 143 and 161; read-only 1 001 halves 147 and 148, 501 floats 116 and 121
+    const bool edges_pay = (size_t)V * sizeof(T) >= (!req_grad ? 2000 : sizeof(T) == 2 ? 3500 : 2300);
     if ((vec_ok || edges_pay) && nch <= kMaxChunks && stream_bytes + 2048 <= (size_t)kSmemLimit && !(env && env[0] == '0')) {
         const auto k = vec_ok ? logsoftmax_gather_stream_kernel<T, false> : logsoftmax_gather_stream_kernel<T, true>;
         e = ensure_dynamic_smem(k, stream_bytes);

@@ -1085,6 +1085,25 @@ def test_logsoftmax_gather_of_unaligned_rows(ops, V, dtype, offset, columns):
         assert ((after.double() - p).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("V", [2051, 33001])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_logsoftmax_gather_of_unaligned_rows_with_a_large_offset(ops, V, dtype):
+    """Logits around 4 000: their differences are exact, so log-probabilities and the softmax are as good as around 0 (a rounded
+    product of the largest logit and log2(e) would put 2e-4 on both).  Fast exponentials, float32 sums: 1e-5 of a
+    log-probability's scale, 2e-5 of a probability (and a half's rounding)."""
+    g = torch.Generator(DEV).manual_seed(V)
+    rows, columns = 6, 40
+    offset = torch.tensor([0, 999, -4001, 4003, 3999.5, -2500.25], device=DEV)[:, None]
+    logits = (torch.randn(rows, V, device=DEV, generator=g) * 3 + offset).to(dtype)[None].contiguous()
+    sel = torch.randint(0, V, (1, rows, columns), device=DEV, generator=g)
+    want = torch.log_softmax(logits.double(), -1)
+    got = ops.get_pcfg_kernel().logsoftmax_gather(logits, sel, True)
+    picked, p = want.gather(2, sel), want.exp()
+    assert ((got.double() - picked).abs() <= 1e-5 * picked.abs().clamp(min=1)).all()
+    bound = 2e-5 * p + (2.0 ** -11 * p + 2.0 ** -24 if dtype == torch.float16 else 1e-38)
+    assert ((logits.double() - p).abs() <= bound).all()
+
+
 def test_copy_real_rows_sends_the_real_nodes_only(ops):
     """pcfgnat_copy_real_rows: rows l < length arrive, the others keep what they held; lengths beyond the tensor
     and below zero are clamped; full sentences next to each other go as one copy; a sentence range."""
