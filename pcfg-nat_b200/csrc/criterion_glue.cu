@@ -153,8 +153,11 @@ __global__ void loss_stats_exchange_kernel(const float *__restrict__ loss, const
 //
 // Bound by latency, one sentence per block.  The T x L match mask is most of what is written: a warp takes a row at a time, from a
 // copy of the alignment in shared memory and in words of four cells where the rows allow it (a division and a read of the
-// alignment per cell, 256 threads and one thread per node's rank before: 12.0 -> 7.0 us for 64 sentences, L = 256, T = 76).
-constexpr int kSelectThreads = 1024;
+// alignment per cell and one thread per node's rank before).  Threads by the graph: small blocks start sooner and share SMs, 64 and
+// 400 sentences, 256 / 512 / 1024 threads, us: 33 nodes 3.3 / 3.5 / 4.2 and 3.8 / 4.7 / 7.7, 64 nodes 3.6 / 3.6 / 4.4 and
+// 4.1 / 5.1 / 8.2, 128 nodes 4.6 / 4.1 / 5.1 and 5.9 / 6.4 / 9.9, 256 nodes 7.9 / 6.4 / 6.7 and 13.1 / 12.5 / 14.3 (before 3.3 and 3.6,
+// 3.8 and 4.1, 5.6 and 7.3, 11.8 and 19.2).
+constexpr int kSelectThreads = 512;
 __global__ void __launch_bounds__(kSelectThreads)
     glance_select_kernel(const int64_t *__restrict__ path, const int64_t *__restrict__ pred, const int64_t *__restrict__ tgt, const
                          int64_t *__restrict__ prev, const int64_t *__restrict__ tl, const float *__restrict__ noise, const float
@@ -181,7 +184,7 @@ __global__ void __launch_bounds__(kSelectThreads)
     same = block_sum(same, scratch);  // exact: a count below 2^24; its barriers also publish sm_noise and aligned_to
     auto hit = [&](int l, int t) { return staged ? aligned_to[l] == t : pb[l] == t; };
     const bool words = (L & 3) == 0 && (reinterpret_cast<uintptr_t>(matchmask) & 3) == 0;
-    for (int t = threadIdx.x >> 5; t < T; t += kSelectThreads / 32) {
+    for (int t = threadIdx.x >> 5; t < T; t += blockDim.x / 32) {
         uint8_t *row = matchmask + ((size_t)b * T + t) * L;
         if (words) {
             for (int l = 4 * (threadIdx.x & 31); l < L; l += 128) {
@@ -220,7 +223,7 @@ __global__ void __launch_bounds__(kSelectThreads)
         same_num[b] = same_i;
         glance_num[b] = k;
     }
-    for (int l0 = 0; l0 < L; l0 += kSelectThreads / 4) {  // four lanes per node
+    for (int l0 = 0; l0 < L; l0 += blockDim.x / 4) {  // four lanes per node
         const int l = l0 + threadIdx.x / 4;
         const float mine = sm_noise[l < L ? l : 0];
         int larger = 0;
@@ -277,8 +280,9 @@ int launch_glance_select(const int64_t *path, const int64_t *pred, const int64_t
     const size_t smem = (size_t)L * (staged ? sizeof(float) + sizeof(int) : sizeof(float));
     // what a launch may ask for without opting in is 48 KB with the kernel's own 128 bytes (6 129 to 6 144 nodes are between)
     if (smem > 47 * 1024 && ensure_dynamic_smem(glance_select_kernel, smem) != cudaSuccess) return PCFGNAT_ERR_TOO_LARGE;
-    glance_select_kernel<<<B, kSelectThreads, smem, st>>>(path, pred, tgt, prev, tl, noise, uniform, strategy, context_p, L, T,
-                                                          staged, matchmask, oracle, same_num, glance_num, keep, glat_prev);
+    const int threads = L < 96 ? kSelectThreads / 2 : kSelectThreads;
+    glance_select_kernel<<<B, threads, smem, st>>>(path, pred, tgt, prev, tl, noise, uniform, strategy, context_p, L, T,
+                                                  staged, matchmask, oracle, same_num, glance_num, keep, glat_prev);
     return cuda_rc(cudaGetLastError());
 }
 
