@@ -111,13 +111,14 @@ __host__ __device__ constexpr int viterbi_overshoot(int G, int NC) { return 31 +
 // whatever lies behind a node's row gives -inf or NaN with it, which never wins.  Both kinds of terms go as pairs: a child's
 // links lie side by side and so do S[len - 1] and S[len - 2] in column len (a node stores its value into two columns).  Peers wait
 // for the value alone: the maximum is sent, and which term it was, with the reference's order of ties, is looked up in the held
-// terms while it is on its way (the terms of a node's first 128 children; of further ones value and term are carried
-// together).
+// terms while it is on its way (the terms of a node's first 128 children; of further ones value and term are carried together, or
+// in LONG chains, of more than 256 nodes, the value alone and the first 32 children that have it, whose terms are formed again:
+// 530 nodes on sixteen CTAs 632 -> 588 us, eight sentences of 320 on eight 242 -> 228.
 //
 // Bound by the latency of a length (loads, the chain of maxima, shuffles, exchange and barrier).  With value and key carried
 // through every comparison, 1024 threads and one load and addition per term before: 64 sentences of up to 120 nodes 82 -> 68 us,
 // 24 of 128 74 -> 57, 56 of up to 160 144 -> 119, one of 256 on eight CTAs 175 -> 141.
-template <int G>
+template <int G, bool LONG>
 __device__ __forceinline__ bool viterbi_lengths(float2 *col, const float2 *lk, const float *s_oa, float *own_v, uint16_t *own_k,
                                                 uint64_t *col_bar, int n_len, int Mb, int my_rows, int NC, int crank, int Q,
                                                 int cs, int pitch) {
@@ -156,22 +157,32 @@ __device__ __forceinline__ bool viterbi_lengths(float2 *col, const float2 *lk, c
 #pragma unroll
                 for (int j = 0; j < U; j++) best = fmaxf(best, fmaxf(held[k * U + j].x, held[k * U + j].y));  // NaN never wins
             }
-            float far = neg_inf();  // further children: value and trip together
+            float far = neg_inf();  // further children: the largest, and its trip or (LONG) that of the first 32 that have it
             int far_at = INT_MAX;
 #pragma unroll 1
             for (int i = HELD; i < trips; i += U) {
                 float2 t[U];
 #pragma unroll
                 for (int j = 0; j < U; j++) t[j] = terms(i + j);
+                if (LONG) {
+                    float most = neg_inf();
 #pragma unroll
-                for (int j = 0; j < U; j++) {
-                    if (t[j].x > far) {
-                        far = t[j].x;
-                        far_at = 2 * (i + j);
+                    for (int j = 0; j < U; j++) most = fmaxf(most, fmaxf(t[j].x, t[j].y));
+                    if (most > far) {
+                        far = most;
+                        far_at = i;
                     }
-                    if (t[j].y > far) {
-                        far = t[j].y;
-                        far_at = 2 * (i + j) + 1;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < U; j++) {
+                        if (t[j].x > far) {
+                            far = t[j].x;
+                            far_at = 2 * (i + j);
+                        }
+                        if (t[j].y > far) {
+                            far = t[j].y;
+                            far_at = 2 * (i + j) + 1;
+                        }
                     }
                 }
             }
@@ -215,6 +226,14 @@ __device__ __forceinline__ bool viterbi_lengths(float2 *col, const float2 *lk, c
             }
             if (!zero) {  // which term it was, while the value is on its way
                 int at = far == best ? far_at : INT_MAX;
+                if (LONG && at != INT_MAX) {
+                    at = INT_MAX;
+#pragma unroll
+                    for (int j = U - 1; j >= 0; j--) {
+                        const float2 t = terms(far_at + j);
+                        at = t.x == best ? 2 * (far_at + j) : t.y == best ? 2 * (far_at + j) + 1 : at;
+                    }
+                }
 #pragma unroll
                 for (int k = HELD / U - 1; k >= 0; k--) {
                     if (k * U < trips) {
@@ -241,6 +260,7 @@ __device__ __forceinline__ bool viterbi_lengths(float2 *col, const float2 *lk, c
     return arrived;
 }
 
+template <bool LONG>
 __global__ void __launch_bounds__(kVitThreads, 1)
     viterbi_cluster_kernel(const float *__restrict__ ob_lprob, const float *__restrict__ links,
                            const int64_t *__restrict__ ol, int L, float *S, int64_t *R, int64_t *Lt, int64_t *Mt,
@@ -333,7 +353,7 @@ __global__ void __launch_bounds__(kVitThreads, 1)
     const int n_len = m / 4;
     const int G = viterbi_lanes(my_rows, warps);  // no fewer than the launch made room for
 #define PCFGNAT_VITERBI_CASE(G_) \
-    viterbi_lengths<G_>(col, lk, s_oa, own_v, own_k, col_bar, n_len, Mb, my_rows, NC, crank, Q, cs, pitch)
+    viterbi_lengths<G_, LONG>(col, lk, s_oa, own_v, own_k, col_bar, n_len, Mb, my_rows, NC, crank, Q, cs, pitch)
     const bool arrived = G == 4 ? PCFGNAT_VITERBI_CASE(4) : G == 8 ? PCFGNAT_VITERBI_CASE(8) : PCFGNAT_VITERBI_CASE(16);
 #undef PCFGNAT_VITERBI_CASE
     if (!arrived && lane == 0) flag(status, PCFGNAT_STATUS_TIMEOUT);
@@ -550,21 +570,15 @@ int launch_trace(const float *S, const float *penalty, int64_t *pred_out, const 
 
 // How a CTA of n that share a sentence lays out its nodes' rows; smem 0: they do not fit.
 struct VitRows {
-    int cap, stride, cs;
+    int cap, stride, cs, warps;
     size_t smem;
 };
 
-// Warps of a block; with more CTAs than SMs no more than the nodes need, so that CTAs share SMs: 1000 sentences of 16 nodes
-// 49 -> 24 us, 300 of 64 105 -> 78.
-static int viterbi_warps(int rows, bool crowded) {
-    const int least = (rows + 31) / 32 * 4;
-    return crowded && least < kVitThreads / 32 ? least : kVitThreads / 32;
-}
-
-static VitRows viterbi_rows(int Mc, int Q, int n, int width, bool crowded) {
+static VitRows viterbi_layout(int Mc, int Q, int n, int width, int warps) {
     VitRows r;
     r.cap = (Mc + n - 1) / n;  // also right for mixed widths: n is 1 there, every CTA may hold a chain
-    const int G = viterbi_lanes(r.cap, viterbi_warps(r.cap, crowded));
+    r.warps = warps;
+    const int G = viterbi_lanes(r.cap, warps);
     r.cs = Mc + viterbi_overshoot(G, width);
     for (int banks = 1; banks >= 0; banks--) {  // the rows that a half-warp reads in different banks where there is room for that
         r.stride = Mc;
@@ -575,6 +589,19 @@ static VitRows viterbi_rows(int Mc, int Q, int n, int width, bool crowded) {
     }
     r.smem = 0;
     return r;
+}
+
+// With more CTAs than SMs no more warps than the nodes need, so that CTAs share SMs: 1000 sentences of 16 nodes 49 -> 24 us, 300 of
+// 64 105 -> 78.  CTAs whose tables leave no room for a second one get all: 16 sentences of 430 nodes 1 798 -> 1 017 us, 32
+// of 320 957 -> 698.
+static VitRows viterbi_rows(int Mc, int Q, int n, int width, bool crowded) {
+    constexpr int all = kVitThreads / 32;
+    const int least = ((Mc + n - 1) / n + 31) / 32 * 4;
+    if (crowded && least < all) {
+        const VitRows r = viterbi_layout(Mc, Q, n, width, least);
+        if (r.smem && 2 * (r.smem + 1024) <= (size_t)kSmemLimit) return r;
+    }
+    return viterbi_layout(Mc, Q, n, width, all);
 }
 
 int launch_viterbi(const float *ob, const float *links, const int64_t *ol, int B, int L, float *S, int64_t *R,
@@ -610,26 +637,28 @@ int launch_viterbi(const float *ob, const float *links, const int64_t *ol, int B
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    const auto kernel = Mc > 256 ? viterbi_cluster_kernel<true> : viterbi_cluster_kernel<false>;
     // the launch with n CTAs per sentence; returns the clusters that run at once, 0 where there is no such launch
     const auto configure = [&](int n, const VitRows &rows) {
         const int launch_nc = mixed(n) ? 2 : n;
         cfg.gridDim = dim3((unsigned)((mixed(n) ? wide + (B - wide + 1) / 2 : B) * launch_nc));
         cfg.dynamicSmemBytes = rows.smem;
-        cfg.blockDim = dim3(32 * viterbi_warps(rows.cap, crowded(n)));
+        cfg.blockDim = dim3(32 * rows.warps);
         attr[0].val.clusterDim.x = (unsigned)launch_nc;
         int clusters = 0;
-        if (ensure_dynamic_smem(viterbi_cluster_kernel, rows.smem) != cudaSuccess ||
-            (n > 8 && cudaFuncSetAttribute(viterbi_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
-            cudaOccupancyMaxActiveClusters(&clusters, viterbi_cluster_kernel, &cfg) != cudaSuccess) {
+        if (ensure_dynamic_smem(kernel, rows.smem) != cudaSuccess ||
+            (n > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+            cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) {
             cudaGetLastError();
             return 0;
         }
         return clusters;
     };
-    // Sixteen CTAs where a chain is long and all sentences still run at once: one sentence of 257 nodes 175 -> 156 us, five of
-    // 380 348 -> 281, but nine of 300, for whose clusters there is no room, 226 -> 352.
-    if (nc == 8 && Mc > 256) {
-        const VitRows rows = viterbi_rows(Mc, Q, 16, 16, crowded(16));
+    // Sixteen CTAs where a chain is long and all sentences still run at once, every CTA on an SM of its own: one sentence of 257
+    // nodes 175 -> 156 us, five of 380 348 -> 281, but nine of 300, for whose clusters there is no room, 226 -> 352, and 16 of 257,
+    // whose CTAs would share SMs, 329 -> 390.
+    if (nc == 8 && Mc > 256 && !crowded(16)) {
+        const VitRows rows = viterbi_rows(Mc, Q, 16, 16, false);
         if (rows.smem && configure(16, rows) >= B) nc = 16;
     }
     for (; nc <= 16; nc *= 2) {
@@ -637,7 +666,7 @@ int launch_viterbi(const float *ob, const float *links, const int64_t *ol, int B
         if (rows.smem == 0) continue;
         if (configure(nc, rows) < 1) continue;  // this cluster size cannot be scheduled here: try the next one
         const int order = mixed(nc) ? wide : (crowded(nc) && B <= 256 ? B : -1);
-        return cuda_rc(cudaLaunchKernelEx(&cfg, viterbi_cluster_kernel, ob, links, ol, L, S, R, Lt, Mt, status, Mc, rows.cs, rows.cap,
+        return cuda_rc(cudaLaunchKernelEx(&cfg, kernel, ob, links, ol, L, S, R, Lt, Mt, status, Mc, rows.cs, rows.cap,
                                           rows.stride, B, order));
     }
     const size_t smem_cols = (size_t)3 * cs * sizeof(float);

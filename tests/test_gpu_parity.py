@@ -317,6 +317,29 @@ def test_viterbi_signed_zeros_and_crowded_grids(ops, monkeypatch, B, L):
     assert ops.read_status(DEV) == 0
 
 
+@pytest.mark.parametrize("B, L", [(3, 512), (2, 516), (16, 514), (24, 562), (20, 700), (1, 1060)])
+def test_viterbi_of_long_chains(ops, monkeypatch, B, L):
+    """Chains at and beyond 256 main-chain nodes, whose children past the first 128 are kept as a block's maximum, on the numbers
+    of CTAs and lanes that the library picks for few and many sentences; few distinct values: many ties within a block and between
+    blocks.  Tables bit for bit those of the kernel that reads the transitions from global memory."""
+    monkeypatch.delenv("PCFGNAT_DP_KERNEL", raising=False)
+    monkeypatch.delenv("PCFGNAT_DP_CLUSTER_SIZE", raising=False)
+    g = torch.Generator(DEV).manual_seed(L + B)
+    ob = -0.25 * torch.randint(0, 3, (B, L), device=DEV, generator=g).float()
+    links = -0.5 * torch.randint(0, 4, (B, L, 2, L), device=DEV, generator=g).float()
+    at = torch.arange(L, device=DEV)
+    links.masked_fill_((at[None, :] <= at[:, None])[None, :, None, :], float("-inf"))
+    ol = torch.randint(L // 3, L + 1, (B,), device=DEV, generator=g)
+    ol[0] = L
+    k = ops.get_pcfg_kernel()
+    got = k.pcfg_viterbi(ob, links, ol, 1)
+    monkeypatch.setenv("PCFGNAT_DP_KERNEL", "rows")
+    want = k.pcfg_viterbi(ob, links, ol, 1)
+    assert np.array_equal(_bits(got[0].cpu().numpy()), _bits(want[0].cpu().numpy()))
+    assert all(torch.equal(x, y) for x, y in zip(got[1:], want[1:]))
+    assert ops.read_status(DEV) == 0
+
+
 @pytest.mark.parametrize("name", ["ref_viterbi_ragged.npz", "ref_viterbi_mid.npz"])
 def test_viterbi_against_reference_golden(vit_kernel, ops, name):
     g = _g(name)
