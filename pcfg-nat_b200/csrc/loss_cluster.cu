@@ -1008,26 +1008,39 @@ int launch_inside(const float *match_all, const float *links, const int64_t *ol,
     return PCFGNAT_ERR_UNSUPPORTED;
 }
 
-// Reference order with G lanes per node; PCFGNAT_ERR_UNSUPPORTED when the tables or the nodes of a CTA do not fit.
+// Reference order with G lanes per node: a CTA's tables on clusters of `width`, nc CTAs per sentence; smem 0: they do not fit.
+struct ExactTables {
+    int rows_cap, cs, pitch;
+    size_t smem;
+};
+template <int G>
+ExactTables exact_tables(int Mc, int W, int nc, int width) {
+    ExactTables t;
+    t.rows_cap = (Mc + nc - 1) / nc;
+    t.cs = Mc + ExactShape<G>::pad(width);
+    // the eight-byte cells that a half-warp reads for its nodes in distinct banks, on a CTA that has a sentence to itself
+    t.pitch = t.cs;
+    while (G < 16 && (t.pitch + nc) % 16 != G) t.pitch++;
+    t.smem = ((size_t)4 * t.cs + (size_t)t.rows_cap * t.pitch) * sizeof(float2) + (size_t)3 * t.rows_cap * W * sizeof(float);
+    if (t.smem > (size_t)kSmemLimit - 1024) t.smem = 0;
+    return t;
+}
+
+// PCFGNAT_ERR_UNSUPPORTED when the tables or the nodes of a CTA do not fit.  small: as few threads as stage the links in time.
 template <int G>
 int launch_exact(const float *match_all, const float *links, const int64_t *ol, const int64_t *tl, int B, int L, int T,
-                 float *S, float *C, float *loss, int *status, cudaStream_t st, int nc, int wide, bool mixed, bool crowded) {
-    const int Mc = main_slots(L, 1), Lt = L - Mc, W = T + 2;
+                 float *S, float *C, float *loss, int *status, cudaStream_t st, int nc, int wide, bool mixed, bool small) {
+    const int Mc = main_slots(L, 1), Lt = L - Mc;
     const int width = mixed ? 2 : nc;  // CTAs of a cluster
-    const int rows_cap = (Mc + nc - 1) / nc;
-    const int cs = Mc + ExactShape<G>::pad(width);
-    // the eight-byte cells that a half-warp reads for its nodes in distinct banks, on a CTA that has a sentence to itself
-    int pitch = cs;
-    while (G < 16 && (pitch + nc) % 16 != G) pitch++;
-    size_t smem = ((size_t)4 * cs + (size_t)rows_cap * pitch) * sizeof(float2) + (size_t)3 * rows_cap * W * sizeof(float);
-    if (wide >= 0 && smem < (size_t)B * sizeof(int)) smem = (size_t)B * sizeof(int);  // the costs that rank the sentences
-    int threads = (rows_cap + ExactShape<G>::kNodes - 1) / ExactShape<G>::kNodes * 32;  // all nodes in one pass
-    if (smem > (size_t)kSmemLimit - 1024 || threads > kExactThreads) return PCFGNAT_ERR_UNSUPPORTED;
-    const int least = crowded ? 128 : 256;  // fewer take longer to stage the links
+    ExactTables t = exact_tables<G>(Mc, T + 2, nc, width);
+    int threads = (t.rows_cap + ExactShape<G>::kNodes - 1) / ExactShape<G>::kNodes * 32;  // all nodes in one pass
+    if (t.smem == 0 || threads > kExactThreads) return PCFGNAT_ERR_UNSUPPORTED;
+    if (wide >= 0 && t.smem < (size_t)B * sizeof(int)) t.smem = (size_t)B * sizeof(int);  // the costs that rank the sentences
+    const int least = small ? 128 : 256;  // fewer take longer to stage the links
     threads = threads <= least ? least : (threads + 127) / 128 * 128;
     const int clusters = mixed ? wide + (B - wide + 1) / 2 : B;
-    return launch_cluster(inside_exact_kernel<G>, threads, clusters, width, smem, st, match_all, links, ol, tl, L, T, S, C, loss,
-                          status, Mc, Lt, cs, rows_cap, pitch, B, wide);
+    return launch_cluster(inside_exact_kernel<G>, threads, clusters, width, t.smem, st, match_all, links, ol, tl, L, T, S, C, loss,
+                          status, Mc, Lt, t.cs, t.rows_cap, t.pitch, B, wide);
 }
 
 // Inside pass in the reference's order on as many CTAs per sentence as leave all sentences on the GPU at once, on more where
@@ -1046,11 +1059,14 @@ int launch_loss_fwd_exact(const float *match_all, const float *links, const int6
         // Fewer lanes per node share more of the fixed costs, more lanes shorten the longest row.  Where every CTA has an SM to
         // itself: 24 nodes of 96 on a CTA (24 sentences) 76 / 70 / 68 us with 4 / 8 / 16 lanes, 48 nodes (100 sentences)
         // 37 / 34.5 / -, 64 of 128 (56 sentences) 128 / 133 / -.  With more CTAs than SMs the four-lane blocks, smaller, share
-        // SMs: 300 sentences of 32 nodes 22 / 22 / 33 us, of 64 nodes 58 / 82 / -.
-        const int rc = crowded || rows > 48
-                           ? launch_exact<4>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, nc, order, wide > 0, crowded)
-                       : rows > 32 ? launch_exact<8>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, nc, order, wide > 0, crowded)
-                                   : launch_exact<16>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, nc, order, wide > 0, crowded);
+        // SMs: 300 sentences of 32 nodes 22 / 22 / 33 us, of 64 nodes 58 / 82 / -; but not where the tables fill more than
+        // half of an SM: 32 sentences of 320 nodes 3 512 / 2 146 us with
+        // 4 / 8.
+        const bool small = crowded && 2 * (exact_tables<4>(Mc, T + 2, nc, wide > 0 ? 2 : nc).smem + 1024) <= (size_t)kSmemLimit;
+        const int rc = small || rows > 48
+                           ? launch_exact<4>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, nc, order, wide > 0, small)
+                       : rows > 32 ? launch_exact<8>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, nc, order, wide > 0, small)
+                                   : launch_exact<16>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, nc, order, wide > 0, small);
         if (rc != PCFGNAT_ERR_UNSUPPORTED) return rc;
     }
     return PCFGNAT_ERR_UNSUPPORTED;

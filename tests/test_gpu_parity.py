@@ -634,6 +634,29 @@ def test_inside_table_edges(ops, monkeypatch, B, L, T):
     assert torch.isfinite(S).any()
 
 
+@pytest.mark.parametrize("B, L, T", [(32, 640, 12), (20, 700, 30), (24, 640, 40), (2, 900, 430)])
+def test_inside_table_of_long_chains(ops, monkeypatch, B, L, T):
+    """More CTAs than SMs, of which no two fit an SM, and the chains that the lanes of a node cannot take (a warp per node, on
+    clusters of sixteen): tables bit for bit those of the kernel with a thread row per node."""
+    for name in ("PCFGNAT_DP_KERNEL", "PCFGNAT_DP_CLUSTER_SIZE"):
+        monkeypatch.delenv(name, raising=False)
+    g = torch.Generator(DEV).manual_seed(L + B)
+    match, links = 2 * torch.randn(B, L, T, device=DEV, generator=g) - 6, torch.randn(B, L, 2, L, device=DEV, generator=g) - 4
+    at = torch.arange(L, device=DEV)
+    links.masked_fill_((at[None, :] <= at[:, None])[None, :, None, :], float("-inf"))
+    ol = torch.randint(L // 3, L + 1, (B,), device=DEV, generator=g)
+    ol[0] = L
+    tl = torch.randint(T // 2, T + 1, (B,), device=DEV, generator=g)
+    tl[0] = T
+    k = ops.get_pcfg_kernel()
+    S, C = k.pcfg_loss(match, links, ol, tl, 1)
+    monkeypatch.setenv("PCFGNAT_DP_KERNEL", "rows")
+    want_S, want_C = k.pcfg_loss(match, links, ol, tl, 1)
+    assert np.array_equal(_bits(S.cpu().numpy()), _bits(want_S.cpu().numpy()))
+    assert np.array_equal(_bits(C.cpu().numpy()), _bits(want_C.cpu().numpy()))
+    assert ops.read_status(DEV) == 0 and torch.isfinite(S).any()
+
+
 @pytest.mark.parametrize("batch", [97, 6])  # one CTA per sentence; a cluster of CTAs per sentence
 @pytest.mark.parametrize("L_even", [True, False])
 def test_outside_pass_with_fused_gradients_matches_the_gradient_kernel(ops, syn, monkeypatch, L_even, batch):
