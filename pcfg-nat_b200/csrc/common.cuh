@@ -98,6 +98,9 @@ inline int cuda_rc(cudaError_t e) { return e == cudaSuccess ? PCFGNAT_OK : PCFGN
 // therefore starts with chain_begin(): wait until that kernel has finished and its memory is visible, then let the
 // next kernel of the chain be scheduled in turn.  What is saved is the launch latency between the kernels.  Without
 // the launch attribute both instructions do nothing.
+// The order of the two matters: a kernel may read, before its own wait, only what was complete when its predecessor let it be
+// scheduled, and the linear-space outside pass, which is always launched early, stages the lengths, emissions and transitions
+// before it waits.  It may because the inside pass has waited for whatever made those before it lets anything follow.
 __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -1072,6 +1072,7 @@ int launch_linear(const LinearGeometry &g, const float *match_all, const float *
     int rc = launch_linear_cluster(inside_linear_kernel<CHUNKS>, clusters, nc, g.smem_in, false, st, match_all, links, ol, tl, L, T,
                                    Y, frames, loss, mg, status, Mc, g.cs, g.rows_cap, B, g.wide);
     if (rc) return rc;
+    // (The inside pass waits for its own predecessor before it lets this one start: chain_begin(), common.cuh.)
     // Both passes fill an SM.  The outside pass's clusters, which can start once all of the inside pass's have, take the SMs that
     // its short sentences leave, find their sentence, stage their matrices from the inputs and wait there: 43.1 -> 41.7 us for a
     // training step of 2 sentences, 954 -> 937 us for 90 on the graph of 8 nodes a source token, 398 -> 391 us for 8 of

@@ -2186,6 +2186,41 @@ def test_outside_pass_that_starts_before_the_inside_pass_has_ended(ops, syn, mon
     ops.read_status(DEV)
 
 
+@pytest.mark.parametrize("B", [2, 90])
+def test_early_outside_pass_behind_a_kernel_that_makes_the_emissions(B):
+    """With every kernel of the chain launched early (PCFGNAT_PDL=1, read once per process): the outside pass stages emissions that
+    the projection's last kernel has just written.  Batches follow one another without a synchronisation, each with other emissions
+    in the same memory; losses and gradients bit for bit those of calls that wait for one another."""
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+
+    program = f"""
+import torch, __graft_entry__ as entry
+syn = entry.load_package().synthetic
+from pcfg_nat_b200.custom_ops import pcfg_loss as ops
+b = syn.make_batch(syn.Workload("chain", batch={B}, vocab=1000, hidden=64, src_min=6, src_max=30, hidden_std=1.0), seed=5)
+d = lambda t: t.to("cuda:0")
+hidden, weight, links, ol, targets, tl = map(d, (b.hidden, b.weight, b.links, b.output_length, b.targets, b.target_length))
+k = ops.get_pcfg_kernel()
+states = [torch.roll(hidden, i, 0) * (1 + i / 8) for i in range(6)]
+def batch(h, wait):
+    match = k.proj_logsoftmax_gather(h, weight, targets, ol, tl)["match"]
+    if wait: torch.cuda.synchronize()
+    return k.pcfg_loss_fwd_bwd(match, links, ol, tl)
+want = [[x.clone() for x in batch(h, True)] for h in states]
+torch.cuda.synchronize()
+got = [batch(h, False) for _ in range(3) for h in states]
+torch.cuda.synchronize()
+for i, out in enumerate(got):
+    assert all(torch.equal(x.nan_to_num(7.0), y.nan_to_num(7.0)) for x, y in zip(out, want[i % 6])), i
+"""
+    env = dict(os.environ, PCFGNAT_PDL="1")
+    r = subprocess.run([sys.executable, "-c", program], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+
+
 @pytest.mark.parametrize("B, L, T", [(20, 314, 238), (1, 322, 304), (2, 384, 238)])
 def test_linear_space_loss_at_the_limit_of_shared_memory(ops, monkeypatch, B, L, T):
     """Shapes whose tables come within a hundred bytes of the shared memory that the kernels' own variables leave."""
