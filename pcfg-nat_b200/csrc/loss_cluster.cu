@@ -961,14 +961,6 @@ int mixed_width_count(int B, int Mc) {
     return sms - B;
 }
 
-// True when the inside pass should run on the cluster kernel although cluster_kernels_pay() is false: batches
-// between half the SMs and all of them, where the costliest sentences get a second CTA (mixed widths).
-bool inside_mixed_widths_pay(int B, int L, int T) {
-    const int Mc = main_slots(L, 1);
-    const ClusterGeometry g = cluster_geometry(B, Mc, T + 2);
-    return g.nc == 1 && mixed_width_count(B, Mc) > 0 && g.smem_in <= (size_t)kSmemLimit - 1024;
-}
-
 // True when the batch is small enough that several CTAs per sentence are available (cluster size >= 2),
 // or the chain is too long for the single-CTA kernels to keep its links in shared memory.
 bool cluster_kernels_pay(int B, int L, int T) {

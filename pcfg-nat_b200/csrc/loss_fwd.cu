@@ -217,7 +217,7 @@ int launch_loss_fwd(const float *match_all, const float *links, const int64_t *o
                     int T, float *S, float *C, float *loss, int *status, cudaStream_t st) {
     if (B == 0) return PCFGNAT_OK;
     // Kernel families, all producing bit-identical tables: 4 to 16 lanes per node on clusters (loss_cluster.cu), a warp per node
-    // on clusters where few sentences leave several SMs per sentence or the chain is long, phase-balanced single CTA
+    // on clusters of sixteen where those do not fit, phase-balanced single CTA
     // (loss_balanced.cu, on request only: measured slower here) and the row-per-thread kernel below, which
     // has no size limit because it can read links from global memory.
     const DpKernel choice = dp_kernel_choice();
@@ -227,7 +227,8 @@ int launch_loss_fwd(const float *match_all, const float *links, const int64_t *o
         // of batches with one CTA per sentence the shortest chains stay with the kernel below, which fits more sentences on an
         // SM: 1000 of 16 nodes 18.6 us against 27.4, 128 of 12 nodes 18.1 against 18.5, but 128 of 20 nodes 20.3 against 19.1
         if (pays || main_slots(L, 1) > 16) rc = launch_loss_fwd_exact(match_all, links, ol, tl, B, L, T, S, C, loss, status, st);
-        if (rc == PCFGNAT_ERR_UNSUPPORTED && (pays || inside_mixed_widths_pay(B, L, T)))
+        // the warp per node: chains of 340 main-chain nodes with 600 tokens to 620 with 20, whose pairs do not fit sixteen CTAs
+        if (rc == PCFGNAT_ERR_UNSUPPORTED && pays)
             rc = launch_loss_fwd_cluster(match_all, links, ol, tl, B, L, T, S, C, loss, status, st);
         if (rc != PCFGNAT_ERR_UNSUPPORTED) return rc;
     }

@@ -634,7 +634,7 @@ def test_inside_table_edges(ops, monkeypatch, B, L, T):
     assert torch.isfinite(S).any()
 
 
-@pytest.mark.parametrize("B, L, T", [(32, 640, 12), (20, 700, 30), (24, 640, 40), (2, 900, 430)])
+@pytest.mark.parametrize("B, L, T", [(32, 640, 12), (20, 700, 30), (24, 640, 40), (2, 1170, 40), (3, 820, 400)])
 def test_inside_table_of_long_chains(ops, monkeypatch, B, L, T):
     """More CTAs than SMs, of which no two fit an SM, and the chains that the lanes of a node cannot take (a warp per node, on
     clusters of sixteen): tables bit for bit those of the kernel with a thread row per node."""
