@@ -26,9 +26,10 @@
 // 2.3e-7 (rms; 2.3e-7 to 2.5e-7 with the float32 kernels), the gradients by 1.5e-7 to 2.0e-7 of their norm (2.0e-7 to 2.7e-7) and
 // every row of them (a node and head) by 1.9e-7 of its own norm in the median, also where the rows of links_grad are 1e12
 // apart (2.3e-7).
-// All five are bound by the issue of their instructions and the latency between them (45 % of the slots, 8 to 16 warps an
-// SM).  90 sentences, M = 161, 8 x 64 features: 33 + 60 us forward, 357 us with extract_links.cu's three; 13 + 100 + 59 us
-// backward, 643 us with its two, 33 of zero fills and 41 of conversions, which these need none of.
+// All five are bound by the issue of their instructions and the latency between them (38 to 56 % of the slots of an SM that has
+// work, 12 to 20 warps; the tensor pipe 12 to 22 %).  90 sentences, M = 161, 8 x 64 features: 33 + 60 us forward, 357 us with
+// extract_links.cu's three; 14 + 109 + 63 us backward, 643 us with its two, 33 of zero fills and 41 of conversions, which these
+// need none of.
 #include <cuda_fp16.h>
 
 #include <initializer_list>

@@ -423,8 +423,8 @@ __global__ void __launch_bounds__(kCThreads, 1)
 // term costs one load of eight bytes of either and half of a packed addition.  The terms of the first 128 children stay in
 // registers between the maximum and the sum; those of further children are formed twice.
 //
-// Bound by the latency of a step on the longest row (57 % of the issue slots with eight lanes; the exponentials, expf for the
-// bits, are half of the instructions).  With the exponentials handed over through shared memory and 1024 threads before
+// Bound by the latency of a step on the longest row (42 % of the issue slots of an SM that has work, 64 sentences, M = 128, four
+// lanes).  With the exponentials handed over through shared memory and 1024 threads before
 // (sixteen or eight lanes, a pass per 64 or 128 nodes), and a warp per node below 32 nodes: 64 sentences, M = 128, T = 76: 191
 // -> 123 us; 90 sentences, M <= 80: 84 -> 64; 16 sentences, M = 128 on eight CTAs each 213 -> 96; 160 sentences, M <= 80 (the
 // row-per-thread kernel of loss_fwd.cu before) 189 -> 75.  For the first of these: terms formed twice for all children 137 us, a

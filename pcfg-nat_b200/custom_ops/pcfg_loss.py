@@ -789,7 +789,7 @@ class _Kernel:
         M = nodes.numel()
         lib = _cabi.lib()
         kept_bytes = lib.pcfgnat_links_fused_kept_bytes(M, B, H, D, int(keep)) if dt == torch.float16 else 0
-        if kept_bytes:  # a shape that the one-launch kernel takes
+        if kept_bytes:  # a shape that the kernels without score matrices take
             with torch.cuda.device(dev):
                 links = torch.empty((B, L, 2, L), dtype=torch.float32, device=dev)
                 kept = torch.empty(kept_bytes, dtype=torch.uint8, device=dev)
@@ -1216,8 +1216,8 @@ class ProjLogsoftmaxGatherFunc(Function):
 class ExtractLinksFunc(Function):
     """links = extract_links(link features) with a hand-written backward: the reference gets its gradient from autograd
     through the ~30 operators of the model's extract_links (models/...pcfg.py:163-199), which keeps several
-    [B, L, 2, L, heads] tensors alive; here the backward recomputes a row's quantities from the compact per-head score
-    matrices the forward kept."""
+    [B, L, 2, L, heads] tensors alive; here the backward recomputes a row's quantities from what the forward kept: the packed
+    features and the rows' sums (half-precision features), or compact per-head score matrices."""
 
     @staticmethod
     def forward(ctx, query, key_left, key_right, gate_logits, prev_output_tokens, pad_index, left_tree_mask, right_tree_mask,

@@ -350,7 +350,8 @@ class LossStep(_GraphedStep):
             from . import _cabi
             with torch.cuda.device(self.device):
                 dp = _cabi.lib().pcfgnat_loss_fwd_bwd_kernels(B, L, T, 1)
-            # with link features: feature gather, score products, links, and the two backward kernels
+            # with link features five: feature gather, score products, links, and the two backward kernels, or without score
+            # matrices two forward and three backward
             self.kernels_per_step = 4 + (dp if dp > 0 else 3) + (2 if self.force_emit else 0) + (5 if link_features else 0)
         self.proj_backward_note = None
         if self.proj_backward:
