@@ -1054,7 +1054,8 @@ int launch_loss_fwd_exact(const float *match_all, const float *links, const int6
         // SMs: 300 sentences of 32 nodes 22 / 22 / 33 us, of 64 nodes 58 / 82 / -; but not where the tables fill more than
         // half of an SM: 32 sentences of 320 nodes 3 512 / 2 146 us with
         // 4 / 8.
-        const bool small = crowded && 2 * (exact_tables<4>(Mc, T + 2, nc, wide > 0 ? 2 : nc).smem + 1024) <= (size_t)kSmemLimit;
+        const size_t four = exact_tables<4>(Mc, T + 2, nc, wide > 0 ? 2 : nc).smem;
+        const bool small = crowded && four && 2 * (four + 1024) <= (size_t)kSmemLimit;
         const int rc = small || rows > 48
                            ? launch_exact<4>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, nc, order, wide > 0, small)
                        : rows > 32 ? launch_exact<8>(match_all, links, ol, tl, B, L, T, S, C, loss, status, st, nc, order, wide > 0, small)

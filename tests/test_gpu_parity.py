@@ -1056,6 +1056,23 @@ def test_loss_step_with_projection_backward_of_an_odd_vocabulary(pkg, ops, syn):
         assert float((got - want).norm() / want.norm()) < 2e-3
 
 
+@pytest.mark.parametrize("T", [8192, 8200])
+def test_projection_with_more_targets_than_are_sorted_in_shared_memory(ops, T):
+    """Targets ranked from shared memory and, beyond 8 192, from global memory (ids outside the vocabulary among them): emissions
+    against float64 from half-precision operands, float32 sums of 64 products: 1e-4."""
+    g = torch.Generator(DEV).manual_seed(T)
+    hidden, weight = torch.randn(1, 4, 64, device=DEV, generator=g).half(), (torch.randn(301, 64, device=DEV, generator=g) * 0.2).half()
+    targets = torch.randint(0, 301, (1, T), device=DEV, generator=g)
+    ops.read_status(DEV)
+    got = ops.proj_logsoftmax_gather(hidden, weight, targets, None, None)["match"]
+    want = torch.log_softmax(hidden.double() @ weight.double().t(), -1).gather(2, targets[:, None].expand(-1, 4, -1))
+    assert (got.double() - want).abs().max() <= 1e-4 and ops.read_status(DEV) == 0
+    targets[0, 7], targets[0, T - 1] = 301, -1
+    got = ops.proj_logsoftmax_gather(hidden, weight, targets, None, None)["match"]
+    assert torch.isnan(got[0, :, [7, T - 1]]).all() and (got[0, :, 8:T - 1].double() - want[0, :, 8:T - 1]).abs().max() <= 1e-4
+    assert ops.read_status(DEV) != 0
+
+
 @pytest.mark.parametrize("V", [33, 513, 1001])
 def test_projection_backward_of_an_odd_vocabulary_and_one_row(pkg, ops, V):
     """One real row, as n_rows and as the whole tensor, and a step whose batch has one real node or none; bounds of the test of
