@@ -1188,20 +1188,13 @@ __global__ void __launch_bounds__(32 * kChildWarps)
 }
 
 inline int tiles_of(int M) { return M > 0 ? (M + kTile - 1) / kTile : 1; }
-// A block walks its children one step after the other, which takes the longer the chain is, however few the sentences are and
-// with eight heads as with two; extract_links.cu's kernels spread a few long sentences over the GPU.  Forward and backward, a graph of
-// calls (us, these / those), features of 64 and nodes of the chain: 8 heads, 41 nodes: one sentence 45 / 41, four 46 / 43, eight
-// 46 / 46; 256: four 115 / 118, eight 125 / 203; 513: two 218 / 183, three 227 / 266.  4 heads, 256: four 106 / 86, six
-// 108 / 110, eight 111 / 125; 513: three 200 / 176, four 199 / 199.  2 heads, 256: eight 106 / 98, twelve 111 / 129; 401: eight
-// 159 / 174.  One head, 257: 16 sentences 113 / 142.  Chains of one or two tiles, or with features of 32 or two heads of three, are as
-// fast or faster here at any size (and twelve heads of three tiles 51 / 46 for one sentence, 50 / 73 for twelve).
+// A block walks its children one step after the other, which takes the longer the chain is, however few the sentences are;
+// extract_links.cu's kernels spread a few long sentences over the GPU.  Forward and backward (us, these / those): one sentence of
+// 257 nodes, eight heads 117 / 85, four 117 / 134, four with one head 101 / 85, 16 with one head 113 / 142; of 121 nodes, four
+// heads: four sentences 66 / 60, 16 67 / 94; of 61: 47 / 47 and 48 / 53; chains of up to three tiles are faster here at any size.
 inline bool fused_shape_ok(int M, int B, int H, int D) {
     if ((D != 32 && D != 64) || (long long)H * D > kMaxWidth || M > kMaxChain) return false;
-    const int tiles = tiles_of(M);
-    if (tiles < 4) return tiles < 3 || D == 32 || H < 4 || H > kFusedWarps || B >= 8;
-    const long long blocks = (long long)B * tiles;
-    return blocks * (H < 4 ? H : 4) >= 256 &&
-           blocks * ((H < kFusedWarps ? H : kFusedWarps) + 2) * (D == 32 ? 5 : 4) >= 40 * (3 * tiles + 16 < 85 ? 3 * tiles + 16 : 85);
+    return tiles_of(M) < 4 || (long long)B * tiles_of(M) * (H < 4 ? H : 4) >= 256;
 }
 
 // Pieces of one block of memory, 16 bytes each at least
