@@ -1191,7 +1191,10 @@ inline int tiles_of(int M) { return M > 0 ? (M + kTile - 1) / kTile : 1; }
 // A block walks its children one step after the other, which takes the longer the chain is, however few the sentences are;
 // extract_links.cu's kernels spread a few long sentences over the GPU.  Forward and backward (us, these / those): one sentence of
 // 257 nodes, eight heads 117 / 85, four 117 / 134, four with one head 101 / 85, 16 with one head 113 / 142; of 121 nodes, four
-// heads: four sentences 66 / 60, 16 67 / 94; of 61: 47 / 47 and 48 / 53; chains of up to three tiles are faster here at any size.
+// heads: four sentences 66 / 60, 16 67 / 94; of 61: 47 / 47 and 48 / 53.  On the device alone, in a graph of calls, the line would lie elsewhere for few sentences: one of
+// 41 nodes and eight heads 45 / 41, four of 256 and four heads 106 / 86, two of 513 213 / 141.  But these are five launches and seven
+// allocations where the others are eight kernels, three conversions and twice the allocations: a training pass from Python over two
+// sentences of 33 nodes 705 / 785 us, over four of 257 and four heads 690 / 775, over two of 513 2 134 / 2 116.
 inline bool fused_shape_ok(int M, int B, int H, int D) {
     if ((D != 32 && D != 64) || (long long)H * D > kMaxWidth || M > kMaxChain) return false;
     return tiles_of(M) < 4 || (long long)B * tiles_of(M) * (H < 4 ? H : 4) >= 256;
